@@ -32,6 +32,7 @@ SOURCES = {
     "bk_noalloc.cu": [],
     "bk_layer.cu": ["--fmad=false"],
     "bk_pq2.cu": [],
+    "bk_pq2_gemm.cu": [],
     "bk_prefill.cu": [],
     "bk_prefill_umma.cu": [],
     "bk_p2p.cu": [],

@@ -319,6 +319,7 @@ void bk_ctx_destroy(bk_ctx *ctx) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_layer) cudaFree(ctx->d_layer);
     if (ctx->d_prefill) cudaFree(ctx->d_prefill);
+    if (ctx->d_pq2_x) cudaFree(ctx->d_pq2_x);
     if (ctx->h_desc) cudaFreeHost(ctx->h_desc);
     if (ctx->d_desc) cudaFree(ctx->d_desc);
     for (int i = 0; i < kDescSlots; i++)
@@ -1265,10 +1266,13 @@ static bk_status pq2_check(bk_ctx *ctx, const char *who, const void *payload, si
     return BK_OK;
 }
 
-// y of range s: [n_tok][n_rows_s]; two tokens share one pass over the weights
+// y of range s: [n_tok][n_rows_s].  One or two tokens take the weight-streaming kernel (two share one pass), more
+// the tensor-core product.
 static bk_status pq2_run_multi(bk_ctx *ctx, int n_seg, const bk_pq2_seg *segs, int64_t ne0, const float *x_dev, int32_t n_tok) {
     const size_t rb = pq2_row_bytes(ne0);
-    for (int t0 = 0; t0 < n_tok; t0 += 2) {
+    const int per_call = n_tok >= kPq2GemmMin ? kPq2GemmTokens : 2;
+    for (int t0 = 0; t0 < n_tok; t0 += per_call) {
+        const int nt = std::min(per_call, n_tok - t0);
         const uint8_t *rows[4];
         float *y[4];
         int n_rows[4];
@@ -1277,7 +1281,9 @@ static bk_status pq2_run_multi(bk_ctx *ctx, int n_seg, const bk_pq2_seg *segs, i
             n_rows[i] = (int)segs[i].n_rows;
             y[i] = segs[i].y_dev + (size_t)t0 * segs[i].n_rows;
         }
-        bk_status st = launch_pq2_matvec(ctx, n_seg, rows, n_rows, y, (int)ne0, x_dev + (size_t)t0 * ne0, std::min(2, n_tok - t0));
+        const float *x = x_dev + (size_t)t0 * ne0;
+        const bk_status st = n_tok >= kPq2GemmMin ? launch_pq2_gemm(ctx, n_seg, rows, n_rows, y, (int)ne0, x, nt)
+                                                  : launch_pq2_matvec(ctx, n_seg, rows, n_rows, y, (int)ne0, x, nt);
         if (st != BK_OK) return st;
     }
     return BK_OK;

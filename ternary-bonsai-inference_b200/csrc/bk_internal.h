@@ -79,6 +79,8 @@ struct bk_ctx {
     size_t d_layer_floats = 0;
     float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention's context chunks
     size_t d_prefill_floats = 0;
+    uint8_t *d_pq2_x = nullptr;            // split activations of the batched PQ2_0 product, then a scale per token
+    size_t pq2_x_bytes = 0;
     // split-K scratch of the decode kernel: partial results and arrival counters
     float *d_partials = nullptr;
     unsigned *d_counters = nullptr;
@@ -284,6 +286,12 @@ bk_status launch_rms_norm_rows(bk_ctx *ctx, const NormSeg &s0, const NormSeg &s1
 size_t pq2_row_bytes(int64_t ne0);
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                             const float *x, int n_tok);
+// The same for a block of up to kPq2GemmTokens tokens on the tensor cores (bk_pq2_gemm.cu).
+// From 5 tokens on (q + k + v and output rows of a layer: 4 tokens 47 us in pairs, 54 us here; 6 tokens 70 and 54);
+// 1024 tokens a pass bound the scratch (21 MB at ne0 5120).
+constexpr int kPq2GemmTokens = 1024, kPq2GemmMin = 5;
+bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
+                          const float *x, int n_tok);
 // Batched causal attention of a block of prompt tokens over a 4- or 3-bit planar cache (bk_prefill.cu).
 bool prefill_mma_supported(const DecodeArgs &a);
 bk_status launch_prefill_mma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha);
