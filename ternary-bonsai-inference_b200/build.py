@@ -38,8 +38,9 @@ SOURCES = {
     "bk_p2p.cu": [],
     "bk_host_tables.cpp": [],
     "bk_snapshot.cpp": [],
+    "bk_hostpipe.cpp": [],
 }
-HEADERS = ["bk_internal.h", "bk_device.cuh", "bk_decode_common.cuh", "bk_mma_common.cuh", "bk_umma.cuh", os.path.join(ROOT, "include", "bonsai_kv.h")]
+HEADERS = ["bk_internal.h", "bk_device.cuh", "bk_decode_common.cuh", "bk_mma_common.cuh", "bk_umma.cuh", "bk_hostpipe.h", os.path.join(ROOT, "include", "bonsai_kv.h")]
 
 
 def nvcc():

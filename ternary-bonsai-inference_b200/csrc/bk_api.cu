@@ -12,6 +12,7 @@
 
 #include <cuda_fp16.h>
 
+#include "bk_hostpipe.h"
 #include "bk_internal.h"
 
 namespace bk {
@@ -308,6 +309,7 @@ void bk_ctx_destroy(bk_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    host_pipe_destroy(ctx->pipe);
     ctx->ropes.clear();
     if (ctx->d_givens) cudaFree(ctx->d_givens);
     if (ctx->d_codebooks) cudaFree(ctx->d_codebooks);
@@ -565,20 +567,25 @@ static bk_status cache_copy(bk_cache *c, int layer, int seq, int pos0, int n_pos
     if (st != BK_OK) return st;
     if (n_pos == 0) return BK_OK;
     const size_t r0 = (size_t)pos0 * c->cfg.n_kv, nr = (size_t)n_pos * c->cfg.n_kv;
-    const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-    auto cp = [&](void *host, void *dev, size_t bytes) -> cudaError_t {
-        return to_host ? cudaMemcpyAsync(host, dev, bytes, kind, ctx->stream)
-                       : cudaMemcpyAsync(dev, host, bytes, kind, ctx->stream);
+    HostSeg segs[4];
+    size_t n = 0, total = 0;
+    auto add = [&](void *host, void *dev, size_t bytes) {
+        segs[n++] = HostSeg{host, dev, bytes};
+        total += bytes;
     };
-    if (k_rows) BK_CUDA(ctx, cp(k_rows, c->k_rows(layer, seq) + r0 * c->k_row_bytes, nr * c->k_row_bytes));
-    if (v_rows) BK_CUDA(ctx, cp(v_rows, c->v_rows(layer, seq) + r0 * c->v_row_bytes, nr * c->v_row_bytes));
-    if (k_norms && c->d_kn) BK_CUDA(ctx, cp(k_norms, c->k_norms(layer, seq) + r0, nr * 4));
-    if (v_norms && c->d_vn) BK_CUDA(ctx, cp(v_norms, c->v_norms(layer, seq) + r0, nr * 4));
-    {
-        const bk_status st_sync = sync_and_check(ctx);
-        if (st_sync != BK_OK) return st_sync;
+    if (k_rows) add(k_rows, c->k_rows(layer, seq) + r0 * c->k_row_bytes, nr * c->k_row_bytes);
+    if (v_rows) add(v_rows, c->v_rows(layer, seq) + r0 * c->v_row_bytes, nr * c->v_row_bytes);
+    if (k_norms && c->d_kn) add(k_norms, c->k_norms(layer, seq) + r0, nr * 4);
+    if (v_norms && c->d_vn) add(v_norms, c->v_norms(layer, seq) + r0, nr * 4);
+    if (total >= kHostPipeMin) {
+        if (to_host) return host_pipe_d2h(ctx, segs, n);
+        st = host_pipe_h2d(ctx, segs, n);
+        return st != BK_OK ? st : sync_and_check(ctx);
     }
-    return BK_OK;
+    for (size_t i = 0; i < n; i++)
+        BK_CUDA(ctx, to_host ? cudaMemcpyAsync(segs[i].host, segs[i].dev, segs[i].bytes, cudaMemcpyDeviceToHost, ctx->stream)
+                             : cudaMemcpyAsync(segs[i].dev, segs[i].host, segs[i].bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return sync_and_check(ctx);
 }
 
 bk_status bk_cache_download(bk_cache *c, int32_t layer, int32_t seq, int32_t pos0, int32_t n_pos, void *k_rows,
@@ -654,9 +661,14 @@ bk_status bk_append_host(bk_cache *c, int32_t layer, int32_t seq, int32_t rope_p
     if (st != BK_OK) return st;
     const size_t per = (size_t)n_tokens * c->cfg.n_kv * kHd * sizeof(float);
     if ((st = ensure_stage(ctx, 2 * per)) != BK_OK) return st;
-    memcpy(ctx->h_stage, k_host, per);
-    memcpy((char *)ctx->h_stage + per, v_host, per);
-    BK_CUDA(ctx, cudaMemcpyAsync(ctx->d_stage, ctx->h_stage, 2 * per, cudaMemcpyHostToDevice, ctx->stream));
+    if (2 * per >= kHostPipeMin) {
+        const HostSeg in[2] = {{const_cast<float *>(k_host), ctx->d_stage, per}, {const_cast<float *>(v_host), (char *)ctx->d_stage + per, per}};
+        if ((st = host_pipe_h2d(ctx, in, 2)) != BK_OK) return st;
+    } else {
+        memcpy(ctx->h_stage, k_host, per);
+        memcpy((char *)ctx->h_stage + per, v_host, per);
+        BK_CUDA(ctx, cudaMemcpyAsync(ctx->d_stage, ctx->h_stage, 2 * per, cudaMemcpyHostToDevice, ctx->stream));
+    }
     st = bk_append(c, layer, seq, rope_pos, n_tokens, (const float *)ctx->d_stage,
                    (const float *)((char *)ctx->d_stage + per));
     if (st != BK_OK) return st;
@@ -1448,6 +1460,13 @@ bk_status bk_kvq_quantize(bk_ctx *ctx, int32_t hd, int32_t bits, int32_t n_vec, 
     const size_t ox = io.take(xb), op = io.take(pb), on = io.take(nb);
     if ((st = ensure_stage(ctx, io.used)) != BK_OK) return st;
     char *h = (char *)ctx->h_stage, *d = (char *)ctx->d_stage;
+    if (xb >= kHostPipeMin) {
+        const HostSeg in{const_cast<float *>(x), d + ox, xb};
+        if ((st = host_pipe_h2d(ctx, &in, 1)) != BK_OK) return st;
+        if ((st = launch_quantize(ctx, bits, n_vec, (const float *)(d + ox), (uint8_t *)(d + op), (float *)(d + on))) != BK_OK) return st;
+        const HostSeg out[2] = {{packed, d + op, pb}, {norms, d + on, nb}};
+        return host_pipe_d2h(ctx, out, 2);
+    }
     memcpy(h + ox, x, xb);
     BK_CUDA(ctx, cudaMemcpyAsync(d + ox, h + ox, xb, cudaMemcpyHostToDevice, ctx->stream));
     if ((st = launch_quantize(ctx, bits, n_vec, (const float *)(d + ox), (uint8_t *)(d + op), (float *)(d + on))) != BK_OK)
@@ -1473,6 +1492,13 @@ bk_status bk_kvq_dequantize(bk_ctx *ctx, int32_t hd, int32_t bits, int32_t n_vec
     const size_t op = io.take(pb), on = io.take(nb), ox = io.take(xb);
     if ((st = ensure_stage(ctx, io.used)) != BK_OK) return st;
     char *h = (char *)ctx->h_stage, *d = (char *)ctx->d_stage;
+    if (xb >= kHostPipeMin) {
+        const HostSeg in[2] = {{const_cast<uint8_t *>(packed), d + op, pb}, {const_cast<float *>(norms), d + on, nb}};
+        if ((st = host_pipe_h2d(ctx, in, 2)) != BK_OK) return st;
+        if ((st = launch_dequantize(ctx, bits, n_vec, (const uint8_t *)(d + op), (const float *)(d + on), (float *)(d + ox))) != BK_OK) return st;
+        const HostSeg out_seg{out, d + ox, xb};
+        return host_pipe_d2h(ctx, &out_seg, 1);
+    }
     memcpy(h + op, packed, pb);
     memcpy(h + on, norms, nb);
     BK_CUDA(ctx, cudaMemcpyAsync(d + op, h + op, ox - op, cudaMemcpyHostToDevice, ctx->stream));

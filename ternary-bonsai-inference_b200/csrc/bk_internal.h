@@ -50,6 +50,9 @@ struct RopeTable {
     ~RopeTable();
 };
 
+struct HostPipe;  // pinned slots and copy threads of bulk host transfers (bk_hostpipe.cpp)
+void host_pipe_destroy(HostPipe *p);
+
 enum RowKind : int { ROW_F32 = 0, ROW_F16 = 1, ROW_PLANAR = 2 };
 
 }  // namespace bk
@@ -79,6 +82,7 @@ struct bk_ctx {
     size_t d_layer_floats = 0;
     float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention's context chunks
     size_t d_prefill_floats = 0;
+    bk::HostPipe *pipe = nullptr;          // made by the first bulk host transfer
     uint8_t *d_pq2_x = nullptr;            // split activations of the batched PQ2_0 product, then a scale per token
     size_t pq2_x_bytes = 0;
     // split-K scratch of the decode kernel: partial results and arrival counters

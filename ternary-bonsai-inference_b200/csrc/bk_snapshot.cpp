@@ -12,11 +12,13 @@
 // n_layers, n_kv, hd, reserved[3]; then n_layers words with the number of cached positions of
 // each layer; then the layers' payloads.  Everything is host code over bk_cache_download /
 // bk_cache_upload; the file or socket that carries the buffer is the caller's.
+#include <sys/mman.h>
+
 #include <cstring>
 #include <string>
 #include <vector>
 
-#include "bk_internal.h"
+#include "bk_hostpipe.h"
 
 namespace {
 
@@ -31,6 +33,24 @@ struct Side {
 
 size_t side_bytes(const Side &s, size_t rows) {
     return rows * s.row_bytes + (s.kind == bk::ROW_PLANAR ? rows * sizeof(float) : 0);  // same total in both layouts
+}
+
+// The ranges of a layout-0 payload at `host`: per layer K rows (and norms), then V rows (and norms).
+template <class Rows>
+std::vector<bk::HostSeg> all_ranges(const bk_cache *c, int seq, uint8_t *host, const Rows &n_pos) {
+    std::vector<bk::HostSeg> segs;
+    auto add = [&](void *dev, size_t bytes) {
+        if (bytes) segs.push_back(bk::HostSeg{host, dev, bytes});
+        host += bytes;
+    };
+    for (int l = 0; l < c->cfg.n_layers; l++) {
+        const size_t rows = (size_t)n_pos(l) * c->cfg.n_kv;
+        add(c->k_rows(l, seq), rows * c->k_row_bytes);
+        if (c->k_kind == bk::ROW_PLANAR) add(c->k_norms(l, seq), rows * 4);
+        add(c->v_rows(l, seq), rows * c->v_row_bytes);
+        if (c->v_kind == bk::ROW_PLANAR) add(c->v_norms(l, seq), rows * 4);
+    }
+    return segs;
 }
 
 }  // namespace
@@ -71,6 +91,17 @@ bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void 
         off += 4;
     }
     const Side sides[2] = {{c->k_kind, c->k_row_bytes}, {c->v_kind, c->v_row_bytes}};
+    if (layout == 0) {  // every range goes where it lies in the buffer: one transfer for all layers
+        // A fresh buffer of this size costs more in page faults than in copying: ask for huge pages where it can have them.
+        constexpr uintptr_t kHuge = 2 << 20;
+        const uintptr_t lo = ((uintptr_t)buf + kHuge - 1) & ~(kHuge - 1), hi = ((uintptr_t)buf + need) & ~(kHuge - 1);
+        if (hi > lo) (void)madvise((void *)lo, hi - lo, MADV_HUGEPAGE);
+        std::vector<HostSeg> segs = all_ranges(c, seq, out + off, [&](int l) { return c->n_pos[c->slab(l, seq)]; });
+        bk_status st = bind_device(ctx);
+        if (st == BK_OK && !segs.empty()) st = host_pipe_d2h(ctx, segs.data(), segs.size());
+        if (st == BK_OK && written) *written = need;
+        return st;
+    }
     std::vector<uint8_t> rows_tmp;
     std::vector<float> norms_tmp;
     for (int l = 0; l < c->cfg.n_layers; l++) {
@@ -82,8 +113,8 @@ bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void 
             const bool planar = sd.kind == ROW_PLANAR;
             uint8_t *dst = out + off;
             void *rows_dst = dst;
-            float *norms_dst = planar ? reinterpret_cast<float *>(dst + rows * sd.row_bytes) : nullptr;
-            if (planar && layout == 1) {  // gather into temporaries, interleave below
+            float *norms_dst = nullptr;
+            if (planar) {  // gather into temporaries, interleave below
                 rows_tmp.resize(rows * sd.row_bytes);
                 norms_tmp.resize(rows);
                 rows_dst = rows_tmp.data();
@@ -92,7 +123,7 @@ bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void 
             const bk_status st = side == 0 ? bk_cache_download(c, l, seq, 0, np, rows_dst, norms_dst, nullptr, nullptr)
                                            : bk_cache_download(c, l, seq, 0, np, nullptr, nullptr, rows_dst, norms_dst);
             if (st != BK_OK) return st;
-            if (planar && layout == 1) {
+            if (planar) {
                 const size_t rb = sd.row_bytes;
                 for (size_t r = 0; r < rows; r++) {
                     memcpy(dst + r * (rb + 4), rows_tmp.data() + r * rb, rb);
@@ -139,6 +170,14 @@ bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size
         need += side_bytes(sides[0], rows) + side_bytes(sides[1], rows);
     }
     if (buf_bytes < need) return fail(ctx, BK_ERR_INVALID, "bk_cache_snapshot_load: truncated");
+    if (layout == 0) {
+        const std::vector<HostSeg> segs = all_ranges(c, seq, const_cast<uint8_t *>(in) + off, [&](int l) { return (int)np[l]; });
+        bk_status st = bind_device(ctx);
+        if (st == BK_OK && !segs.empty()) st = host_pipe_h2d(ctx, segs.data(), segs.size());
+        if (st == BK_OK) st = sync_and_check(ctx);
+        for (int l = 0; l < c->cfg.n_layers && st == BK_OK; l++) st = bk_cache_set_n_pos(c, l, seq, (int32_t)np[l]);
+        return st;
+    }
     std::vector<uint8_t> rows_tmp;
     std::vector<float> norms_tmp;
     for (int l = 0; l < c->cfg.n_layers; l++) {
@@ -149,8 +188,8 @@ bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size
                 const bool planar = sd.kind == ROW_PLANAR;
                 const uint8_t *src = in + off;
                 const void *rows_src = src;
-                const float *norms_src = planar ? reinterpret_cast<const float *>(src + rows * sd.row_bytes) : nullptr;
-                if (planar && layout == 1) {
+                const float *norms_src = nullptr;
+                if (planar) {
                     const size_t rb = sd.row_bytes;
                     rows_tmp.resize(rows * rb);
                     norms_tmp.resize(rows);
@@ -159,10 +198,6 @@ bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size
                         memcpy(&norms_tmp[r], src + r * (rb + 4) + rb, 4);
                     }
                     rows_src = rows_tmp.data();
-                    norms_src = norms_tmp.data();
-                } else if (planar) {  // the norms may sit at an address that is not 4-byte aligned for float access
-                    norms_tmp.resize(rows);
-                    memcpy(norms_tmp.data(), src + rows * sd.row_bytes, rows * 4);
                     norms_src = norms_tmp.data();
                 }
                 const bk_status st = side == 0

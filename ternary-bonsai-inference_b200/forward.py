@@ -29,6 +29,11 @@ def _i32_array(values):
     return a.ctypes.data_as(C.POINTER(C.c_int32)), a
 
 
+# A bytes object of a given size with its content still to be written, and where that content lies.
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_bytes_at = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
+
+
 class AttnCache:
     """Device KV cache of the full-attention layers (K roped, V raw)."""
 
@@ -163,10 +168,10 @@ class AttnCache:
     def snapshot(self, seq=0, layout=0):
         """All layers of one sequence as bytes (layout 0: the reference's CPU stores, 1: its device rows)."""
         n = self.ctx.lib.bk_cache_snapshot_bytes(self.h, seq)
-        buf = np.zeros(max(n, 1), np.uint8)
+        blob = _new_bytes(None, n)  # written once, by the library, before anybody else sees it
         written = C.c_size_t(0)
-        self.ctx.check(self.ctx.lib.bk_cache_snapshot_save(self.h, seq, layout, buf.ctypes.data, n, C.byref(written)))
-        return buf[:written.value].tobytes()
+        self.ctx.check(self.ctx.lib.bk_cache_snapshot_save(self.h, seq, layout, _bytes_at(blob), n, C.byref(written)))
+        return blob if written.value == n else blob[:written.value]
 
     def restore(self, blob, seq=0):
         """Load a snapshot taken from a cache of the same mode and head geometry; sets n_pos."""

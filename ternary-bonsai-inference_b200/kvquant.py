@@ -117,8 +117,8 @@ class PlanarQuant:
         """-> (packed uint8 [.., packed_len], norm float32 [..])"""
         a, single = self._batch(x, self.hd, np.float32)
         n = a.shape[0]
-        packed = np.zeros((n, self.packed_len()), np.uint8)
-        norms = np.zeros(n, np.float32)
+        packed = np.empty((n, self.packed_len()), np.uint8)
+        norms = np.empty(n, np.float32)
         c = self.ctx
         c.check(c.lib.bk_kvq_quantize(c.h, self.hd, self.bits, n, a.ctypes.data, packed.ctypes.data, norms.ctypes.data))
         return (packed[0], norms[0]) if single else (packed, norms)
@@ -126,14 +126,14 @@ class PlanarQuant:
     def dequantize(self, packed, norm):
         p, single = self._batch(packed, self.packed_len(), np.uint8)
         nrm = np.ascontiguousarray(norm, np.float32).reshape(-1)
-        out = np.zeros((p.shape[0], self.hd), np.float32)
+        out = np.empty((p.shape[0], self.hd), np.float32)
         c = self.ctx
         c.check(c.lib.bk_kvq_dequantize(c.h, self.hd, self.bits, p.shape[0], p.ctypes.data, nrm.ctypes.data, out.ctypes.data))
         return out[0] if single else out
 
     def _rot(self, x, inverse):
         a, single = self._batch(x, self.hd, np.float32)
-        out = np.zeros_like(a)
+        out = np.empty_like(a)
         c = self.ctx
         c.check(c.lib.bk_kvq_rotate(c.h, self.hd, a.shape[0], inverse, a.ctypes.data, out.ctypes.data))
         return out[0] if single else out
