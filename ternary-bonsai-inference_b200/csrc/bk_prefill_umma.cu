@@ -1,36 +1,34 @@
 // Batched (prefill) attention over a 4-, 3- or 2-bit planar cache, or an f16 or f32 cache, on the
-// 5th-generation tensor cores: the same work split, operands and arithmetic as bk_prefill.cu
-// (which documents them and stays as the mma.sync form), with both contractions issued as
-// tcgen05.mma and the accumulators in tensor memory.
+// 5th-generation tensor cores: the same work split and operands as bk_prefill.cu (which documents them and
+// stays as the mma.sync form), with both contractions issued as tcgen05.mma and the accumulators in tensor memory.
 //
-// One CTA = 128 query rows (M = 128) of one kv head over one context chunk; 8 warps.  Per tile
-// of 32 positions:
-//   1. all warps dequantize the packed K rows once into shared memory as f16 (for 4 bit also the
-//      rounding remainders, as rows 32-63 of the same K-major, 128-byte-swizzled operand tile);
-//   2. one thread issues S[128 x 32] = Q . K^T as 16 K-steps x (q_hi [k_hi; k_lo] with N = 64, then
-//      q_lo k_hi with N = 32) into tensor-memory columns and commits to an mbarrier; while those
-//      MMAs run, all warps dequantize V (hi and lo tiles, read later as the MN-major B operand);
-//   3. warps 0-3 (thread = query row: tensor-memory lane r is row r) read their row of S with
-//      tcgen05.ld, scale by ||k||, apply the causal limit, update the running reference R of
-//      s + log2 ||v|| LAZILY (only when the row maximum exceeds R by more than 8: the weights
-//      p = 2^(t - R) * 64 then stay below 2^14 in f16), rescale their row of O in tensor memory when
-//      R moved, and write the weights as f16 hi + lo into the no-swizzle K-major P tiles;
-//   4. the same thread issues O[128 x 256] += P . V as 2 K-steps x (p_hi v_hi + p_lo v_hi + p_hi v_lo)
-//      into 256 tensor-memory columns and commits.
-// f16 caches (BITS = 16) skip the dequantization: the TMA engine drops their rows, which are the
-// operands as stored, into two shared-memory stages through the cache's swizzled tensor maps.
-// f32 caches (BITS = 32) take the place of the dequantization with a split of every float into f16 hi + lo
-// (both K parts side by side as for 4 bit, both V parts as for 4 bit).
-// For packed and f32 caches the K rows of tile t + 1 are dequantized right after the O products of tile t are
-// issued (the K tile is free once S of tile t is complete), so that step runs under the tensor cores' work.
-// Every mbarrier wait is bounded (a time-out raises the context's error flag and the kernel runs
-// on to its end, where the tensor memory is always released).  The packed rows of the next tile
-// are fetched into registers (f16: into the other stage) while the current one is computed.
+// One CTA = 128 query rows (M = 128) of one kv head over one context chunk, tile by tile of 32 positions.  What
+// bounds it: for 4-bit and f32 rows six 128 x 32 x 256 products per tile (hi.hi, hi.lo, lo.hi twice), 1536 clocks of
+// the tensor cores, and about as much traffic of shared memory; so nothing may wait for anything else, and shared
+// memory has to be spared.  Thirteen warps in three roles, coupled by mbarriers only:
+//   * warps 4-11 (producers) turn packed rows into f16 operand tiles (for 4 bit with the rounding remainders, for
+//     f32 rows hi + lo parts) in a ring of five slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
+//     16-byte pieces of a row go out in an order that depends on its lane, or the eight lanes of a row would meet on
+//     two of eight bank groups.  f16 rows are operands as stored and are dropped in by the TMA engine.
+//   * warp 12 issues the products: S(t + 1) = Q . K^T goes ahead of O += P(t) . V, so the tensor cores work on S(t + 1)
+//     under the softmax of tile t.  The small terms of S come first: the accumulator truncates, and does so at
+//     the size of what it holds.
+//   * warps 0-3 (thread = query row = tensor-memory lane) read S, scale by ||k||, apply the causal limit, move the
+//     running reference R of s + log2 ||v|| LAZILY (only when the row maximum exceeds R by more than 8: the weights
+//     p = 2^(t - R) * 64 then stay below 2^14 in f16; their row of O is then rescaled in place) and write the
+//     weights as f16 hi + lo.
+// Tensor memory (all 512 columns): O 256 | q_hi 128 | S 2 x 32 | P (hi, lo) 2 x 32.  q_hi and P are A operands from
+// there: a product with N = 32 otherwise re-reads 4 KiB of q for 1 KiB of K.  q_lo stays in shared memory.
+// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.4 -> 6.2 ms, a 777-token f32 prompt in
+// one block 737 -> 301 us; before, one role after the other per tile, with every MMA operand moved to uniform registers.
+// Every mbarrier wait is bounded: one that runs out raises the context's error flag, the others of the CTA stop
+// waiting, and the kernel runs on to its end, where the tensor memory is always released.
 #include <cuda_fp16.h>
 #include <math_constants.h>
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "bk_device.cuh"
 #include "bk_internal.h"
@@ -41,7 +39,7 @@ namespace bk {
 
 namespace {
 
-constexpr int kUW = 8, kUT = kUW * 32;
+constexpr int kSoftWarps = 4, kProdWarps = 8, kMmaWarp = kSoftWarps + kProdWarps, kUWarps = kMmaWarp + 1, kUT = kUWarps * 32;
 constexpr int kRows = 128;  // query rows per CTA = tensor-memory lanes
 constexpr int kTK = 32;     // positions per tile
 constexpr float kPScale = 64.0f;
@@ -49,20 +47,25 @@ constexpr float kLazy = 8.0f;  // the reference moves when a row maximum exceeds
 
 constexpr uint32_t kQSlab = kRows * 128, kQTile = 4 * kQSlab;  // 16 KiB per 64-coordinate slab, 64 KiB per tile
 constexpr uint32_t kKVSlab = kTK * 128, kKVTile = 4 * kKVSlab;  // 4 KiB, 16 KiB
-constexpr uint32_t kPChunk = (kRows / 8) * 128, kPTile = 4 * kPChunk;  // 2 KiB per 8 positions, 8 KiB
+// Operand slots.  Five: K(t) then takes the place of V(t - 4), so what the softmax reads of tile t - 4 (its norms, kept for
+// four tiles) is read before the producers are at tile t.
+constexpr int kSlots = 5, kNormTiles = 4;
+constexpr uint32_t kSlotBytes = 2 * kKVTile;  // hi and lo tile
 // offsets from the 1024-byte aligned base
-constexpr uint32_t oQhi = 0, oQlo = kQTile, oKhi = 2 * kQTile, oKlo = oKhi + kKVTile, oVhi = oKlo + kKVTile,
-                   oVlo = oVhi + kKVTile, oPhi = oVlo + kKVTile, oPlo = oPhi + kPTile, oSmall = oPlo + kPTile;
+constexpr uint32_t oQlo = 0, oSlots = kQTile, oSmall = oSlots + kSlots * kSlotBytes;
 struct SmallU {
-    float kn[kTK], lv[kTK];  // ||k|| and log2 ||v|| of the tile's positions
     float givens[kHd];
-    __half table[16], table_lo[16];
-    unsigned long long bar_s, bar_o;
-    unsigned long long bar_t[2];  // f16 caches: the TMA engine fills two K/V stages
+    float kn[kNormTiles][kTK], lv[kNormTiles][kTK];  // ||k|| and log2 ||v|| of a tile's positions
+    unsigned long long full[kSlots], empty[kSlots];  // operand slots
+    unsigned long long norms[kNormTiles];            // kn, lv of a tile written
+    unsigned long long s_full[2], p_full[2], o_done[2], drain;
+    float mul[kRows];  // what a row's sums are multiplied by at the end
     uint32_t tmem_slot;
+    int gave_up;
 };
-constexpr uint32_t kUmmaSmem = oSmall + sizeof(SmallU) + 1024;  // + alignment slack
-constexpr uint32_t kTmemCols = 512, kColS = 0, kColO = 64;  // S: 32 (+32 for the k_lo term) columns, O: 256
+constexpr uint32_t kUmmaSmem = oSmall + 3072;
+static_assert(sizeof(SmallU) <= 3072 && kUmmaSmem <= 227 * 1024, "shared memory of a CTA");
+constexpr uint32_t kTmemCols = 512, kColO = 0, kColQ = 256, kColS = 384, kColP = 448;
 
 __device__ __forceinline__ uint32_t sw_off(int rows, int row, int chunk) {  // as tile_off in bk_prefill.cu
     return (uint32_t)((chunk >> 3) * rows * 128 + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
@@ -81,12 +84,24 @@ __device__ __forceinline__ uint32_t expand16u(uint32_t y) {  // eight 2-bit indi
     y = (y | (y << 2)) & 0x33333333u;
     return y;
 }
-// 32 coordinates (four words of eight nibbles) -> 32 halfs as four 16-byte chunks of a tile row.
+// The first `rot` (0..3) of four words go to the end: the piece order of a lane, see dequant_store_shfl.
+__device__ __forceinline__ void rotate4(uint32_t (&w)[4], int rot) {
+    if (rot & 1) {
+        const uint32_t t = w[0];
+        w[0] = w[1], w[1] = w[2], w[2] = w[3], w[3] = t;
+    }
+    if (rot & 2) {
+        const uint32_t t0 = w[0], t1 = w[1];
+        w[0] = w[2], w[1] = w[3], w[2] = t0, w[3] = t1;
+    }
+}
+// 32 coordinates (four words of eight nibbles, rotated by `rot`) -> 32 halfs as four 16-byte chunks of a tile row.
+// The eight lanes of a row store chunks 4 c + ((j + c / 2) & 3) together, one per bank group (4 c + j would put them on two).
 // The table sits in registers: lane i holds (hi | lo << 16) of centroid i & 15, one shuffle looks
 // both parts of an index up, and no shared-memory bank is involved.
 template <bool LO>
 __device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint32_t tab, uint8_t *tile_hi, uint8_t *tile_lo, int rows,
-                                                   int row_hi, int row_lo, int chunk0) {
+                                                   int row_hi, int row_lo, int chunk0, int rot) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         uint32_t h[4], l[4];
@@ -97,8 +112,9 @@ __device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint3
             h[e] = __byte_perm(v0, v1, 0x5410);
             l[e] = __byte_perm(v0, v1, 0x7632);
         }
-        *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, row_hi, chunk0 + j)) = make_uint4(h[0], h[1], h[2], h[3]);
-        if (LO) *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, chunk0 + j)) = make_uint4(l[0], l[1], l[2], l[3]);
+        const int chunk = chunk0 + ((j + rot) & 3);
+        *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, row_hi, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
+        if (LO) *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, chunk)) = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
 
@@ -113,16 +129,13 @@ struct PrefillUArgs {
 template <int BITS, int NREP, bool VF32 = false>
 __global__ void __launch_bounds__(kUT, 1)
 prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t sm[];
     const DecodeArgs &a = pa.d;
-    const uint32_t base0 = (uint32_t)__cvta_generic_to_shared(smem_raw), base = (base0 + 1023u) & ~1023u;
-    uint8_t *sm = smem_raw + (base - base0);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm), small = base + oSmall;
     SmallU &ss = *reinterpret_cast<SmallU *>(sm + oSmall);
-    const uint32_t bar_s = base + oSmall + (uint32_t)offsetof(SmallU, bar_s), bar_o = base + oSmall + (uint32_t)offsetof(SmallU, bar_o);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // BITS = 16 stands for an f16 cache: its rows ARE the operands, so the TMA engine drops them into
-    // two shared-memory stages in the swizzled layout and nothing is dequantized (no table, no norms,
-    // no Givens rotation); everything else is the same kernel.
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    // BITS = 16 stands for an f16 cache: its rows ARE the operands, so the TMA engine drops them into the slots in
+    // the swizzled layout and nothing is dequantized (no table, no norms, no Givens rotation).
     constexpr bool kF16 = BITS == 16;
     // BITS = 32 stands for an f32 cache: its rows are split into f16 hi + lo on their way into the operand tiles
     // (the lo tiles are the ones the 4-bit rows use for their rounding remainders); like f16 rows they are
@@ -137,11 +150,6 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     // lo tiles: the rounding remainders of the 4-bit table (see bk_prefill.cu: it is only good to 1e-4), the lo parts
     // of f32 rows; beside raw V rows (several times larger than dequantized ones) the 3-bit table carries them too
     constexpr bool kLoTiles = BITS == 4 || kF32 || VF32;
-    // The K operand holds k_hi in rows 0-31 of every slab and, for 4 bit, k_lo in rows 32-63: one MMA
-    // with N = 64 then yields q_hi k_hi and q_hi k_lo side by side (q is re-read from shared memory
-    // once instead of twice, and that read is what an N = 32 MMA waits for).
-    constexpr int kKRows = kLoTiles ? 64 : 32;
-    constexpr uint32_t kKSlab = kKRows * 128;
 
     // ---- which item (as in the mma.sync kernel) ---------------------------------------------
     const int item = blockIdx.x;
@@ -155,43 +163,96 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
 
     // ---- tables, barriers, tensor memory ----------------------------------------------------
     for (int i = tid; i < kHd; i += kUT) ss.givens[i] = a.givens[i];
-    if (tid < 16) {
-        const float c = kRaw ? 0.f : a.book[tid & ((1 << (kRaw ? 4 : BITS)) - 1)] * pa.lut_alpha;
-        const __half h = __float2half_rn(c);
-        ss.table[tid] = h;
-        ss.table_lo[tid] = __float2half_rn(c - __half2float(h));
-    }
-    if (kRaw && tid < kTK) {  // no norms: ||k|| = 1, log2 ||v|| = 0
-        ss.kn[tid] = 1.f;
-        ss.lv[tid] = 0.f;
-    }
-    const uint32_t bar_t = base + oSmall + (uint32_t)offsetof(SmallU, bar_t);
+    auto bar_at = [&](size_t off, int i) { return small + (uint32_t)off + 8u * (uint32_t)i; };
+    const uint32_t bar_full = bar_at(offsetof(SmallU, full), 0), bar_empty = bar_at(offsetof(SmallU, empty), 0),
+                   bar_norms = bar_at(offsetof(SmallU, norms), 0), bar_s = bar_at(offsetof(SmallU, s_full), 0),
+                   bar_p = bar_at(offsetof(SmallU, p_full), 0), bar_o = bar_at(offsetof(SmallU, o_done), 0),
+                   bar_drain = bar_at(offsetof(SmallU, drain), 0);
     if (tid == 0) {
-        mbar_init(bar_s, 1);
-        mbar_init(bar_o, 1);
-        mbar_init(bar_t, 1);
-        mbar_init(bar_t + 8, 1);
+        for (int i = 0; i < kSlots; i++) {
+            mbar_init(bar_full + 8 * i, kF16 ? 1 : kProdWarps);
+            mbar_init(bar_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < kNormTiles; i++) mbar_init(bar_norms + 8 * i, 2);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(bar_s + 8 * i, 1);
+            mbar_init(bar_p + 8 * i, kSoftWarps);
+            mbar_init(bar_o + 8 * i, 1);
+        }
+        mbar_init(bar_drain, 1);
+        ss.gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    if (warp == 0) tmem_alloc(base + oSmall + (uint32_t)offsetof(SmallU, tmem_slot), kTmemCols);
+    if (warp == 0) tmem_alloc(small + (uint32_t)offsetof(SmallU, tmem_slot), kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = ss.tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, ss.tmem_slot, 0);
     const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
 
-    // O starts at zero (it is rescaled before the first product is added)
-    if (warp < 4) {
-        uint32_t z[32];
-#pragma unroll
-        for (int j = 0; j < 32; j++) z[j] = 0u;
-        for (int b = 0; b < 8; b++) tmem_st32(my_tmem + kColO + 32 * b, z);
-        tmem_wait_st();
-    }
+    // bounded wait; after one has run out (never expected) the others of the CTA do not start to wait
+    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+        volatile int *gave_up = &ss.gave_up;
+        int polls = 0;
+        while (!mbar_try_wait(bar, parity)) {
+            if (*gave_up) return false;
+            if (++polls > kWaitPolls) {
+                *gave_up = 1;
+                raise_error(pa.err_flag, 4);
+                return false;
+            }
+        }
+        return true;
+    };
 
-    // ---- q rows -> the two q tiles (rope, Givens, scale, f16 hi/lo); staged through the K tile ----
+    // ---- a producer thread's share of a packed tile: position pt / 8, coordinates 32 (pt % 8) .. + 31 ------
+    const int pt = (tid - 32 * kSoftWarps) & 255, my_row = pt >> 3, my_c = pt & 7, rot = my_c >> 1;
+    const bool producer = warp >= kSoftWarps && warp < kMmaWarp;
+    const size_t seq_rows = (size_t)pa.seq * a.seq_stride_rows;
+    auto row_of = [&](int tile, int r) {  // rows past the cache's end are never used: any row of it will do
+        return seq_rows + (size_t)min(c0 + tile * kTK + r, a.n_ctx - 1) * a.n_kv + kv;
+    };
+    uint32_t pk[4], pv[4];  // packed K of one tile and packed V of the tile before, on their way
+    float pn = 0.f;
+    // f32 rows: the thread's 128 bytes, its four 16-byte operand pieces in the lane's order
+    [[maybe_unused]] float4 fk[kF32 ? 8 : 1], fv[kVRows32 ? 8 : 1];
+    auto fetch_f32 = [&](float4 *dst, const uint8_t *rows, int tile) {
+        const float4 *src = reinterpret_cast<const float4 *>(rows + row_of(tile, my_row) * 1024) + 8 * my_c;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            dst[2 * j] = __ldg(src + 2 * ((j + rot) & 3));
+            dst[2 * j + 1] = __ldg(src + 2 * ((j + rot) & 3) + 1);
+        }
+    };
+    auto fetch_packed = [&](uint32_t (&w)[4], const uint8_t *rows, int tile) {
+        const uint8_t *p = rows + row_of(tile, my_row) * kRowBytes;
+        if constexpr (BITS == 4) {
+            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(p) + my_c);
+            w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+        } else if constexpr (BITS == 3) {
+            const uint32_t *p3 = reinterpret_cast<const uint32_t *>(p) + 3 * my_c;
+            w[0] = __ldg(p3), w[1] = __ldg(p3 + 1), w[2] = __ldg(p3 + 2), w[3] = 0;
+        } else {  // 2 bit: 32 coordinates are 8 bytes
+            const uint2 x = __ldg(reinterpret_cast<const uint2 *>(p) + my_c);
+            w[0] = x.x, w[1] = x.y, w[2] = w[3] = 0;
+        }
+    };
+    auto fetch_k = [&](int tile) {
+        if constexpr (kF32) {
+            fetch_f32(fk, a.k_rows, tile);
+        } else if constexpr (!kF16) {
+            fetch_packed(pk, a.k_rows, tile);
+            if (pt < (VF32 ? kTK : 2 * kTK)) pn = __ldg((pt < kTK ? a.k_norms : a.v_norms) + row_of(tile, pt & (kTK - 1)));
+        }
+    };
+    auto fetch_v = [&](int tile) {
+        if constexpr (kVRows32) fetch_f32(fv, a.v_rows, tile);
+        else if constexpr (!kF16) fetch_packed(pv, a.v_rows, tile);
+    };
+
+    // ---- q rows -> q_hi (through slots 0 and 1, then to tensor memory) and q_lo: rope, Givens, scale, f16 hi/lo ----
     {
-        float *stage = reinterpret_cast<float *>(sm + oKhi) + warp * (kHd + 8);  // rows are padded by one float per 32 (see pad())
+        float *stage = reinterpret_cast<float *>(sm + oSlots + 2 * kSlotBytes) + warp * (kHd + 8);  // rows are padded by one float per 32 (see pad())
         auto pad = [](int i) { return i + (i >> 5); };  // lanes 8 coordinates apart land in different banks
         const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / pa.lut_alpha;
         const int half = a.n_rot >> 1;
@@ -210,7 +271,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             }
         };
         prefetch(warp);
-        for (int r = warp; r < kRows; r += kUW) {
+        for (int r = warp; r < kRows; r += kUWarps) {
             const bool real = r < n_rows;
             if (real) {
                 float2 rc[4];
@@ -218,7 +279,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 for (int i = 0; i < 8; i++) stage[pad(lane + 32 * i)] = xn[i];
 #pragma unroll
                 for (int i = 0; i < 4; i++) rc[i] = rn[i];
-                prefetch(r + kUW);
+                prefetch(r + kUWarps);
                 __syncwarp();
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -253,233 +314,255 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 lw[p] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
             }
             const uint32_t off = sw_off(kRows, r, lane);
-            *reinterpret_cast<uint4 *>(sm + oQhi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            *reinterpret_cast<uint4 *>(sm + oSlots + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
             *reinterpret_cast<uint4 *>(sm + oQlo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             __syncwarp();
         }
     }
-
-    fence_smem_to_async_proxy();  // (f16: the TMA engine writes where the staging rows were)
-    __syncthreads();  // the staging area becomes the K tile
-
-    // ---- per-thread share of a packed tile: position tid / 8, coordinates 32 (tid % 8) .. + 31 ----
-    const int my_row = tid >> 3, my_c = tid & 7;
-    const size_t seq_rows = (size_t)pa.seq * a.seq_stride_rows;
-    uint32_t pk[4], pv[4];
-    float pn = 0.f;
-    // f32: the thread's 128 bytes of a K row or of a V row (one buffer: K of this tile until it is split, then
-    // V of this tile, then K of the next one)
-    [[maybe_unused]] float4 pf[kVRows32 ? 8 : 1];
-    [[maybe_unused]] auto fetch_f32 = [&](int tile, bool v_side) {
-        const int pos = min(c0 + tile * kTK + my_row, a.n_ctx - 1);
-        const size_t row = seq_rows + (size_t)pos * a.n_kv + kv;
-        const float4 *src = reinterpret_cast<const float4 *>((v_side ? a.v_rows : a.k_rows) + row * 1024) + 8 * my_c;
+    fence_smem_to_async_proxy();
+    __syncthreads();
+    const int my_q = (warp & 3) * 32 + lane;  // query row of a softmax thread
+    if (warp < kSoftWarps) {
 #pragma unroll
-        for (int i = 0; i < (kVRows32 ? 8 : 1); i++) pf[i] = __ldg(src + i);
-    };
-    // f32: split the buffer into f16 hi + lo and store both as four 16-byte chunks of a tile row; rows at or past
-    // `end` are stored as zeros (they may hold anything, and 0 * Inf would poison the accumulators)
-    [[maybe_unused]] auto split_store_f32 = [&](uint8_t *tile_hi, uint8_t *tile_lo, int rows, int row_hi, int row_lo, bool live) {
+        for (int b = 0; b < 4; b++) {
+            uint32_t r[32];
 #pragma unroll
-        for (int j = 0; j < (kVRows32 ? 4 : 0); j++) {
-            const float x[8] = {pf[2 * j].x, pf[2 * j].y, pf[2 * j].z, pf[2 * j].w, pf[2 * j + 1].x, pf[2 * j + 1].y, pf[2 * j + 1].z, pf[2 * j + 1].w};
-            uint32_t h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const float x0 = live ? x[2 * e] : 0.f, x1 = live ? x[2 * e + 1] : 0.f;
-                const __half2 hv = __floats2half2_rn(x0, x1);
-                const float2 hf = __half22float2(hv);
-                const __half2 lv = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
-                h[e] = *reinterpret_cast<const uint32_t *>(&hv);
-                l[e] = *reinterpret_cast<const uint32_t *>(&lv);
+            for (int j = 0; j < 8; j++) {
+                const uint4 x = *reinterpret_cast<const uint4 *>(sm + oSlots + sw_off(kRows, my_q, 8 * b + j));
+                r[4 * j] = x.x, r[4 * j + 1] = x.y, r[4 * j + 2] = x.z, r[4 * j + 3] = x.w;
             }
-            *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, row_hi, 4 * my_c + j)) = make_uint4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, 4 * my_c + j)) = make_uint4(l[0], l[1], l[2], l[3]);
+            tmem_st32(my_tmem + kColQ + 32 * b, r);
         }
-    };
-    auto fetch = [&](int tile) {
-        if constexpr (kF16) return;
-        if constexpr (kF32) {
-            fetch_f32(tile, false);
-            return;
-        }
-        const int pos = min(c0 + tile * kTK + my_row, a.n_ctx - 1);
-        const size_t row = seq_rows + (size_t)pos * a.n_kv + kv;
-        const uint8_t *kr = a.k_rows + row * kRowBytes, *vr = a.v_rows + row * kRowBytes;
-        if constexpr (VF32) {  // only the K row is packed (vr is not used: the V row is fetched as floats below)
-            if constexpr (BITS == 4) {
-                const uint4 x = __ldg(reinterpret_cast<const uint4 *>(kr) + my_c);
-                pk[0] = x.x; pk[1] = x.y; pk[2] = x.z; pk[3] = x.w;
-            } else {
-                const uint32_t *k3 = reinterpret_cast<const uint32_t *>(kr) + 3 * my_c;
-                pk[0] = __ldg(k3); pk[1] = __ldg(k3 + 1); pk[2] = __ldg(k3 + 2); pk[3] = 0;
-            }
-        } else if constexpr (BITS == 4) {
-            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(kr) + my_c), y = __ldg(reinterpret_cast<const uint4 *>(vr) + my_c);
-            pk[0] = x.x; pk[1] = x.y; pk[2] = x.z; pk[3] = x.w;
-            pv[0] = y.x; pv[1] = y.y; pv[2] = y.z; pv[3] = y.w;
-        } else if constexpr (BITS == 3) {
-            const uint32_t *k3 = reinterpret_cast<const uint32_t *>(kr) + 3 * my_c, *v3 = reinterpret_cast<const uint32_t *>(vr) + 3 * my_c;
-            pk[0] = __ldg(k3); pk[1] = __ldg(k3 + 1); pk[2] = __ldg(k3 + 2); pk[3] = 0;
-            pv[0] = __ldg(v3); pv[1] = __ldg(v3 + 1); pv[2] = __ldg(v3 + 2); pv[3] = 0;
-        } else {  // 2 bit: 32 coordinates are 8 bytes
-            const uint2 x = __ldg(reinterpret_cast<const uint2 *>(kr) + my_c), y = __ldg(reinterpret_cast<const uint2 *>(vr) + my_c);
-            pk[0] = x.x; pk[1] = x.y; pk[2] = pk[3] = 0;
-            pv[0] = y.x; pv[1] = y.y; pv[2] = pv[3] = 0;
-        }
-        if (tid < (VF32 ? kTK : 2 * kTK)) {
-            const int p2 = min(c0 + tile * kTK + (tid & (kTK - 1)), a.n_ctx - 1);
-            pn = __ldg((tid < kTK ? a.k_norms : a.v_norms) + seq_rows + (size_t)p2 * a.n_kv + kv);
-        }
-        if constexpr (VF32) fetch_f32(tile, true);
-    };
-    auto widen = [&](uint32_t (&w)[4]) {
-        if constexpr (BITS == 3) {
-            const uint32_t u0 = w[0], u1 = w[1], u2 = w[2];
-            w[0] = expand24u(u0);
-            w[1] = expand24u(__funnelshift_r(u0, u1, 24));
-            w[2] = expand24u(__funnelshift_r(u1, u2, 16));
-            w[3] = expand24u(u2 >> 8);
-        } else if constexpr (BITS == 2) {  // sixteen indices per word -> two words of eight nibbles
-            const uint32_t u0 = w[0], u1 = w[1];
-            w[0] = expand16u(u0);
-            w[1] = expand16u(u0 >> 16);
-            w[2] = expand16u(u1);
-            w[3] = expand16u(u1 >> 16);
-        }
-    };
-    auto wait_bar = [&](uint32_t bar, uint32_t parity) {
-        int polls = 0;
-        while (!mbar_try_wait(bar, parity)) {
-            if (++polls > kWaitPolls) {  // never expected; leave a mark and go on rather than hang
-                if (lane == 0) raise_error(pa.err_flag, 4);
-                break;
-            }
-        }
-    };
-
-    // this thread's query row (warps 0-3): causal limit, running reference and sum
-    const int my_q = (warp & 3) * 32 + lane;
-    const int lim = (warp < 4 && my_q < n_rows) ? pa.pos0 + tok0 + my_q / NREP + 1 : 0;
-    float R = -CUDART_INF_F, lsum = 0.f;
-    const uint32_t tab = (uint32_t)__half_as_ushort(ss.table[lane & 15]) | ((uint32_t)__half_as_ushort(ss.table_lo[lane & 15]) << 16);
-    const uint32_t idesc_s = umma_idesc_f16(kRows, kTK, 0, 0), idesc_s2 = umma_idesc_f16(kRows, kKRows, 0, 0);
-    const uint32_t idesc_o = umma_idesc_f16(kRows, kHd, 0, 1);
-
-    // f16: one thread has the TMA engine copy tile `tile` (32 rows x 512 bytes of K and of V, as
-    // 16 boxes of 16 rows x 128 bytes) into stage st; completion on bar_t[st].
-    auto issue_tma = [&](int tile, int st) {
-        const uint32_t bar = bar_t + (uint32_t)st * 8u, dstk = base + oKhi + (uint32_t)st * 2u * kKVTile, dstv = dstk + kKVTile;
-        mbar_expect_tx(bar, 2 * kKVTile);
-        const int gpos = a.layer_pos0 + pa.seq * a.n_ctx + c0 + tile * kTK;
-#pragma unroll
-        for (int sl = 0; sl < 4; sl++)
-#pragma unroll
-            for (int hf = 0; hf < 2; hf++) {
-                tma_tile_x(dstk + sl * kKVSlab + hf * 2048, &tm_k, sl * 128, kv, gpos + 16 * hf, bar);
-                tma_tile_x(dstv + sl * kKVSlab + hf * 2048, &tm_v, sl * 128, kv, gpos + 16 * hf, bar);
-            }
-    };
-    // Packed (or f32) caches: K of tile t + 1 is dequantized right after the O products of tile t are issued, so
-    // that it runs under them (the K tile is free once S of tile t is complete, which the softmax has waited for);
-    // the norms of the tile travel with it.
-    [[maybe_unused]] auto dequant_k = [&](int tile) {
-        if constexpr (kF32) {
-            split_store_f32(sm + oKhi, sm + oKhi, kKRows, my_row, my_row + 32, c0 + tile * kTK + my_row < c1);
-            fetch_f32(tile, true);  // this tile's V rows travel while the S products are issued
-        } else if constexpr (!kF16) {
-            widen(pk);
-            dequant_store_shfl<kLoTiles>(pk, tab, sm + oKhi, sm + oKhi, kKRows, my_row, my_row + 32, 4 * my_c);
-            if (tid < kTK) ss.kn[tid] = pn;
-            else if (tid < 2 * kTK) ss.lv[tid - kTK] = VF32 ? 0.f : fast_log2(fmaxf(pn, 1e-30f));
-        }
-        fence_smem_to_async_proxy();
-    };
-    if constexpr (kF16) {
-        if (tid == 0 && n_tiles > 0) issue_tma(0, 0);
-    } else {
-        if (n_tiles > 0) {
-            fetch(0);
-            dequant_k(0);
-        }
-        __syncthreads();
+        tmem_wait_st();
+        fence_smem_to_async_proxy();  // (f16: the TMA engine writes where q_hi was read)
     }
-    for (int tile = 0; tile < n_tiles; tile++) {
-        const uint32_t parity = (uint32_t)tile & 1u;
-        const int st = kF16 ? (tile & 1) : 0;
-        const uint32_t k_off = kF16 ? oKhi + (uint32_t)st * 2u * kKVTile : oKhi, v_off = kF16 ? k_off + kKVTile : oVhi;
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+
+    float R = -CUDART_INF_F, lsum = 0.f;  // a query row's running reference and sum
+    if (warp == kMmaWarp) {
+        // ---- the products -----------------------------------------------------------------------------------
+        constexpr int kKRows = kLoTiles ? 64 : 32;  // a K slab holds k_hi in rows 0-31 and k_lo in rows 32-63
+        constexpr uint32_t kKSlab = kKRows * 128;
+        const uint32_t idesc_s = umma_idesc_f16(kRows, kTK, 0, 0), idesc_o = umma_idesc_f16(kRows, kHd, 0, 1);
+        uint32_t slot = 0, use = 0;
+        auto next_slot = [&]() {
+            if (++slot == kSlots) slot = 0, use ^= 1u;
+        };
+        auto issue_s = [&](int tile) -> bool {
+            if (!__all_sync(0xffffffffu, wait(bar_full + 8 * slot, use))) return false;
+            tc_fence_after_sync();
+            const uint32_t d = tmem + kColS + (uint32_t)(tile & 1) * 32u, kb = base + oSlots + slot * kSlotBytes;
+            const uint64_t kd = umma_smem_desc(kb, 16, 1024, kUmmaSwizzle128), ql = umma_smem_desc(base + oQlo, 16, 1024, kUmmaSwizzle128);
+            if (elect_one()) {  // (the address field of a descriptor counts 16-byte units)
+#pragma unroll
+                for (int ks = 0; ks < 16; ks++)
+                    umma_f16_ss(d, ql + (((ks >> 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0);
+                if constexpr (kLoTiles) {
+#pragma unroll
+                    for (int ks = 0; ks < 16; ks++)
+                        umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + 4096 + (ks & 3) * 32) >> 4), idesc_s, true);
+                }
+#pragma unroll
+                for (int ks = 0; ks < 16; ks++)
+                    umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s, true);
+                umma_commit(bar_s + 8 * (tile & 1));
+                umma_commit(bar_empty + 8 * slot);
+            }
+            __syncwarp();
+            next_slot();
+            return true;
+        };
+        bool ok = n_tiles == 0 || issue_s(0);
+        for (int tile = 0; ok && tile < n_tiles; tile++) {
+            // (S(tile + 1) goes where S(tile - 1) was, which the softmax had read when P(tile - 1) was awaited)
+            if (tile + 1 < n_tiles && !issue_s(tile + 1)) break;
+            ok = wait(bar_full + 8 * slot, use);
+            ok = ok && wait(bar_p + 8 * (tile & 1), (uint32_t)(tile >> 1) & 1u);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t p = tmem + kColP + (uint32_t)(tile & 1) * 32u, vb = base + oSlots + slot * kSlotBytes;
+            const uint64_t vd = umma_smem_desc(vb, kKVSlab, 1024, kUmmaSwizzle128);
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < 2; kk++) {
+                    umma_f16_ts(tmem + kColO, p + 8 * kk, vd + ((kk * 2048) >> 4), idesc_o, tile > 0 || kk > 0);
+                    umma_f16_ts(tmem + kColO, p + 16 + 8 * kk, vd + ((kk * 2048) >> 4), idesc_o, true);
+                    if constexpr (kLoTiles) umma_f16_ts(tmem + kColO, p + 8 * kk, vd + ((kKVTile + kk * 2048) >> 4), idesc_o, true);
+                }
+                umma_commit(bar_o + 8 * (tile & 1));
+                umma_commit(bar_empty + 8 * slot);
+            }
+            __syncwarp();
+            next_slot();
+        }
+        // nothing in flight is left behind, whatever happened above
+        if (elect_one()) umma_commit(bar_drain);
+        __syncwarp();
+        for (int polls = 0; !mbar_try_wait(bar_drain, 0) && polls < kWaitPolls; polls++) {}
+    } else if (producer) {
+        // ---- operand tiles ------------------------------------------------------------------------------------
+        uint32_t slot = 0, use = 0;
+        auto next_slot = [&]() {
+            if (++slot == kSlots) slot = 0, use++;
+        };
+        auto slot_free = [&]() { return use == 0 || wait(bar_empty + 8 * slot, (use - 1) & 1u); };
         if constexpr (kF16) {
-            // ---- 1. the next tile starts travelling (its stage was released when bar_o was awaited);
-            // this tile has landed; rows past the chunk's end may hold anything and are zeroed
-            if (tid == 0 && tile + 1 < n_tiles) issue_tma(tile + 1, st ^ 1);
-            wait_bar(bar_t + (uint32_t)st * 8u, (uint32_t)(tile >> 1) & 1u);
-            const int valid = c1 - (c0 + tile * kTK);
-            if (valid < kTK) {
-                for (int i = tid; i < 2 * 4 * kTK * 8; i += kUT) {
-                    const int tl = i >> 10, slab = (i >> 8) & 3, r = (i >> 3) & 31, c = i & 7;
-                    if (r >= valid) *reinterpret_cast<uint4 *>(sm + k_off + tl * kKVTile + slab * kKVSlab + r * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+            if (warp == kSoftWarps) {
+                // a tile that is whole: 8 boxes of 16 rows x 128 bytes by the TMA engine; the last one when rows of it are past
+                // the chunk's end (they may hold anything, and 0 * Inf would poison the accumulators): by the warp, with zeros
+                auto put = [&](int tile, const CUtensorMap *map, const uint8_t *rows) -> bool {
+                    if (!__all_sync(0xffffffffu, slot_free())) return false;
+                    const int valid = c1 - (c0 + tile * kTK);
+                    const uint32_t bar = bar_full + 8 * slot, dst = base + oSlots + slot * kSlotBytes;
+                    if (valid >= kTK) {
+                        if (elect_one()) {
+                            mbar_expect_tx(bar, kKVTile);
+                            const int gpos = a.layer_pos0 + pa.seq * a.n_ctx + c0 + tile * kTK;
+#pragma unroll
+                            for (int sl = 0; sl < 4; sl++)
+#pragma unroll
+                                for (int hf = 0; hf < 2; hf++) tma_tile_x(dst + sl * kKVSlab + hf * 2048, map, sl * 128, kv, gpos + 16 * hf, bar);
+                        }
+                    } else {
+                        for (int r = 0; r < kTK; r++) {
+                            uint4 x = make_uint4(0, 0, 0, 0);
+                            if (r < valid) x = __ldg(reinterpret_cast<const uint4 *>(rows + row_of(tile, r) * 512) + lane);
+                            *reinterpret_cast<uint4 *>(sm + oSlots + slot * kSlotBytes + sw_off(kTK, r, lane)) = x;
+                        }
+                        fence_smem_to_async_proxy();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar);
+                    }
+                    __syncwarp();
+                    next_slot();
+                    return true;
+                };
+                bool ok = n_tiles == 0 || put(0, &tm_k, a.k_rows);
+                for (int tile = 0; ok && tile < n_tiles; tile++) {
+                    if (tile + 1 < n_tiles) ok = put(tile + 1, &tm_k, a.k_rows);
+                    ok = ok && put(tile, &tm_v, a.v_rows);
+                }
+                if (!ok) {  // gave up: leave no copy in flight behind (every slot that was filled before this one)
+                    const uint32_t filled = use * kSlots + slot;
+                    for (uint32_t i = filled > kSlots ? filled - kSlots : 0; i < filled; i++) {
+                        int polls = 0;
+                        while (!mbar_try_wait(bar_full + 8 * (i % kSlots), (i / kSlots) & 1u) && ++polls < kWaitPolls) {}
+                    }
                 }
             }
-            fence_smem_to_async_proxy();
-            __syncthreads();
-        }  // (packed and f32 caches: K of this tile was dequantized at the end of the previous iteration)
-
-        // ---- 2. S = Q . K^T, and V is dequantized while it runs ---------------------------------------
-        if (tid == 0) {
-            tc_fence_after_sync();
+        } else {
+            const float cent = kRaw ? 0.f : a.book[lane & ((1 << (kRaw ? 4 : BITS)) - 1)] * pa.lut_alpha;
+            const __half cent_hi = __float2half_rn(cent);
+            const uint32_t tab = (uint32_t)__half_as_ushort(cent_hi) | ((uint32_t)__half_as_ushort(__float2half_rn(cent - __half2float(cent_hi))) << 16);
+            // split the fetched floats into f16 hi + lo and store both as four 16-byte chunks of a tile row; rows at or past
+            // the chunk's end are stored as zeros (they may hold anything, and 0 * Inf would poison the accumulators)
+            auto split_store = [&](const float4 *f, uint8_t *tile_hi, uint8_t *tile_lo, int rows, int row_lo, bool live) {
 #pragma unroll
-            for (int ks = 0; ks < 16; ks++) {
-                const uint32_t qo = (uint32_t)(ks >> 2) * kQSlab + (uint32_t)(ks & 3) * 32u;
-                const uint32_t ko = (uint32_t)(ks >> 2) * kKSlab + (uint32_t)(ks & 3) * 32u;
-                const uint64_t qh = umma_smem_desc(base + oQhi + qo, 16, 1024, kUmmaSwizzle128);
-                const uint64_t ql = umma_smem_desc(base + oQlo + qo, 16, 1024, kUmmaSwizzle128);
-                const uint64_t kd = umma_smem_desc(base + k_off + ko, 16, 1024, kUmmaSwizzle128);
-                umma_f16_ss(tmem + kColS, qh, kd, idesc_s2, ks > 0);  // columns 0-31: q_hi k_hi, 32-63: q_hi k_lo
-                umma_f16_ss(tmem + kColS, ql, kd, idesc_s, true);     // columns 0-31 += q_lo k_hi
+                for (int j = 0; j < 4; j++) {
+                    const float x[8] = {f[2 * j].x, f[2 * j].y, f[2 * j].z, f[2 * j].w, f[2 * j + 1].x, f[2 * j + 1].y, f[2 * j + 1].z, f[2 * j + 1].w};
+                    uint32_t h[4], l[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float x0 = live ? x[2 * e] : 0.f, x1 = live ? x[2 * e + 1] : 0.f;
+                        const __half2 hv = __floats2half2_rn(x0, x1);
+                        const float2 hf = __half22float2(hv);
+                        const __half2 lv = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
+                        h[e] = *reinterpret_cast<const uint32_t *>(&hv);
+                        l[e] = *reinterpret_cast<const uint32_t *>(&lv);
+                    }
+                    const int ch = 4 * my_c + ((j + rot) & 3);
+                    *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, my_row, ch)) = make_uint4(h[0], h[1], h[2], h[3]);
+                    *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, ch)) = make_uint4(l[0], l[1], l[2], l[3]);
+                }
+            };
+            auto widen = [&](uint32_t (&w)[4]) {
+                if constexpr (BITS == 3) {
+                    const uint32_t u0 = w[0], u1 = w[1], u2 = w[2];
+                    w[0] = expand24u(u0);
+                    w[1] = expand24u(__funnelshift_r(u0, u1, 24));
+                    w[2] = expand24u(__funnelshift_r(u1, u2, 16));
+                    w[3] = expand24u(u2 >> 8);
+                } else if constexpr (BITS == 2) {  // sixteen indices per word -> two words of eight nibbles
+                    const uint32_t u0 = w[0], u1 = w[1];
+                    w[0] = expand16u(u0);
+                    w[1] = expand16u(u0 >> 16);
+                    w[2] = expand16u(u1);
+                    w[3] = expand16u(u1 >> 16);
+                }
+                rotate4(w, rot);
+            };
+            auto put_done = [&]() {
+                fence_smem_to_async_proxy();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * slot);
+                next_slot();
+            };
+            auto live = [&](int tile) { return c0 + tile * kTK + my_row < c1; };
+            auto put_k = [&](int tile) -> bool {
+                if (!slot_free()) return false;
+                __syncwarp();
+                uint8_t *dst = sm + oSlots + slot * kSlotBytes;
+                if constexpr (kF32) {
+                    split_store(fk, dst, dst, 64, my_row + 32, live(tile));
+                } else {
+                    widen(pk);
+                    dequant_store_shfl<kLoTiles>(pk, tab, dst, dst, kLoTiles ? 64 : 32, my_row, my_row + 32, 4 * my_c, rot);
+                    if (pt < 2 * kTK) {
+                        if (pt < kTK) ss.kn[tile % kNormTiles][pt] = pn;
+                        else ss.lv[tile % kNormTiles][pt - kTK] = VF32 ? 0.f : fast_log2(fmaxf(pn, 1e-30f));
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_norms + 8 * (tile % kNormTiles));
+                    }
+                }
+                put_done();
+                if (tile + 1 < n_tiles) fetch_k(tile + 1);
+                return true;
+            };
+            auto put_v = [&](int tile) -> bool {
+                if (!slot_free()) return false;
+                __syncwarp();
+                uint8_t *dst = sm + oSlots + slot * kSlotBytes;
+                if constexpr (kVRows32) {
+                    split_store(fv, dst, dst + kKVTile, kTK, my_row, live(tile));
+                } else {
+                    widen(pv);
+                    dequant_store_shfl<kLoTiles>(pv, tab, dst, dst + kKVTile, kTK, my_row, my_row, 4 * my_c, rot);
+                }
+                put_done();
+                if (tile + 1 < n_tiles) fetch_v(tile + 1);
+                return true;
+            };
+            if (n_tiles > 0) fetch_k(0), fetch_v(0);
+            bool ok = n_tiles == 0 || put_k(0);
+            for (int tile = 0; __all_sync(0xffffffffu, ok) && tile < n_tiles; tile++) {
+                if (tile + 1 < n_tiles) ok = __all_sync(0xffffffffu, put_k(tile + 1));
+                ok = ok && put_v(tile);
             }
-            umma_commit(bar_s);
         }
-        __syncwarp();
-        if constexpr (!kF16) {
-            // the previous tile's O products read the V tiles and the P buffers and write O: they must be complete
-            // before V is overwritten here and before the softmax below rescales O or rewrites P
-            if (tile > 0) {
-                wait_bar(bar_o, (uint32_t)(tile - 1) & 1u);
-                tc_fence_after_sync();
-            }
-        }
-        if constexpr (kVRows32) {
-            split_store_f32(sm + oVhi, sm + oVlo, kTK, my_row, my_row, c0 + tile * kTK + my_row < c1);
-            if (tile + 1 < n_tiles) fetch(tile + 1);
-            fence_smem_to_async_proxy();
-        } else if constexpr (!kF16) {
-            widen(pv);
-            dequant_store_shfl<kLoTiles>(pv, tab, sm + oVhi, sm + oVlo, kTK, my_row, my_row, 4 * my_c);
-            if (tile + 1 < n_tiles) fetch(tile + 1);
-            fence_smem_to_async_proxy();
-        }
-
-        // ---- 3. softmax: thread = query row ---------------------------------------------------------
-        if (warp < 4) {
-            wait_bar(bar_s, parity);
+    } else {
+        // ---- softmax: thread = query row ------------------------------------------------------------------------
+        const int lim = my_q < n_rows ? pa.pos0 + tok0 + my_q / NREP + 1 : 0;
+        for (int tile = 0; tile < n_tiles; tile++) {
+            const uint32_t buf = (uint32_t)tile & 1u, par = (uint32_t)(tile >> 1) & 1u;
+            bool ok = wait(bar_s + 8 * buf, par);
+            if constexpr (!kRaw) ok = ok && wait(bar_norms + 8 * (tile % kNormTiles), (uint32_t)(tile / kNormTiles) & 1u);
+            if (tile >= 2) ok = ok && wait(bar_o + 8 * buf, par ^ 1u);  // P of two tiles ago has been used
+            if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after_sync();
             uint32_t sr[32];
-            tmem_ld32(my_tmem + kColS, sr);
-            if constexpr (kLoTiles) {
-                uint32_t s2[32];
-                tmem_ld32(my_tmem + kColS + 32, s2);
-#pragma unroll
-                for (int j = 0; j < 32; j++) sr[j] = __float_as_uint(__uint_as_float(sr[j]) + __uint_as_float(s2[j]));
-            }
-            const int pb = c0 + tile * kTK;
+            tmem_ld32(my_tmem + kColS + 32 * buf, sr);
+            const float *kn = ss.kn[tile % kNormTiles], *lv = ss.lv[tile % kNormTiles];
+            const int n_ok = min(c1, lim) - (c0 + tile * kTK);  // positions of the tile that this row sees
             float t[32];
             float mx = -CUDART_INF_F;
 #pragma unroll
             for (int j = 0; j < 32; j++) {
-                const float s = __uint_as_float(sr[j]) * ss.kn[j];
+                const float s = kRaw ? __uint_as_float(sr[j]) : __uint_as_float(sr[j]) * kn[j];
                 sr[j] = __float_as_uint(s);
-                const int p = pb + j;
-                t[j] = (p < c1 && p < lim) ? s + ss.lv[j] : -CUDART_INF_F;
+                t[j] = j < n_ok ? (kVPlanar ? s + lv[j] : s) : -CUDART_INF_F;
                 mx = fmaxf(mx, t[j]);
             }
             // lazy reference: move it only when this row's maximum ran ahead by more than kLazy
@@ -488,94 +571,73 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 const float newR = move ? mx : R;
                 const float f = (move && R > -CUDART_INF_F) ? fast_exp2(R - newR) : (move ? 0.f : 1.f);
                 lsum *= f;
-                for (int b = 0; b < 8; b++) {
-                    uint32_t o[32];
-                    tmem_ld32(my_tmem + kColO + 32 * b, o);
+                if (tile > 0) {  // (the first product of a CTA does not add to O)
+                    if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
+                    tc_fence_after_sync();
+                    for (int b = 0; b < 8; b++) {
+                        uint32_t o[32];
+                        tmem_ld32(my_tmem + kColO + 32 * b, o);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-                    tmem_st32(my_tmem + kColO + 32 * b, o);
+                        for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                        tmem_st32(my_tmem + kColO + 32 * b, o);
+                    }
                 }
-                tmem_wait_st();
                 R = newR;
             }
             const float ref = R > -CUDART_INF_F ? R : 0.f;
-            // weights: chunk c = positions 8c .. 8c+7 -> 16 bytes at c * 2048 + (row / 8) * 128 + (row % 8) * 16
-            uint8_t *p_hi = sm + oPhi + (my_q >> 3) * 128 + (my_q & 7) * 16, *p_lo = sm + oPlo + (my_q >> 3) * 128 + (my_q & 7) * 16;
+            // weights of positions 2 e, 2 e + 1: hi parts in column e, lo parts in column 16 + e
+            uint32_t pw[32];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t hw[4], lw[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int j = 8 * c + 2 * e;
-                    const float w0 = fast_exp2(t[j] - ref) * kPScale, w1 = fast_exp2(t[j + 1] - ref) * kPScale;
-                    if (t[j] > -CUDART_INF_F) lsum += fast_exp2(__uint_as_float(sr[j]) - ref);
-                    if (t[j + 1] > -CUDART_INF_F) lsum += fast_exp2(__uint_as_float(sr[j + 1]) - ref);
-                    const __half2 h = __floats2half2_rn(w0, w1);
-                    const float2 hf = __half22float2(h);
-                    const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
-                    hw[e] = *reinterpret_cast<const uint32_t *>(&h);
-                    lw[e] = *reinterpret_cast<const uint32_t *>(&l);
+            for (int e = 0; e < 16; e++) {
+                const int j = 2 * e;
+                float w0 = fast_exp2(t[j] - ref), w1 = fast_exp2(t[j + 1] - ref);
+                if constexpr (kVPlanar) {
+                    if (j < n_ok) lsum += fast_exp2(__uint_as_float(sr[j]) - ref);
+                    if (j + 1 < n_ok) lsum += fast_exp2(__uint_as_float(sr[j + 1]) - ref);
+                } else {
+                    lsum += w0;
+                    lsum += w1;
                 }
-                *reinterpret_cast<uint4 *>(p_hi + c * kPChunk) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                *reinterpret_cast<uint4 *>(p_lo + c * kPChunk) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                w0 *= kPScale;
+                w1 *= kPScale;
+                const __half2 h = __floats2half2_rn(w0, w1);
+                const float2 hf = __half22float2(h);
+                const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
+                pw[e] = *reinterpret_cast<const uint32_t *>(&h);
+                pw[16 + e] = *reinterpret_cast<const uint32_t *>(&l);
             }
+            tmem_st32(my_tmem + kColP + 32 * buf, pw);
+            tmem_wait_st();
             tc_fence_before_sync();
-            fence_smem_to_async_proxy();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_p + 8 * buf);
         }
-        __syncthreads();
-
-        // ---- 4. O += P . V ----------------------------------------------------------------------------
-        if (tid == 0) {
-            tc_fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < 2; kk++) {
-                const uint64_t ph = umma_smem_desc(base + oPhi + kk * 2 * kPChunk, kPChunk, 128, kUmmaSwizzleNone);
-                const uint64_t pl = umma_smem_desc(base + oPlo + kk * 2 * kPChunk, kPChunk, 128, kUmmaSwizzleNone);
-                const uint64_t vh = umma_smem_desc(base + v_off + kk * 2048, kKVSlab, 1024, kUmmaSwizzle128);
-                umma_f16_ss(tmem + kColO, ph, vh, idesc_o, true);
-                umma_f16_ss(tmem + kColO, pl, vh, idesc_o, true);
-                if constexpr (kLoTiles) {
-                    const uint64_t vl = umma_smem_desc(base + oVlo + kk * 2048, kKVSlab, 1024, kUmmaSwizzle128);
-                    umma_f16_ss(tmem + kColO, ph, vl, idesc_o, true);
-                }
-            }
-            umma_commit(bar_o);
-        }
-        __syncwarp();
-        if constexpr (kF16) {
-            wait_bar(bar_o, parity);  // everybody: the tiles and the P buffers may be overwritten, O may be rescaled
-            tc_fence_after_sync();
-        } else {
-            if (tile + 1 < n_tiles) dequant_k(tile + 1);  // under the O products just issued
-            __syncthreads();
-        }
-    }
-    if constexpr (!kF16) {
-        if (n_tiles > 0) {  // the last tile's O products
-            wait_bar(bar_o, (uint32_t)(n_tiles - 1) & 1u);
-            tc_fence_after_sync();
-        }
-    }
-
-    // ---- epilogue: thread = query row ------------------------------------------------------------------
-    if (warp < 4) {  // every lane takes part in the warp-collective tensor-memory loads, rows past the block only skip the stores
-        const bool real = my_q < n_rows;
-        const size_t out_row = real ? (size_t)(tok0 + my_q / NREP) * a.n_head + kv * NREP + my_q % NREP : 0;
         const float unscale = 1.0f / (kPScale * (kVPlanar ? pa.lut_alpha : 1.0f));  // (raw V rows carry no table scale)
+        ss.mul[my_q] = pa.n_chunks == 1 ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
+        if (pa.n_chunks > 1 && my_q < n_rows) {
+            float *dst = pa.scratch + (((size_t)(tok0 + my_q / NREP) * a.n_head + kv * NREP + my_q % NREP) * pa.n_chunks + chunk) * (kHd + 2);
+            dst[kHd] = R;
+            dst[kHd + 1] = lsum;
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();  // (the issuing warp has seen all its products complete)
+    tc_fence_after_sync();
+
+    // ---- epilogue: warps 0-11, 32 query rows x 32 columns at a time through a padded shared-memory block, so that the
+    // global stores of a warp cover one row's 128 bytes instead of 32 rows' 8 bytes
+    if (warp < kMmaWarp) {
         const bool whole = pa.n_chunks == 1;
-        const float mul = whole ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
-        float *dst = whole ? a.out + out_row * kHd : pa.scratch + (out_row * pa.n_chunks + chunk) * (kHd + 2);
-        // 32 rows x 32 columns at a time through a padded shared-memory block, so that the global
-        // stores of a warp cover one row's 128 bytes instead of 32 rows' 8 bytes
-        float *stg = reinterpret_cast<float *>(sm + oKhi) + (warp & 3) * (32 * 33);
+        const float mul = ss.mul[my_q];
+        float *stg = reinterpret_cast<float *>(sm + oSlots) + warp * (32 * 33);
         const int wrow0 = (warp & 3) * 32;
-        for (int b = 0; b < 8; b++) {
+        for (int b = warp >> 2; b < 8; b += 3) {
             uint32_t o[32];
             tmem_ld32(my_tmem + kColO + 32 * b, o);
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
                 const int d = 32 * b + j;
-                float o0 = __uint_as_float(o[j]) * mul, o1 = __uint_as_float(o[j + 1]) * mul;
+                float o0 = n_tiles > 0 ? __uint_as_float(o[j]) * mul : 0.f, o1 = n_tiles > 0 ? __uint_as_float(o[j + 1]) * mul : 0.f;
                 if (whole && kVPlanar) {
                     float r0, r1;
                     givens_inv(o0, o1, ss.givens[d], ss.givens[d + 1], r0, r1);
@@ -594,10 +656,6 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 drow[32 * b + lane] = stg[rr * 33 + lane];
             }
             __syncwarp();
-        }
-        if (real && !whole) {
-            dst[kHd] = R;
-            dst[kHd + 1] = lsum;
         }
     }
     tc_fence_before_sync();
@@ -664,6 +722,31 @@ bool prefill_umma_supported(const DecodeArgs &a) {
     return (planar || f16 || f32 || k_only) && a.h_tmap_k && a.h_tmap_v && (n_rep == 1 || n_rep == 2 || n_rep == 4 || n_rep == 6);
 }
 
+// Into how many chunks the context is cut: the count with the least estimated time.  A CTA has an SM to itself and costs
+// kFixed tiles' worth of set-up, q preparation and epilogue beside its tiles; what a launch then takes is bounded both by full rounds of its
+// longest item and by its work spread evenly plus one longest item (items are handed out longest first).  Merging costs a
+// launch and one read of every chunk's rows.
+static int plan_chunks(int n_sms, int pos0, int n_tokens, int tq, int n_kv, int n_head) {
+    constexpr double kFixed = 6.0, kMergeLaunch = 3.0, kMergeRow = 1.0 / 2048;
+    const int n_blocks = (n_tokens + tq - 1) / tq, vis = pos0 + n_tokens;
+    // no more than about four items per SM, which also bounds the scratch
+    const int most = std::max(1, std::min({64, vis / 256, (4 * n_sms + n_blocks * n_kv - 1) / (n_blocks * n_kv)}));
+    const double mean_vis = pos0 + 0.5 * (n_tokens + tq);
+    double best = 0.0;
+    int chunks = 1;
+    for (int c = 1; c <= most; c++) {
+        const double longest = kFixed + (double)((vis + c * kTK - 1) / (c * kTK)), items = (double)n_blocks * n_kv * c;
+        const double mean = kFixed + std::max(1.0, mean_vis / (c * kTK));
+        const double t = std::min(std::ceil(items / n_sms) * longest, items * mean / n_sms + longest) +
+                         (c > 1 ? kMergeLaunch + kMergeRow * c * n_tokens * n_head / 24 : 0.0);
+        if (c == 1 || t < best) {
+            best = t;
+            chunks = c;
+        }
+    }
+    return chunks;
+}
+
 bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha) {
     if (n_tokens <= 0) return BK_OK;
     const int n_rep = a.n_head / a.n_kv;
@@ -676,9 +759,7 @@ bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos
     pa.n_blocks = (n_tokens + pa.tq - 1) / pa.tq;
     pa.lut_alpha = alpha;
     pa.err_flag = ctx->d_err;
-    const int vis = pos0 + n_tokens;
-    int chunks = (4 * ctx->n_sms + pa.n_blocks * a.n_kv - 1) / (pa.n_blocks * a.n_kv);  // about four CTAs per SM: the causal triangle leaves them unequal
-    chunks = std::max(1, std::min(chunks, std::min(64, vis / 256)));
+    const int chunks = plan_chunks(ctx->n_sms, pos0, n_tokens, pa.tq, a.n_kv, a.n_head);
     pa.n_chunks = chunks;
     if (chunks > 1) {
         const size_t need = (size_t)n_tokens * a.n_head * chunks * (kHd + 2);

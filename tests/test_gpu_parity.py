@@ -1000,6 +1000,17 @@ def test_prefill_mma_sync_variant_and_empty_chunks(bk, oracle, monkeypatch, tag,
         ctx.close()
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [MODES[2], MODES[3], MODES[1], MODES[0], MODES[4]])
+def test_prefill_tile_edges(bk, gpu_ctx, oracle, tag, mode, bits, vq):
+    """Context lengths around the 32-position tile and from one tile up to more tiles than the operand ring has
+    slots, so that the first, the last and the ragged tile, and every slot's reuse, are met."""
+    for n in (4, 31, 32, 33, 64, 65, 95, 96, 97, 129, 191, 192, 225):
+        n_tok = min(n, 8)
+        got, want = prefill_both(bk, gpu_ctx, oracle, tag, mode, bits, vq, n - n_tok, n_tok, seed=n)
+        for i in range(n_tok):
+            assert_close(got[i], want[i], f"{tag} n={n} token {i}")
+
+
 def test_prefill_other_group_sizes_and_long_context(bk, gpu_ctx, oracle):
     for n_head, n_kv in ((4, 4), (8, 4), (8, 2)):
         got, want = prefill_both(bk, gpu_ctx, oracle, "planar4", MODE_PLANAR, 4, True, 500, 70, seed=n_head, n_head=n_head, n_kv=n_kv)
