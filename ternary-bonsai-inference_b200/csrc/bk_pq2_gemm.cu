@@ -17,9 +17,10 @@
 //     scale * block sum, grouped as the reference's scalar path does it (src/kernels.rs:633-650); the tensor
 //     core never accumulates more than 16 MMAs, which keeps its truncating f32 adds from building up a bias.
 //     Two D buffers alternate: the drain of one step runs under the MMAs of the next.
-// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 512 tokens 228 us = 470
+// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 512 tokens 290 us = 370
 // TFLOP/s of useful work (two passes of it on the tensor cores), 5760 us as pairs of tokens; 16 tokens 55 us against
-// 187.  Rounding against float64: 1.4e-7 of the result's 2-norm (1.0e-7 one token at a time).
+// 187.  Rounding against float64: 1.0e-7 of the result's 2-norm, as one token at a time (with x20 outliers in x 1.0e-7 against
+// 2.6e-7); 1.4e-7, and 240 us, with one running sum over all blocks.
 // A step is (row tile of 128, block of 128); a CTA works on one or two row tiles (two share every B block: 32
 // instead of 64 bytes per clock and SM from L2, which is what the L2 delivers) and one token tile of 16..128.
 // The sum over blocks is sequential whatever the tiling, so a result does not depend on it bit for bit.
@@ -41,6 +42,7 @@ constexpr int kGemmBlock = 128, kGemmBlockBytes = 34;
 constexpr int kGemmSegBlocks = 4;                 // blocks of a row staged together
 constexpr int kGemmRowWords = 36;                 // words of a staged row: nine 16-byte pieces hold any four blocks of an aligned row
 constexpr int kGemmMaxSegs = 4;
+constexpr int kGemmGroup = 8;                     // blocks that are added up before their sum goes to y
 constexpr uint32_t kColsD = 128, kColA = 256, kColsA = 64;  // tensor-memory columns: D0 | D1 | four A stages
 
 struct GemmArgs {
@@ -349,11 +351,43 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
                         for (int j = 0; j < 8; j++) ac[(c0 + c) * 8 + j] = fmaf(sc, __uint_as_float(v[8 * c + j]), ac[(c0 + c) * 8 + j]);
             }
         };
+        // The sums so far join y and start again at zero: one running f32 sum over all blocks rounds at the size of the whole
+        // result forty times (1.4e-7 of the 2-norm against 1.0e-7).  Eight elements at a time are read back, which are the registers
+        // there are; an element belongs to one thread.  (red.add instead of the read was slower: 28 clocks a warp.)
+        // kLag iterations on, a group's last block is drained; a rest of fewer than three blocks joins the last group, with either MT.
+        constexpr int kLag = MT == 1 ? 2 : 1;
+        int next_flush = kGemmGroup + kLag;
+        bool first = true;
+        auto flush = [&](int b) {
+            if (first) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // what came before on the stream may still read y until here
+            const int t0 = tok_tile * N + half * NH, left = a.n_tok - t0;
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                const int row = row0 + m * 128 + r;
+                if (row < seg_rows) {
+                    float *yp = a.y[sg] + (size_t)t0 * seg_rows + row;
+#pragma unroll
+                    for (int j0 = 0; j0 < NH; j0 += 8) {
+                        float old[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) old[j] = (!first && j0 + j < left) ? __ldcg(yp + (size_t)(j0 + j) * seg_rows) : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 8; j++)  // (the scale is a power of two)
+                            if (j0 + j < left) __stcg(yp + (size_t)(j0 + j) * seg_rows, fmaf(acc[m][j0 + j], __ldg(a.tok_scale + t0 + j0 + j), old[j]));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < NH; j++) acc[m][j] = 0.f;
+            }
+            first = false;
+            next_flush = b + kGemmGroup;
+        };
         // one iteration per block: unpack the block's steps, drain the steps of two steps ago.  An A stage is reused
         // four steps on, after the drain of its step, which waited for its MMAs.
         float sc1[MT] = {}, sc2 = 0.f;  // block scales of the steps that are unpacked and not yet drained
         fetch(0);
         for (int b = 0; b < nb; b++) {
+            if (b == next_flush && b - kLag + 3 <= nb) flush(b);
             float now[MT];
 #pragma unroll
             for (int m = 0; m < MT; m++) now[m] = sc0[m];
@@ -378,18 +412,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
             if (nb > 1) drain(nb - 2, acc[0], sc2);
             drain(nb - 1, acc[0], sc1[0]);
         }
-        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // what came before on the stream may still read y until here
-        const int t0 = tok_tile * N + half * NH;
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            const int row = row0 + m * 128 + r;
-            if (row < seg_rows) {
-                float *yp = a.y[sg] + (size_t)t0 * seg_rows + row;
-#pragma unroll
-                for (int j = 0; j < NH; j++)
-                    if (t0 + j < a.n_tok) yp[(size_t)j * seg_rows] = acc[m][j] * __ldg(a.tok_scale + t0 + j);
-            }
-        }
+        flush(nb);
     }
     tc_fence_before_sync();
     __syncthreads();

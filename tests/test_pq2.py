@@ -191,10 +191,11 @@ def test_gpu_pq2_multi_equals_separate_calls(bk, gpu_ctx):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("ne0,n_rows,n_tok,base", [(128, 1, 5, 0), (128, 130, 6, 3), (200, 129, 15, 1), (512, 128, 16, 0), (640, 257, 17, 1), (5120, 300, 33, 2),
-                                                   (1280, 2000, 128, 0), (768, 255, 129, 0), (384, 40, 1025, 1), (128, 40000, 100, 0), (5120, 40, 512, 5)])
+                                                   (1280, 2000, 128, 0), (768, 255, 129, 0), (384, 40, 1025, 1), (128, 40000, 100, 0), (5120, 40, 512, 5),
+                                                   (1024, 300, 20, 0), (1152, 300, 128, 0), (1280, 20000, 512, 0), (1408, 300, 90, 0), (2432, 140, 40, 0)])
 def test_gpu_pq2_token_block_product(bk, gpu_ctx, ne0, n_rows, n_tok, base):
-    """The tensor-core product at the edges of its tiles (128 rows, 16..128 tokens, segments of four blocks, 1024 tokens
-    a pass, rows off a word boundary).  Bound: f16 pairs hold x to 2^-22 of each element and the per-block sums are
+    """The tensor-core product at the edges of its tiles (128 rows, 16..128 tokens, segments of four and groups of eight blocks,
+    1024 tokens a pass, rows off a word boundary).  Bound: f16 pairs hold x to 2^-22 of each element and the per-block sums are
     rounded to f32 (2^-24 of sum |x||w|, up to 16 times a block, then once a block): 2e-6 of sum |x||w|."""
     payload, codes, scales, x = synth(bk, 7 * ne0 + n_rows + n_tok, n_rows + base, ne0, n_tok)
     t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
