@@ -109,11 +109,14 @@ struct HostPipe {
         }
     }
     void push(const Task &t) {
-        {
+        busy.fetch_add(1);
+        try {
             std::lock_guard<std::mutex> lk(m);
             q.push_back(t);
             waiting.fetch_add(1);
-            busy.fetch_add(1);
+        } catch (...) {  // no memory to queue it: now
+            run(t);
+            return;
         }
         cv.notify_one();
     }
@@ -184,8 +187,8 @@ struct Part {
     size_t n;
 };
 
-// Cut the ranges into slots; ranges that follow one another in host memory share a slot.
-void cut(const HostSeg *segs, size_t n_seg, std::vector<Piece> &pieces, std::vector<Part> &parts) {
+// Cut the ranges into slots; ranges that follow one another in host memory share a slot.  False without memory for the lists.
+bool cut(const HostSeg *segs, size_t n_seg, std::vector<Piece> &pieces, std::vector<Part> &parts) try {
     for (size_t i = 0; i < n_seg; i++) {
         size_t at = 0;
         while (at < segs[i].bytes) {
@@ -200,6 +203,9 @@ void cut(const HostSeg *segs, size_t n_seg, std::vector<Piece> &pieces, std::vec
             at += n;
         }
     }
+    return true;
+} catch (const std::bad_alloc &) {
+    return false;
 }
 }  // namespace
 
@@ -221,7 +227,7 @@ bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
     if (st != BK_OK) return st;
     std::vector<Piece> pieces;
     std::vector<Part> parts;
-    cut(segs, n_seg, pieces, parts);
+    if (!cut(segs, n_seg, pieces, parts)) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
     // A fresh destination: fault its huge pages in on different threads first.  Copies of neighbouring pieces would fault on the
     // same page at once, and each clears 2 MB for it.
     for (size_t k = 0; k < pieces.size(); k++) {
@@ -267,7 +273,7 @@ bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, const st
     if (st != BK_OK) return st;
     std::vector<Piece> pieces;
     std::vector<Part> parts;
-    cut(segs, n_seg, pieces, parts);
+    if (!cut(segs, n_seg, pieces, parts)) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
     cudaError_t e = cudaSuccess;
     size_t pushed = 0, issued = 0, bytes = 0;
     while (issued < pieces.size() && e == cudaSuccess && st == BK_OK) {
