@@ -7,20 +7,22 @@
 // the tensor cores, and about as much traffic of shared memory; so nothing may wait for anything else, and shared
 // memory has to be spared.  Thirteen warps in three roles, coupled by mbarriers only:
 //   * warps 4-11 (producers) turn packed rows into f16 operand tiles (for 4 bit with the rounding remainders, for
-//     f32 rows hi + lo parts) in a ring of five slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
+//     f32 rows hi + lo parts) in a ring of four slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
 //     16-byte pieces of a row go out in an order that depends on its lane, or the eight lanes of a row would meet on
 //     two of eight bank groups.  f16 rows are operands as stored and are dropped in by the TMA engine.
 //   * warp 12 issues the products: S(t + 1) = Q . K^T goes ahead of O += P(t) . V, so the tensor cores work on S(t + 1)
-//     under the softmax of tile t.  The small terms of S come first: the accumulator truncates, and does so at
-//     the size of what it holds.
+//     under the softmax of tile t.  The small terms of S have columns of their own: the accumulator truncates, and does
+//     so at the size of what it holds.
 //   * warps 0-3 (thread = query row = tensor-memory lane) read S, scale by ||k||, apply the causal limit, move the
 //     running reference R of s + log2 ||v|| LAZILY (only when the row maximum exceeds R by more than 8: the weights
 //     p = 2^(t - R) * 64 then stay below 2^14 in f16; their row of O is then rescaled in place) and write the
 //     weights as f16 hi + lo.
-// Tensor memory (all 512 columns): O 256 | q_hi 128 | S 2 x 32 | P (hi, lo) 2 x 32.  q_hi and P are A operands from
-// there: a product with N = 32 otherwise re-reads 4 KiB of q for 1 KiB of K.  q_lo stays in shared memory.
-// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.4 -> 6.2 ms, a 777-token f32 prompt in
-// one block 737 -> 301 us; before, one role after the other per tile, with every MMA operand moved to uniform registers.
+// Tensor memory (all 512 columns): O 256 | half of q_hi 64 | S 2 x (32 + 32) | P (hi, lo) 2 x 32.  A product with N = 32 costs as
+// much as one with N = 64 (32 clocks), so q_hi meets k_hi and k_lo side by side; P and as much of q_hi as there are columns for
+// are A operands from tensor memory, which spares shared memory 4 KiB a product.
+// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.4 -> 5.6 ms, a 777-token f32 prompt in
+// one block 737 -> 302 us.  Before, one role after the other per tile with every MMA operand moved to uniform registers; the roles
+// with products of N = 32 and q fetched row by row 6.2 ms.
 // Every mbarrier wait is bounded: one that runs out raises the context's error flag, the others of the CTA stop
 // waiting, and the kernel runs on to its end, where the tensor memory is always released.
 #include <cuda_fp16.h>
@@ -42,17 +44,17 @@ namespace {
 constexpr int kSoftWarps = 4, kProdWarps = 8, kMmaWarp = kSoftWarps + kProdWarps, kUWarps = kMmaWarp + 1, kUT = kUWarps * 32;
 constexpr int kRows = 128;  // query rows per CTA = tensor-memory lanes
 constexpr int kTK = 32;     // positions per tile
-constexpr float kPScale = 64.0f;
+constexpr float kPScale = 64.0f, kPScaleLog2 = 6.0f;
 constexpr float kLazy = 8.0f;  // the reference moves when a row maximum exceeds it by more than this (log2 units)
 
 constexpr uint32_t kQSlab = kRows * 128, kQTile = 4 * kQSlab;  // 16 KiB per 64-coordinate slab, 64 KiB per tile
 constexpr uint32_t kKVSlab = kTK * 128, kKVTile = 4 * kKVSlab;  // 4 KiB, 16 KiB
-// Operand slots.  Five: K(t) then takes the place of V(t - 4), so what the softmax reads of tile t - 4 (its norms, kept for
-// four tiles) is read before the producers are at tile t.
-constexpr int kSlots = 5, kNormTiles = 4;
+// Operand slots.  Four: K(t) then takes the place of K(t - 2), whose S products were issued when the softmax had read tile
+// t - 4, so the norms of four tiles can be kept.
+constexpr int kSlots = 4, kNormTiles = 4;
 constexpr uint32_t kSlotBytes = 2 * kKVTile;  // hi and lo tile
 // offsets from the 1024-byte aligned base
-constexpr uint32_t oQlo = 0, oSlots = kQTile, oSmall = oSlots + kSlots * kSlotBytes;
+constexpr uint32_t oQlo = 0, oQhi2 = kQTile, oSlots = oQhi2 + kQTile / 2, oSmall = oSlots + kSlots * kSlotBytes;
 struct SmallU {
     float givens[kHd];
     float kn[kNormTiles][kTK], lv[kNormTiles][kTK];  // ||k|| and log2 ||v|| of a tile's positions
@@ -65,7 +67,7 @@ struct SmallU {
 };
 constexpr uint32_t kUmmaSmem = oSmall + 3072;
 static_assert(sizeof(SmallU) <= 3072 && kUmmaSmem <= 227 * 1024, "shared memory of a CTA");
-constexpr uint32_t kTmemCols = 512, kColO = 0, kColQ = 256, kColS = 384, kColP = 448;
+constexpr uint32_t kTmemCols = 512, kColO = 0, kColQ = 256, kColS = 320, kColP = 448;
 
 __device__ __forceinline__ uint32_t sw_off(int rows, int row, int chunk) {  // as tile_off in bk_prefill.cu
     return (uint32_t)((chunk >> 3) * rows * 128 + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
@@ -97,8 +99,8 @@ __device__ __forceinline__ void rotate4(uint32_t (&w)[4], int rot) {
 }
 // 32 coordinates (four words of eight nibbles, rotated by `rot`) -> 32 halfs as four 16-byte chunks of a tile row.
 // The eight lanes of a row store chunks 4 c + ((j + c / 2) & 3) together, one per bank group (4 c + j would put them on two).
-// The table sits in registers: lane i holds (hi | lo << 16) of centroid i & 15, one shuffle looks
-// both parts of an index up, and no shared-memory bank is involved.
+// The table sits in registers: lane i holds (hi | lo << 16) of centroid i & 15, one shuffle looks both parts of an index
+// up, and no shared-memory bank is involved.  (A shuffle takes the low five bits of the lane number; the fifth, the next index's, does not matter.)
 template <bool LO>
 __device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint32_t tab, uint8_t *tile_hi, uint8_t *tile_lo, int rows,
                                                    int row_hi, int row_lo, int chunk0, int rot) {
@@ -107,8 +109,8 @@ __device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint3
         uint32_t h[4], l[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-            const uint32_t v0 = __shfl_sync(0xffffffffu, tab, (w[j] >> (8 * e)) & 15u);
-            const uint32_t v1 = __shfl_sync(0xffffffffu, tab, (w[j] >> (8 * e + 4)) & 15u);
+            const uint32_t v0 = __shfl_sync(0xffffffffu, tab, w[j] >> (8 * e));
+            const uint32_t v1 = __shfl_sync(0xffffffffu, tab, w[j] >> (8 * e + 4));
             h[e] = __byte_perm(v0, v1, 0x5410);
             l[e] = __byte_perm(v0, v1, 0x7632);
         }
@@ -160,6 +162,21 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     const int L = ((vis + pa.n_chunks - 1) / pa.n_chunks + kTK - 1) / kTK * kTK;
     const int c0 = chunk * L, c1 = min(c0 + L, vis);
     const int n_tiles = c1 > c0 ? (c1 - c0 + kTK - 1) / kTK : 0;
+
+    // ---- the query rows start travelling: every row's round trip at once -----------------------------------
+    const int half = a.n_rot >> 1;
+    {
+        const float *q0 = a.q + ((size_t)tok0 * a.n_head + kv * NREP) * kHd;
+        auto row_src = [&](int r) { return q0 + ((size_t)(r / NREP) * a.n_head + r % NREP) * kHd; };
+        if (((uintptr_t)a.q & 15) == 0) {
+            for (int i = tid; i < n_rows * (kHd / 4); i += kUT)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + oSlots + 16u * i), "l"(row_src(i / (kHd / 4)) + 4 * (i % (kHd / 4)))
+                             : "memory");
+        } else {
+            for (int i = tid; i < n_rows * kHd; i += kUT)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(base + oSlots + 4u * i), "l"(row_src(i / kHd) + i % kHd) : "memory");
+        }
+    }
 
     // ---- tables, barriers, tensor memory ----------------------------------------------------
     for (int i = tid; i < kHd; i += kUT) ss.givens[i] = a.givens[i];
@@ -250,73 +267,51 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         else if constexpr (!kF16) fetch_packed(pv, a.v_rows, tile);
     };
 
-    // ---- q rows -> q_hi (through slots 0 and 1, then to tensor memory) and q_lo: rope, Givens, scale, f16 hi/lo ----
+    // ---- q rows -> q_hi and q_lo: rope, Givens, scale, f16 hi/lo; a warp takes a row, the 32 bytes of a lane are coordinates
+    // 8 lane .. + 7; the half of q_hi for tensor memory goes where the row was ---------------------------------------
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
     {
-        float *stage = reinterpret_cast<float *>(sm + oSlots + 2 * kSlotBytes) + warp * (kHd + 8);  // rows are padded by one float per 32 (see pad())
-        auto pad = [](int i) { return i + (i >> 5); };  // lanes 8 coordinates apart land in different banks
         const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / pa.lut_alpha;
-        const int half = a.n_rot >> 1;
-        // the next row's q and rope values travel while the current row is processed
-        float xn[8];
-        float2 rn[4];
-        auto prefetch = [&](int r) {
-            if (r < n_rows) {
-                const int tok = tok0 + r / NREP, head = kv * NREP + r % NREP;
-                const float *src = a.q + ((size_t)tok * a.n_head + head) * kHd;
-                const float2 *cs = a.rope + (size_t)(pa.pos0 + tok) * half;
-#pragma unroll
-                for (int i = 0; i < 8; i++) xn[i] = __ldg(src + lane + 32 * i);
-#pragma unroll
-                for (int i = 0; i < 4; i++) rn[i] = (lane + 32 * i < half) ? __ldg(cs + lane + 32 * i) : make_float2(1.f, 0.f);
-            }
-        };
-        prefetch(warp);
+        // the rope entries of the warp's next two rows travel (up to 32 per row; wider rotations read the rest where they need it)
+        auto rope_row = [&](int r) { return a.rope + (size_t)(pa.pos0 + tok0 + r / NREP) * half; };
+        auto rope_of = [&](int r) { return r < n_rows && lane < half ? __ldg(rope_row(r) + lane) : make_float2(1.f, 0.f); };
+        float2 c0r = rope_of(warp), c1r = rope_of(warp + kUWarps);
         for (int r = warp; r < kRows; r += kUWarps) {
-            const bool real = r < n_rows;
-            if (real) {
-                float2 rc[4];
-#pragma unroll
-                for (int i = 0; i < 8; i++) stage[pad(lane + 32 * i)] = xn[i];
-#pragma unroll
-                for (int i = 0; i < 4; i++) rc[i] = rn[i];
-                prefetch(r + kUWarps);
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int j = lane + 32 * i;
-                    if (j < half) {
-                        float x0 = stage[pad(j)], x1 = stage[pad(j + half)];
-                        rope_pair(x0, x1, rc[i]);
-                        stage[pad(j)] = x0;
-                        stage[pad(j + half)] = x1;
-                    }
+            float *row = reinterpret_cast<float *>(sm + oSlots) + r * kHd;
+            uint32_t hw[4] = {}, lw[4] = {};
+            const float2 c2r = rope_of(r + 2 * kUWarps);
+            if (r < n_rows) {
+                for (int j = lane; j < half; j += 32) {
+                    float x0 = row[j], x1 = row[j + half];
+                    rope_pair(x0, x1, j < 32 ? c0r : __ldg(rope_row(r) + j));
+                    row[j] = x0;
+                    row[j + half] = x1;
                 }
                 __syncwarp();
-            }
-            uint32_t hw[4], lw[4];
+                const float4 x0 = reinterpret_cast<const float4 *>(row)[2 * lane], x1 = reinterpret_cast<const float4 *>(row)[2 * lane + 1];
+                const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                float o0 = 0.f, o1 = 0.f;
-                if (real) {
-                    const int d = 8 * lane + 2 * p;
-                    if constexpr (kRaw) {
-                        o0 = stage[pad(d)];
-                        o1 = stage[pad(d + 1)];
-                    } else {
-                        givens_fwd(stage[pad(d)], stage[pad(d + 1)], ss.givens[d], ss.givens[d + 1], o0, o1);
+                for (int p = 0; p < 4; p++) {
+                    float o0 = x[2 * p], o1 = x[2 * p + 1];
+                    if constexpr (!kRaw) {
+                        const int d = 8 * lane + 2 * p;
+                        givens_fwd(x[2 * p], x[2 * p + 1], ss.givens[d], ss.givens[d + 1], o0, o1);
                     }
                     o0 *= qscale;
                     o1 *= qscale;
+                    const __half h0 = __float2half_rn(o0), h1 = __float2half_rn(o1);
+                    const __half l0 = __float2half_rn(o0 - __half2float(h0)), l1 = __float2half_rn(o1 - __half2float(h1));
+                    hw[p] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
+                    lw[p] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
                 }
-                const __half h0 = __float2half_rn(o0), h1 = __float2half_rn(o1);
-                const __half l0 = __float2half_rn(o0 - __half2float(h0)), l1 = __float2half_rn(o1 - __half2float(h1));
-                hw[p] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
-                lw[p] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
+                __syncwarp();
             }
-            const uint32_t off = sw_off(kRows, r, lane);
-            *reinterpret_cast<uint4 *>(sm + oSlots + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-            *reinterpret_cast<uint4 *>(sm + oQlo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-            __syncwarp();
+            c0r = c1r;
+            c1r = c2r;
+            uint4 *hi = lane < 16 ? reinterpret_cast<uint4 *>(row) + (lane ^ (r & 7)) : reinterpret_cast<uint4 *>(sm + oQhi2 + sw_off(kRows, r, lane - 16));
+            *hi = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            *reinterpret_cast<uint4 *>(sm + oQlo + sw_off(kRows, r, lane)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
     }
     fence_smem_to_async_proxy();
@@ -324,11 +319,11 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     const int my_q = (warp & 3) * 32 + lane;  // query row of a softmax thread
     if (warp < kSoftWarps) {
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
+        for (int b = 0; b < 2; b++) {
             uint32_t r[32];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const uint4 x = *reinterpret_cast<const uint4 *>(sm + oSlots + sw_off(kRows, my_q, 8 * b + j));
+                const uint4 x = reinterpret_cast<const uint4 *>(sm + oSlots + my_q * (kHd * 4))[(8 * b + j) ^ (my_q & 7)];
                 r[4 * j] = x.x, r[4 * j + 1] = x.y, r[4 * j + 2] = x.z, r[4 * j + 3] = x.w;
             }
             tmem_st32(my_tmem + kColQ + 32 * b, r);
@@ -345,7 +340,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         // ---- the products -----------------------------------------------------------------------------------
         constexpr int kKRows = kLoTiles ? 64 : 32;  // a K slab holds k_hi in rows 0-31 and k_lo in rows 32-63
         constexpr uint32_t kKSlab = kKRows * 128;
-        const uint32_t idesc_s = umma_idesc_f16(kRows, kTK, 0, 0), idesc_o = umma_idesc_f16(kRows, kHd, 0, 1);
+        const uint32_t idesc_s = umma_idesc_f16(kRows, kTK, 0, 0), idesc_s2 = umma_idesc_f16(kRows, kKRows, 0, 0), idesc_o = umma_idesc_f16(kRows, kHd, 0, 1);
         uint32_t slot = 0, use = 0;
         auto next_slot = [&]() {
             if (++slot == kSlots) slot = 0, use ^= 1u;
@@ -353,20 +348,21 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         auto issue_s = [&](int tile) -> bool {
             if (!__all_sync(0xffffffffu, wait(bar_full + 8 * slot, use))) return false;
             tc_fence_after_sync();
-            const uint32_t d = tmem + kColS + (uint32_t)(tile & 1) * 32u, kb = base + oSlots + slot * kSlotBytes;
+            // columns 0-31: q_hi k_hi; 32-63: the small terms
+            const uint32_t d = tmem + kColS + (uint32_t)(tile & 1) * 64u, kb = base + oSlots + slot * kSlotBytes;
             const uint64_t kd = umma_smem_desc(kb, 16, 1024, kUmmaSwizzle128), ql = umma_smem_desc(base + oQlo, 16, 1024, kUmmaSwizzle128);
+            const uint64_t qh2 = umma_smem_desc(base + oQhi2, 16, 1024, kUmmaSwizzle128);
             if (elect_one()) {  // (the address field of a descriptor counts 16-byte units)
 #pragma unroll
-                for (int ks = 0; ks < 16; ks++)
-                    umma_f16_ss(d, ql + (((ks >> 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s, ks > 0);
-                if constexpr (kLoTiles) {
+                for (int ks = 0; ks < 8; ks++)
+                    umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s2, ks > 0);
 #pragma unroll
-                    for (int ks = 0; ks < 16; ks++)
-                        umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + 4096 + (ks & 3) * 32) >> 4), idesc_s, true);
-                }
+                for (int ks = 8; ks < 16; ks++)
+                    umma_f16_ss(d, qh2 + ((((ks >> 2) - 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s2, true);
 #pragma unroll
                 for (int ks = 0; ks < 16; ks++)
-                    umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s, true);
+                    umma_f16_ss(d + 32, ql + (((ks >> 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s,
+                                kLoTiles || ks > 0);
                 umma_commit(bar_s + 8 * (tile & 1));
                 umma_commit(bar_empty + 8 * slot);
             }
@@ -388,9 +384,9 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 2; kk++) {
-                    umma_f16_ts(tmem + kColO, p + 8 * kk, vd + ((kk * 2048) >> 4), idesc_o, tile > 0 || kk > 0);
-                    umma_f16_ts(tmem + kColO, p + 16 + 8 * kk, vd + ((kk * 2048) >> 4), idesc_o, true);
-                    if constexpr (kLoTiles) umma_f16_ts(tmem + kColO, p + 8 * kk, vd + ((kKVTile + kk * 2048) >> 4), idesc_o, true);
+                    umma_f16_ts(tmem + kColO, p + 16 * kk, vd + ((kk * 2048) >> 4), idesc_o, tile > 0 || kk > 0);
+                    umma_f16_ts(tmem + kColO, p + 16 * kk + 8, vd + ((kk * 2048) >> 4), idesc_o, true);
+                    if constexpr (kLoTiles) umma_f16_ts(tmem + kColO, p + 16 * kk, vd + ((kKVTile + kk * 2048) >> 4), idesc_o, true);
                 }
                 umma_commit(bar_o + 8 * (tile & 1));
                 umma_commit(bar_empty + 8 * slot);
@@ -552,19 +548,26 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             if (tile >= 2) ok = ok && wait(bar_o + 8 * buf, par ^ 1u);  // P of two tiles ago has been used
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after_sync();
-            uint32_t sr[32];
-            tmem_ld32(my_tmem + kColS + 32 * buf, sr);
+            uint32_t sr[32], t[32];
+            tmem_ld32(my_tmem + kColS + 64 * buf, sr);
+            tmem_ld32(my_tmem + kColS + 64 * buf + 32, t);
             const float *kn = ss.kn[tile % kNormTiles], *lv = ss.lv[tile % kNormTiles];
-            const int n_ok = min(c1, lim) - (c0 + tile * kTK);  // positions of the tile that this row sees
-            float t[32];
             float mx = -CUDART_INF_F;
 #pragma unroll
             for (int j = 0; j < 32; j++) {
-                const float s = kRaw ? __uint_as_float(sr[j]) : __uint_as_float(sr[j]) * kn[j];
+                float s = __uint_as_float(sr[j]) + __uint_as_float(t[j]);
+                if constexpr (!kRaw) s *= kn[j];
                 sr[j] = __float_as_uint(s);
-                t[j] = j < n_ok ? (kVPlanar ? s + lv[j] : s) : -CUDART_INF_F;
-                mx = fmaxf(mx, t[j]);
+                t[j] = __float_as_uint(kVPlanar ? s + lv[j] : s);
             }
+            const int n_ok = min(c1, lim) - (c0 + tile * kTK);  // positions of the tile that this row sees
+            if (!__all_sync(0xffffffffu, n_ok >= kTK)) {
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (j >= n_ok) sr[j] = t[j] = __float_as_uint(-CUDART_INF_F);
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(t[j]));
             // lazy reference: move it only when this row's maximum ran ahead by more than kLazy
             const bool move = mx > -CUDART_INF_F && (R == -CUDART_INF_F || mx > R + kLazy);
             if (__any_sync(0xffffffffu, move)) {  // tensor-memory traffic is warp-collective
@@ -574,45 +577,48 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 if (tile > 0) {  // (the first product of a CTA does not add to O)
                     if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
                     tc_fence_after_sync();
-                    for (int b = 0; b < 8; b++) {
-                        uint32_t o[32];
-                        tmem_ld32(my_tmem + kColO + 32 * b, o);
+                    for (int b = 0; b < 16; b++) {
+                        uint32_t o[16];
+                        tmem_ld16(my_tmem + kColO + 16 * b, o);
 #pragma unroll
-                        for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-                        tmem_st32(my_tmem + kColO + 32 * b, o);
+                        for (int j = 0; j < 16; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                        tmem_st16(my_tmem + kColO + 16 * b, o);
                     }
                 }
                 R = newR;
             }
-            const float ref = R > -CUDART_INF_F ? R : 0.f;
-            // weights of positions 2 e, 2 e + 1: hi parts in column e, lo parts in column 16 + e
-            uint32_t pw[32];
+            const float ref = (R > -CUDART_INF_F ? R : 0.f) - kPScaleLog2;
+            // weights, two positions a column: for each K-step of 16 positions eight columns of hi parts and eight of lo parts;
+            // lsum carries their scale
 #pragma unroll
-            for (int e = 0; e < 16; e++) {
-                const int j = 2 * e;
-                float w0 = fast_exp2(t[j] - ref), w1 = fast_exp2(t[j + 1] - ref);
-                if constexpr (kVPlanar) {
-                    if (j < n_ok) lsum += fast_exp2(__uint_as_float(sr[j]) - ref);
-                    if (j + 1 < n_ok) lsum += fast_exp2(__uint_as_float(sr[j + 1]) - ref);
-                } else {
-                    lsum += w0;
-                    lsum += w1;
+            for (int kk = 0; kk < 2; kk++) {
+                uint32_t pw[16];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int j = 16 * kk + 2 * e;
+                    const float w0 = fast_exp2(__uint_as_float(t[j]) - ref), w1 = fast_exp2(__uint_as_float(t[j + 1]) - ref);
+                    if constexpr (kVPlanar) {
+                        lsum += fast_exp2(__uint_as_float(sr[j]) - ref);
+                        lsum += fast_exp2(__uint_as_float(sr[j + 1]) - ref);
+                    } else {
+                        lsum += w0;
+                        lsum += w1;
+                    }
+                    const __half2 h = __floats2half2_rn(w0, w1);
+                    const float2 hf = __half22float2(h);
+                    const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
+                    pw[e] = *reinterpret_cast<const uint32_t *>(&h);
+                    pw[8 + e] = *reinterpret_cast<const uint32_t *>(&l);
                 }
-                w0 *= kPScale;
-                w1 *= kPScale;
-                const __half2 h = __floats2half2_rn(w0, w1);
-                const float2 hf = __half22float2(h);
-                const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
-                pw[e] = *reinterpret_cast<const uint32_t *>(&h);
-                pw[16 + e] = *reinterpret_cast<const uint32_t *>(&l);
+                tmem_st16(my_tmem + kColP + 32 * buf + 16 * kk, pw);
             }
-            tmem_st32(my_tmem + kColP + 32 * buf, pw);
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p + 8 * buf);
         }
         const float unscale = 1.0f / (kPScale * (kVPlanar ? pa.lut_alpha : 1.0f));  // (raw V rows carry no table scale)
+        lsum *= 1.0f / kPScale;
         ss.mul[my_q] = pa.n_chunks == 1 ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
         if (pa.n_chunks > 1 && my_q < n_rows) {
             float *dst = pa.scratch + (((size_t)(tok0 + my_q / NREP) * a.n_head + kv * NREP + my_q % NREP) * pa.n_chunks + chunk) * (kHd + 2);
@@ -663,28 +669,56 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-// One CTA of 128 threads per output row: merge the chunks' triples, rotate back, write.
-__global__ void __launch_bounds__(128) prefill_umma_merge_kernel(const float *scratch, const float *givens, int n_chunks, float *out) {
-    const size_t row = blockIdx.x;
-    const int pr = threadIdx.x;
-    const float *basep = scratch + row * n_chunks * (kHd + 2);
-    float M = -CUDART_INF_F;
-    for (int c = 0; c < n_chunks; c++) M = fmaxf(M, basep[(size_t)c * (kHd + 2) + kHd]);
-    float a0 = 0.f, a1 = 0.f, Ls = 0.f;
+// Merge the chunks' triples, rotate back, write: a warp per output row, so that the references and sums of up to 64 chunks
+// are one or two loads and the rows' loads do not wait for them.  A chunk that the row does not see counts as zeros whatever it holds.
+constexpr int kMergeWarps = 8;
+__global__ void __launch_bounds__(kMergeWarps * 32) prefill_umma_merge_kernel(const float *scratch, const float *givens, int n_chunks, int n_out, float *out) {
+    const int row = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= n_out) return;
+    const float *basep = scratch + (size_t)row * n_chunks * (kHd + 2);
+    float m[2], f[2], l[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int c = lane + 32 * h;
+        m[h] = c < n_chunks ? basep[(size_t)c * (kHd + 2) + kHd] : -CUDART_INF_F;
+        l[h] = c < n_chunks ? basep[(size_t)c * (kHd + 2) + kHd + 1] : 0.f;
+    }
+    float M = fmaxf(m[0], m[1]);
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    float Ls = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        f[h] = m[h] > -CUDART_INF_F ? exp2f(m[h] - M) : 0.f;
+        if (f[h] > 0.f) Ls = fmaf(l[h], f[h], Ls);
+    }
+    for (int o = 16; o > 0; o >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, o);
+    float2 acc[4] = {};  // coordinates 2 lane, 2 lane + 1 of each quarter
+#pragma unroll 4
     for (int c = 0; c < n_chunks; c++) {
-        const float *p = basep + (size_t)c * (kHd + 2);
-        const float m = p[kHd];
-        if (!(m > -CUDART_INF_F)) continue;
-        const float f = exp2f(m - M);
-        const float2 v = *reinterpret_cast<const float2 *>(p + 2 * pr);
-        a0 = fmaf(v.x, f, a0);
-        a1 = fmaf(v.y, f, a1);
-        Ls = fmaf(p[kHd + 1], f, Ls);
+        const float2 *p = reinterpret_cast<const float2 *>(basep + (size_t)c * (kHd + 2)) + lane;
+        const float fc = __shfl_sync(0xffffffffu, c < 32 ? f[0] : f[1], c & 31);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 v = p[32 * i];
+            acc[i].x = fmaf(fc > 0.f ? v.x : 0.f, fc, acc[i].x);
+            acc[i].y = fmaf(fc > 0.f ? v.y : 0.f, fc, acc[i].y);
+        }
     }
     const float inv = Ls > 0.f ? 1.0f / Ls : 0.f;
-    float o0 = a0 * inv, o1 = a1 * inv;
-    if (givens) givens_inv(a0 * inv, a1 * inv, givens[2 * pr], givens[2 * pr + 1], o0, o1);  // planar V only
-    *reinterpret_cast<float2 *>(out + row * kHd + 2 * pr) = make_float2(o0, o1);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int d = 64 * i + 2 * lane;
+        float o0 = acc[i].x * inv, o1 = acc[i].y * inv;
+        if (givens) {  // planar V only
+            float r0, r1;
+            givens_inv(o0, o1, givens[d], givens[d + 1], r0, r1);
+            o0 = r0;
+            o1 = r1;
+        }
+        float *dst = out + (size_t)row * kHd + d;  // (the caller's alignment is only that of a float)
+        dst[0] = o0;
+        dst[1] = o1;
+    }
 }
 
 template <int BITS, int NREP, bool VF32 = false>
@@ -703,8 +737,9 @@ bk_status launch_umma_one(bk_ctx *ctx, const PrefillUArgs &pa) {
     ctx->launches++;
     BK_CUDA(ctx, cudaGetLastError());
     if (pa.n_chunks > 1) {
-        prefill_umma_merge_kernel<<<pa.n_tokens * pa.d.n_head, 128, 0, ctx->stream>>>(pa.scratch, (BITS == 16 || BITS == 32 || VF32) ? nullptr : pa.d.givens,
-                                                                                      pa.n_chunks, pa.d.out);
+        const int n_out = pa.n_tokens * pa.d.n_head;
+        prefill_umma_merge_kernel<<<(n_out + kMergeWarps - 1) / kMergeWarps, kMergeWarps * 32, 0, ctx->stream>>>(
+            pa.scratch, (BITS == 16 || BITS == 32 || VF32) ? nullptr : pa.d.givens, pa.n_chunks, n_out, pa.d.out);
         ctx->launches++;
         BK_CUDA(ctx, cudaGetLastError());
     }
