@@ -215,6 +215,50 @@ def test_append_special_vectors(bk, gpu_ctx, oracle):
         cache.close()
 
 
+@pytest.mark.parametrize("n", [7, 400])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_append_vectors_of_any_magnitude(bk, gpu_ctx, oracle, bits, n):
+    """Rows from 1e-25 to 1e25 (norms that vanish or overflow), one-hot rows, and rows with infinities and NaN, in the
+    small and the bulk form of the append: indices as the scan gives them, norms bit for bit (NaN as NaN)."""
+    rng = np.random.default_rng(100 * bits + n)
+    k, v = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    for x in (k, v):
+        x *= (10.0 ** rng.uniform(-25, 25, (n, NKV, 1))).astype(np.float32)
+        x[0, 0], x[1, 1], x[2, 2] = 0, 0, 0
+        x[1, 1, 77], x[2, 2, 200] = 1.0, -3.0
+        x[3, 0, 9], x[4, 1, 250], x[5, 2, 130], x[6, 3, 131] = np.inf, -np.inf, np.nan, np.inf
+        x[6, 3, 132] = np.nan
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(f"planar{bits}"), n_layers=1, n_ctx=n)
+    ref = oracle.cache(MODE_PLANAR, bits, True)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    cache.append(0, k, v)
+    got, want = cache.dump_kv(0), ref.dump(0)
+    for key in want:
+        if want[key].dtype == np.float32:
+            nan = np.isnan(want[key])
+            assert np.array_equal(np.isnan(got[key]), nan) and np.array_equal(bits_of(got[key])[~nan], bits_of(want[key])[~nan]), key
+        else:
+            assert np.array_equal(got[key], want[key]), key
+    cache.close()
+
+
+@pytest.mark.parametrize("n_vec", [255, 256, 257, 512, 513, 8192, 8193, 20001])
+def test_bulk_host_transfers_at_slot_edges(bk, gpu_ctx, n_vec):
+    """Calls whose vectors (1 KB each) fill less than, just, and just more than the smallest bulk transfer, a pinned slot,
+    and the whole ring of slots: the same bytes as in calls that are too small for any of it."""
+    rng = np.random.default_rng(n_vec)
+    x = rng.standard_normal((n_vec, HD)).astype(np.float32)
+    pq = bk.PlanarQuant(HD, 4, gpu_ctx)
+    packed, norms = pq.quantize(x)
+    back = pq.dequantize(packed, norms)
+    for p in range(0, n_vec, 200):
+        pp, nn = pq.quantize(x[p:p + 200])
+        assert np.array_equal(np.asarray(packed).reshape(n_vec, -1)[p:p + 200], np.asarray(pp).reshape(len(nn), -1))
+        assert np.array_equal(bits_of(np.asarray(norms)[p:p + 200]), bits_of(np.asarray(nn)))
+        assert np.array_equal(bits_of(np.asarray(back).reshape(n_vec, HD)[p:p + 200]), bits_of(np.asarray(pq.dequantize(pp, nn)).reshape(-1, HD)))
+
+
 def test_append_at_far_positions(bk, gpu_ctx, oracle):
     """Rope positions up to the 262144-token training context; rows land at the next index."""
     cache = bk.AttnCache(gpu_ctx, bk.parse_mode("planar4"), n_layers=1, n_ctx=8, rope_positions=262144)
