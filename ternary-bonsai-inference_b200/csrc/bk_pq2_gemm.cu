@@ -18,8 +18,8 @@
 //     core never accumulates more than 16 MMAs, which keeps its truncating f32 adds from building up a bias.
 //     Two D buffers alternate: the drain of one step runs under the MMAs of the next.
 // Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 512 tokens 290 us = 370
-// TFLOP/s of useful work (two passes of it on the tensor cores), 5760 us as pairs of tokens; 16 tokens 55 us (before the
-// sums went in groups) against 187.  Rounding against float64: 1.0e-7 of the result's 2-norm, as one token at a time (with x20 outliers in x 1.0e-7 against
+// TFLOP/s of useful work (two passes of it on the tensor cores), 5760 us as pairs of tokens; 5 tokens 58 us against 64
+// (where the line lies: 4 tokens as pairs take 46), 16 tokens 59 against 180, 128 tokens 129 against 1440.  Rounding against float64: 1.0e-7 of the result's 2-norm, as one token at a time (with x20 outliers in x 1.0e-7 against
 // 2.6e-7); 1.4e-7, and 240 us, with one running sum over all blocks.
 // A step is (row tile of 128, block of 128); a CTA works on one or two row tiles (two share every B block: 32
 // instead of 64 bytes per clock and SM from L2, which is what the L2 delivers) and one token tile of 16..128.
