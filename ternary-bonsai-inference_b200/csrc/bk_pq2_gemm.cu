@@ -23,7 +23,7 @@
 // 2.6e-7); 1.4e-7, and 240 us, with one running sum over all blocks.
 // A step is (row tile of 128, block of 128); a CTA works on one or two row tiles (two share every B block: 32
 // instead of 64 bytes per clock and SM from L2, which is what the L2 delivers) and one token tile of 16..128.
-// The sum over blocks is sequential whatever the tiling, so a result does not depend on it bit for bit.
+// The sum over blocks takes the same order and groups whatever the tiling, so a result does not depend on it bit for bit.
 #include <algorithm>
 #include <atomic>
 #include <cuda_fp16.h>
