@@ -288,6 +288,8 @@ bk_status launch_rms_norm_rows(bk_ctx *ctx, const NormSeg &s0, const NormSeg &s1
 
 // PQ2_0 ternary rows (bk_pq2.cu): bytes per row, and y[t][r] = x[t] . row r for up to 2 tokens and 4 row ranges a launch.
 size_t pq2_row_bytes(int64_t ne0);
+// BK_ERR_UNSUPPORTED for rows too long for the products of n_tok tokens.
+bk_status pq2_rows_fit(bk_ctx *ctx, int ne0, int n_tok);
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                             const float *x, int n_tok);
 // The same for a block of up to kPq2GemmTokens tokens on the tensor cores (bk_pq2_gemm.cu).

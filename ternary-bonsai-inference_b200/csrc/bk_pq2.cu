@@ -292,6 +292,17 @@ bk_status launch_nt(bk_ctx *ctx, const Pq2Args &a, int grid, size_t smem) {
 
 size_t pq2_row_bytes(int64_t ne0) { return (size_t)((ne0 + kPqQK - 1) / kPqQK) * kPqBlockBytes; }
 
+// Shared memory of a CTA, and of it what the tables and the digits of nt tokens take.
+constexpr size_t kPqSmem = 227 * 1024;
+static size_t pq2_stage_bytes(int nb) { return ((size_t)kPqTileRows * nb * kPqBlockBytes + 16 + 127) / 128 * 128; }
+
+bk_status pq2_rows_fit(bk_ctx *ctx, int ne0, int n_tok) {
+    const int nb = (ne0 + kPqQK - 1) / kPqQK;
+    if (pq_off_stage(nb, n_tok <= 1 ? 1 : 2) + pq2_stage_bytes(nb) > kPqSmem)
+        return fail(ctx, BK_ERR_UNSUPPORTED, "pq2_matvec: rows too long for a shared-memory stage of 16 rows");
+    return BK_OK;
+}
+
 // Up to four row ranges with the same ne0 (rows[s]: device pointer to the first row, n_rows[s] rows,
 // y[s] [n_tok][n_rows[s]]); x [n_tok][ne0], n_tok 1..2.
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
@@ -318,15 +329,14 @@ bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, 
     for (int sgi = used; sgi <= kPqMaxSegs; sgi++) a.seg_tile0[sgi] = tiles;
     a.n_tiles = tiles;
     if (tiles == 0) return BK_OK;
-    const size_t tile_bytes = (size_t)kPqTileRows * a.row_bytes;
-    a.stage_stride = (int)((tile_bytes + 16 + 127) / 128 * 128);
+    const bk_status st = pq2_rows_fit(ctx, ne0, n_tok);
+    if (st != BK_OK) return st;
+    a.stage_stride = (int)pq2_stage_bytes(a.nb);
     const int nt = n_tok <= 1 ? 1 : 2;
     const size_t fixed = pq_off_stage(a.nb, nt);
-    const size_t limit = 227 * 1024;
+    const size_t limit = kPqSmem;
     a.stages = fixed + (size_t)kPqGroupStages * a.stage_stride <= limit ? kPqGroupStages : 1;
     const size_t per_group = (size_t)a.stages * a.stage_stride;
-    if (fixed + per_group > limit)
-        return fail(ctx, BK_ERR_UNSUPPORTED, "pq2_matvec: rows too long for a shared-memory stage of 16 rows");
     // One CTA per SM; it runs as many groups of 8 warps (each with its own tiles and stages) as the
     // matrix has tiles for and shared memory has room for.
     int groups = (int)std::min<size_t>(kPqMaxGroups, (limit - fixed) / per_group);

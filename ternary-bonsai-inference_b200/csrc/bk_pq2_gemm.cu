@@ -502,6 +502,8 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
         used++;
     }
     if (used == 0) return BK_OK;
+    const bk_status fit = pq2_rows_fit(ctx, ne0, n_tok);  // one limit for every number of tokens from two on
+    if (fit != BK_OK) return fit;
     int mt = 1, nc = 1;
     plan_gemm(ctx->n_sms, used, rows_used, a.nb, n_tok, &mt, &nc);
     const int n = 16 * nc, tok_tiles = (n_tok + n - 1) / n;

@@ -205,3 +205,16 @@ def test_gpu_pq2_token_block_product(bk, gpu_ctx, ne0, n_rows, n_tok, base):
     norm = np.abs(x.astype(np.float64)) @ np.abs(w).T
     assert np.max(np.abs(got - truth) / (norm + 1e-30)) <= 2e-6
     t.free()
+
+
+@pytest.mark.gpu
+def test_gpu_pq2_row_length_limit(bk, gpu_ctx):
+    """Rows of 157 blocks fit the product of one token and not that of two: whatever the number of tokens from two on,
+    the call is refused."""
+    payload, _, _, x = synth(bk, 5, 3, 157 * 128, 6)
+    t = bk.Pq2Tensor(gpu_ctx, payload, 157 * 128)
+    assert t.matmul_n(x[:1], 1).shape == (1, 3)
+    for n_tok in (2, 4, 5, 6):
+        with pytest.raises(bk.BonsaiKvError, match="rows too long"):
+            t.matmul_n(x[:n_tok], n_tok)
+    t.free()
