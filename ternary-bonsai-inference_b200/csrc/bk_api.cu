@@ -1278,7 +1278,7 @@ static bk_status pq2_check(bk_ctx *ctx, const char *who, const void *payload, si
     return BK_OK;
 }
 
-// y of range s: [n_tok][n_rows_s].  One or two tokens take the weight-streaming kernel (two share one pass), more
+// y of range s: [n_tok][n_rows_s].  Up to four tokens take the weight-streaming kernel (two share one pass), more
 // the tensor-core product.
 static bk_status pq2_run_multi(bk_ctx *ctx, int n_seg, const bk_pq2_seg *segs, int64_t ne0, const float *x_dev, int32_t n_tok) {
     const size_t rb = pq2_row_bytes(ne0);

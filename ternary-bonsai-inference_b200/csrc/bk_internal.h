@@ -293,7 +293,7 @@ bk_status pq2_rows_fit(bk_ctx *ctx, int ne0, int n_tok);
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                             const float *x, int n_tok);
 // The same for a block of up to kPq2GemmTokens tokens on the tensor cores (bk_pq2_gemm.cu).
-// From 5 tokens on (q + k + v and output rows of a layer: 4 tokens 47 us in pairs, 58 us here; 6 tokens 68 and 58);
+// From 5 tokens on (q + k + v and output rows of a layer: 4 tokens 45 us in pairs, 52 us here; 5 tokens 62 and 52);
 // 1024 tokens a pass bound the scratch (21 MB at ne0 5120).
 constexpr int kPq2GemmTokens = 1024, kPq2GemmMin = 5;
 bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,

@@ -1,32 +1,40 @@
 // PQ2_0 ternary rows times a block of activations (prompt or speculative tokens) on the 5th-generation
 // tensor cores: y[t][r] = sum_j x[t][j] * W[base_row + r][j] for n_tok tokens at once
 // (src/kernels.rs:333-420 `pq2_matmul_n`; row format src/kernels.rs:204-229).  bk_pq2.cu is the form for
-// one or two tokens, where the weight stream is the cost and every launch reads it once per pair of tokens.
+// one to four tokens, where the weight stream is the cost and every launch reads it once per pair of tokens.
 //
-// What bounds it: with hundreds of tokens the multiply-adds, 2 tensor-core terms each; with a few tokens the
-// unpacking of the weights.  The layout follows from three numbers:
-//   * Weights are the A operand, IN TENSOR MEMORY: M = 128 rows, a thread's tensor-memory lane is a row, so
-//     unpacking is register work (a mask and an f16 FMA give two weights -1, 0, 1, 2) and a tcgen05.st; no shared-memory pass, and the MMA reads only B from shared memory.
-//   * Activations are the B operand, as f16 hi + mid parts of x scaled by a power of two per token (at least
-//     22 bits of every element, and 2^-40 of the token's largest one as the floor, so no less than the
-//     25-bit fixed point per block of the one-token form gives: its grid is 2^-24 of a block's largest element).
-//     A first kernel writes them once, already permuted (the order of the K slots is free and is chosen so that the
-//     unpacking needs no shuffles) and swizzled, one contiguous piece per (token tile, block of 128): the
-//     main kernel fetches a block with ONE bulk copy.
-//   * The block scale is the row's, so the accumulator is drained after every block of 128 and added up in f32 as
-//     scale * block sum, grouped as the reference's scalar path does it (src/kernels.rs:633-650); the tensor
-//     core never accumulates more than 16 MMAs, which keeps its truncating f32 adds from building up a bias.
-//     Two D buffers alternate: the drain of one step runs under the MMAs of the next.
-// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 512 tokens 290 us = 370
-// TFLOP/s of useful work (two passes of it on the tensor cores), 5760 us as pairs of tokens; 5 tokens 58 us against 64
-// (where the line lies: 4 tokens as pairs take 46), 16 tokens 59 against 180, 128 tokens 129 against 1440.  Rounding against float64: 1.0e-7 of the result's 2-norm, as one token at a time (with x20 outliers in x 1.0e-7 against
-// 2.6e-7); 1.4e-7, and 240 us, with one running sum over all blocks.
+// The block sums are exact integers, as there: x is fixed point, X = round(x * 2^(27 - e)) with 2^e the power of two
+// above the largest |x| of the token's block of 128 (three bits more than the form for few tokens keeps).
+//
+// What bounds it: what the sixteen warps that unpack weights and drain sums have to issue (0.72 of all issue slots with 512
+// tokens, the tensor cores 0.41 busy with four 8-bit products per weight and token); with a few tokens the round trips of a
+// step.  The layout:
+//   * X has 28 bits and an operand has 8, so X is cut into four digits, X = d0 - 64 d1 + 2^14 (d2 - 64 d3), each within
+//     -128..127.  The weights are unpacked twice, as -1, 0, 1, 2 and times -64 (which fits 8 bits): d0 and d1 then meet in one
+//     accumulator, d2 and d3 in another, and both stay within 2^21, exact in s32 and in f32.
+//   * Weights are the A operand, IN TENSOR MEMORY: M = 128 rows, a thread's tensor-memory lane is a row, so unpacking is
+//     register work (four codes in a byte permute's selector give four weights) and a tcgen05.st; no shared-memory pass, and
+//     the MMA reads only B from shared memory.
+//   * X is the B operand.  A first kernel writes the digits once, already permuted (the order of the K slots is free and is
+//     chosen so that the unpacking needs no shuffles) and swizzled, one contiguous piece per (token tile, block of 128): the
+//     main kernel fetches a block with ONE bulk copy, and a tile's block scales (2^(e - 27)) with one more.
+//   * Both scales are the block's, so the accumulators are drained after every block of 128: the two sums become one f32
+//     (one rounding) that is added up as scale * sum, as the reference's scalar path groups it (src/kernels.rs:633-650).
+//     Two pairs of accumulators alternate: the drain of one step runs under the MMAs of the other's next.  128 columns a
+//     pair are what the operand stages leave, hence at most 64 tokens a tile.
+// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 to 16 tokens 52 us (62 and 176 as
+// pairs of tokens; 4 tokens as pairs take 45, which is where the line lies), 64 tokens 68 (702), 128 tokens 101 (1410), 512
+// tokens 308 (5750), 1024 tokens 536.  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
+// 57, 86, 129, 287 and 574.  Error against float64, 2-norm: 7.4e-8 on normal data, 8.0e-8 with x20 outliers in x, 4.5e-8 without
+// a bias on products of one sign; 1.02e-7, 2.4e-7 and 5.0e-8 as pairs of tokens; 1.01e-7, 1.0e-7 and 6.5e-8 (bias -5e-8) in the
+// form before, which also lost blocks that lie 2^40 below the token's largest element.
 // A step is (row tile of 128, block of 128); a CTA works on one or two row tiles (two share every B block: 32
-// instead of 64 bytes per clock and SM from L2, which is what the L2 delivers) and one token tile of 16..128.
+// instead of 64 bytes per clock and SM from L2, which is what the L2 delivers) and one token tile of 16..64.
 // The sum over blocks takes the same order and groups whatever the tiling, so a result does not depend on it bit for bit.
 #include <algorithm>
 #include <atomic>
 #include <cuda_fp16.h>
+#include <math_constants.h>
 
 #include "bk_device.cuh"
 #include "bk_internal.h"
@@ -37,118 +45,167 @@ namespace bk {
 
 namespace {
 
-constexpr int kGemmThreads = 320;                 // 8 warps that unpack and drain, one that issues MMAs, one that loads B
+constexpr int kWorkWarps = 16;                    // unpack and drain
+constexpr int kMmaWarp = kWorkWarps, kLoadWarp = kWorkWarps + 1, kGemmThreads = (kWorkWarps + 2) * 32;
 constexpr int kGemmBlock = 128, kGemmBlockBytes = 34;
 constexpr int kGemmSegBlocks = 4;                 // blocks of a row staged together
 constexpr int kGemmRowWords = 36;                 // words of a staged row: nine 16-byte pieces hold any four blocks of an aligned row
 constexpr int kGemmMaxSegs = 4;
-constexpr int kGemmGroup = 8;                     // blocks that are added up before their sum goes to y
-constexpr uint32_t kColsD = 128, kColA = 256, kColsA = 64;  // tensor-memory columns: D0 | D1 | four A stages
+constexpr int kGemmMaxSegments = 64;              // of four blocks in a row (the length limit leaves 36)
+constexpr uint32_t kGemmStageW = 2 * 2 * 128 * kGemmRowWords * 4;  // staged weights of the two owners
+// Shared memory of the sums of the segments done, [row tile][token][row].
+__host__ __device__ constexpr uint32_t gemm_sum_bytes(int mt, int n) { return (uint32_t)(mt * n) * 512u; }
+constexpr int kGemmFrac = 27;                     // X = round(x * 2^(kGemmFrac - e))
+// tensor-memory columns: per owner a pair of sums (low | high), then per owner two A stages (weights | times -64)
+constexpr uint32_t kColsD = 128, kColHi = 64, kColA = 256, kColsA = 64;
 
 struct GemmArgs {
     const uint8_t *rows[kGemmMaxSegs];
     float *y[kGemmMaxSegs];
-    int seg_rows[kGemmMaxSegs], seg_tile0[kGemmMaxSegs + 1];
-    const uint8_t *xb;        // [token tile][block][hi|mid][2 slabs of 64 slots][n][128 B, swizzled]
-    const float *tok_scale;   // [token tile * n]: what a token's sums are multiplied by
+    int seg_rows[kGemmMaxSegs], seg_tile0[kGemmMaxSegs];
+    int y_stride[kGemmMaxSegs];  // rows of a token in y (the range may be a part of them)
+    const uint8_t *xb;        // [token tile][block][digit][n][128 B, swizzled]
+    const float *x_scale;     // [token tile][block][n]: 2^(e - kGemmFrac), NaN for a block with an infinity or a NaN in it
     int nb, row_bytes, n_tok, n_stages_b;
     int vec;                  // bit s: the rows of range s all start on 16-byte boundaries
     int *err_flag;
 };
 
-// x -> scaled hi and mid parts in the order and swizzle of the B operand.  One CTA per (padded) token.
-// Slot k = 16 i + 2 p + h of a block holds weight 16 i + p + 8 h (see unpack16()), so the eight slots of a
-// 16-byte chunk are four consecutive elements and the four that lie eight further on, alternating.
-__global__ void __launch_bounds__(256) pq2_split_x_kernel(const float *x, int ne0, int nb, int n_tok, int n, uint8_t *xb, float *tok_scale) {
+// x -> digits in the order and swizzle of the B operand, and the block scales.  One thread per 16 elements of a (padded) token,
+// eight per block.  Slots 16 i + 4 p .. + 3 of a block hold the elements 16 i + o, 16 i + o + 2, .. + 4, .. + 6 with
+// o = 0, 8, 1, 9 for p = 0..3 (see unpack16()), so the sixteen elements of a thread are one 16-byte chunk of each digit.
+__global__ void __launch_bounds__(256) pq2_split_x_kernel(const float *x, int ne0, int nb, int n_tok, int n, int n_pad, uint8_t *xb, float *x_scale) {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    __shared__ float wmax[8];
-    const int tok = blockIdx.x, tile = tok / n, r = tok - tile * n, tid = threadIdx.x;
-    const float *xr = x + (size_t)tok * ne0;
-    const bool real = tok < n_tok;
-    const bool vec = (ne0 & 3) == 0 && ((uintptr_t)x & 15) == 0;
-    const int chunks = nb * 16;
-    auto load = [&](int c, float (&v)[8]) {
-        const int j = (c >> 1) * 16 + (c & 1) * 4;  // and j + 8
-        if (real && vec && j + 12 <= ne0) {
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(xr + j)), b = __ldg(reinterpret_cast<const float4 *>(xr + j + 8));
-            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-        } else {
+    const int idx = blockIdx.x * 256 + threadIdx.x, tok = idx / (nb * 8), c = idx - tok * (nb * 8), blk = c >> 3, i = c & 7;
+    const int tile = tok / n, r = tok - tile * n, j0 = 16 * c;
+    float v[16];
+    if (tok < n_tok && (ne0 & 3) == 0 && ((uintptr_t)x & 15) == 0 && j0 + 16 <= ne0) {
+        const float4 *p = reinterpret_cast<const float4 *>(x + (size_t)tok * ne0 + j0);
 #pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = (real && j + i + (i & 4) < ne0) ? xr[j + i + (i & 4)] : 0.f;
+        for (int k = 0; k < 4; k++) {
+            const float4 f = __ldg(p + k);
+            v[4 * k] = f.x, v[4 * k + 1] = f.y, v[4 * k + 2] = f.z, v[4 * k + 3] = f.w;
         }
-    };
-    float v[8], am = 0.f;
-    for (int c = tid; c < chunks; c += 256) {
-        load(c, v);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) am = fmaxf(am, fabsf(v[i]));
+        for (int k = 0; k < 16; k++) v[k] = (tok < n_tok && j0 + k < ne0) ? x[(size_t)tok * ne0 + j0 + k] : 0.f;
     }
-    for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-    if ((tid & 31) == 0) wmax[tid >> 5] = am;
-    __syncthreads();
-    am = wmax[0];
+    float am = 0.f;
 #pragma unroll
-    for (int i = 1; i < 8; i++) am = fmaxf(am, wmax[i]);
+    for (int k = 0; k < 16; k++) am = fabsf(v[k]) <= am ? am : (fabsf(v[k]) < CUDART_INF_F ? fabsf(v[k]) : CUDART_INF_F);
+    for (int o = 4; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));  // the block's eight threads
+    if (tok >= n_pad) return;
     int e = 0;
-    if (am > 0.f && am < INFINITY) frexpf(am, &e);  // am = f * 2^e, f in [0.5, 1)
-    const int up = max(-126, min(15 - e, 127));     // the largest element lands in [2^14, 2^15)
+    if (am > 0.f && am < CUDART_INF_F) frexpf(am, &e);  // am = f * 2^e, f in [0.5, 1)
+    const int up = min(kGemmFrac - e, 127);             // (blocks below 2^-100: the grid stays at 2^-127)
     const float s = ldexpf(1.0f, up);
-    if (tid == 0) tok_scale[tok] = ldexpf(1.0f, -up);
-    for (int c = tid; c < chunks; c += 256) {
-        load(c, v);
-        uint32_t hi[4], mid[4];
+    if (i == 0) x_scale[((size_t)tile * nb + blk) * n + r] = am < CUDART_INF_F ? ldexpf(1.0f, -up) : CUDART_NAN_F;
+    uint32_t d[4][4] = {};
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const float a = v[p] * s, b = v[p + 4] * s;
-            const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-            const __half2 h2 = __halves2half2(ha, hb);
-            const __half2 m2 = __halves2half2(__float2half_rn(a - __half2float(ha)), __float2half_rn(b - __half2float(hb)));
-            hi[p] = *reinterpret_cast<const uint32_t *>(&h2);
-            mid[p] = *reinterpret_cast<const uint32_t *>(&m2);
+    for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int X = __float2int_rn(v[(p & 1) * 8 + (p >> 1) + 2 * q] * s);      // |X| < 2^27
+            const int h = (X + 8192) >> 14, l = X - h * 16384;                        // -8192..8192, -8192..8191
+            const int d1 = min(-((l + 32) >> 6), 127), d3 = min(-((h + 32) >> 6), 127);  // what 127 cuts off fits the digit below
+            d[0][p] |= (uint32_t)((l + 64 * d1) & 255) << (8 * q);
+            d[1][p] |= (uint32_t)(d1 & 255) << (8 * q);
+            d[2][p] |= (uint32_t)((h + 64 * d3) & 255) << (8 * q);
+            d[3][p] |= (uint32_t)(d3 & 255) << (8 * q);
         }
-        const int blk = c >> 4, slab = (c >> 3) & 1, ch = c & 7;
-        uint8_t *dst = xb + ((size_t)tile * nb + blk) * (size_t)n * 512 + (size_t)slab * n * 128 + (size_t)r * 128 + ((ch ^ (r & 7)) << 4);
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4 *>(dst + (size_t)n * 256) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-    }
+    uint8_t *dst = xb + ((size_t)tile * nb + blk) * (size_t)n * 512 + (size_t)r * 128 + ((i ^ (r & 7)) << 4);
+#pragma unroll
+    for (int k = 0; k < 4; k++) *reinterpret_cast<uint4 *>(dst + (size_t)k * n * 128) = make_uint4(d[k][0], d[k][1], d[k][2], d[k][3]);
 }
 
+// Tensor-memory loads without the wait.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+}
 
-// Sixteen 2-bit codes -> eight registers of two f16 weights (code - 1): register p = codes p and p + 8.  A code that
-// is masked where it lies and put under the exponent of 1024 is the f16 number 1024 + 4^i code; one f16 FMA brings
-// it to code - 1 exactly.  (Nine integer operations for sixteen weights; shift, mask and byte permute took 23 and, at half
-// the issue rate of the FMA pipe, were most of a step.)
-__device__ __forceinline__ void unpack16(uint32_t w, uint32_t *out) {
-    const uint32_t w2 = w >> 10;
+// Sixteen 2-bit codes -> four registers of four 8-bit weights (code - 1) and four of the same times -64.  The codes are
+// the selectors of a byte permute of the four weights: a nibble with one code in it picks a byte.  Registers in order:
+// codes 0 2 4 6, 8 10 12 14, 1 3 5 7, 9 11 13 15.
+__device__ __forceinline__ void unpack16(uint32_t w, uint32_t *one, uint32_t *wide) {
+    const uint32_t even = w & 0x33333333u, odd = (w >> 2) & 0x33333333u;
+    const uint32_t sel[4] = {even, even >> 16, odd, odd >> 16};
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
-        const int i = p < 5 ? p : p - 5;
-        const uint32_t u = ((p < 5 ? w : w2) & (0x00030003u << (2 * i))) | 0x64006400u;
-        const float f = 1.0f / (float)(1 << (2 * i));
-        const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&u), __float2half2_rn(f), __float2half2_rn(-(1024.0f * f + 1.0f)));
-        out[p] = *reinterpret_cast<const uint32_t *>(&r);
+    for (int p = 0; p < 4; p++) {
+        one[p] = __byte_perm(0x020100ffu, 0u, sel[p]);
+        wide[p] = __byte_perm(0x80c00040u, 0u, sel[p]);
     }
 }
 
-// MT row tiles per CTA, N = 16 NC tokens.
+// Two f32 operations in one instruction (the draining warps are bound by what they issue).
+struct F2 {
+    float x, y;
+};
+__device__ __forceinline__ uint64_t join2(F2 a) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ F2 split2(uint64_t r) {
+    F2 a;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t int2_to_f2(uint32_t a, uint32_t b) { return join2(F2{__int2float_rn((int)a), __int2float_rn((int)b)}); }
+
+// MT row tiles per CTA, N = 16 NC tokens.  Sixteen warps in two halves of eight ("owners") work on alternate steps, each with
+// its own sums and operand stages, so that the round trips of a step (operand stores, the MMAs, reading the sums back) are under
+// the other half's step: sixteen warps that share every step took 465 us for 512 tokens, two owners 340.
+// With two row tiles an owner has one of them; with one, the owners take every other unit of up to eight blocks.
 template <int MT, int NC>
 __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    constexpr int N = 16 * NC, NH = 8 * NC;  // tokens of the tile, and of one warpgroup
+    constexpr int N = 16 * NC, NH = 8 * NC;  // tokens of the tile, and of one warp
     constexpr uint32_t kBlockB = (uint32_t)N * 512u;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
-    // barriers: B full [4] | B free [4] | A full [4] | D full [2] | D free [2]; then the tensor-memory address and a give-up flag
-    const uint32_t bar_bf = sbase, bar_be = sbase + 32, bar_af = sbase + 64, bar_df = sbase + 96, bar_de = sbase + 112, slot = sbase + 128;
-    volatile int *gave_up = reinterpret_cast<volatile int *>(sm + 132);
-    const int nst = a.n_stages_b, nb = a.nb, n_steps = nb * MT;
-    const uint32_t off_b = 1024u, off_w = off_b + (uint32_t)nst * kBlockB;
+    // barriers: B full [4] | B free [4] | A full [owner][2] | D full [2] | D free [2] | turn [2] | block scales | drain; then the
+    // tensor-memory address and a give-up flag
+    const uint32_t bar_bf = sbase, bar_be = sbase + 32, bar_af = sbase + 64, bar_df = sbase + 96, bar_de = sbase + 112, bar_turn = sbase + 128,
+                   bar_sc = sbase + 144, bar_drain = sbase + 152, slot = sbase + 160;
+    volatile int *gave_up = reinterpret_cast<volatile int *>(sm + 164);
+    const int nst = a.n_stages_b, nb = a.nb, n_seg = (nb + kGemmSegBlocks - 1) / kGemmSegBlocks;
+    const uint32_t off_b = 1024u, off_w = off_b + (uint32_t)nst * kBlockB, off_t = off_w + kGemmStageW, off_s = off_t + gemm_sum_bytes(MT, N);
+    // The segments form units of one or two, whose sums are kept apart; a pair of units has the same size as far as the row
+    // goes.  Neither depends on the tiling.  The steps go in rounds of one per owner: round q is block q of both row tiles, or,
+    // with one row tile, block q % 4 of the (q / 4)-th segment of the owner's units, which are every other one.
+    const int n_half = (n_seg + 1) / 2, n_pairs = (n_half + 1) / 2;
+    volatile uint8_t *seg_order = sm + 168, *unit_end = sm + 168 + 2 * kGemmMaxSegments;  // [owner][i]: i-th segment (one row tile); [segment]
+    if (tid < n_half) {
+        // pair p has the segments 2 f .. 2 f + 2 h - 1
+        const int p = ((tid + 1) * n_pairs - 1) / n_half, f = p * n_half / n_pairs, h = (p + 1) * n_half / n_pairs - f;
+        for (int o = 0; o < 2; o++) {
+            const int seg = 2 * f + o * h + tid - f;
+            seg_order[o * kGemmMaxSegments + tid] = (uint8_t)seg;
+            unit_end[seg] = tid - f == h - 1 || seg == n_seg - 1;
+        }
+    }
+    const int n_rounds = MT == 2 ? nb : n_half * kGemmSegBlocks;
+    auto segment = [&](int i, int owner) { return MT == 2 ? i : (int)seg_order[owner * kGemmMaxSegments + i]; };
+    auto block_of = [&](int q, int owner) { return MT == 2 ? q : segment(q >> 2, owner) * kGemmSegBlocks + (q & 3); };
 
     if (tid == 0) {
         for (int i = 0; i < 4; i++) {
@@ -159,15 +216,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
         for (int i = 0; i < 2; i++) {
             mbar_init(bar_df + 8 * i, 1);
             mbar_init(bar_de + 8 * i, 8);
+            mbar_init(bar_turn + 8 * i, 8);
         }
+        mbar_init(bar_sc, 1);
+        mbar_init(bar_drain, 1);
         *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == 8) tmem_alloc(slot, 512);
+    if (warp == kMmaWarp) tmem_alloc(slot, 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(sm + 128), 0);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t *>(sm + 160), 0);
 
     // bounded wait; after one has run out (never expected) the others of the CTA do not start to wait
     auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
@@ -182,6 +242,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
         }
         return true;
     };
+    auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, wait(bar, parity)); };  // one answer for the warp
 
     const int row_tile = blockIdx.x, tok_tile = blockIdx.y;
     int sg = 0;
@@ -190,57 +251,80 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
     const int row0 = (row_tile - a.seg_tile0[sg]) * (128 * MT), seg_rows = a.seg_rows[sg];
     const uint8_t *wrows = a.rows[sg];
 
-    if (warp == 9) {
-        // B blocks, in order through the ring of stages
+    if (warp == kLoadWarp) {
+        // the tile's block scales, then its B blocks, in order of use through the ring of stages
         const uint8_t *xb = a.xb + (size_t)tok_tile * nb * kBlockB;
         asm volatile("griddepcontrol.wait;\n" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-        int b = 0;
-        for (uint32_t st = 0, use = 0; b < nb; b++) {
-            if (use > 0 && !wait(bar_be + 8 * st, (use - 1) & 1u)) break;
-            if (elect_one()) {
-                mbar_expect_tx(bar_bf + 8 * st, kBlockB);
-                tma_bulk(sbase + off_b + st * kBlockB, xb + (size_t)b * kBlockB, kBlockB, bar_bf + 8 * st);
+        if (elect_one()) {
+            const uint32_t bytes = (uint32_t)nb * N * 4u;
+            mbar_expect_tx(bar_sc, bytes);
+            tma_bulk(sbase + off_s, a.x_scale + (size_t)tok_tile * nb * N, bytes, bar_sc);
+        }
+        __syncwarp();
+        uint32_t st = 0, use = 0;
+        bool ok = true;
+        for (int q = 0; q < n_rounds && ok; q++)
+#pragma unroll
+            for (int o = 0; o < 3 - MT; o++) {
+                const int b = block_of(q, o);
+                if (b >= nb) continue;
+                if (use > 0) ok = ok && wait_all(bar_be + 8 * st, (use - 1) & 1u);
+                if (!ok) break;
+                if (elect_one()) {
+                    mbar_expect_tx(bar_bf + 8 * st, kBlockB);
+                    tma_bulk(sbase + off_b + st * kBlockB, xb + (size_t)b * kBlockB, kBlockB, bar_bf + 8 * st);
+                }
+                __syncwarp();
+                if (++st == (uint32_t)nst) st = 0, use++;
             }
-            __syncwarp();
-            if (++st == (uint32_t)nst) st = 0, use++;
-        }
-        for (int c = max(0, b - nst); c < b && b < nb; c++) {  // gave up: leave no copy in flight behind
-            int polls = 0;
-            while (!mbar_try_wait(bar_bf + 8 * (c % nst), (uint32_t)(c / nst) & 1u) && ++polls < kWaitPolls) {}
-        }
-    } else if (warp == 8) {
-        const uint32_t idesc = umma_idesc_f16(128, N, 0, 0);
+        // no copy in flight is left behind, whatever happened above
+        const int filled = (int)use * nst + (int)st;
+        for (int c = max(0, filled - nst); c < filled; c++)
+            for (int polls = 0; !mbar_try_wait(bar_bf + 8 * (c % nst), (uint32_t)(c / nst) & 1u) && polls < kWaitPolls; polls++) {}
+        for (int polls = 0; !mbar_try_wait(bar_sc, 0) && polls < kWaitPolls; polls++) {}
+    } else if (warp == kMmaWarp) {
+        const uint32_t idesc = umma_idesc_s8(128, N);
         uint32_t st = 0, b_par = 0;
-        for (int s = 0; s < n_steps; s++) {
-            bool ok = true;
-            if (s % MT == 0) ok = wait(bar_bf + 8 * st, b_par);
-            ok = ok && wait(bar_af + 8 * (s & 3), (uint32_t)(s >> 2) & 1u);
-            if (s >= 2) ok = ok && wait(bar_de + 8 * (s & 1), (uint32_t)((s >> 1) - 1) & 1u);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            tc_fence_after_sync();
-            const uint32_t d = tmem + (s & 1) * kColsD, am = tmem + kColA + (s & 3) * kColsA;
-            const uint64_t bd = umma_smem_desc(sbase + off_b + st * kBlockB, 16, 1024, kUmmaSwizzle128);
-            if (elect_one()) {
+        bool ok = true;
+        for (int q = 0; q < n_rounds && ok; q++)
 #pragma unroll
-                for (int term = 1; term >= 0; term--)  // the small parts first
+            for (int o = 0; o < 2; o++) {  // round q is every owner's q-th step
+                if (block_of(q, o) >= nb) continue;
+                if (MT == 1 || o == 0) ok = ok && wait_all(bar_bf + 8 * st, b_par);
+                ok = ok && wait_all(bar_af + 16 * o + 8 * (q & 1), (uint32_t)(q >> 1) & 1u);
+                if (q > 0) ok = ok && wait_all(bar_de + 8 * o, (uint32_t)(q - 1) & 1u);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t d = tmem + o * kColsD, am = tmem + kColA + o * (2 * kColsA) + (q & 1) * kColsA;
+                const uint64_t bd = umma_smem_desc(sbase + off_b + st * kBlockB, 16, 1024, kUmmaSwizzle128);
+                const bool last_use = MT == 1 || o == 1;
+                if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 8; k++)  // (the address field of a descriptor counts 16-byte units)
-                        umma_f16_ts(d, am + 8 * k, bd + (uint64_t)((term * (N * 256) + (k >> 2) * (N * 128) + (k & 3) * 32) >> 4), idesc,
-                                    !(term == 1 && k == 0));
-                umma_commit(bar_df + 8 * (s & 1));
-                if (s % MT == MT - 1) umma_commit(bar_be + 8 * st);
+                    for (int dg = 0; dg < 4; dg++)  // digits 0 and 1: low sums, 2 and 3: high ones; the odd ones meet the weights times -64
+#pragma unroll
+                        for (int k = 0; k < 4; k++)  // (the address field of a descriptor counts 16-byte units)
+                            umma_i8_ts(d + (dg >> 1) * kColHi, am + (dg & 1) * 32 + 8 * k, bd + (uint64_t)((dg * (N * 128) + k * 32) >> 4), idesc,
+                                       !((dg & 1) == 0 && k == 0));
+                    umma_commit(bar_df + 8 * o);
+                    if (last_use) umma_commit(bar_be + 8 * st);
+                }
+                __syncwarp();
+                if (last_use && ++st == (uint32_t)nst) st = 0, b_par ^= 1u;
             }
-            __syncwarp();
-            if (s % MT == MT - 1 && ++st == (uint32_t)nst) st = 0, b_par ^= 1u;
-        }
+        // no product in flight is left behind, whatever happened above
+        if (elect_one()) umma_commit(bar_drain);
+        __syncwarp();
+        for (int polls = 0; !mbar_try_wait(bar_drain, 0) && polls < kWaitPolls; polls++) {}
     } else {
-        const int quad = warp & 3, half = warp >> 2, r = quad * 32 + lane;  // tensor-memory lane = row of the tile
-        uint32_t *wst = reinterpret_cast<uint32_t *>(sm + off_w);           // [2][MT * 128][kGemmRowWords]
-        const int n_seg = (nb + kGemmSegBlocks - 1) / kGemmSegBlocks;
-        // The two warps of a quadrant stage its 32 rows.  Rows on 16-byte boundaries (their length is then a multiple of
-        // eight blocks): the nine 16-byte pieces around four blocks, which start at the segment's first byte or, every other
-        // segment, 8 bytes before it.  Other rows: the words that overlap the blocks.
+        const int owner = warp >> 3, quad = warp & 3, half = (warp >> 2) & 1, r = quad * 32 + lane;  // tensor-memory lane = row of the tile
+        const int trow0 = row0 + (MT == 2 ? owner * 128 : 0);                                        // first row of the owner's tile
+        auto seg_of = [&](int k) { return segment(k, owner); };
+        const int n_local = MT == 2 ? n_seg : (seg_of(n_half - 1) < n_seg ? n_half : n_half - 1);    // segments of the owner
+        uint32_t *wst = reinterpret_cast<uint32_t *>(sm + off_w) + owner * (2 * 128 * kGemmRowWords);  // [2][128][kGemmRowWords]
+        // The two warps of a quadrant stage its 32 rows, a segment of four blocks at a time.  Rows on 16-byte boundaries (their
+        // length is then a multiple of eight blocks): the nine 16-byte pieces around the blocks, which start at the segment's
+        // first byte or, every other segment, 8 bytes before it.  Other rows: the words that overlap the blocks.
         const bool vec = (a.vec >> sg) & 1;
         const int t64 = half * 32 + lane;
         uint32_t src[5];
@@ -250,173 +334,171 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
             src[i] = (uint32_t)rr * a.row_bytes + (uint32_t)(idx - rr * 9) * 16u;
         }
         auto stage_w = [&](int k) {
-            const int blocks = min(kGemmSegBlocks, nb - k * kGemmSegBlocks), bytes = blocks * kGemmBlockBytes;
+            const int seg = seg_of(k), blocks = min(kGemmSegBlocks, nb - seg * kGemmSegBlocks), bytes = blocks * kGemmBlockBytes;
+            const int rb = quad * 32;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(wst) + (uint32_t)(((k & 1) * 128 + rb) * kGemmRowWords) * 4u;
+            const uint8_t *p0 = wrows + (size_t)(trow0 + rb) * a.row_bytes + (size_t)seg * (kGemmSegBlocks * kGemmBlockBytes);
+            const int rows = min(32, seg_rows - trow0 - rb);
+            if (vec) {
+                p0 -= (seg & 1) * 8;
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
-                const int rb = m * 128 + quad * 32;
-                const uint32_t dst = sbase + off_w + (uint32_t)(((k & 1) * MT * 128 + rb) * kGemmRowWords) * 4u;
-                const uint8_t *p0 = wrows + (size_t)(row0 + rb) * a.row_bytes + (size_t)k * (kGemmSegBlocks * kGemmBlockBytes);
-                const int rows = min(32, seg_rows - row0 - rb);
-                if (vec) {
-                    p0 -= (k & 1) * 8;
-#pragma unroll
-                    for (int i = 0; i < 5; i++)
-                        if (t64 + 64 * i < rows * 9)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t)(t64 + 64 * i) * 16u), "l"(p0 + src[i]) : "memory");
-                } else {
-                    for (int rr = half; rr < rows; rr += 2) {
-                        const uint8_t *p = p0 + (size_t)rr * a.row_bytes;
-                        const uint32_t sh = (uint32_t)((uintptr_t)p & 2u);
-                        for (int wd = lane; wd * 4 < (int)sh + bytes; wd += 32)
-                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + (uint32_t)(rr * kGemmRowWords + wd) * 4u), "l"(p - sh + 4 * wd)
-                                         : "memory");
-                    }
+                for (int i = 0; i < 5; i++)
+                    if (t64 + 64 * i < rows * 9)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + (uint32_t)(t64 + 64 * i) * 16u), "l"(p0 + src[i]) : "memory");
+            } else {
+                for (int rr = half; rr < rows; rr += 2) {
+                    const uint8_t *p = p0 + (size_t)rr * a.row_bytes;
+                    const uint32_t sh = (uint32_t)((uintptr_t)p & 2u);
+                    for (int wd = lane; wd * 4 < (int)sh + bytes; wd += 32)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + (uint32_t)(rr * kGemmRowWords + wd) * 4u), "l"(p - sh + 4 * wd)
+                                     : "memory");
                 }
             }
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         };
-        auto quad_sync = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quad) : "memory"); };
-        stage_w(0);
+        auto quad_sync = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(1 + owner * 4 + quad) : "memory"); };
+        if (n_local > 0) stage_w(0);
 
-        float acc[MT][NH];
+        uint64_t acc[NH / 2];  // pairs of tokens
 #pragma unroll
-        for (int m = 0; m < MT; m++)
-#pragma unroll
-            for (int j = 0; j < NH; j++) acc[m][j] = 0.f;
+        for (int j = 0; j < NH / 2; j++) acc[j] = 0;
         const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
         // where a segment starts in the staged row, in bytes: see stage_w (rows start on even addresses; a row's
         // misalignment is the same in every segment, 136 bytes on)
-        uint32_t row_sh[MT];
-#pragma unroll
-        for (int m = 0; m < MT; m++) row_sh[m] = vec ? 0u : (uint32_t)((uintptr_t)(wrows + (size_t)(row0 + m * 128 + r) * a.row_bytes) & 2u);
+        const uint32_t row_sh = vec ? 0u : (uint32_t)((uintptr_t)(wrows + (size_t)(trow0 + r) * a.row_bytes) & 2u);
 
-        // this warp's half of block b of the thread's rows, from the staged words, and the block scales
-        uint32_t w[MT][4];
-        float sc0[MT];
-        auto fetch = [&](int b) {
-            const int k = b / kGemmSegBlocks;
-            if (b % kGemmSegBlocks == 0) {
+        // this warp's half of block i of the owner's segment k, from the staged words, and the block's weight scale
+        uint32_t w[4];
+        float sc_next;
+        auto fetch = [&](int k, int i) {
+            if (i == 0) {
                 asm volatile("cp.async.wait_group 0;\n" ::: "memory");
                 quad_sync();  // both warps' pieces are in, and both have left the segment before
-                if (k + 1 < n_seg) stage_w(k + 1);
+                if (k + 1 < n_local) stage_w(k + 1);
             }
+            const uint32_t *row = wst + (size_t)((k & 1) * 128 + r) * kGemmRowWords;
+            const uint32_t byte = (vec ? (uint32_t)(seg_of(k) & 1) * 8u : row_sh) + (uint32_t)i * kGemmBlockBytes;
+            sc_next = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(reinterpret_cast<const uint8_t *>(row) + byte)));
+            const uint32_t cb = byte + 2u + (uint32_t)half * 16u, cs = (cb & 2u) * 8u;
+            const uint32_t *cw = row + (cb >> 2);
+            uint32_t v[5];
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
-                const uint32_t *row = wst + (size_t)((k & 1) * MT * 128 + m * 128 + r) * kGemmRowWords;
-                const uint32_t byte = (vec ? (uint32_t)(k & 1) * 8u : row_sh[m]) + (uint32_t)(b - k * kGemmSegBlocks) * kGemmBlockBytes;
-                sc0[m] = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(reinterpret_cast<const uint8_t *>(row) + byte)));
-                const uint32_t cb = byte + 2u + (uint32_t)half * 16u, cs = (cb & 2u) * 8u;
-                const uint32_t *cw = row + (cb >> 2);
-                uint32_t v[5];
+            for (int j = 0; j < 4; j++) v[j] = cw[j];
+            v[4] = cs ? cw[4] : 0u;
 #pragma unroll
-                for (int i = 0; i < 4; i++) v[i] = cw[i];
-                v[4] = cs ? cw[4] : 0u;
-#pragma unroll
-                for (int i = 0; i < 4; i++) w[m][i] = __funnelshift_r(v[i], v[i + 1], cs);
-            }
+            for (int j = 0; j < 4; j++) w[j] = __funnelshift_r(v[j], v[j + 1], cs);
         };
-        // ... unpacked into the A stage of step s
-        auto unpack = [&](int s, int m) {
-            uint32_t regs[32];
+        // ... unpacked into the operand stage of the owner's step t.  The stage's last user is step t - 2, whose sums have been drained.
+        auto unpack = [&](int t) {
+            const uint32_t at = lane_base + kColA + (uint32_t)owner * (2 * kColsA) + (uint32_t)(t & 1) * kColsA + (uint32_t)half * 16u;
+            uint32_t one[16], wide[16];
 #pragma unroll
-            for (int i = 0; i < 4; i++) unpack16(w[m][i], regs + 8 * i);
-            tmem_st32(lane_base + kColA + (uint32_t)(s & 3) * kColsA + (uint32_t)half * 32u, regs);
+            for (int i = 0; i < 4; i++) unpack16(w[i], one + 4 * i, wide + 4 * i);
+            tmem_st16(at, one);
+            tmem_st16(at + 32u, wide);
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_af + 8 * (s & 3));
+            if (lane == 0) mbar_arrive(bar_af + 16 * owner + 8 * (t & 1));
         };
-        bool ok = true;
-        auto drain = [&](int s, float (&ac)[NH], float sc) {
-            ok = ok && wait(bar_df + 8 * (s & 1), (uint32_t)(s >> 1) & 1u);
+        bool ok = wait(bar_sc, 0);
+        auto drain = [&](int t, int b, float sc) {
+            ok = ok && wait(bar_df + 8 * owner, (uint32_t)t & 1u);
             __syncwarp();
             tc_fence_after_sync();
-            const uint32_t d = lane_base + (uint32_t)(s & 1) * kColsD + (uint32_t)half * NH;
+            const uint32_t d = lane_base + (uint32_t)owner * kColsD + (uint32_t)half * NH;
+            const uint32_t xs = sbase + off_s + (uint32_t)(b * N + half * NH) * 4u;
 #pragma unroll
-            for (int c0 = 0; c0 < NC; c0 += 4) {
-                uint32_t v[32];
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c0 + c < NC) tmem_ld8(d + 8u * (c0 + c), v + 8 * c);
+            for (int c0 = 0; c0 < NC; c0 += 2) {
+                uint32_t lo[16], hi[16];
+                if (c0 + 1 < NC) {
+                    tmem_ld16_async(d + 8u * c0, lo);
+                    tmem_ld16_async(d + kColHi + 8u * c0, hi);
+                } else {
+                    tmem_ld8(d + 8u * c0, lo);
+                    tmem_ld8(d + kColHi + 8u * c0, hi);
+                }
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (c0 + 4 >= NC) {
+                if (c0 + 2 >= NC) {
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_de + 8 * (s & 1));
+                    if (lane == 0) mbar_arrive(bar_de + 8 * owner);
                 }
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (c0 + c < NC)
+                for (int c4 = 0; c4 < 4; c4++)
+                    if (2 * c0 + c4 < 2 * NC) {
+                        const uint4 x4 = lds128(xs + 16u * (2 * c0 + c4));
+                        const uint64_t xv[2] = {(uint64_t)x4.x | (uint64_t)x4.y << 32, (uint64_t)x4.z | (uint64_t)x4.w << 32};
 #pragma unroll
-                        for (int j = 0; j < 8; j++) ac[(c0 + c) * 8 + j] = fmaf(sc, __uint_as_float(v[8 * c + j]), ac[(c0 + c) * 8 + j]);
-            }
-        };
-        // The sums so far join y and start again at zero: one running f32 sum over all blocks rounds at the size of the whole
-        // result forty times (1.4e-7 of the 2-norm against 1.0e-7).  Eight elements at a time are read back, which are the registers
-        // there are; an element belongs to one thread.  (red.add instead of the read was slower: 28 clocks a warp.)
-        // kLag iterations on, a group's last block is drained; a rest of fewer than three blocks joins the last group, with either MT.
-        constexpr int kLag = MT == 1 ? 2 : 1;
-        int next_flush = kGemmGroup + kLag;
-        bool first = true;
-        auto flush = [&](int b) {
-            if (first) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // what came before on the stream may still read y until here
-            const int t0 = tok_tile * N + half * NH, left = a.n_tok - t0;
-#pragma unroll
-            for (int m = 0; m < MT; m++) {
-                const int row = row0 + m * 128 + r;
-                if (row < seg_rows) {
-                    float *yp = a.y[sg] + (size_t)t0 * seg_rows + row;
-#pragma unroll
-                    for (int j0 = 0; j0 < NH; j0 += 8) {
-                        float old[8];
-#pragma unroll
-                        for (int j = 0; j < 8; j++) old[j] = (!first && j0 + j < left) ? __ldcg(yp + (size_t)(j0 + j) * seg_rows) : 0.f;
-#pragma unroll
-                        for (int j = 0; j < 8; j++)  // (the scale is a power of two)
-                            if (j0 + j < left) __stcg(yp + (size_t)(j0 + j) * seg_rows, fmaf(acc[m][j0 + j], __ldg(a.tok_scale + t0 + j0 + j), old[j]));
+                        for (int j = 0; j < 2; j++) {
+                            const int k = 4 * c4 + 2 * j;
+                            const uint64_t sum = fma2(int2_to_f2(hi[k], hi[k + 1]), join2(F2{16384.0f, 16384.0f}), int2_to_f2(lo[k], lo[k + 1]));
+                            acc[4 * c0 + k / 2] = fma2(mul2(join2(F2{sc, sc}), xv[j]), sum, acc[4 * c0 + k / 2]);
+                        }
                     }
-                }
-#pragma unroll
-                for (int j = 0; j < NH; j++) acc[m][j] = 0.f;
             }
-            first = false;
-            next_flush = b + kGemmGroup;
         };
-        // one iteration per block: unpack the block's steps, drain the steps of two steps ago.  An A stage is reused
-        // four steps on, after the drain of its step, which waited for its MMAs.
-        float sc1[MT] = {}, sc2 = 0.f;  // block scales of the steps that are unpacked and not yet drained
-        fetch(0);
-        for (int b = 0; b < nb; b++) {
-            if (b == next_flush && b - kLag + 3 <= nb) flush(b);
-            float now[MT];
-#pragma unroll
-            for (int m = 0; m < MT; m++) now[m] = sc0[m];
-            unpack(MT * b, 0);
-            if constexpr (MT == 2) {
-                if (b > 0) drain(2 * b - 2, acc[0], sc1[0]);
-                unpack(2 * b + 1, 1);
-                if (b + 1 < nb) fetch(b + 1);
-                if (b > 0) drain(2 * b - 1, acc[1], sc1[1]);
-                sc1[1] = now[1];
-            } else {
-                if (b + 1 < nb) fetch(b + 1);
-                if (b > 1) drain(b - 2, acc[0], sc2);
-                sc2 = sc1[0];
+        // A unit's sums join the ones before it in shared memory, in the order of the units, and leave for y after the last: one running
+        // f32 sum over all blocks would round at the size of the whole result forty times.  With one row tile the owners take turns.
+        float *tot = reinterpret_cast<float *>(sm + off_t) + (size_t)((MT == 2 ? owner * N : 0) + half * NH) * 128 + r;
+        auto flush = [&](int unit, bool last) {
+            if (MT == 1 && unit > 0) {
+                ok = ok && wait(bar_turn + 8 * (1 - owner), (uint32_t)((unit - 1) >> 1) & 1u);
+                __syncwarp();
             }
-            sc1[0] = now[0];
+            F2 v[NH / 2];
+#pragma unroll
+            for (int j = 0; j < NH / 2; j++) {
+                v[j] = split2(acc[j]);
+                acc[j] = 0;
+                if (unit > 0) v[j].x += tot[2 * j * 128], v[j].y += tot[(2 * j + 1) * 128];
+            }
+            if (!last) {
+#pragma unroll
+                for (int j = 0; j < NH / 2; j++) tot[2 * j * 128] = v[j].x, tot[(2 * j + 1) * 128] = v[j].y;
+                if (MT == 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_turn + 8 * owner);
+                }
+                return;
+            }
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");  // what came before on the stream may still read y until here
+            const int t0 = tok_tile * N + half * NH, left = a.n_tok - t0, row = trow0 + r, stride = a.y_stride[sg];
+            if (row < seg_rows) {
+                float *yp = a.y[sg] + (size_t)t0 * stride + row;
+#pragma unroll
+                for (int j = 0; j < NH; j++)
+                    if (j < left) yp[(size_t)j * stride] = j & 1 ? v[j / 2].y : v[j / 2].x;
+            }
+        };
+        // one iteration per step: the next step's operand goes out before this step's sums are awaited
+        if (n_local > 0) {
+            fetch(0, 0);
+            unpack(0);
         }
-        if constexpr (MT == 2) {
-            drain(2 * nb - 2, acc[0], sc1[0]);
-            drain(2 * nb - 1, acc[1], sc1[1]);
-        } else {
-            if (nb > 1) drain(nb - 2, acc[0], sc2);
-            drain(nb - 1, acc[0], sc1[0]);
+        float sc = n_local > 0 ? sc_next : 0.f;
+        int unit = MT == 2 ? 0 : owner;
+        for (int k = 0; k < n_local; k++) {
+            const int seg = seg_of(k), blocks = min(kGemmSegBlocks, nb - seg * kGemmSegBlocks);
+            for (int i = 0; i < blocks; i++) {
+                const int t = k * kGemmSegBlocks + i;
+                const bool more = i + 1 < blocks;
+                if (more || k + 1 < n_local) {
+                    fetch(more ? k : k + 1, more ? i + 1 : 0);
+                    unpack(t + 1);
+                }
+                drain(t, seg * kGemmSegBlocks + i, sc);
+                sc = sc_next;
+            }
+            if (unit_end[seg]) {
+                flush(unit, seg == n_seg - 1);
+                unit += 3 - MT;
+            }
         }
-        flush(nb);
     }
     tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 8) tmem_dealloc(tmem, 512);
+    __syncthreads();  // (every product and every copy has come to its end)
+    if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
 }
 
 template <int MT, int NC>
@@ -450,38 +532,53 @@ bk_status launch_gemm_nc(bk_ctx *ctx, int nc, const GemmArgs &a, dim3 grid, size
         case 1: return launch_gemm<MT, 1>(ctx, a, grid, smem);
         case 2: return launch_gemm<MT, 2>(ctx, a, grid, smem);
         case 3: return launch_gemm<MT, 3>(ctx, a, grid, smem);
-        case 4: return launch_gemm<MT, 4>(ctx, a, grid, smem);
-        case 5: return launch_gemm<MT, 5>(ctx, a, grid, smem);
-        case 6: return launch_gemm<MT, 6>(ctx, a, grid, smem);
-        case 7: return launch_gemm<MT, 7>(ctx, a, grid, smem);
-        default: return launch_gemm<MT, 8>(ctx, a, grid, smem);
+        default: return launch_gemm<MT, 4>(ctx, a, grid, smem);
     }
 }
 
 }  // namespace
 
-// Row tiles per CTA and token-tile width for a product: the pair with the least estimated time.  A step (row tile,
-// block) costs 8 clocks a token on the tensor cores, 16 with one row tile per CTA (its B blocks then come from L2 at
-// twice the rate the L2 delivers), but never less than unpacking and draining take; work goes out in rounds of one
-// CTA per SM.
-static void plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n_tok, int *mt_out, int *nc_out) {
+static size_t gemm_smem(int mt, int n, int nb, int stages) {
+    return 1024 + (size_t)stages * n * 512 + kGemmStageW + gemm_sum_bytes(mt, n) + (size_t)nb * n * sizeof(float);
+}
+static int gemm_stages(int mt, int n, int nb) {  // of B that shared memory has room for: four at most, two at least or the tile is not used
+    int stages = 4;
+    while (stages > 0 && gemm_smem(mt, n, nb, stages) > 227 * 1024) stages--;
+    return stages;
+}
+
+struct GemmPlan {
+    int mt = 1, nc = 1;
+    int64_t main_tiles = 0;  // how many of the launch's tiles of 128 mt rows; the rows of the others go to a second launch with one row tile per CTA
+};
+// Row tiles per CTA and token-tile width for a product: what has the least estimated time.  Work goes out in rounds of one CTA per SM.  A step
+// (row tile, block) takes what unpacking and draining issue, about 480 + 12 n clocks, or 700 + 11 n when two row tiles do not share a B block (L2).
+// Where two row tiles a CTA leave a last round nearly empty, its rows go out as tiles of half the size: q, k and v of 512 tokens are
+// 448 items for 148 SMs, 219 us in four rounds and 199 us as three rounds and one of half the length.
+static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n_tok) {
+    GemmPlan plan;
     double best = 1e300;
-    for (int mt = 1; mt <= 2; mt++)
-        for (int nc = 1; nc <= 8; nc++) {
-            const int n = 16 * nc;
-            if (nc > 1 && n - 16 >= n_tok) break;
-            int64_t tiles = 0;
-            for (int i = 0; i < n_seg; i++) tiles += (n_rows[i] + 128 * mt - 1) / (128 * mt);
-            const int64_t items = tiles * ((n_tok + n - 1) / n);
-            const double rounds = (double)((items + n_sms - 1) / n_sms);
-            const double step = std::max((mt == 1 ? 16.0 : 8.0) * n, 260.0 + 1.3 * n);
-            const double cost = rounds * (step * mt * nb + 4000.0);
-            if (cost < best) {
-                best = cost;
-                *mt_out = mt;
-                *nc_out = nc;
-            }
-        }
+    for (int nc = 1; nc <= 4; nc++) {
+        const int n = 16 * nc;
+        if (nc > 1 && n - 16 >= n_tok) break;
+        int64_t tiles[3] = {};
+        for (int i = 0; i < n_seg; i++)
+            for (int mt = 1; mt <= 2; mt++) tiles[mt] += (n_rows[i] + 128 * mt - 1) / (128 * mt);
+        const int64_t tok_tiles = (n_tok + n - 1) / n;
+        const double round[3] = {0.0, (700.0 + 11.0 * n) * nb + 6000.0, (480.0 + 12.0 * n) * 2 * nb + 6000.0};
+        auto rounds = [&](int64_t row_tiles) { return (double)((row_tiles * tok_tiles + n_sms - 1) / n_sms); };
+        auto take = [&](int mt, int64_t main_tiles, double cost) {
+            if (cost >= best) return;
+            best = cost;
+            plan = GemmPlan{mt, nc, main_tiles};
+        };
+        for (int mt = 1; mt <= 2; mt++)
+            if (gemm_stages(mt, n, nb) >= 2) take(mt, tiles[mt], rounds(tiles[mt]) * round[mt]);
+        const int64_t whole = tiles[2] * tok_tiles / n_sms, main_tiles = whole * n_sms / tok_tiles;
+        if (whole > 0 && main_tiles < tiles[2] && gemm_stages(2, n, nb) >= 2)
+            take(2, main_tiles, (double)whole * round[2] + rounds(2 * (tiles[2] - main_tiles)) * round[1]);
+    }
+    return plan;
 }
 
 // Up to four row ranges with the same ne0 against n_tok activations (n_tok <= kPq2GemmTokens).
@@ -497,27 +594,18 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
         if (n_rows[i] <= 0) continue;
         a.rows[used] = rows[i];
         a.y[used] = y[i];
-        rows_used[used] = a.seg_rows[used] = n_rows[i];
+        rows_used[used] = n_rows[i];
         if (((uintptr_t)rows[i] | (uintptr_t)a.row_bytes) % 16 == 0) a.vec |= 1 << used;
         used++;
     }
     if (used == 0) return BK_OK;
     const bk_status fit = pq2_rows_fit(ctx, ne0, n_tok);  // one limit for every number of tokens from two on
     if (fit != BK_OK) return fit;
-    int mt = 1, nc = 1;
-    plan_gemm(ctx->n_sms, used, rows_used, a.nb, n_tok, &mt, &nc);
-    const int n = 16 * nc, tok_tiles = (n_tok + n - 1) / n;
-    int tiles = 0;
-    for (int i = 0; i < kGemmMaxSegs; i++) {
-        a.seg_tile0[i] = tiles;
-        if (i < used) tiles += (a.seg_rows[i] + 128 * mt - 1) / (128 * mt);
-        else a.seg_tile0[i] = INT32_MAX;
-    }
-    const size_t w_bytes = (size_t)2 * mt * 128 * kGemmRowWords * 4, b_bytes = (size_t)n * 512;
-    const size_t limit = 227 * 1024;
-    a.n_stages_b = (int)std::min<size_t>(4, (limit - 1024 - w_bytes) / b_bytes);
-    // the activations' parts, one scale per padded token
-    const size_t xb_bytes = (size_t)tok_tiles * a.nb * b_bytes, need = xb_bytes + (size_t)tok_tiles * n * sizeof(float);
+    const GemmPlan plan = plan_gemm(ctx->n_sms, used, rows_used, a.nb, n_tok);
+    const int n = 16 * plan.nc, tok_tiles = (n_tok + n - 1) / n;
+    const size_t b_bytes = (size_t)n * 512, s_bytes = (size_t)a.nb * n * sizeof(float);
+    // the digits, one scale per block of every padded token
+    const size_t xb_bytes = (size_t)tok_tiles * a.nb * b_bytes, need = xb_bytes + (size_t)tok_tiles * s_bytes;
     if (ctx->pq2_x_bytes < need) {
         BK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->d_pq2_x) cudaFree(ctx->d_pq2_x);
@@ -526,11 +614,11 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
         BK_CUDA(ctx, cudaMalloc((void **)&ctx->d_pq2_x, need));
         ctx->pq2_x_bytes = need;
     }
-    float *tok_scale = reinterpret_cast<float *>(ctx->d_pq2_x + xb_bytes);
+    float *x_scale = reinterpret_cast<float *>(ctx->d_pq2_x + xb_bytes);
     a.xb = ctx->d_pq2_x;
-    a.tok_scale = tok_scale;
+    a.x_scale = x_scale;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tok_tiles * n));
+    cfg.gridDim = dim3((unsigned)(((size_t)tok_tiles * n * a.nb * 8 + 255) / 256));
     cfg.blockDim = dim3(256);
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
@@ -538,11 +626,40 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, pq2_split_x_kernel, x, ne0, a.nb, n_tok, n, ctx->d_pq2_x, tok_scale));
+    BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, pq2_split_x_kernel, x, ne0, a.nb, n_tok, n, tok_tiles * n, ctx->d_pq2_x, x_scale));
     ctx->launches++;
-    const size_t smem = 1024 + (size_t)a.n_stages_b * b_bytes + w_bytes;
-    const dim3 grid((unsigned)tiles, (unsigned)tok_tiles);
-    return mt == 1 ? launch_gemm_nc<1>(ctx, nc, a, grid, smem) : launch_gemm_nc<2>(ctx, nc, a, grid, smem);
+    // the ranges' first main_tiles tiles, then what is left of them
+    GemmArgs part[2] = {a, a};
+    int tiles[2] = {0, 0};
+    const int part_mt[2] = {plan.mt, 1};
+    int64_t left = plan.main_tiles;
+    for (int i = 0; i < kGemmMaxSegs; i++) {
+        int done = 0;
+        for (int h = 0; h < 2; h++) {
+            GemmArgs &g = part[h];
+            g.seg_tile0[i] = i < used ? tiles[h] : INT32_MAX;
+            if (i >= used) continue;
+            const int per = 128 * part_mt[h], want = rows_used[i] - done;
+            const int64_t take = h == 0 ? std::min<int64_t>((want + per - 1) / per, left) : (want + per - 1) / per;
+            g.rows[i] = a.rows[i] + (size_t)done * a.row_bytes;
+            g.y[i] = a.y[i] + done;
+            g.seg_rows[i] = (int)std::min<int64_t>(want, take * per);
+            g.y_stride[i] = rows_used[i];
+            tiles[h] += (int)take;
+            if (h == 0) left -= take;
+            done += g.seg_rows[i];
+        }
+    }
+    for (int h = 0; h < 2; h++) {
+        if (tiles[h] == 0) continue;
+        GemmArgs &g = part[h];
+        g.n_stages_b = gemm_stages(part_mt[h], n, a.nb);
+        const size_t smem = gemm_smem(part_mt[h], n, a.nb, g.n_stages_b);
+        const dim3 grid((unsigned)tiles[h], (unsigned)tok_tiles);
+        const bk_status st = part_mt[h] == 1 ? launch_gemm_nc<1>(ctx, plan.nc, g, grid, smem) : launch_gemm_nc<2>(ctx, plan.nc, g, grid, smem);
+        if (st != BK_OK) return st;
+    }
+    return BK_OK;
 }
 
 }  // namespace bk

@@ -53,6 +53,20 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
         : "memory");
 }
 
+// s8 x s8 -> s32, M = 128 (one CTA), N a multiple of 16, both operands K-major (K = 32 per instruction).
+__device__ __forceinline__ uint32_t umma_idesc_s8(int M, int N) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// D[tmem] (+)= A[tmem] . B[smem] in integers; issued by ONE thread.
+__device__ __forceinline__ void umma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+
 // True in one lane of a converged warp.  MMA and bulk-copy loops are run by a WHOLE warp with only the instruction
 // itself under this predicate: the loop state then stays in uniform registers, which the instructions take.  A loop
 // inside `if (lane == 0)` moves every operand over first and issued one MMA per 63 clocks.

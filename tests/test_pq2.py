@@ -6,6 +6,8 @@ reference ships three summation orders for this product (decoded-row dot, scalar
 and bounds their mutual difference by 1e-4 relative in its own test (src/kernels.rs:855-906);
 the norm-wise form used here is the same bound without the blow-up on outputs that cancel to ~0.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -218,3 +220,122 @@ def test_gpu_pq2_row_length_limit(bk, gpu_ctx):
         with pytest.raises(bk.BonsaiKvError, match="rows too long"):
             t.matmul_n(x[:n_tok], n_tok)
     t.free()
+
+
+def product(bk, ctx, t, x, base=0, n_rows=None, x_shift=0):
+    """The product on device buffers, with x placed x_shift floats behind a 256-byte boundary."""
+    n_tok, ne0 = x.shape
+    n_rows = t.n_rows - base if n_rows is None else n_rows
+    dx = ctx.to_device(np.concatenate([np.zeros(x_shift, np.float32), x.ravel()]))
+    dy = ctx.alloc(max(n_tok * n_rows * 4, 4))
+    t.matvec_device(dx.ptr + 4 * x_shift, dy.ptr, n_tok, base, n_rows)
+    y = dy.download((n_tok, n_rows), np.float32)
+    dx.free()
+    dy.free()
+    return y
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tok", [4, 5, 70])
+def test_gpu_pq2_blocks_of_unlike_size(bk, gpu_ctx, n_tok):
+    """A block of x a factor of 1e13 above the others, and rows whose weights there are zero: the other blocks count in full.
+    Bound: x is held to 2^-25 of its own block's largest element (about 4 times its mean size: 2^-23 of |x||w|) and the f32 sums of
+    ten blocks round by 2^-24 each: 2e-6 of sum |x||w|."""
+    rng = np.random.default_rng(n_tok)
+    _, codes, scales, x = synth(bk, 11, 200, 1280, n_tok)
+    codes[::2, :128] = 1
+    x[:, :128] *= 1e13
+    x[:, 256:512] *= 2.0 ** rng.integers(-40, 1, (n_tok, 1))
+    t = bk.Pq2Tensor(gpu_ctx, bk.pack_pq2(codes, scales), 1280)
+    w = dense(codes, scales, 1280)
+    got, x64 = product(bk, gpu_ctx, t, x), x.astype(np.float64)
+    assert np.max(np.abs(got - x64 @ w.T) / (np.abs(x64) @ np.abs(w).T)) <= 2e-6
+    t.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tok", [4, 64])
+def test_gpu_pq2_sums_are_not_biased(bk, gpu_ctx, n_tok):
+    """Products of one sign: exact block sums and sums rounded to nearest leave no mean error.  The errors of 300 x n_tok outputs are about 5e-8
+    each and cancel to 2e-9 or less; truncated sums showed 5e-8."""
+    _, _, scales, x = synth(bk, 12, 300, 5120, n_tok)
+    codes, x = np.full((300, 5120), 2, np.uint8), np.abs(x) + np.float32(0.5)
+    t = bk.Pq2Tensor(gpu_ctx, bk.pack_pq2(codes, scales), 5120)
+    truth = x.astype(np.float64) @ dense(codes, scales, 5120).T
+    assert abs(np.mean((product(bk, gpu_ctx, t, x) - truth) / truth)) <= 1e-8
+    t.free()
+
+
+@pytest.mark.gpu
+def test_gpu_pq2_zero_and_non_finite_tokens(bk, gpu_ctx):
+    """A token of zeros gives zeros, one with an infinity or a NaN in it gives NaN, and neither touches the others."""
+    payload, _, _, x = synth(bk, 13, 130, 640, 20)
+    t = bk.Pq2Tensor(gpu_ctx, payload, 640)
+    clean = product(bk, gpu_ctx, t, x)
+    x[3], x[7, 5], x[8, 639], x[9, 130] = 0, np.nan, np.inf, -np.inf
+    got = product(bk, gpu_ctx, t, x)
+    assert not got[3].any() and np.isnan(got[7:10]).all()
+    rest = [i for i in range(20) if i not in (3, 7, 8, 9)]
+    assert np.array_equal(got[rest], clean[rest])
+    t.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ne0,shift,off", [(1026, 0, 0), (1027, 0, 0), (1024, 1, 0), (1024, 2, 0), (1024, 0, 4), (1024, 3, 2), (2048, 0, 8)])
+def test_gpu_pq2_token_block_alignment(bk, gpu_ctx, ne0, shift, off):
+    """x off a 16-byte boundary, rows of an odd length, weights off 16- and 4-byte boundaries: bit for bit the aligned call's result."""
+    payload, codes, scales, x = synth(bk, 14, 150, ne0, 21)
+    t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
+    want = product(bk, gpu_ctx, t, x)
+    w, x64 = dense(codes, scales, ne0), x.astype(np.float64)
+    assert np.max(np.abs(want - x64 @ w.T) / (np.abs(x64) @ np.abs(w).T + 1e-30)) <= 2e-6  # as in the token-block test
+    moved = gpu_ctx.to_device(np.concatenate([np.zeros(off, np.uint8), payload]))
+    dx, dy = gpu_ctx.to_device(np.concatenate([np.zeros(shift, np.float32), x.ravel()])), gpu_ctx.alloc(want.nbytes)
+    gpu_ctx.check(gpu_ctx.lib.bk_pq2_matvec(gpu_ctx.h, moved.ptr + off, payload.size, ne0, 0, 150, dx.ptr + 4 * shift, 21, dy.ptr))
+    assert np.array_equal(dy.download(want.shape, np.float32), want)
+    for b in (moved, dx, dy):
+        b.free()
+    t.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb", [1, 2, 4, 5, 8, 9, 12, 13, 16, 17, 20, 33, 40])
+def test_gpu_pq2_tiling_does_not_show(bk, gpu_ctx, nb):
+    """One or two row tiles a CTA, 16 to 64 tokens a tile, rows handed to a second launch: the first tokens of a long block
+    come out bit for bit as in a short one.  14336 rows x 512 tokens take the split launch, 300 rows single row tiles."""
+    rng = np.random.default_rng(nb)
+    n_rows, ne0 = 14336 + 3, nb * 128
+    payload = rng.integers(0, 256, (n_rows, nb, 34), dtype=np.uint8)
+    payload[..., :2] = rng.uniform(0.01, 2.0, (n_rows, nb, 1)).astype(np.float16).view(np.uint8)
+    x = rng.standard_normal((512, ne0)).astype(np.float32)
+    t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
+    whole = product(bk, gpu_ctx, t, x)
+    for n_tok in (5, 40, 130):
+        assert np.array_equal(product(bk, gpu_ctx, t, x[:n_tok]), whole[:n_tok]), n_tok
+    for base in (0, 14039):
+        assert np.array_equal(product(bk, gpu_ctx, t, x[:33], base, 300), whole[:33, base:base + 300]), base
+    t.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tok", [5, 17, 200])
+def test_gpu_pq2_multi_token_block_equals_separate_calls(bk, gpu_ctx, n_tok):
+    """Ranges of odd row counts, one of them off a 16-byte boundary, in one launch: bit for bit the separate calls."""
+    ne0 = 1280
+    payload, _, _, x = synth(bk, 15, 1000, ne0, n_tok)
+    buf = gpu_ctx.to_device(np.concatenate([np.zeros(6, np.uint8), payload]))
+    dx = gpu_ctx.to_device(x)
+    ranges = [(6, 0, 333), (0, 0, 1), (6, 400, 257), (0, 0, 0)]  # (offset, base row, rows); row bytes 340, so offset 0 holds other rows
+    multi = [gpu_ctx.alloc(max(n_tok * n, 1) * 4) for _, _, n in ranges]
+    segs = (bk.pq2._Seg * len(ranges))()
+    for sg, y, (off, base, n) in zip(segs, multi, ranges):
+        sg.payload_dev, sg.payload_bytes, sg.base_row, sg.n_rows, sg.y_dev = buf.ptr + off, payload.size, base, n, y.ptr
+    gpu_ctx.check(gpu_ctx.lib.bk_pq2_matvec_multi(gpu_ctx.h, len(ranges), ctypes.cast(segs, ctypes.c_void_p), ne0, dx.ptr, n_tok))
+    for y, (off, base, n) in zip(multi, ranges):
+        if n:
+            one = gpu_ctx.alloc(n_tok * n * 4)
+            gpu_ctx.check(gpu_ctx.lib.bk_pq2_matvec(gpu_ctx.h, buf.ptr + off, payload.size, ne0, base, n, dx.ptr, n_tok, one.ptr))
+            assert np.array_equal(y.download((n_tok, n), np.float32).view(np.uint32), one.download((n_tok, n), np.float32).view(np.uint32)), (off, base)
+            one.free()
+    for b in (buf, dx, *multi):
+        b.free()
