@@ -289,6 +289,9 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
     const size_t cnt_bytes = (size_t)kCtrTotal * sizeof(unsigned);
     if ((e = cudaMalloc(&ctx->d_counters, cnt_bytes)) != cudaSuccess) return bail(e, "cudaMalloc counters");
     if ((e = cudaMemset(ctx->d_counters, 0, cnt_bytes)) != cudaSuccess) return bail(e, "clear counters");
+    const size_t run_bytes = (size_t)ctx->n_sms * kPrefillRunFloats * sizeof(float);
+    if ((e = cudaMalloc(&ctx->d_prefill_runs, run_bytes + ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc prefill sums");
+    if ((e = cudaMemset((char *)ctx->d_prefill_runs + run_bytes, 0, ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "clear prefill sums");
     {
         void *herr = nullptr, *derr = nullptr;
         if ((e = cudaHostAlloc(&herr, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) return bail(e, "cudaHostAlloc error word");
@@ -321,6 +324,7 @@ void bk_ctx_destroy(bk_ctx *ctx) {
     if (ctx->d_stage) cudaFree(ctx->d_stage);
     if (ctx->d_layer) cudaFree(ctx->d_layer);
     if (ctx->d_prefill) cudaFree(ctx->d_prefill);
+    if (ctx->d_prefill_runs) cudaFree(ctx->d_prefill_runs);
     if (ctx->d_pq2_x) cudaFree(ctx->d_pq2_x);
     if (ctx->h_desc) cudaFreeHost(ctx->h_desc);
     if (ctx->d_desc) cudaFree(ctx->d_desc);

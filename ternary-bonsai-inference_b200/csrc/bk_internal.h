@@ -50,6 +50,9 @@ struct RopeTable {
     ~RopeTable();
 };
 
+// A CTA's f32 sums in the prefill attention: 128 query rows of 256 coordinates.
+constexpr size_t kPrefillRunFloats = 128 * 256;
+
 struct HostPipe;  // pinned slots and copy threads of bulk host transfers (bk_hostpipe.cpp)
 void host_pipe_destroy(HostPipe *p);
 
@@ -82,6 +85,7 @@ struct bk_ctx {
     size_t d_layer_floats = 0;
     float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention's context chunks
     size_t d_prefill_floats = 0;
+    float *d_prefill_runs = nullptr;       // prefill attention: kPrefillRunFloats per SM, then an int per SM (taken or not)
     bk::HostPipe *pipe = nullptr;          // made by the first bulk host transfer
     uint8_t *d_pq2_x = nullptr;            // split activations of the batched PQ2_0 product, then a scale per token
     size_t pq2_x_bytes = 0;

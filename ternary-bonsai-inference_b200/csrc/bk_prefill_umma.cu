@@ -20,9 +20,9 @@
 // Tensor memory (all 512 columns): O 256 | half of q_hi 64 | S 2 x (32 + 32) | P (hi, lo) 2 x 32.  A product with N = 32 costs as
 // much as one with N = 64 (32 clocks), so q_hi meets k_hi and k_lo side by side; P and as much of q_hi as there are columns for
 // are A operands from tensor memory, which spares shared memory 4 KiB a product.
-// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.4 -> 5.6 ms, a 777-token f32 prompt in
-// one block 737 -> 302 us.  Before, one role after the other per tile with every MMA operand moved to uniform registers; the roles
-// with products of N = 32 and q fetched row by row 6.2 ms.
+// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.3 -> 5.9 ms, a 777-token f32 prompt in
+// one block 741 -> 309 us.  Before, one role after the other per tile with every MMA operand moved to uniform registers.  Without
+// the runs of collect_o 5.5 ms and 287 us.
 // Every mbarrier wait is bounded: one that runs out raises the context's error flag, the others of the CTA stop
 // waiting, and the kernel runs on to its end, where the tensor memory is always released.
 #include <cuda_fp16.h>
@@ -46,6 +46,8 @@ constexpr int kRows = 128;  // query rows per CTA = tensor-memory lanes
 constexpr int kTK = 32;     // positions per tile
 constexpr float kPScale = 64.0f, kPScaleLog2 = 6.0f;
 constexpr float kLazy = 8.0f;  // the reference moves when a row maximum exceeds it by more than this (log2 units)
+constexpr size_t kRunFloats = kPrefillRunFloats;  // a CTA's sums of the runs done, [4 coordinates][row][4]
+static_assert(kRunFloats == (size_t)kRows * kHd, "a place per row and coordinate");
 
 constexpr uint32_t kQSlab = kRows * 128, kQTile = 4 * kQSlab;  // 16 KiB per 64-coordinate slab, 64 KiB per tile
 constexpr uint32_t kKVSlab = kTK * 128, kKVTile = 4 * kKVSlab;  // 4 KiB, 16 KiB
@@ -64,6 +66,7 @@ struct SmallU {
     float mul[kRows];  // what a row's sums are multiplied by at the end
     uint32_t tmem_slot;
     int gave_up;
+    int run_slot;
 };
 constexpr uint32_t kUmmaSmem = oSmall + 3072;
 static_assert(sizeof(SmallU) <= 3072 && kUmmaSmem <= 227 * 1024, "shared memory of a CTA");
@@ -125,6 +128,9 @@ struct PrefillUArgs {
     int seq, pos0, n_tokens, tq, n_blocks, n_chunks;
     float lut_alpha;
     float *scratch;
+    float *runs;      // a place of kRunFloats per resident CTA, and which of them are taken
+    int *runs_taken;
+    int n_runs;
     int *err_flag;
 };
 
@@ -153,6 +159,8 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     // of f32 rows; beside raw V rows (several times larger than dequantized ones) the 3-bit table carries them too
     constexpr bool kLoTiles = BITS == 4 || kF32 || VF32;
 
+    constexpr int kRun = kLoTiles ? 16 : 20;  // tiles that O collects, at most, before it is added up in f32 (see collect_o)
+
     // ---- which item (as in the mma.sync kernel) ---------------------------------------------
     const int item = blockIdx.x;
     // the blocks late in the prompt see the most rows: they go first
@@ -162,6 +170,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     const int L = ((vis + pa.n_chunks - 1) / pa.n_chunks + kTK - 1) / kTK * kTK;
     const int c0 = chunk * L, c1 = min(c0 + L, vis);
     const int n_tiles = c1 > c0 ? (c1 - c0 + kTK - 1) / kTK : 0;
+    const int n_runs = (n_tiles + kRun - 1) / kRun, run_len = n_runs > 1 ? (n_tiles + n_runs - 1) / n_runs : kRun;
 
     // ---- the query rows start travelling: every row's round trip at once -----------------------------------
     const int half = a.n_rot >> 1;
@@ -198,6 +207,21 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         }
         mbar_init(bar_drain, 1);
         ss.gave_up = 0;
+        ss.run_slot = 0;
+        if (n_runs > 1) {
+            // a place for the sums: there are as many as SMs, a CTA fills an SM and gives its place back at its end, so one is free
+            uint32_t i;
+            asm("mov.u32 %0, %%smid;\n" : "=r"(i));
+            int tries = 0;
+            for (i %= (uint32_t)pa.n_runs; atomicExch(pa.runs_taken + i, 1) != 0; i = i + 1 == (uint32_t)pa.n_runs ? 0 : i + 1)
+                if (++tries > kWaitPolls) {  // (never expected)
+                    ss.gave_up = 1;
+                    raise_error(pa.err_flag, 4);
+                    break;
+                }
+            __threadfence();
+            ss.run_slot = (int)i;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) tmem_alloc(small + (uint32_t)offsetof(SmallU, tmem_slot), kTmemCols);
@@ -205,6 +229,8 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, ss.tmem_slot, 0);
+    auto run_sums = [&]() { return reinterpret_cast<float4 *>(pa.runs + (size_t)ss.run_slot * kRunFloats); };
+    float *run_mul = reinterpret_cast<float *>(sm + oQlo);  // [row], where q_lo was: the runs' factor at the end
     const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
 
     // bounded wait; after one has run out (never expected) the others of the CTA do not start to wait
@@ -371,6 +397,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             return true;
         };
         bool ok = n_tiles == 0 || issue_s(0);
+        int run_start = 0;
         for (int tile = 0; ok && tile < n_tiles; tile++) {
             // (S(tile + 1) goes where S(tile - 1) was, which the softmax had read when P(tile - 1) was awaited)
             if (tile + 1 < n_tiles && !issue_s(tile + 1)) break;
@@ -384,7 +411,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 2; kk++) {
-                    umma_f16_ts(tmem + kColO, p + 16 * kk, vd + ((kk * 2048) >> 4), idesc_o, tile > 0 || kk > 0);
+                    umma_f16_ts(tmem + kColO, p + 16 * kk, vd + ((kk * 2048) >> 4), idesc_o, tile != run_start || kk > 0);
                     umma_f16_ts(tmem + kColO, p + 16 * kk + 8, vd + ((kk * 2048) >> 4), idesc_o, true);
                     if constexpr (kLoTiles) umma_f16_ts(tmem + kColO, p + 16 * kk, vd + ((kKVTile + kk * 2048) >> 4), idesc_o, true);
                 }
@@ -392,6 +419,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 umma_commit(bar_empty + 8 * slot);
             }
             __syncwarp();
+            if (tile == run_start) run_start += run_len;
             next_slot();
         }
         // nothing in flight is left behind, whatever happened above
@@ -541,8 +569,37 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     } else {
         // ---- softmax: thread = query row ------------------------------------------------------------------------
         const int lim = my_q < n_rows ? pa.pos0 + tok0 + my_q / NREP + 1 : 0;
+        float run_R = -CUDART_INF_F;  // the reference of the sums of the runs done
+        int run_start = 0;
+        // O collects a run of tiles, joins the sums of the runs before, rounded to nearest, and starts again: its adds truncate at the
+        // size of what it holds, so its error grows with the tiles it collects.  Against float64, channels with x20 outliers: 777
+        // tokens into an f32 cache 1.36e-6 of the result (1.69e-6 without runs, 1.49e-6 with runs of up to 20 tiles), 4608 in blocks
+        // of 512 2.0e-6 (3.5e-6, 2.2e-6); V of one sign, 4608 tokens, 2.8e-6 (7.9e-6).  Without lo tiles a run may be longer: fewer
+        // products.  The sums stay in L2; a launch pays 5 us for the first and the last pass over them and 4 for each between: the
+        // 4608 tokens 6.2 -> 6.7 ms (four layers), 777 tokens 287 -> 309 us.  The same by shorter chunks: 7.1 ms and 341 us.
+        auto collect_o = [&](bool first) {
+            const float f = run_R > -CUDART_INF_F ? fast_exp2(run_R - R) : 0.f;
+            for (int b = 0; b < 8; b++) {
+                float4 *at = run_sums() + (8 * b) * kRows + my_q;
+                float4 old[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) old[j] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(at + j * kRows);
+                uint32_t o[32];
+                tmem_ld32(my_tmem + kColO + 32 * b, o);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    __stcg(at + j * kRows, make_float4(fmaf(old[j].x, f, __uint_as_float(o[4 * j])), fmaf(old[j].y, f, __uint_as_float(o[4 * j + 1])),
+                                                       fmaf(old[j].z, f, __uint_as_float(o[4 * j + 2])), fmaf(old[j].w, f, __uint_as_float(o[4 * j + 3]))));
+            }
+            run_R = R;
+        };
         for (int tile = 0; tile < n_tiles; tile++) {
             const uint32_t buf = (uint32_t)tile & 1u, par = (uint32_t)(tile >> 1) & 1u;
+            if (tile == run_start && tile > 0) {  // (the next product, which starts O again, waits for this tile's weights)
+                if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
+                tc_fence_after_sync();
+                collect_o(tile == run_len);
+            }
             bool ok = wait(bar_s + 8 * buf, par);
             if constexpr (!kRaw) ok = ok && wait(bar_norms + 8 * (tile % kNormTiles), (uint32_t)(tile / kNormTiles) & 1u);
             if (tile >= 2) ok = ok && wait(bar_o + 8 * buf, par ^ 1u);  // P of two tiles ago has been used
@@ -574,7 +631,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 const float newR = move ? mx : R;
                 const float f = (move && R > -CUDART_INF_F) ? fast_exp2(R - newR) : (move ? 0.f : 1.f);
                 lsum *= f;
-                if (tile > 0) {  // (the first product of a CTA does not add to O)
+                if (tile != run_start) {  // (the first product of a run does not add to O)
                     if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
                     tc_fence_after_sync();
                     for (int b = 0; b < 16; b++) {
@@ -612,6 +669,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 }
                 tmem_st16(my_tmem + kColP + 32 * buf + 16 * kk, pw);
             }
+            if (tile == run_start) run_start += run_len;
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
@@ -619,6 +677,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         }
         const float unscale = 1.0f / (kPScale * (kVPlanar ? pa.lut_alpha : 1.0f));  // (raw V rows carry no table scale)
         lsum *= 1.0f / kPScale;
+        if (n_runs > 1) run_mul[my_q] = run_R > -CUDART_INF_F ? fast_exp2(run_R - R) : 0.f;
         ss.mul[my_q] = pa.n_chunks == 1 ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
         if (pa.n_chunks > 1 && my_q < n_rows) {
             float *dst = pa.scratch + (((size_t)(tok0 + my_q / NREP) * a.n_head + kv * NREP + my_q % NREP) * pa.n_chunks + chunk) * (kHd + 2);
@@ -634,12 +693,22 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     // global stores of a warp cover one row's 128 bytes instead of 32 rows' 8 bytes
     if (warp < kMmaWarp) {
         const bool whole = pa.n_chunks == 1;
-        const float mul = ss.mul[my_q];
+        const float mul = ss.mul[my_q], rmul = n_runs > 1 ? run_mul[my_q] : 0.f;
         float *stg = reinterpret_cast<float *>(sm + oSlots) + warp * (32 * 33);
         const int wrow0 = (warp & 3) * 32;
         for (int b = warp >> 2; b < 8; b += 3) {
             uint32_t o[32];
             tmem_ld32(my_tmem + kColO + 32 * b, o);
+            if (n_runs > 1) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float4 x = __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
+                    o[4 * j] = __float_as_uint(fmaf(x.x, rmul, __uint_as_float(o[4 * j])));
+                    o[4 * j + 1] = __float_as_uint(fmaf(x.y, rmul, __uint_as_float(o[4 * j + 1])));
+                    o[4 * j + 2] = __float_as_uint(fmaf(x.z, rmul, __uint_as_float(o[4 * j + 2])));
+                    o[4 * j + 3] = __float_as_uint(fmaf(x.w, rmul, __uint_as_float(o[4 * j + 3])));
+                }
+            }
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
                 const int d = 32 * b + j;
@@ -666,6 +735,10 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     }
     tc_fence_before_sync();
     __syncthreads();
+    if (tid == 0 && n_runs > 1) {
+        __threadfence();
+        atomicExch(pa.runs_taken + ss.run_slot, 0);
+    }
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
@@ -796,6 +869,9 @@ bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos
     pa.err_flag = ctx->d_err;
     const int chunks = plan_chunks(ctx->n_sms, pos0, n_tokens, pa.tq, a.n_kv, a.n_head);
     pa.n_chunks = chunks;
+    pa.runs = ctx->d_prefill_runs;
+    pa.runs_taken = reinterpret_cast<int *>(ctx->d_prefill_runs + ctx->n_sms * kRunFloats);
+    pa.n_runs = ctx->n_sms;
     if (chunks > 1) {
         const size_t need = (size_t)n_tokens * a.n_head * chunks * (kHd + 2);
         if (ctx->d_prefill_floats < need) {

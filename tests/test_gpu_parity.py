@@ -1055,6 +1055,80 @@ def test_prefill_tile_edges(bk, gpu_ctx, oracle, tag, mode, bits, vq):
             assert_close(got[i], want[i], f"{tag} n={n} token {i}")
 
 
+def roped(bk, ctx, x):
+    """Vectors [n, 4 m, 256] roped at positions 0..n-1, as an f32 cache holds its K rows."""
+    n = x.shape[0]
+    cache = bk.AttnCache(ctx, bk.parse_mode("f32"), n_layers=1, n_ctx=n)
+    out = []
+    for h in range(0, x.shape[1], NKV):
+        cache.reset()
+        cache.append(0, x[:, h:h + NKV], x[:, h:h + NKV])
+        out.append(cache.dump_kv(0)["k"])
+    cache.close()
+    return np.concatenate(out, 1)
+
+
+def prefill_against_float64(bk, ctx, tag, q, k, v, block, tokens):
+    """(result, float64 attention over the rows as stored) of some tokens of a prompt that goes in block by block."""
+    n = q.shape[0]
+    cache = bk.AttnCache(ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    got = np.empty((n, NH, HD), np.float32)
+    for p in range(0, n, block):
+        cache.append(0, k[p:p + block], v[p:p + block])
+        got[p:p + block] = cache.prefill_attend(0, q[p:p + block], p)
+    d = cache.dump_kv(0)
+    cache.close()
+    if tag == "f32":
+        ks, vs = d["k"], d["v"]
+    elif tag == "f16":
+        ks, vs = d["k16"].view(np.float16), d["v16"].view(np.float16)
+    else:
+        pq = bk.PlanarQuant(HD, int(tag[6]), ctx)
+        ks = pq.dequantize(d["kq"].reshape(n * NKV, -1), d["kn"].ravel()).reshape(n, NKV, HD)
+        vs = pq.dequantize(d["vq"].reshape(n * NKV, -1), d["vn"].ravel()).reshape(n, NKV, HD)
+    qr = roped(bk, ctx, q)[tokens].astype(np.float64)
+    want = np.empty((len(tokens), NH, HD))
+    for h in range(NH):
+        s = qr[:, h] @ ks[:, h // (NH // NKV)].astype(np.float64).T / 16.0
+        s[np.arange(n)[None, :] > np.asarray(tokens)[:, None]] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want[:, h] = (w / w.sum(1, keepdims=True)) @ vs[:, h // (NH // NKV)].astype(np.float64)
+    return got[tokens].astype(np.float64), want
+
+
+@pytest.mark.parametrize("n", [480, 512, 513, 545, 641, 1030])
+@pytest.mark.parametrize("tag", ["f32", "f16", "planar4", "planar2"])
+def test_prefill_runs(bk, gpu_ctx, tag, n):
+    """Contexts around one and two runs of 16 or 20 tiles of 32 positions, whose sums are kept apart.  K grows along the prompt, and one position
+    near its end outweighs all the others for every other token, so that the rows' references move between runs and within
+    them.  Bound: scores of up to 2^6 from truncated adds, 2^-24 of them each (16 of them), as a relative error of the weights: 4e-5
+    at most, a tenth of it as a 2-norm."""
+    rng = np.random.default_rng(n)
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    k *= np.linspace(0.1, 1.0, n, dtype=np.float32)[:, None, None]
+    q[n - 8::2, :, 64:] *= 0.25
+    k[n - 30, :, 64:] = q[n - 2, ::NH // NKV, 64:] * 6.0
+    tokens = [0, 31, 32, 479, n - 9, n - 8, n - 2, n - 1]
+    got, want = prefill_against_float64(bk, gpu_ctx, tag, q, k, v, n, tokens)
+    for i, t in enumerate(tokens):
+        assert np.linalg.norm(got[i] - want[i]) <= 4e-6 * np.linalg.norm(want[i]), (t, np.linalg.norm(got[i] - want[i]) / np.linalg.norm(want[i]))
+
+
+@pytest.mark.parametrize("tag,bound", [("f32", 6e-6), ("f16", 6e-6), ("planar4", 1e-5)])
+def test_prefill_sums_of_one_sign(bk, gpu_ctx, tag, bound):
+    """V of one sign over a long context: the adds of the tensor cores truncate, but no further than a run of 512 or 640 positions.  Bound:
+    a product loses up to 2^-26 of O's binade, half of it on average, at half of O's final size: 640 * 2^-26 / 2 = 5e-6 (the 4-bit rows'
+    remainders are more products).  Collected over the whole context it would be eight times that, and was 1.2e-5 and more."""
+    rng = np.random.default_rng(5)
+    n = 4608
+    k, _ = synth_kv(rng, n, outliers=False)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    v = (1 + 0.1 * rng.standard_normal((n, NKV, HD))).astype(np.float32)
+    got, want = prefill_against_float64(bk, gpu_ctx, tag, q, k * np.float32(0.1), v, 512, list(range(n - 24, n)))
+    assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
 def test_prefill_other_group_sizes_and_long_context(bk, gpu_ctx, oracle):
     for n_head, n_kv in ((4, 4), (8, 4), (8, 2)):
         got, want = prefill_both(bk, gpu_ctx, oracle, "planar4", MODE_PLANAR, 4, True, 500, 70, seed=n_head, n_head=n_head, n_kv=n_kv)
