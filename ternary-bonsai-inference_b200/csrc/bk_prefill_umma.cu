@@ -526,8 +526,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             };
             auto live = [&](int tile) { return c0 + tile * kTK + my_row < c1; };
             auto put_k = [&](int tile) -> bool {
-                if (!slot_free()) return false;
-                __syncwarp();
+                if (!__all_sync(0xffffffffu, slot_free())) return false;  // one answer for the warp, also when a wait runs out
                 uint8_t *dst = sm + oSlots + slot * kSlotBytes;
                 if constexpr (kF32) {
                     split_store(fk, dst, dst, 64, my_row + 32, live(tile));
@@ -546,8 +545,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 return true;
             };
             auto put_v = [&](int tile) -> bool {
-                if (!slot_free()) return false;
-                __syncwarp();
+                if (!__all_sync(0xffffffffu, slot_free())) return false;  // one answer for the warp, also when a wait runs out
                 uint8_t *dst = sm + oSlots + slot * kSlotBytes;
                 if constexpr (kVRows32) {
                     split_store(fv, dst, dst + kKVTile, kTK, my_row, live(tile));
@@ -561,8 +559,8 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             };
             if (n_tiles > 0) fetch_k(0), fetch_v(0);
             bool ok = n_tiles == 0 || put_k(0);
-            for (int tile = 0; __all_sync(0xffffffffu, ok) && tile < n_tiles; tile++) {
-                if (tile + 1 < n_tiles) ok = __all_sync(0xffffffffu, put_k(tile + 1));
+            for (int tile = 0; ok && tile < n_tiles; tile++) {
+                if (tile + 1 < n_tiles) ok = put_k(tile + 1);
                 ok = ok && put_v(tile);
             }
         }
