@@ -289,6 +289,7 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
     const size_t cnt_bytes = (size_t)kCtrTotal * sizeof(unsigned);
     if ((e = cudaMalloc(&ctx->d_counters, cnt_bytes)) != cudaSuccess) return bail(e, "cudaMalloc counters");
     if ((e = cudaMemset(ctx->d_counters, 0, cnt_bytes)) != cudaSuccess) return bail(e, "clear counters");
+    if ((e = cudaMalloc(&ctx->d_pq2_x, kPq2ScratchBytes)) != cudaSuccess) return bail(e, "cudaMalloc pq2 scratch");
     const size_t run_bytes = (size_t)ctx->n_sms * kPrefillRunFloats * sizeof(float);
     if ((e = cudaMalloc(&ctx->d_prefill_runs, run_bytes + ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc prefill sums");
     if ((e = cudaMemset((char *)ctx->d_prefill_runs + run_bytes, 0, ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "clear prefill sums");
@@ -1286,7 +1287,7 @@ static bk_status pq2_check(bk_ctx *ctx, const char *who, const void *payload, si
 // the tensor-core product.
 static bk_status pq2_run_multi(bk_ctx *ctx, int n_seg, const bk_pq2_seg *segs, int64_t ne0, const float *x_dev, int32_t n_tok) {
     const size_t rb = pq2_row_bytes(ne0);
-    const int per_call = n_tok >= kPq2GemmMin ? kPq2GemmTokens : 2;
+    const int per_call = n_tok >= kPq2GemmMin ? pq2_gemm_tokens((int)ne0) : 2;
     for (int t0 = 0; t0 < n_tok; t0 += per_call) {
         const int nt = std::min(per_call, n_tok - t0);
         const uint8_t *rows[4];

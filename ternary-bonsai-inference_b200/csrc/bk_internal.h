@@ -87,8 +87,7 @@ struct bk_ctx {
     size_t d_prefill_floats = 0;
     float *d_prefill_runs = nullptr;       // prefill attention: kPrefillRunFloats per SM, then an int per SM (taken or not)
     bk::HostPipe *pipe = nullptr;          // made by the first bulk host transfer
-    uint8_t *d_pq2_x = nullptr;            // split activations of the batched PQ2_0 product, then a scale per token
-    size_t pq2_x_bytes = 0;
+    uint8_t *d_pq2_x = nullptr;            // digits and block scales of x in the token-block PQ2_0 product (kPq2ScratchBytes)
     // split-K scratch of the decode kernel: partial results and arrival counters
     float *d_partials = nullptr;
     unsigned *d_counters = nullptr;
@@ -296,10 +295,13 @@ size_t pq2_row_bytes(int64_t ne0);
 bk_status pq2_rows_fit(bk_ctx *ctx, int ne0, int n_tok);
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                             const float *x, int n_tok);
-// The same for a block of up to kPq2GemmTokens tokens on the tensor cores (bk_pq2_gemm.cu).
+// The same for a block of up to pq2_gemm_tokens() tokens on the tensor cores (bk_pq2_gemm.cu).
 // From 5 tokens on (q + k + v and output rows of a layer: 4 tokens 45 us in pairs, 52 us here; 5 tokens 62 and 52);
-// 1024 tokens a pass bound the scratch (21 MB at ne0 5120).
+// The scratch is made with the context, so that no call allocates or waits for the stream: 1024 tokens of up to 59 blocks a
+// pass, fewer of longer rows.
 constexpr int kPq2GemmTokens = 1024, kPq2GemmMin = 5;
+constexpr size_t kPq2ScratchBytes = 32 << 20;
+int pq2_gemm_tokens(int ne0);  // tokens a pass, a multiple of 64
 bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                           const float *x, int n_tok);
 // Batched causal attention of a block of prompt tokens over a 4- or 3-bit planar cache (bk_prefill.cu).

@@ -581,7 +581,14 @@ static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n
     return plan;
 }
 
-// Up to four row ranges with the same ne0 against n_tok activations (n_tok <= kPq2GemmTokens).
+// A token has 512 bytes of digits and a scale a block; a tile is filled up with up to 63 tokens of zeros.
+static constexpr size_t kXBytes = 512 + sizeof(float);
+int pq2_gemm_tokens(int ne0) {
+    const int64_t nb = ((int64_t)ne0 + kGemmBlock - 1) / kGemmBlock, room = (int64_t)(kPq2ScratchBytes / (nb * kXBytes)) - 63;
+    return (int)std::max<int64_t>(64, std::min<int64_t>(kPq2GemmTokens, room / 64 * 64));  // (rows that leave fewer are refused)
+}
+
+// Up to four row ranges with the same ne0 against n_tok activations (n_tok <= pq2_gemm_tokens(ne0)).
 bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0, const float *x,
                           int n_tok) {
     GemmArgs a{};
@@ -604,16 +611,9 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
     const GemmPlan plan = plan_gemm(ctx->n_sms, used, rows_used, a.nb, n_tok);
     const int n = 16 * plan.nc, tok_tiles = (n_tok + n - 1) / n;
     const size_t b_bytes = (size_t)n * 512, s_bytes = (size_t)a.nb * n * sizeof(float);
-    // the digits, one scale per block of every padded token
-    const size_t xb_bytes = (size_t)tok_tiles * a.nb * b_bytes, need = xb_bytes + (size_t)tok_tiles * s_bytes;
-    if (ctx->pq2_x_bytes < need) {
-        BK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (ctx->d_pq2_x) cudaFree(ctx->d_pq2_x);
-        ctx->d_pq2_x = nullptr;
-        ctx->pq2_x_bytes = 0;
-        BK_CUDA(ctx, cudaMalloc((void **)&ctx->d_pq2_x, need));
-        ctx->pq2_x_bytes = need;
-    }
+    // the digits, then one scale per block of every padded token
+    const size_t xb_bytes = (size_t)tok_tiles * a.nb * b_bytes;
+    if (xb_bytes + (size_t)tok_tiles * s_bytes > kPq2ScratchBytes) return fail(ctx, BK_ERR_UNSUPPORTED, "pq2_matvec: more tokens than a pass takes");
     float *x_scale = reinterpret_cast<float *>(ctx->d_pq2_x + xb_bytes);
     a.xb = ctx->d_pq2_x;
     a.x_scale = x_scale;

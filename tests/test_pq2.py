@@ -339,3 +339,28 @@ def test_gpu_pq2_multi_token_block_equals_separate_calls(bk, gpu_ctx, n_tok):
             one.free()
     for b in (buf, dx, *multi):
         b.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tok", [2, 5, 100])
+def test_gpu_pq2_first_call_can_be_captured(bk, n_tok):
+    """The first product of a context goes into a CUDA graph: no call allocates or waits for the stream."""
+    import torch
+    ctx = bk.Context(0)
+    payload, _, _, x = synth(bk, 16, 300, 640, n_tok)
+    t = bk.Pq2Tensor(ctx, payload, 640)
+    dx, dy = ctx.to_device(x), ctx.to_device(np.zeros((n_tok, 300), np.float32))
+    ctx.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    stream = torch.cuda.ExternalStream(ctx.lib.bk_ctx_stream(ctx.h))
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        t.matvec_device(dx.ptr, dy.ptr, n_tok)
+    with torch.cuda.stream(stream):
+        graph.replay()
+    ctx.synchronize()
+    assert np.array_equal(dy.download((n_tok, 300), np.float32), product(bk, ctx, t, x))
+    del graph
+    t.free()
+    dx.free()
+    dy.free()
+    ctx.close()
