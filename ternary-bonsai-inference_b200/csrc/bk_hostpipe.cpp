@@ -74,11 +74,9 @@ struct HostPipe {
             busy.fetch_sub(1, std::memory_order_release);
             return;
         }
-        if (t.after) {
-            const cudaError_t e = cudaEventSynchronize(t.after);
-            if (e != cudaSuccess) err.store((int)e);
-        }
-        if (t.to_slot) copy_streaming(t.dst, t.src, t.n);
+        const cudaError_t e = t.after ? cudaEventSynchronize(t.after) : cudaSuccess;
+        if (e != cudaSuccess) err.store((int)e);  // (what the slot holds is an earlier transfer's)
+        else if (t.to_slot) copy_streaming(t.dst, t.src, t.n);
         else memcpy(t.dst, t.src, t.n);
         t.done->store(1, std::memory_order_release);
         busy.fetch_sub(1, std::memory_order_release);
@@ -217,11 +215,24 @@ static bool is_pinned(const void *host) {
     return yes;
 }
 
-bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
-    if (n_seg > 0 && is_pinned(segs[0].host)) {
-        for (size_t i = 0; i < n_seg; i++) BK_CUDA(ctx, cudaMemcpyAsync(segs[i].host, segs[i].dev, segs[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        return sync_and_check(ctx);
+// After an error: the copies that did go out still read or write the caller's memory and the slots.
+static bk_status give_up(bk_ctx *ctx, cudaError_t e, const char *what) {
+    cudaStreamSynchronize(ctx->stream);
+    return cuda_fail(ctx, e, what);
+}
+
+// Without slots.
+static bk_status copy_direct(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, bool to_host) {
+    for (size_t i = 0; i < n_seg; i++) {
+        const cudaError_t e = to_host ? cudaMemcpyAsync(segs[i].host, segs[i].dev, segs[i].bytes, cudaMemcpyDeviceToHost, ctx->stream)
+                                      : cudaMemcpyAsync(segs[i].dev, segs[i].host, segs[i].bytes, cudaMemcpyHostToDevice, ctx->stream);
+        if (e != cudaSuccess) return give_up(ctx, e, to_host ? "copy to the host" : "copy to the device");
     }
+    return sync_and_check(ctx);
+}
+
+bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
+    if (n_seg > 0 && is_pinned(segs[0].host)) return copy_direct(ctx, segs, n_seg, true);
     HostPipe *p;
     bk_status st = get_pipe(ctx, &p);
     if (st != BK_OK) return st;
@@ -237,10 +248,9 @@ bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
     }
     cudaError_t e = cudaSuccess;
     size_t i = 0;
-    for (; i < pieces.size() && e == cudaSuccess; i++) {
+    for (; i < pieces.size(); i++) {
         const int s = (int)(i % kSlots);
         if (i >= kSlots) p->finish(s);
-        p->done[s].store(0);
         char *at = p->slot(s);
         for (size_t k = 0; k < pieces[i].count && e == cudaSuccess; k++) {
             const Part &pt = parts[pieces[i].first + k];
@@ -248,26 +258,19 @@ bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
             at += pt.n;
         }
         if (e == cudaSuccess) e = cudaEventRecord(p->ev[s], ctx->stream);
+        if (e != cudaSuccess) break;
+        p->done[s].store(0);
         p->push(HostPipe::Task{pieces[i].host, p->slot(s), pieces[i].n, p->ev[s], false, &p->done[s]});
     }
     for (size_t k = i > kSlots ? i - kSlots : 0; k < i; k++) p->finish((int)(k % kSlots));
     p->drain();
-    if (e == cudaSuccess) e = (cudaError_t)p->err.exchange(0);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "copy to the host");
-    return sync_and_check(ctx);
+    const cudaError_t helper = (cudaError_t)p->err.exchange(0);
+    if (e == cudaSuccess) e = helper;
+    return e != cudaSuccess ? give_up(ctx, e, "copy to the host") : sync_and_check(ctx);
 }
 
-bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, const std::function<bk_status(size_t)> &arrived) {
-    if (n_seg > 0 && is_pinned(segs[0].host)) {
-        size_t bytes = 0;
-        for (size_t i = 0; i < n_seg; i++) {
-            BK_CUDA(ctx, cudaMemcpyAsync(segs[i].dev, segs[i].host, segs[i].bytes, cudaMemcpyHostToDevice, ctx->stream));
-            bytes += segs[i].bytes;
-            const bk_status st = arrived ? arrived(bytes) : BK_OK;
-            if (st != BK_OK) return st;
-        }
-        return sync_and_check(ctx);
-    }
+bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
+    if (n_seg > 0 && is_pinned(segs[0].host)) return copy_direct(ctx, segs, n_seg, false);
     HostPipe *p;
     bk_status st = get_pipe(ctx, &p);
     if (st != BK_OK) return st;
@@ -275,8 +278,8 @@ bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, const st
     std::vector<Part> parts;
     if (!cut(segs, n_seg, pieces, parts)) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
     cudaError_t e = cudaSuccess;
-    size_t pushed = 0, issued = 0, bytes = 0;
-    while (issued < pieces.size() && e == cudaSuccess && st == BK_OK) {
+    size_t pushed = 0, issued = 0;
+    while (issued < pieces.size() && e == cudaSuccess) {
         for (; pushed < pieces.size() && pushed - issued < kSlots && e == cudaSuccess; pushed++) {
             const int s = (int)(pushed % kSlots);
             if (pushed >= kSlots) {  // the slot's last copy to the device
@@ -298,16 +301,12 @@ bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, const st
             at += pt.n;
         }
         if (e == cudaSuccess) e = cudaEventRecord(p->ev[s], ctx->stream);
-        bytes += pieces[issued].n;
         issued++;
-        if (e == cudaSuccess && arrived) st = arrived(bytes);
     }
     for (; issued < pushed; issued++) p->finish((int)(issued % kSlots));  // (after an error)
     // the slots are the next transfer's: they must be read by then
-    cudaError_t e2 = cudaEventSynchronize(p->ev[(pieces.size() + kSlots - 1) % kSlots]);
-    if (e == cudaSuccess && !pieces.empty()) e = e2;
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "copy to the device");
-    return st;
+    if (e == cudaSuccess && !pieces.empty()) e = cudaEventSynchronize(p->ev[(pieces.size() - 1) % kSlots]);
+    return e != cudaSuccess ? give_up(ctx, e, "copy to the device") : BK_OK;
 }
 
 }  // namespace bk

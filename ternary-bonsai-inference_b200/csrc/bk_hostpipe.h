@@ -1,8 +1,6 @@
 // Bulk transfers between pageable caller memory and the device (bk_hostpipe.cpp).
 #pragma once
 
-#include <functional>
-
 #include "bk_internal.h"
 
 namespace bk {
@@ -18,8 +16,7 @@ constexpr size_t kHostPipeMin = 256 << 10;
 // The ranges, in order, after what is on the stream; returns when the bytes are in host memory (and checks the
 // context's error word).
 bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg);
-// The ranges, in order, on the stream; returns when the caller's memory has been read and the copies are through.  `arrived`
-// (optional) is called with the bytes issued so far after each piece, to enqueue work on them.
-bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg, const std::function<bk_status(size_t)> &arrived = nullptr);
+// The ranges, in order, on the stream; returns when the caller's memory has been read and the copies are through.
+bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg);
 
 }  // namespace bk
