@@ -14,6 +14,7 @@
 #include <deque>
 #include <mutex>
 #include <new>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -150,10 +151,22 @@ void host_pipe_destroy(HostPipe *p) {
     delete p;
 }
 
+bk_status out_of_memory(bk_ctx *ctx, const char *who) noexcept {
+    try {
+        return fail(ctx, BK_ERR_OOM, std::string(who) + ": host allocation failed");
+    } catch (...) {
+        return BK_ERR_OOM;
+    }
+}
+
 static bk_status get_pipe(bk_ctx *ctx, HostPipe **out) {
     if (!ctx->pipe) {
-        HostPipe *p = new (std::nothrow) HostPipe();
-        if (!p) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
+        HostPipe *p;
+        try {
+            p = new HostPipe();  // (its queue allocates as well)
+        } catch (const std::bad_alloc &) {
+            return out_of_memory(ctx, "host pipe");
+        }
         p->device = ctx->device;
         cudaError_t e = cudaMallocHost((void **)&p->mem, kSlots * kSlotBytes);
         for (int i = 0; i < kSlots && e == cudaSuccess; i++) e = cudaEventCreateWithFlags(&p->ev[i], cudaEventDisableTiming);
@@ -238,7 +251,7 @@ bk_status host_pipe_d2h(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
     if (st != BK_OK) return st;
     std::vector<Piece> pieces;
     std::vector<Part> parts;
-    if (!cut(segs, n_seg, pieces, parts)) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
+    if (!cut(segs, n_seg, pieces, parts)) return out_of_memory(ctx, "host pipe");
     // A fresh destination: fault its huge pages in on different threads first.  Copies of neighbouring pieces would fault on the
     // same page at once, and each clears 2 MB for it.
     for (size_t k = 0; k < pieces.size(); k++) {
@@ -276,7 +289,7 @@ bk_status host_pipe_h2d(bk_ctx *ctx, const HostSeg *segs, size_t n_seg) {
     if (st != BK_OK) return st;
     std::vector<Piece> pieces;
     std::vector<Part> parts;
-    if (!cut(segs, n_seg, pieces, parts)) return fail(ctx, BK_ERR_OOM, "host pipe: allocation failed");
+    if (!cut(segs, n_seg, pieces, parts)) return out_of_memory(ctx, "host pipe");
     cudaError_t e = cudaSuccess;
     size_t pushed = 0, issued = 0;
     while (issued < pieces.size() && e == cudaSuccess) {

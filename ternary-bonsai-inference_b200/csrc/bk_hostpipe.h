@@ -10,6 +10,9 @@ struct HostSeg {
     void *dev;
     size_t bytes;
 };
+// BK_ERR_OOM with the name of who ran out; the message is dropped when there is no memory for it either.
+bk_status out_of_memory(bk_ctx *ctx, const char *who) noexcept;
+
 // Transfers of less than this are not worth the hand-over to other threads.
 constexpr size_t kHostPipeMin = 256 << 10;
 

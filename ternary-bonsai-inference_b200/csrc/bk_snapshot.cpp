@@ -15,6 +15,7 @@
 #include <sys/mman.h>
 
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -68,7 +69,7 @@ size_t bk_cache_snapshot_bytes(const bk_cache *c, int32_t seq) {
     return total;
 }
 
-bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void *buf, size_t buf_bytes, size_t *written) {
+bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void *buf, size_t buf_bytes, size_t *written) try {
     using namespace bk;
     if (!c) return fail(nullptr, BK_ERR_INVALID, "bk_cache_snapshot_save: cache is null");
     bk_ctx *ctx = c->ctx;
@@ -135,9 +136,11 @@ bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void 
     }
     if (written) *written = off;
     return BK_OK;
+} catch (const std::bad_alloc &) {
+    return bk::out_of_memory(c->ctx, "bk_cache_snapshot_save");
 }
 
-bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size_t buf_bytes) {
+bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size_t buf_bytes) try {
     using namespace bk;
     if (!c) return fail(nullptr, BK_ERR_INVALID, "bk_cache_snapshot_load: cache is null");
     bk_ctx *ctx = c->ctx;
@@ -211,6 +214,8 @@ bk_status bk_cache_snapshot_load(bk_cache *c, int32_t seq, const void *buf, size
         if (st != BK_OK) return st;
     }
     return BK_OK;
+} catch (const std::bad_alloc &) {
+    return bk::out_of_memory(c->ctx, "bk_cache_snapshot_load");
 }
 
 }  // extern "C"

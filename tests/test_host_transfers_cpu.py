@@ -102,3 +102,50 @@ def test_failed_copy_of_pinned_memory_leaves_nothing_in_flight(fake, ctx, to_hos
     plan(fake, copy=2)
     assert transfer(fake, ctx, to_host, host, dev, [1000, 2000, 3000]) == BK_ERR_CUDA
     assert fake.fake_in_flight() == 0
+
+
+def caches(fake, ctx, n_pos, n_ctx, bits=4):
+    """Two caches of the same geometry with other contents; positions per layer of sequence 0."""
+    n = (C.c_int * len(n_pos))(*n_pos)
+    return [C.c_void_p(fake.fake_cache(ctx, len(n_pos), 2, n_ctx, bits, n, seed)) for seed in (1, 2)]
+
+
+def save(fake, cache, seq, layout):
+    n = fake.bk_cache_snapshot_bytes(cache, seq)
+    buf, written = np.zeros(n, np.uint8), C.c_size_t(0)
+    assert fake.bk_cache_snapshot_save(cache, seq, layout, C.c_void_p(buf.ctypes.data), C.c_size_t(n), C.byref(written)) == 0 and written.value == n
+    return buf
+
+
+@pytest.mark.parametrize("n_pos", [[7000, 0, 1, 9000, 257, 0], [0, 0], [40000]])
+def test_snapshot_of_unequal_layers(fake, ctx, n_pos):
+    """Snapshots of up to 20 MB with empty and short layers: the rows come back into another cache, and the row-by-row layout
+    that does not use the bulk transfer agrees."""
+    a, b = caches(fake, ctx, n_pos, 40000 if len(n_pos) == 1 else 9000)
+    blob, rows = save(fake, a, 0, 0), save(fake, a, 0, 1)
+    assert fake.bk_cache_snapshot_load(b, 1, C.c_void_p(blob.ctypes.data), C.c_size_t(blob.size)) == 0
+    assert [fake.fake_n_pos(b, il, 1) for il in range(len(n_pos))] == n_pos
+    assert np.array_equal(save(fake, b, 1, 0), blob) and np.array_equal(save(fake, b, 1, 1), rows)
+    for c in (a, b):
+        fake.fake_cache_free(c)
+
+
+def test_snapshot_without_memory_for_its_lists(fake, ctx):
+    """Whichever allocation of a save or a load fails, the call says so; no exception passes the C boundary."""
+    a, b = caches(fake, ctx, [3000] * 9, 3000)
+    for layout in (0, 1):
+        blob = save(fake, a, 0, layout)
+        for call in (lambda: fake.bk_cache_snapshot_save(a, 0, layout, C.c_void_p(blob.ctypes.data), C.c_size_t(blob.size), None),
+                     lambda: fake.bk_cache_snapshot_load(b, 0, C.c_void_p(blob.ctypes.data), C.c_size_t(blob.size))):
+            failed = 0
+            for k in range(200):
+                plan(fake, alloc=k)
+                st = call()
+                plan(fake)
+                assert st in (0, BK_ERR_OOM), (layout, k, st)
+                failed += st != 0
+                if st == 0:
+                    break
+            assert st == 0 and failed > 0
+    for c in (a, b):
+        fake.fake_cache_free(c)
