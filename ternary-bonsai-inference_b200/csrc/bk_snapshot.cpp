@@ -12,8 +12,6 @@
 // n_layers, n_kv, hd, reserved[3]; then n_layers words with the number of cached positions of
 // each layer; then the layers' payloads.  Everything is host code over bk_cache_download /
 // bk_cache_upload; the file or socket that carries the buffer is the caller's.
-#include <sys/mman.h>
-
 #include <cstring>
 #include <new>
 #include <string>
@@ -93,10 +91,6 @@ bk_status bk_cache_snapshot_save(bk_cache *c, int32_t seq, int32_t layout, void 
     }
     const Side sides[2] = {{c->k_kind, c->k_row_bytes}, {c->v_kind, c->v_row_bytes}};
     if (layout == 0) {  // every range goes where it lies in the buffer: one transfer for all layers
-        // A fresh buffer of this size costs more in page faults than in copying: ask for huge pages where it can have them.
-        constexpr uintptr_t kHuge = 2 << 20;
-        const uintptr_t lo = ((uintptr_t)buf + kHuge - 1) & ~(kHuge - 1), hi = ((uintptr_t)buf + need) & ~(kHuge - 1);
-        if (hi > lo) (void)madvise((void *)lo, hi - lo, MADV_HUGEPAGE);
         std::vector<HostSeg> segs = all_ranges(c, seq, out + off, [&](int l) { return c->n_pos[c->slab(l, seq)]; });
         bk_status st = bind_device(ctx);
         if (st == BK_OK && !segs.empty()) st = host_pipe_d2h(ctx, segs.data(), segs.size());

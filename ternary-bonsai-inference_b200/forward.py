@@ -34,6 +34,20 @@ _new_bytes = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(("PyBytes_FromSt
 _bytes_at = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
 
 
+_madvise = getattr(C.CDLL(None), "madvise", None)
+_HUGE_PAGE, _MADV_HUGEPAGE = 2 << 20, 14
+
+
+def _new_large_bytes(n):
+    """_new_bytes(None, n) that asks for huge pages: filling a fresh buffer of megabytes costs more in page faults than in copying."""
+    blob = _new_bytes(None, n)
+    lo = -(-_bytes_at(blob) // _HUGE_PAGE) * _HUGE_PAGE
+    hi = (_bytes_at(blob) + n) // _HUGE_PAGE * _HUGE_PAGE
+    if _madvise is not None and hi > lo:
+        _madvise(C.c_void_p(lo), C.c_size_t(hi - lo), _MADV_HUGEPAGE)
+    return blob
+
+
 class AttnCache:
     """Device KV cache of the full-attention layers (K roped, V raw)."""
 
@@ -168,7 +182,7 @@ class AttnCache:
     def snapshot(self, seq=0, layout=0):
         """All layers of one sequence as bytes (layout 0: the reference's CPU stores, 1: its device rows)."""
         n = self.ctx.lib.bk_cache_snapshot_bytes(self.h, seq)
-        blob = _new_bytes(None, n)  # written once, by the library, before anybody else sees it
+        blob = _new_large_bytes(n)  # written once, by the library, before anybody else sees it
         written = C.c_size_t(0)
         self.ctx.check(self.ctx.lib.bk_cache_snapshot_save(self.h, seq, layout, _bytes_at(blob), n, C.byref(written)))
         return blob if written.value == n else blob[:written.value]

@@ -21,7 +21,7 @@ struct Op {
 };
 std::recursive_mutex mu;
 std::deque<Op> queue;
-long n_copies, n_syncs, fail_copy = -1, fail_sync = -1, fail_new = -1;
+long n_copies, n_syncs, n_advice, fail_copy = -1, fail_sync = -1, fail_new = -1;
 std::thread::id new_thread;
 std::vector<std::pair<const char *, size_t>> pinned;
 struct Event {
@@ -46,6 +46,7 @@ void operator delete(void *p) noexcept { free(p); }
 void operator delete(void *p, size_t) noexcept { free(p); }
 
 extern "C" {
+int madvise(void *, size_t, int) { return n_advice++, 0; }
 cudaError_t cudaMallocHost(void **p, size_t n) { return *p = malloc(n), memset(*p, 0xee, n), cudaSuccess; }
 cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
@@ -129,6 +130,7 @@ __attribute__((visibility("default"))) void fake_plan(long copy, long sync, long
     fail_copy = copy, fail_sync = sync, fail_new = alloc;
     new_thread = std::this_thread::get_id();
 }
+__attribute__((visibility("default"))) long fake_advice() { return n_advice; }
 __attribute__((visibility("default"))) void fake_pin(const void *p, size_t n) { pinned.emplace_back((const char *)p, n); }
 __attribute__((visibility("default"))) long fake_in_flight() {
     std::lock_guard<std::recursive_mutex> lk(mu);

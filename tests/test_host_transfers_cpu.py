@@ -22,7 +22,7 @@ def fake(tmp_path_factory):
                     os.path.join(CSRC, "bk_hostpipe.cpp"), os.path.join(CSRC, "bk_snapshot.cpp"), "-o", so], check=True)
     lib = C.CDLL(so)
     lib.fake_ctx.restype = lib.fake_cache.restype = C.c_void_p
-    lib.fake_in_flight.restype = C.c_long
+    lib.fake_in_flight.restype = lib.fake_advice.restype = C.c_long
     lib.bk_cache_snapshot_bytes.restype = C.c_size_t
     return lib
 
@@ -126,6 +126,7 @@ def test_snapshot_of_unequal_layers(fake, ctx, n_pos):
     assert fake.bk_cache_snapshot_load(b, 1, C.c_void_p(blob.ctypes.data), C.c_size_t(blob.size)) == 0
     assert [fake.fake_n_pos(b, il, 1) for il in range(len(n_pos))] == n_pos
     assert np.array_equal(save(fake, b, 1, 0), blob) and np.array_equal(save(fake, b, 1, 1), rows)
+    assert fake.fake_advice() == 0  # the buffers are the caller's: how they are paged is not the library's business
     for c in (a, b):
         fake.fake_cache_free(c)
 
