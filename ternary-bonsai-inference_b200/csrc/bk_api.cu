@@ -119,19 +119,27 @@ RopeTable::~RopeTable() {
     }
 }
 
-bk_status ensure_stage(bk_ctx *ctx, size_t bytes) {
-    if (bytes <= ctx->h_stage_bytes && bytes <= ctx->d_stage_bytes) return BK_OK;
+bk_status ensure_stage(bk_ctx *ctx, size_t bytes, bool host) {
+    host = host && bytes > ctx->h_stage_bytes;
+    const bool dev = bytes > ctx->d_stage_bytes;
+    if (!host && !dev) return BK_OK;
     BK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     size_t want = std::max<size_t>(bytes, 1 << 20);
     want = (want + 255) & ~(size_t)255;
-    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
-    if (ctx->d_stage) cudaFree(ctx->d_stage);
-    ctx->h_stage = ctx->d_stage = nullptr;
-    ctx->h_stage_bytes = ctx->d_stage_bytes = 0;
-    BK_CUDA(ctx, cudaMallocHost(&ctx->h_stage, want));
-    ctx->h_stage_bytes = want;
-    BK_CUDA(ctx, cudaMalloc(&ctx->d_stage, want));
-    ctx->d_stage_bytes = want;
+    if (host) {
+        if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+        ctx->h_stage = nullptr;
+        ctx->h_stage_bytes = 0;
+        BK_CUDA(ctx, cudaMallocHost(&ctx->h_stage, want));
+        ctx->h_stage_bytes = want;
+    }
+    if (dev) {
+        if (ctx->d_stage) cudaFree(ctx->d_stage);
+        ctx->d_stage = nullptr;
+        ctx->d_stage_bytes = 0;
+        BK_CUDA(ctx, cudaMalloc(&ctx->d_stage, want));
+        ctx->d_stage_bytes = want;
+    }
     return BK_OK;
 }
 
@@ -665,7 +673,7 @@ bk_status bk_append_host(bk_cache *c, int32_t layer, int32_t seq, int32_t rope_p
     bk_status st = bind(ctx);
     if (st != BK_OK) return st;
     const size_t per = (size_t)n_tokens * c->cfg.n_kv * kHd * sizeof(float);
-    if ((st = ensure_stage(ctx, 2 * per)) != BK_OK) return st;
+    if ((st = ensure_stage(ctx, 2 * per, 2 * per < kHostPipeMin)) != BK_OK) return st;
     if (2 * per >= kHostPipeMin) {
         const HostSeg in[2] = {{const_cast<float *>(k_host), ctx->d_stage, per}, {const_cast<float *>(v_host), (char *)ctx->d_stage + per, per}};
         if ((st = host_pipe_h2d(ctx, in, 2)) != BK_OK) return st;
@@ -1463,7 +1471,7 @@ bk_status bk_kvq_quantize(bk_ctx *ctx, int32_t hd, int32_t bits, int32_t n_vec, 
     const size_t xb = (size_t)n_vec * hd * 4, pb = (size_t)n_vec * 32 * bits, nb = (size_t)n_vec * 4;
     HostIo io{ctx};
     const size_t ox = io.take(xb), op = io.take(pb), on = io.take(nb);
-    if ((st = ensure_stage(ctx, io.used)) != BK_OK) return st;
+    if ((st = ensure_stage(ctx, io.used, xb < kHostPipeMin)) != BK_OK) return st;
     char *h = (char *)ctx->h_stage, *d = (char *)ctx->d_stage;
     if (xb >= kHostPipeMin) {
         const HostSeg in{const_cast<float *>(x), d + ox, xb};
@@ -1495,7 +1503,7 @@ bk_status bk_kvq_dequantize(bk_ctx *ctx, int32_t hd, int32_t bits, int32_t n_vec
     const size_t xb = (size_t)n_vec * hd * 4, pb = (size_t)n_vec * 32 * bits, nb = (size_t)n_vec * 4;
     HostIo io{ctx};
     const size_t op = io.take(pb), on = io.take(nb), ox = io.take(xb);
-    if ((st = ensure_stage(ctx, io.used)) != BK_OK) return st;
+    if ((st = ensure_stage(ctx, io.used, xb < kHostPipeMin)) != BK_OK) return st;
     char *h = (char *)ctx->h_stage, *d = (char *)ctx->d_stage;
     if (xb >= kHostPipeMin) {
         const HostSeg in[2] = {{const_cast<uint8_t *>(packed), d + op, pb}, {const_cast<float *>(norms), d + on, nb}};

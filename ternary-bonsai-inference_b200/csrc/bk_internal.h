@@ -162,7 +162,8 @@ bk_status cuda_fail(bk_ctx *ctx, cudaError_t e, const char *what);
         if (e__ != cudaSuccess) return bk::cuda_fail((ctx), e__, #call); \
     } while (0)
 
-bk_status ensure_stage(bk_ctx *ctx, size_t bytes);
+// Staging of at least `bytes` on the device and, unless the call moves its data through the host pipe, in pinned memory.
+bk_status ensure_stage(bk_ctx *ctx, size_t bytes, bool host = true);
 // Wait for the context's stream, then look at the error word the kernels raise when a bounded wait runs
 // out: BK_ERR_CUDA (and the word and the split-K counters cleared) if one did.
 bk_status sync_and_check(bk_ctx *ctx);

@@ -10,15 +10,13 @@
 //   MN-major, 128-byte swizzle: the same bytes read the other way: a slab holds 64 MN-elements
 //     (128 bytes) per K-row, K-rows 128 bytes apart, 8-row groups 1024 bytes apart (stride byte
 //     offset), the next 64 MN-elements one slab further (leading byte offset = slab bytes).
-//   K-major, no swizzle: core matrices of 8 rows x 16 bytes, contiguous; row groups `sbo` bytes
-//     apart, the two 8-element K halves of a K-step `lbo` bytes apart.
 #pragma once
 
 #include <stdint.h>
 
 namespace bk {
 
-constexpr uint32_t kUmmaSwizzleNone = 0, kUmmaSwizzle128 = 2;
+constexpr uint32_t kUmmaSwizzle128 = 2;
 
 __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
     uint64_t d = 0;
