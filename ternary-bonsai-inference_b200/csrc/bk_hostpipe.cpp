@@ -5,7 +5,9 @@
 // page faults of a fresh destination on top (0.25 us per 4 KB page), so a 34.6 MB snapshot as pageable copies moved
 // 1.2 GB/s per direction; with the copies cut into 512 KB pieces and spread over the threads it takes 1.6 ms out and 1.2 ms
 // back in (28 ms before), a quantize call of 8192 vectors 0.42 ms (1.0 ms before).
+#ifdef __SSE2__
 #include <emmintrin.h>
+#endif
 #include <string.h>
 
 #include <algorithm>
@@ -27,6 +29,9 @@ constexpr int kSlots = 16;
 constexpr size_t kSlotBytes = 512 << 10;
 constexpr int kMaxThreads = 6;
 
+#ifdef __SSE2__
+inline void relax() { _mm_pause(); }
+
 // Into a pinned slot the copy engine reads next: past the caches.  Lines that other cores hold dirty are fetched from
 // them one by one, which held the engine to 4.5 GB/s on slots written with ordinary stores (52 GB/s from memory).
 void copy_streaming(void *dst, const void *src, size_t n) {
@@ -44,6 +49,10 @@ void copy_streaming(void *dst, const void *src, size_t n) {
     while (n--) *d++ = *s++;
     _mm_sfence();
 }
+#else
+inline void relax() { std::this_thread::yield(); }
+void copy_streaming(void *dst, const void *src, size_t n) { memcpy(dst, src, n); }
+#endif
 }  // namespace
 
 // Owned by one context and used by one thread at a time, like the context; the helpers end with it.
@@ -95,7 +104,7 @@ struct HostPipe {
         for (;;) {
             Task t;
             // the next task of a running transfer follows within microseconds: look for it before going to sleep
-            for (int i = 0; i < 2000 && waiting.load(std::memory_order_relaxed) == 0; i++) _mm_pause();
+            for (int i = 0; i < 2000 && waiting.load(std::memory_order_relaxed) == 0; i++) relax();
             {
                 std::unique_lock<std::mutex> lk(m);
                 cv.wait(lk, [&] { return stop || !q.empty(); });
@@ -123,7 +132,7 @@ struct HostPipe {
         Task t;
         while (!done[slot].load(std::memory_order_acquire)) {
             if (take(&t)) run(t);
-            else _mm_pause();
+            else relax();
         }
     }
     // Page touches carry no flag of their own: none may outlive the call, whose caller owns the memory.
@@ -131,7 +140,7 @@ struct HostPipe {
         Task t;
         while (busy.load(std::memory_order_acquire) != 0) {
             if (take(&t)) run(t);
-            else _mm_pause();
+            else relax();
         }
     }
     char *slot(int i) { return mem + (size_t)i * kSlotBytes; }

@@ -13,11 +13,11 @@ BK_ERR_OOM, BK_ERR_CUDA = 3, 2
 SLOT = 512 << 10
 
 
-@pytest.fixture(scope="module")
-def fake(tmp_path_factory):
+@pytest.fixture(scope="module", params=[[], ["-U__SSE2__"]], ids=["sse2", "portable"])
+def fake(request, tmp_path_factory):
     so = str(tmp_path_factory.mktemp("fake") / "host_transfers.so")
     cuda = next(d for d in ("/usr/local/cuda/include", "/usr/include") if os.path.exists(os.path.join(d, "cuda_runtime.h")))
-    subprocess.run(["g++", "-std=c++20", "-O1", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-Wno-changes-meaning", "-I", cuda,
+    subprocess.run(["g++", *request.param, "-std=c++20", "-O1", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-Wno-changes-meaning", "-I", cuda,
                     "-I", os.path.join(ROOT, "include"), "-I", CSRC, os.path.join(ROOT, "tests", "fake_cuda.cpp"),
                     os.path.join(CSRC, "bk_hostpipe.cpp"), os.path.join(CSRC, "bk_snapshot.cpp"), "-o", so], check=True)
     lib = C.CDLL(so)
