@@ -259,6 +259,45 @@ def test_bulk_host_transfers_at_slot_edges(bk, gpu_ctx, n_vec):
         assert np.array_equal(bits_of(np.asarray(back).reshape(n_vec, HD)[p:p + 200]), bits_of(np.asarray(pq.dequantize(pp, nn)).reshape(-1, HD)))
 
 
+@pytest.mark.parametrize("n_vec", [100, 300, 9000])
+def test_host_transfers_of_pinned_memory(bk, gpu_ctx, n_vec):
+    """Page-locked arguments, below and above the size of a bulk transfer, next to pageable ones: the same bytes."""
+    rng = np.random.default_rng(n_vec)
+    x = rng.standard_normal((n_vec, HD)).astype(np.float32)
+    pq = bk.PlanarQuant(HD, 4, gpu_ctx)
+    packed, norms = pq.quantize(x)
+    back = pq.dequantize(packed, norms)
+    px, pp, pn, pb = (gpu_ctx.pinned(a.shape, a.dtype) for a in (x, packed, norms, back))
+    px.array[...] = x
+    gpu_ctx.check(gpu_ctx.lib.bk_kvq_quantize(gpu_ctx.h, HD, 4, n_vec, px.ptr, pp.ptr, pn.ptr))
+    assert np.array_equal(pp.array, packed) and np.array_equal(bits_of(pn.array), bits_of(norms))
+    gpu_ctx.check(gpu_ctx.lib.bk_kvq_dequantize(gpu_ctx.h, HD, 4, n_vec, pp.ptr, norms.ctypes.data, pb.ptr))
+    assert np.array_equal(bits_of(pb.array), bits_of(back))
+    for a in (px, pp, pn, pb):
+        a.free()
+
+
+@pytest.mark.parametrize("tag", ["f32", "planar4"])
+def test_large_snapshot_of_unequal_layers(bk, gpu_ctx, tag):
+    """More bytes than the ring of pinned slots holds, from layers of unlike length, one of them empty: the rows as the row-by-row
+    layout has them, and the same rows in the other sequence after a restore."""
+    lens = [9000, 0, 31, 6001]
+    a = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=4, n_ctx=9000, n_seqs=2)
+    rng = np.random.default_rng(3)
+    for il, n in enumerate(lens):
+        if n:
+            a.append(il, *synth_kv(rng, n))
+    blob = a.snapshot(seq=0)
+    assert len(blob) > 8 << 20
+    a.restore(blob, seq=1)
+    assert [a.n_pos(il, 1) for il in range(4)] == lens
+    assert a.snapshot(seq=1) == blob and a.snapshot(seq=1, layout=1) == a.snapshot(seq=0, layout=1)
+    for il, n in enumerate(lens):
+        if n:
+            compare_dumps(a.dump_kv(il, seq=1, pos0=n - 5, n_pos=5), a.dump_kv(il, seq=0, pos0=n - 5, n_pos=5))
+    a.close()
+
+
 def test_append_at_far_positions(bk, gpu_ctx, oracle):
     """Rope positions up to the 262144-token training context; rows land at the next index."""
     cache = bk.AttnCache(gpu_ctx, bk.parse_mode("planar4"), n_layers=1, n_ctx=8, rope_positions=262144)
@@ -1127,6 +1166,26 @@ def test_prefill_sums_of_one_sign(bk, gpu_ctx, tag, bound):
     v = (1 + 0.1 * rng.standard_normal((n, NKV, HD))).astype(np.float32)
     got, want = prefill_against_float64(bk, gpu_ctx, tag, q, k * np.float32(0.1), v, 512, list(range(n - 24, n)))
     assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("tag", ["f32", "f16", "planar3"])
+def test_prefill_of_unaligned_q(bk, gpu_ctx, tag):
+    """q and the result off a 16-byte boundary: bit for bit the aligned call."""
+    rng = np.random.default_rng(8)
+    n = 100
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    want = cache.prefill_attend(0, q, 0)
+    for off in (1, 2, 3):
+        dq = gpu_ctx.to_device(np.concatenate([np.zeros(off, np.float32), q.ravel()]))
+        do = gpu_ctx.to_device(np.zeros(q.size + off, np.float32))
+        gpu_ctx.check(gpu_ctx.lib.bk_prefill_attn(cache.h, 0, 0, 0, n, dq.ptr + 4 * off, do.ptr + 4 * off))
+        assert np.array_equal(do.download((q.size + off,), np.float32)[off:], want.ravel()), off
+        dq.free()
+        do.free()
+    cache.close()
 
 
 def test_prefill_other_group_sizes_and_long_context(bk, gpu_ctx, oracle):
