@@ -95,7 +95,8 @@ BK_API const char *bk_status_string(bk_status s);
 
 /* Replaces vk::Gpu creation as far as this path needs it (src/gdev.rs:269):
  * binds `device`, creates the stream and uploads the Givens table and the
- * Lloyd-Max codebooks (src/gdev.rs:360-368 uploads the same two tables). */
+ * Lloyd-Max codebooks (src/gdev.rs:360-368 uploads the same two tables), and
+ * makes the scratch of the PQ2_0 products and of a prefill CTA's sums (51 MB). */
 BK_API bk_status bk_ctx_create(int device, bk_ctx **out);
 BK_API void bk_ctx_destroy(bk_ctx *ctx);
 /* Text of the last error on `ctx` (or of the last context-less failure when ctx is NULL). */

@@ -6,8 +6,8 @@
 // The block sums are exact integers, as there: x is fixed point, X = round(x * 2^(27 - e)) with 2^e the power of two
 // above the largest |x| of the token's block of 128 (three bits more than the form for few tokens keeps).
 //
-// What bounds it: what the sixteen warps that unpack weights and drain sums have to issue (0.72 of all issue slots with 512
-// tokens, the tensor cores 0.41 busy with four 8-bit products per weight and token); with a few tokens the round trips of a
+// What bounds it: what the sixteen warps that unpack weights and drain sums have to issue (0.67 of all issue slots with 512
+// tokens, the tensor cores 0.40 busy with four 8-bit products per weight and token); with a few tokens the round trips of a
 // step.  The layout:
 //   * X has 28 bits and an operand has 8, so X is cut into four digits, X = d0 - 64 d1 + 2^14 (d2 - 64 d3), each within
 //     -128..127.  The weights are unpacked twice, as -1, 0, 1, 2 and times -64 (which fits 8 bits): d0 and d1 then meet in one

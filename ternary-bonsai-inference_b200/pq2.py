@@ -3,7 +3,8 @@
 Mirrors src/kernels.rs:204-420 (`pq2_row_bytes`, `pq2_matvec_range`, `pq2_matmul_n`): a tensor
 is its GGUF payload, rows back to back, each row ceil(ne0 / 128) blocks of 34 bytes (f16 scale +
 128 two-bit codes, weight = (code - 1) * scale).  The payload is uploaded once and stays in
-device memory; every product streams it once per group of four activations.
+device memory; a product streams it once per pair of activations, from five on once per tile of
+up to 64.
 """
 import ctypes as C
 
