@@ -6,8 +6,8 @@
 // The block sums are exact integers, as there: x is fixed point, X = round(x * 2^(27 - e)) with 2^e the power of two
 // above the largest |x| of the token's block of 128 (three bits more than the form for few tokens keeps).
 //
-// What bounds it: what the sixteen warps that unpack weights and drain sums have to issue (0.67 of all issue slots with 512
-// tokens, the tensor cores 0.40 busy with four 8-bit products per weight and token); with a few tokens the round trips of a
+// What bounds it: what the sixteen warps that unpack weights and drain sums have to issue (two thirds of all issue slots with
+// 512 tokens, the tensor cores 0.4 busy with four 8-bit products per weight and token); with a few tokens the round trips of a
 // step.  The layout:
 //   * X has 28 bits and an operand has 8, so X is cut into four digits, X = d0 - 64 d1 + 2^14 (d2 - 64 d3), each within
 //     -128..127.  The weights are unpacked twice, as -1, 0, 1, 2 and times -64 (which fits 8 bits): d0 and d1 then meet in one
@@ -23,8 +23,8 @@
 //     Two pairs of accumulators alternate: the drain of one step runs under the MMAs of the other's next.  128 columns a
 //     pair are what the operand stages leave, hence at most 64 tokens a tile.
 // Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 to 16 tokens 52 us (62 and 176 as
-// pairs of tokens; 4 tokens as pairs take 45, which is where the line lies), 64 tokens 68 (702), 128 tokens 101 (1410), 512
-// tokens 308 (5750), 1024 tokens 536.  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
+// pairs of tokens; 4 tokens as pairs take 45, which is where the line lies), 64 tokens 69 (702), 128 tokens 97 (1410), 512
+// tokens 299 (5750), 1024 tokens 516.  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
 // 57, 86, 129, 287 and 574.  Error against float64, 2-norm: 7.4e-8 on normal data, 8.0e-8 with x20 outliers in x, 4.5e-8 without
 // a bias on products of one sign; 1.02e-7, 2.4e-7 and 5.0e-8 as pairs of tokens; 1.01e-7, 1.0e-7 and 6.5e-8 (bias -5e-8) in the
 // form before, which also lost blocks that lie 2^40 below the token's largest element.
@@ -119,17 +119,17 @@ __global__ void __launch_bounds__(256) pq2_split_x_kernel(const float *x, int ne
     for (int k = 0; k < 4; k++) *reinterpret_cast<uint4 *>(dst + (size_t)k * n * 128) = make_uint4(d[k][0], d[k][1], d[k][2], d[k][3]);
 }
 
-// Tensor-memory loads without the wait.
+// A tensor-memory load without the wait.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
+
+__device__ __forceinline__ uint32_t pick_bytes(uint32_t table, uint32_t nibbles) {  // (every nibble 0..3)
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;\n" : "=r"(r) : "r"(table), "r"(nibbles));
+    return r;
 }
 
 // Sixteen 2-bit codes -> four registers of four 8-bit weights (code - 1) and four of the same times -64.  The codes are
@@ -140,8 +140,8 @@ __device__ __forceinline__ void unpack16(uint32_t w, uint32_t *one, uint32_t *wi
     const uint32_t sel[4] = {even, even >> 16, odd, odd >> 16};
 #pragma unroll
     for (int p = 0; p < 4; p++) {
-        one[p] = __byte_perm(0x020100ffu, 0u, sel[p]);
-        wide[p] = __byte_perm(0x80c00040u, 0u, sel[p]);
+        one[p] = pick_bytes(0x020100ffu, sel[p]);
+        wide[p] = pick_bytes(0x80c00040u, sel[p]);
     }
 }
 
@@ -408,34 +408,33 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
             tc_fence_after_sync();
             const uint32_t d = lane_base + (uint32_t)owner * kColsD + (uint32_t)half * NH;
             const uint32_t xs = sbase + off_s + (uint32_t)(b * N + half * NH) * 4u;
+            // eight tokens at a time, the next eight on their way meanwhile (sixteen at a time spill: 308 us for 512 tokens, 299 so)
+            uint32_t lo[2][8], hi[2][8];
+            tmem_ld8(d, lo[0]);
+            tmem_ld8(d + kColHi, hi[0]);
 #pragma unroll
-            for (int c0 = 0; c0 < NC; c0 += 2) {
-                uint32_t lo[16], hi[16];
-                if (c0 + 1 < NC) {
-                    tmem_ld16_async(d + 8u * c0, lo);
-                    tmem_ld16_async(d + kColHi + 8u * c0, hi);
-                } else {
-                    tmem_ld8(d + 8u * c0, lo);
-                    tmem_ld8(d + kColHi + 8u * c0, hi);
-                }
+            for (int c = 0; c < NC; c++) {
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (c0 + 2 >= NC) {
+                if (c + 1 < NC) {
+                    tmem_ld8(d + 8u * (c + 1), lo[(c + 1) & 1]);
+                    tmem_ld8(d + kColHi + 8u * (c + 1), hi[(c + 1) & 1]);
+                } else {
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_de + 8 * owner);
                 }
 #pragma unroll
-                for (int c4 = 0; c4 < 4; c4++)
-                    if (2 * c0 + c4 < 2 * NC) {
-                        const uint4 x4 = lds128(xs + 16u * (2 * c0 + c4));
-                        const uint64_t xv[2] = {(uint64_t)x4.x | (uint64_t)x4.y << 32, (uint64_t)x4.z | (uint64_t)x4.w << 32};
+                for (int c4 = 0; c4 < 2; c4++) {
+                    const uint4 x4 = lds128(xs + 16u * (2 * c + c4));
+                    const uint64_t xv[2] = {(uint64_t)x4.x | (uint64_t)x4.y << 32, (uint64_t)x4.z | (uint64_t)x4.w << 32};
 #pragma unroll
-                        for (int j = 0; j < 2; j++) {
-                            const int k = 4 * c4 + 2 * j;
-                            const uint64_t sum = fma2(int2_to_f2(hi[k], hi[k + 1]), join2(F2{16384.0f, 16384.0f}), int2_to_f2(lo[k], lo[k + 1]));
-                            acc[4 * c0 + k / 2] = fma2(mul2(join2(F2{sc, sc}), xv[j]), sum, acc[4 * c0 + k / 2]);
-                        }
+                    for (int j = 0; j < 2; j++) {
+                        const int k = 4 * c4 + 2 * j;
+                        const uint64_t sum = fma2(int2_to_f2(hi[c & 1][k], hi[c & 1][k + 1]), join2(F2{16384.0f, 16384.0f}),
+                                                  int2_to_f2(lo[c & 1][k], lo[c & 1][k + 1]));
+                        acc[4 * c + k / 2] = fma2(mul2(join2(F2{sc, sc}), xv[j]), sum, acc[4 * c + k / 2]);
                     }
+                }
             }
         };
         // A unit's sums join the ones before it in shared memory, in the order of the units, and leave for y after the last: one running
