@@ -553,7 +553,7 @@ struct GemmPlan {
 // Row tiles per CTA and token-tile width for a product: what has the least estimated time.  Work goes out in rounds of one CTA per SM.  A step
 // (row tile, block) takes what unpacking and draining issue, about 480 + 12 n clocks, or 700 + 11 n when two row tiles do not share a B block (L2).
 // Where two row tiles a CTA leave a last round nearly empty, its rows go out as tiles of half the size: q, k and v of 512 tokens are
-// 448 items for 148 SMs, 219 us in four rounds and 199 us as three rounds and one of half the length.
+// 448 items for 148 SMs: 219 us in four rounds, 204 us as three rounds and one of half the length.
 static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n_tok) {
     GemmPlan plan;
     double best = 1e300;
