@@ -294,9 +294,12 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
         return bail(e, "upload codebooks");
     const size_t part_bytes = (size_t)kMaxItems * kMaxRep * kScratchStride * sizeof(float);
     if ((e = cudaMalloc(&ctx->d_partials, part_bytes)) != cudaSuccess) return bail(e, "cudaMalloc partials");
-    const size_t cnt_bytes = (size_t)kCtrTotal * sizeof(unsigned);
+    const size_t cnt_bytes = (size_t)kCounters * sizeof(unsigned);
     if ((e = cudaMalloc(&ctx->d_counters, cnt_bytes)) != cudaSuccess) return bail(e, "cudaMalloc counters");
     if ((e = cudaMemset(ctx->d_counters, 0, cnt_bytes)) != cudaSuccess) return bail(e, "clear counters");
+    ctx->box_bytes = (size_t)ctx->n_sms * kMaxRep * kBoxFloats * sizeof(float);
+    if ((e = cudaMalloc(&ctx->d_boxes, ctx->box_bytes)) != cudaSuccess) return bail(e, "cudaMalloc boxes");
+    if ((e = cudaMemset(ctx->d_boxes, 0xff, ctx->box_bytes)) != cudaSuccess) return bail(e, "empty boxes");
     if ((e = cudaMalloc(&ctx->d_pq2_x, kPq2ScratchBytes)) != cudaSuccess) return bail(e, "cudaMalloc pq2 scratch");
     const size_t run_bytes = (size_t)ctx->n_sms * kPrefillRunFloats * sizeof(float);
     if ((e = cudaMalloc(&ctx->d_prefill_runs, run_bytes + ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc prefill sums");
@@ -328,6 +331,7 @@ void bk_ctx_destroy(bk_ctx *ctx) {
     if (ctx->d_cell_tabs) cudaFree(ctx->d_cell_tabs);
     if (ctx->d_partials) cudaFree(ctx->d_partials);
     if (ctx->d_counters) cudaFree(ctx->d_counters);
+    if (ctx->d_boxes) cudaFree(ctx->d_boxes);
     if (ctx->h_err) cudaFreeHost(const_cast<int *>(ctx->h_err));
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->d_stage) cudaFree(ctx->d_stage);
@@ -353,9 +357,9 @@ bk_status sync_and_check(bk_ctx *ctx) {
     const int flag = ctx->h_err ? *ctx->h_err : 0;
     if (flag) {
         *ctx->h_err = 0;
-        // a kernel that gave up may have left arrival counters behind: start the next launch from zero
-        cudaMemsetAsync(ctx->d_counters, 0, sizeof(unsigned) * kCtrTotal, ctx->stream);
-        ctx->ctr_dirty[0] = ctx->ctr_dirty[1] = 0;
+        // a kernel that gave up may have left arrival counters or words in the boxes behind: start the next launch from zero
+        cudaMemsetAsync(ctx->d_counters, 0, sizeof(unsigned) * kCounters, ctx->stream);
+        cudaMemsetAsync(ctx->d_boxes, 0xff, ctx->box_bytes, ctx->stream);
         static const char *const what[] = {"", "a tile copy did not arrive", "no room for the tile ring", "the context-split exchange (a peer never sent its rows) or a split-K copy did not arrive",
                                            "a tensor-memory operation of the prefill kernel did not complete", "a weight tile of the PQ2_0 matvec did not arrive",
                                            "the CTAs of a kv head did not all arrive for the split-K combine"};
@@ -783,8 +787,7 @@ void fill_decode_args(const bk_cache *c, int layer, int partial, DecodeArgs *out
     a.xch_err = ctx->d_err;
     a.xch_spin = ctx->xch_polls;
     a.dyn = a.dist = 0;
-    a.counters_other = nullptr;
-    a.other_n = 0;
+    a.boxes = ctx->d_boxes;
     a.k_rows_w = c->k_rows(layer, 0);
     a.v_rows_w = c->v_rows(layer, 0);
     a.k_norms_w = c->k_norms(layer, 0);
@@ -808,7 +811,7 @@ bk_status check_decode_entry(const bk_cache *c, int layer, int slot, const int32
 
 // One launch for up to kMaxSeqsPerLaunch sequences of one class.  Chunk length: generic kernel
 // about 4 CTAs per SM over the whole launch, at least 64 positions each; tensor-core kernel one
-// CTA per SM in one wave (chunks in units of 128 positions), or whole sequences when there are
+// CTA per SM in one wave (chunks in units of 32 positions), or whole sequences when there are
 // at least as many (sequence, kv head) pairs as SMs; never more than max_items work items (the
 // capacity of the split-K scratch behind a.partials).
 bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntry *list, int nb, bool use_mma,
@@ -835,7 +838,7 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
         max_np = std::max(max_np, e.np);
         min_np = std::min(min_np, e.np);
     }
-    const int64_t gran = use_mma ? 128 : 64;
+    const int64_t gran = use_mma ? 32 : 64;  // (a multiple of either tensor-core kernel's tile)
     auto items_for = [&](int64_t len) {
         int64_t items = 0;
         for (int i = 0; i < nb; i++) items += (int64_t)n_kv * ((m.n_pos[i] + len - 1) / len);
@@ -851,9 +854,15 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
         // Fewer pairs than SMs: one wave.  The balanced chunk length, grown until the items fit the SMs, so
         // that all CTAs are resident together (which the slice form of the split-K combine needs) and no
         // second, nearly empty wave doubles the launch.
+        // Short contexts: chunks of at least 96 rows over quantized V (a launch of 36 to 68 CTAs leaves room for the next
+        // launch's set-up; 511 rows 9.8 us, with 32-row chunks 10.2), of 32 rows otherwise (511 rows of f16 7.4 us, with
+        // 96-row chunks 7.6).  Where V is f32 six warps scan tiles of 16 rows, and a chunk above 96 rows is a multiple of
+        // that round (4096 rows: 192-row chunks 13.1 us, 128-row chunks 14.0).
+        const bool v_planar = a.v_kind == ROW_PLANAR, v_f32 = a.v_kind == ROW_F32;
         const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms / n_kv);
         L = (total + target_items - 1) / target_items;
-        L = std::max<int64_t>(gran, (L + gran - 1) / gran * gran);
+        L = std::max<int64_t>(v_planar ? 96 : gran, (L + gran - 1) / gran * gran);
+        if (v_f32 && L > 96) L = (L + 95) / 96 * 96;
         while (items_for(L) > ctx->n_sms && L < max_np) L += gran;
     } else {
         const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms * 4 / n_kv);  // about four CTAs per SM
@@ -872,17 +881,8 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
     if (!use_mma) return launch_decode(ctx, a, m);
     DecodeArgs a2 = a;
     a2.dyn = ctx->dyn_tiles;
-    if (a.counters == ctx->d_counters) {  // (a caller with its own scratch clears it itself before every call)
-        const int set = ctx->ctr_set;
-        a2.counters = ctx->d_counters + (size_t)kCtrSet * (1 + set);
-        a2.counters_other = ctx->d_counters + (size_t)kCtrSet * (2 - set);
-        a2.other_n = ctx->ctr_dirty[1 - set];
-        ctx->ctr_dirty[set] = std::max(ctx->ctr_dirty[set], nb * n_kv);
-        ctx->ctr_dirty[1 - set] = 0;
-        ctx->ctr_set = 1 - set;
-    }
     // every CTA holds a whole SM, so a launch of at most n_sms items is resident all at once
-    a2.dist = (ctx->dist_combine && items <= ctx->n_sms) ? 1 : 0;
+    a2.dist = (ctx->dist_combine && items <= ctx->n_sms && items <= kFactorCap) ? 1 : 0;
     return decode_f16_mma_supported(a) ? launch_decode_f16_mma(ctx, a2, m, a.k_kind == ROW_PLANAR ? ctx->lut_alpha[a.bits] : 1.0f, ctx->qsplit)
                                : launch_decode_p4_mma(ctx, a2, m, ctx->lut_alpha[a.bits], ctx->qsplit, min_np < kMmaMinPos);
 }

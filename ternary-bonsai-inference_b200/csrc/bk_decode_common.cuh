@@ -20,8 +20,7 @@
 
 namespace bk {
 
-constexpr int kFactorCap = 256;  // chunks whose rescale factors are cached in shared memory
-constexpr int kDistSpin = 1 << 21;  // polls of the arrival counter before the slice combine gives up
+constexpr int kBoxPolls = 1 << 21;  // polls of box words before a thread of the slice combine gives up
 
 // Per-CTA time stamps for tuning builds (-DBK_PHASE): stamp i of CTA b lands in g_phase[b][i].
 #ifdef BK_PHASE
@@ -71,13 +70,12 @@ __device__ __forceinline__ void store_word(uint2 *p, float value, unsigned seqno
 }
 
 __device__ __forceinline__ void exchange_slice(const DecodeArgs &a, int n_rep, int slot, int kv, int d0, int dn,
-                                               const float *vals, const float *s_M, const float *s_L, int *s_ok) {
+                                               const float *vals, const float *s_M, const float *s_L) {
     constexpr int kStride = kHd + 2;
     const int tid = threadIdx.x, nt = blockDim.x;
     const int world = a.xch_world, rank = a.xch_rank, n_rows = a.n_head, row0 = kv * n_rep;
     const unsigned seqno = a.xch_seqno, par = seqno & 1u;
     const size_t slot_w = (size_t)n_rows * kStride;
-    (void)s_ok;
     BK_STAMP(10);
     for (int r = 0; r < world; r++) {
         uint2 *dst = reinterpret_cast<uint2 *>(a.xch_peer[r]) + ((size_t)par * world + rank) * slot_w + (size_t)row0 * kStride;
@@ -142,158 +140,338 @@ __device__ __forceinline__ void exchange_slice(const DecodeArgs &a, int n_rep, i
     BK_STAMP(12);
 }
 
-// The slice form of the split-K combine.  When every CTA of a (sequence, kv head) is resident at
-// the same time (the launcher sets DecodeArgs::dist only then), nobody leaves after publishing:
-// each CTA waits (bounded) until all n_chunks triples are in the scratch and then combines ONE
-// slice of the output - all heads of the group, `D` consecutive coordinates - from every chunk's
-// triple: one L2 round trip of a few hundred 16-byte loads per CTA instead of one CTA walking
-// through all the triples.  The slices are whole Givens pairs, so the inverse rotation, the
-// division by l and the gate happen here too.  `red` is free shared memory (16-byte aligned, at
-// least 16 KiB); s_f holds kFactorCap * NREP floats.  Returns false when the wait ran out.
+// ---- Set-up shared by the tensor-core kernels ----------------------------------------------------------------
+// One warp prepares one q head: lane l holds coordinates 8 l .. 8 l + 7.  load() issues every load (the rope partners
+// among them, whatever n_rot), so that tile copies can be issued behind them; finish() applies RMSNorm
+// (src/forward.rs:242-243; q is not stored, so a tree sum will do) and rope.  A warp per head needs no barrier between
+// the steps: q was ready 2.5 us after the dependency wait with the CTA's threads spread over all heads, 1.2 us now.
+struct QHead {
+    float x[8], y[8];  // the lane's coordinates and their rope partners
+    __device__ __forceinline__ void load(const float *row, int lane, int half) {
+        const int d = 8 * lane;
+        if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+            const float4 u = __ldg(reinterpret_cast<const float4 *>(row + d)), v = __ldg(reinterpret_cast<const float4 *>(row + d) + 1);
+            x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+            x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; e++) x[e] = __ldg(row + d + e);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            y[e] = 0.f;
+            if (d + e < 2 * half) y[e] = __ldg(row + (d + e < half ? d + e + half : d + e - half));
+        }
+    }
+    __device__ __forceinline__ void finish(int lane, int half, const float *norm_w /* shared memory, or null */, float eps, const float2 *rope_row) {
+        const int d = 8 * lane;
+        if (norm_w) {
+            float ss = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; e++) ss = fmaf(x[e], x[e], ss);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            const float sc = 1.0f / sqrtf(ss / (float)kHd + eps);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                x[e] = x[e] * sc * norm_w[d + e];
+                if (d + e < 2 * half) y[e] = y[e] * sc * norm_w[d + e < half ? d + e + half : d + e - half];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            if (d + e < 2 * half) {
+                const bool first = d + e < half;
+                float x0 = first ? x[e] : y[e], x1 = first ? y[e] : x[e];
+                rope_pair(x0, x1, rope_row[first ? d + e : d + e - half]);
+                x[e] = first ? x0 : x1;
+            }
+    }
+};
+
+// The newest token's K row (role 0) or V row (role 1) of a kv head on its way to the cache: one warp loads it, norms
+// (layer form, src/forward.rs:244-245) and ropes K, and leaves it in sx (shared memory, 16-byte aligned), with the
+// append kernel's arithmetic.
+__device__ __forceinline__ void prepare_new_row(const DecodeArgs &a, int role, int lane, float4 lo, float4 hi, float *sx, const float2 *rope_row) {
+    reinterpret_cast<float4 *>(sx)[lane] = lo;
+    reinterpret_cast<float4 *>(sx)[lane + 32] = hi;
+    __syncwarp();
+    if (role == 0 && a.k_norm_w) {
+        float w[kHd / 32];
+#pragma unroll
+        for (int j = 0; j < kHd / 32; j++) w[j] = __ldg(a.k_norm_w + lane + 32 * j);
+        float sc = 0.f;
+        if (lane == 0) sc = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(serial_sumsq256(sx), (float)kHd), a.eps)));
+        sc = __shfl_sync(0xffffffffu, sc, 0);
+#pragma unroll
+        for (int j = 0; j < kHd / 32; j++) sx[lane + 32 * j] = __fmul_rn(__fmul_rn(sx[lane + 32 * j], sc), w[j]);
+        __syncwarp();
+    }
+    if (role == 0 && !a.no_rope) {
+        const int half = a.n_rot >> 1;
+        for (int j = lane; j < half; j += 32) {
+            float x0 = sx[j], x1 = sx[j + half];
+            rope_pair(x0, x1, rope_row[j]);
+            sx[j] = x0;
+            sx[j + half] = x1;
+        }
+        __syncwarp();
+    }
+}
+// The row in sx as `BITS`-wide indices (src/kvquant.rs:397-412): eight indices per lane; returns the norm (every lane).
+template <int BITS>
+__device__ __forceinline__ float quantize_new_row(const float *sx, int lane, const float *givens, const float *book, uint64_t &packed) {
+    float n = 0.f;
+    if (lane == 0) n = __fsqrt_rn(serial_sumsq256(sx));
+    n = __shfl_sync(0xffffffffu, n, 0);
+    const float inv = (n > 1e-12f) ? __fdiv_rn(1.0f, n) : 0.0f;
+    packed = 0;
+#pragma unroll
+    for (int pr = 0; pr < 4; pr++) {
+        const int i = lane * 4 + pr;  // pair index: coordinates 2i, 2i+1
+        float r0, r1;
+        givens_fwd(__fmul_rn(sx[2 * i], inv), __fmul_rn(sx[2 * i + 1], inv), givens[2 * i], givens[2 * i + 1], r0, r1);
+        packed |= (uint64_t)nearest_centroid_fast<BITS>(r0, book) << (BITS * (2 * pr));
+        packed |= (uint64_t)nearest_centroid_fast<BITS>(r1, book) << (BITS * (2 * pr + 1));
+    }
+    return n;
+}
+
+// Bounded wait for an mbarrier by a whole warp.
+__device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, int lane, int *err_flag) {
+    int polls = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if (++polls > kWaitPolls) {  // never expected; leave a mark and go on rather than hang
+            if (lane == 0) raise_error(err_flag, 1);
+            break;
+        }
+    }
+}
+
+// ---- The slice form of the split-K combine ----------------------------------------------------------------
+// When every CTA of a (sequence, kv head) is resident at the same time (the launcher sets DecodeArgs::dist only
+// then), each CTA sends its chunk's result to the CTAs that combine it and then combines ONE slice of the output
+// itself: all heads of the group, D consecutive coordinates (whole Givens pairs, so the inverse rotation, the
+// division by l and the gate happen here too).
+//
+// The boxes (DecodeArgs::boxes) are empty between launches: every 32-bit word holds kEmptyWord, a NaN pattern that
+// no sender ever stores.  A word therefore validates itself: the owner of a slice reads it until it is not empty,
+// uses it and empties it again.  No counter, no fence between data and flag, no set-up from launch to launch: one
+// trip through L2 instead of three (stores, ticket, loads of the triples).  What bounds this stage is that trip and
+// the barriers around it; per launch (planar4, 9000 rows) publish + arrive + combine took 4.6 us with a ticket
+// counter and take 1.9 us.
+//
+// Boxes of a (sequence, kv head) start at first_item * NREP * kBoxFloats:
+//     values  [slice][chunk][NREP][D]     relative to the chunk's maximum, not normalised
+//     (m, l)  [slice][chunk][NREP][2]     a copy per slice, so that every word has one reader
+constexpr unsigned kEmptyWord = 0xffffffffu;
+// 16-byte columns per head in a slice, as a power of two (the index arithmetic below is shifts), and how many slices that
+// makes.  The context split wants slices on its mailbox's octet grid.
+__host__ __device__ constexpr int slice_lg(int n_chunks, bool exchange) {
+    int lg = exchange ? 1 : 0;
+    while ((kHd / 4 >> lg) > n_chunks) lg++;
+    return lg;
+}
+constexpr bool boxes_fit() {
+    for (int n = 2; n <= kFactorCap; n++)
+        for (int x = 0; x < 2; x++) {
+            const int n_slices = kHd / 4 >> slice_lg(n, x != 0);
+            if (kHd + 2 * n_slices > kBoxFloats || n_slices > n) return false;
+        }
+    return true;
+}
+static_assert(boxes_fit(), "a box does not hold a chunk's values and (m, l) pairs, or a slice has no owner");
+
+__device__ __forceinline__ float box_word(float x) {  // kEmptyWord becomes the ordinary NaN
+    return __float_as_uint(x) == kEmptyWord ? __uint_as_float(0x7fffffffu) : x;
+}
+__device__ __forceinline__ void box_store(float *p, float x) {
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;\n" ::"l"(p), "f"(box_word(x)) : "memory");
+}
+__device__ __forceinline__ float4 box_load4(const float *p) {
+    float4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 box_load2(const float *p) {
+    float2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0,%1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool box_full(float x) { return __float_as_uint(x) != kEmptyWord; }
+__device__ __forceinline__ bool box_full4(float4 v) { return box_full(v.x) && box_full(v.y) && box_full(v.z) && box_full(v.w); }
+
+// sums[r]: this chunk's value of coordinate tid (threads 0..255) of head r; s_M, s_L: its maxima and sums.  `red` is
+// free shared memory (16-byte aligned, kCombineBytes); *s_ok is 1 on entry.  Every thread of the CTA calls.
+// A thread merges a few chunks of one 16-byte column on its own (its own reference, no exchange of maxima), the threads
+// that write the output merge the thread groups: one barrier between the loads and the output.
+constexpr uint32_t kCombineBytes = 12288;
 template <int NREP>
-__device__ __forceinline__ bool combine_slice(const DecodeArgs &a, int slot, int kv, int my_chunk, int n_chunks,
-                                              const float *base /* first chunk's triple */, float *red, float *s_f,
-                                              float *s_M, float *s_L, int *s_flag, unsigned *counter, bool v_planar,
-                                              const float *givens, int *err_flag) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        cuda::atomic_ref<unsigned, cuda::thread_scope_device> cnt(*counter);
-        int polls = 0, ok = 1;
-        while (cnt.load(cuda::memory_order_acquire) < (unsigned)n_chunks) {
-            if (++polls > kDistSpin) {  // never expected: leave a mark, write nothing
-                ok = 0;
-                raise_error(err_flag, 6);
-                break;
-            }
-        }
-        *s_flag = ok;
-    }
-    __syncthreads();
-    BK_STAMP(7);
-    if (!*s_flag) return false;
-    int D4 = (kHd / 4 + n_chunks - 1) / n_chunks;  // 16-byte columns per head in a slice
-    if (a.xch_peer) {  // context split: slices on the mailbox's octet grid, and of a size that divides the row
-        int D8 = 8;
-        while (D8 * n_chunks < kHd) D8 <<= 1;
-        D4 = D8 >> 2;
-    }
-    const int D = 4 * D4, n_slices = (kHd + D - 1) / D;
-    if (my_chunk >= n_slices) return true;
-    const int d0 = my_chunk * D, d4 = min(D4, (kHd - d0) >> 2), dn = 4 * d4;
-    const int n_col = NREP * d4;                     // 16-byte columns of this slice (<= 192 for two chunks)
-    const int n_grp = max(1, 256 / n_col);           // thread groups; group g takes chunks g, g + n_grp, ...
-    const bool act = tid < n_grp * n_col;
-    const int grp = tid / n_col, col = tid - grp * n_col, r_col = col / d4, j_col = col - r_col * d4;
-    // the data loads go out first: they and the (m, l) sweep below share one round trip
-    constexpr int kPre = 4;
-    float4 pre[kPre];
-    const float *src = base + (size_t)r_col * kScratchStride + d0 + 4 * j_col;
+__device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int kv, int my_chunk, int n_chunks, int first_item,
+                                              const float (&sums)[NREP], const float *s_M, const float *s_L, float *red, int *s_ok,
+                                              bool v_planar, const float *givens, int *err_flag) {
+    const int tid = threadIdx.x, nthr = (int)blockDim.x;
+    const int lg = slice_lg(n_chunks, a.xch_peer != nullptr), D4 = 1 << lg, D = 4 * D4, n_slices = kHd / 4 >> lg;
+    float *const boxes = a.boxes + (size_t)first_item * NREP * kBoxFloats;
+    float *const ml = boxes + (size_t)n_slices * n_chunks * NREP * D;
+    // ---- send
+    if (tid < kHd) {
+        const int sl = tid >> (lg + 2);
+        float *dst = boxes + (size_t)(sl * n_chunks + my_chunk) * NREP * D + (tid & (D - 1));
 #pragma unroll
-    for (int u = 0; u < kPre; u++) {
-        const int c = grp + u * n_grp;
-        pre[u] = (act && c < n_chunks) ? __ldcg(reinterpret_cast<const float4 *>(src + (size_t)c * NREP * kScratchStride))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < NREP; r++) box_store(dst + r * D, sums[r]);
     }
+    for (int i = tid; i < n_slices * NREP; i += nthr) {
+        const int sl = i / NREP, r = i - sl * NREP;
+        float *dst = ml + 2 * ((size_t)(sl * n_chunks + my_chunk) * NREP + r);
+        asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1, %2};\n" ::"l"(dst), "f"(box_word(s_M[r])), "f"(box_word(s_L[r])) : "memory");
+    }
+    BK_STAMP(6);
+    if (my_chunk >= n_slices) return;
+    // ---- receive
+    const int d0 = my_chunk * D, n_col = NREP << lg;  // n_col: 16-byte columns of this slice (192 for two chunks)
+    const int j_col = tid & (D4 - 1), rest = tid >> lg, grp = rest / NREP, r_col = rest - grp * NREP;
+    const int n_grp = (256 >> lg) / NREP;             // thread groups; group g takes chunks g, g + n_grp, ...
+    const int n_out = NREP * D;                       // (up to 768 outputs for a slice of half a row)
+    constexpr int kPre = 4;                           // enough for every chunk of up to 168 (a.xch_peer: 84); else several rounds
+    float *src = boxes + ((size_t)my_chunk * n_chunks * NREP + r_col) * D + 4 * j_col;
+    float *my_ml = ml + 2 * (size_t)my_chunk * n_chunks * NREP;
+    // the gate of this thread's first output travels with the first loads
     const float *gate = (a.gate && !a.partial) ? a.gate + ((size_t)slot * a.n_head + (size_t)kv * NREP) * a.gate_stride + d0 : nullptr;
-    if (warp < NREP) {  // one warp per head: global max, every chunk's factor, the merged l
-        const int r = warp;
-        constexpr int kPer = kFactorCap / 32;
-        float2 ml[kPer];
-        float M = -CUDART_INF_F;
-#pragma unroll
-        for (int u = 0; u < kPer; u++) {
-            const int c = lane + 32 * u;
-            ml[u] = make_float2(-CUDART_INF_F, 0.f);
-            if (c < n_chunks) ml[u] = __ldcg(reinterpret_cast<const float2 *>(base + ((size_t)c * NREP + r) * kScratchStride + kHd));
-            M = fmaxf(M, ml[u].x);
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-        float Lsum = 0.f;
-#pragma unroll
-        for (int u = 0; u < kPer; u++) {
-            const int c = lane + 32 * u;
-            const float f = ml[u].x > -CUDART_INF_F ? exp2f(ml[u].x - M) : 0.f;
-            Lsum = fmaf(ml[u].y, f, Lsum);
-            if (c < n_chunks) s_f[c * NREP + r] = f;
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) Lsum += __shfl_xor_sync(0xffffffffu, Lsum, off);
-        if (lane == 0) {
-            s_M[r] = M;
-            s_L[r] = Lsum;
-        }
-    }
-    __syncthreads();
+    float gate0 = 0.f;
+    if (gate && tid < n_out) gate0 = __ldg(gate + (size_t)(tid >> (lg + 2)) * a.gate_stride + (tid & (D - 1)));
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (act) {
+    float M = -CUDART_INF_F, L = 0.f;
+    if (grp < n_grp) {
+        int polls = 0;
         for (int c0 = grp; c0 < n_chunks; c0 += kPre * n_grp) {
-            if (c0 > grp) {
-#pragma unroll
-                for (int u = 0; u < kPre; u++) {
-                    const int c = c0 + u * n_grp;
-                    pre[u] = c < n_chunks ? __ldcg(reinterpret_cast<const float4 *>(src + (size_t)c * NREP * kScratchStride))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
+            float4 v[kPre];
+            float2 x[kPre];
 #pragma unroll
             for (int u = 0; u < kPre; u++) {
                 const int c = c0 + u * n_grp;
-                const float f = c < n_chunks ? s_f[c * NREP + r_col] : 0.f;
-                if (f != 0.f) {  // an empty chunk's accumulator is never looked at
-                    sum.x = fmaf(pre[u].x, f, sum.x);
-                    sum.y = fmaf(pre[u].y, f, sum.y);
-                    sum.z = fmaf(pre[u].z, f, sum.z);
-                    sum.w = fmaf(pre[u].w, f, sum.w);
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                x[u] = make_float2(-CUDART_INF_F, 0.f);
+                if (c < n_chunks) {
+                    v[u] = box_load4(src + (size_t)c * NREP * D);
+                    x[u] = box_load2(my_ml + 2 * (c * NREP + r_col));
                 }
             }
+            bool full;
+            do {  // words that were empty are read again, all of a thread's together
+                full = true;
+#pragma unroll
+                for (int u = 0; u < kPre; u++) {
+                    const int c = c0 + u * n_grp;
+                    if (!(box_full4(v[u]) && box_full(x[u].x) && box_full(x[u].y))) {
+                        v[u] = box_load4(src + (size_t)c * NREP * D);
+                        x[u] = box_load2(my_ml + 2 * (c * NREP + r_col));
+                        full = false;
+                    }
+                }
+            } while (!full && ++polls <= kBoxPolls);
+            float Mn = M;
+#pragma unroll
+            for (int u = 0; u < kPre; u++) Mn = fmaxf(Mn, x[u].x);
+            if (c0 > grp) {
+                const float f = M > -CUDART_INF_F ? fast_exp2(M - Mn) : 0.f;
+                sum.x *= f; sum.y *= f; sum.z *= f; sum.w *= f;
+                L *= f;
+            }
+            M = Mn;
+#pragma unroll
+            for (int u = 0; u < kPre; u++)
+                if (x[u].x > -CUDART_INF_F) {  // an empty chunk's accumulator is never looked at
+                    const float f = fast_exp2(x[u].x - M);
+                    L = fmaf(x[u].y, f, L);
+                    sum.x = fmaf(v[u].x, f, sum.x);
+                    sum.y = fmaf(v[u].y, f, sum.y);
+                    sum.z = fmaf(v[u].z, f, sum.z);
+                    sum.w = fmaf(v[u].w, f, sum.w);
+                }
         }
-        reinterpret_cast<float4 *>(red)[grp * n_col + col] = sum;
+        if (polls > kBoxPolls) {  // never expected: leave a mark, write nothing
+            *s_ok = 0;
+            raise_error(err_flag, 6);
+        }
     }
-    __syncthreads();
-    float *res = red + (size_t)4 * n_grp * n_col;  // [NREP][dn], fixed summation order over the groups
-    const int n_out = NREP * dn, nthr = (int)blockDim.x;  // (up to 768 outputs for a slice of half a row: loop)
-    for (int i = tid; i < n_out; i += nthr) {
-        const int r = i / dn, d = i - r * dn;
-        float t = 0.f;
-        for (int g2 = 0; g2 < n_grp; g2++) t += red[((size_t)g2 * n_col + r * d4 + (d >> 2)) * 4 + (d & 3)];
-        res[i] = t;
+    float2 *s_ml = reinterpret_cast<float2 *>(red);  // [n_grp][NREP]
+    float *s_sum = red + 2 * 256;                     // [n_grp][NREP][D]
+    if (grp < n_grp) {
+        reinterpret_cast<float4 *>(s_sum)[(grp * NREP + r_col) * D4 + j_col] = sum;
+        if (j_col == 0) s_ml[grp * NREP + r_col] = make_float2(M, L);
     }
+    float *s_Mg = s_sum + 1024, *s_Lg = s_Mg + 8, *snd = s_Lg + 8;  // context split: what this slice sends
     __syncthreads();
-    float *snd = res + n_out;  // context split: what this slice sends
-    for (int i = tid; i < n_out; i += nthr) {
-        const int r_o = i / dn, d_o = i - r_o * dn;
-        float o = res[i];
-        if (v_planar) {  // undo the Givens rotation: coordinate d0 + d and its partner (src/forward.rs:349)
+    BK_STAMP(7);
+    if (!*s_ok) return;
+    // ---- merge the groups in a fixed order and write.  Whole warps, because a Givens pair is two neighbouring lanes.
+    for (int i0 = tid & ~31; i0 < n_out; i0 += nthr) {
+        const int i = i0 + (tid & 31), r_o = i < n_out ? i >> (lg + 2) : 0, d_o = i & (D - 1);
+        float Mx = -CUDART_INF_F, Ls = 0.f, o = 0.f;
+        for (int g0 = 0; g0 < n_grp; g0 += 8) {
+            float2 x[8];
+            float v[8], Mn = Mx;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const bool in = i < n_out && g0 + u < n_grp;
+                x[u] = in ? s_ml[(g0 + u) * NREP + r_o] : make_float2(-CUDART_INF_F, 0.f);
+                v[u] = in ? s_sum[(g0 + u) * n_out + i] : 0.f;
+                Mn = fmaxf(Mn, x[u].x);
+            }
+            const float keep = Mx > -CUDART_INF_F ? fast_exp2(Mx - Mn) : 0.f;
+            Ls *= keep;
+            o *= keep;
+            Mx = Mn;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const float f = x[u].x > -CUDART_INF_F ? fast_exp2(x[u].x - Mx) : 0.f;
+                Ls = fmaf(x[u].y, f, Ls);
+                o = fmaf(v[u], f, o);
+            }
+        }
+        if (v_planar) {  // undo the Givens rotation (src/forward.rs:349)
+            const float p = __shfl_xor_sync(0xffffffffu, o, 1);
             const int pr = (d0 + d_o) >> 1;
-            const float c = givens[2 * pr], sn = givens[2 * pr + 1];
             float o0, o1;
-            givens_inv(res[r_o * dn + (d_o & ~1)], res[r_o * dn + (d_o | 1)], c, sn, o0, o1);
-            o = (d_o & 1) ? o1 : o0;
+            givens_inv((i & 1) ? p : o, (i & 1) ? o : p, givens[2 * pr], givens[2 * pr + 1], o0, o1);
+            o = (i & 1) ? o1 : o0;
         }
-        if (a.xch_peer) {
-            snd[i] = o;
-        } else if (a.partial) {
-            a.out[((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kPartStride + d0 + d_o] = o;
-        } else {
-            const float Ls = s_L[r_o];
-            o = Ls > 0.f ? o / Ls : 0.f;
-            // src/forward.rs:379-382 with src/kernels.rs:162: out *= 1 / (1 + exp(-gate))
-            if (gate) o *= 1.0f / (1.0f + expf(-__ldg(gate + (size_t)r_o * a.gate_stride + d_o)));
-            a.out[((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kHd + d0 + d_o] = o;
+        if (i < n_out) {
+            if (a.xch_peer) {
+                snd[i] = o;
+                if (d_o == 0) {
+                    s_Mg[r_o] = Mx;
+                    s_Lg[r_o] = Ls;
+                }
+            } else if (a.partial) {
+                float *po = a.out + ((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kPartStride;
+                po[d0 + d_o] = o;
+                if (d0 + d_o == 0) {
+                    po[kHd] = Mx * 0.6931471805599453f;  // log2 -> ln
+                    po[kHd + 1] = Ls;
+                }
+            } else {
+                o = Ls > 0.f ? o / Ls : 0.f;
+                // src/forward.rs:379-382 with src/kernels.rs:162: out *= 1 / (1 + exp(-gate))
+                if (gate) o *= 1.0f / (1.0f + expf(-(i == tid ? gate0 : __ldg(gate + (size_t)r_o * a.gate_stride + d_o))));
+                a.out[((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kHd + d0 + d_o] = o;
+            }
         }
+    }
+    BK_STAMP(8);
+    // ---- empty the boxes again (behind the output: only the end of the launch waits for it).  Everything this CTA
+    // owns has been read.
+    {
+        float4 *p = reinterpret_cast<float4 *>(boxes + (size_t)my_chunk * n_chunks * NREP * D);
+        const float e = __uint_as_float(kEmptyWord);
+        for (int i = tid; i < n_chunks * n_col; i += nthr) p[i] = make_float4(e, e, e, e);
+        for (int i = tid; i < n_chunks * NREP; i += nthr) reinterpret_cast<float2 *>(my_ml)[i] = make_float2(e, e);
     }
     if (a.xch_peer) {  // context split: this slice goes to every rank and is merged with theirs
         __syncthreads();
-        exchange_slice(a, NREP, slot, kv, d0, dn, snd, s_M, s_L, s_flag);
-        return true;
+        exchange_slice(a, NREP, slot, kv, d0, D, snd, s_Mg, s_Lg);
     }
-    if (a.partial && my_chunk == 0 && tid < NREP) {
-        float *po = a.out + ((size_t)slot * a.n_head + (size_t)kv * NREP + tid) * kPartStride;
-        po[kHd] = s_M[tid] * 0.6931471805599453f;  // log2 -> ln
-        po[kHd + 1] = s_L[tid];
-    }
-    return true;
 }
 
 template <int NREP, bool STREAM = false>
@@ -302,8 +480,20 @@ __device__ __forceinline__ void finish_item(const DecodeArgs &a, int slot, int s
                                             int *s_last, bool v_planar,
                                             const float *givens = nullptr /* shared-memory copy, if the caller has one */,
                                             FinishSmem fs = FinishSmem()) {
-    __shared__ float s_f[kFactorCap * NREP];
-    __shared__ float s_scale[8];
+    // the chunks' factors: at the front of the caller's region in the streamed form, which would otherwise lose a
+    // ring stage to them
+    constexpr uint32_t kFactorBytes = (kFactorCap * NREP + 8) * sizeof(float);
+    float *s_f;
+    if constexpr (STREAM) {
+        s_f = reinterpret_cast<float *>(fs.ptr);
+        fs.ptr += kFactorBytes;
+        fs.addr += kFactorBytes;
+        fs.bytes -= kFactorBytes;
+    } else {
+        __shared__ float s_static[kFactorCap * NREP + 8];
+        s_f = s_static;
+    }
+    float *s_scale = s_f + kFactorCap * NREP;
     // the first 256 threads work; a larger CTA's remaining threads only take part in the barriers
     const int tid = threadIdx.x, nt = 256;
     const bool act = threadIdx.x < 256;
@@ -340,15 +530,6 @@ __device__ __forceinline__ void finish_item(const DecodeArgs &a, int slot, int s
         }
         if (STREAM) asm volatile("fence.proxy.async;\n" ::: "memory");  // this thread's shared-memory traffic before the copies below
         __syncthreads();
-        BK_STAMP(6);
-        if (STREAM && a.dist && fs.ptr && fs.bytes >= 20480 && n_chunks <= kFactorCap) {
-            // every CTA of this (sequence, kv head) stays and combines one slice of the output
-            const float *base0 = a.partials + (size_t)first_item * NREP * kScratchStride;
-            combine_slice<NREP>(a, slot, kv, item - first_item, n_chunks, base0, reinterpret_cast<float *>(fs.ptr), s_f, s_M,
-                                s_L, s_last, &a.counters[s * a.n_kv + kv], v_planar, givens ? givens : a.givens, fs.err_flag);
-            BK_STAMP(8);
-            return;  // (the counter is cleared by the launch after the next one)
-        }
         if (!*s_last) return;
         const float *base = a.partials + (size_t)first_item * NREP * kScratchStride;
         constexpr uint32_t kChunkBytes = NREP * kScratchStride * sizeof(float);
@@ -566,8 +747,7 @@ __device__ __forceinline__ void finish_item(const DecodeArgs &a, int slot, int s
     }
     if (a.xch_peer) {
         // ---- context split: send this kv head's rows to every rank, wait for everybody's, merge ----
-        __shared__ int s_ok;
-        exchange_slice(a, NREP, slot, kv, 0, kHd, s_acc, s_M, s_L, &s_ok);
+        exchange_slice(a, NREP, slot, kv, 0, kHd, s_acc, s_M, s_L);
     } else if (a.partial) {
         float *out = a.out + ((size_t)slot * a.n_head + (size_t)kv * NREP) * kPartStride;
         for (int i = tid0; i < NREP * kHd; i += nt) {

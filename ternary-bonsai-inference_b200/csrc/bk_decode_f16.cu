@@ -74,10 +74,12 @@ constexpr uint32_t kLutBytes = 65536;    // planar K: 256 entries x 256 B, one w
 constexpr int kHeadStride = 276;         // floats per head in the warp-merge area (bank-conflict free)
 constexpr float kWScale = 16384.0f;      // 2^14: V weights are stored as f16 in (0, 2^14]
 
+constexpr int kFragRow = 33;             // a k-step's fragments, padded: the lanes that write one column of it hit different banks
 struct Other {
-    uint2 q_hi_frag[16][32], q_lo_frag[16][32];  // q as B fragments: [k-step][lane]
-    float sq[8 * kHd];                   // q of the group while it is roped
-    float new_row[2][kHd];               // the newest token's k and v of this kv head (fused append)
+    uint2 q_hi_frag[16][kFragRow], q_lo_frag[16][kFragRow];  // q as B fragments: [k-step][lane]
+    alignas(16) float new_row[2][kHd];   // the newest token's k and v of this kv head (fused append)
+    alignas(16) uint8_t new_packed[2][4 * kHd];  // the same as they are stored
+    float new_norm;                      // planar K: the norm of the new row
     float2 rope_row[kHd / 2];            // (cos, sin) of the q position
     float qw[kHd];                       // q RMSNorm weight (layer form of the step)
     float givens[kHd];                   // planar K: (cos, sin) pairs
@@ -87,6 +89,7 @@ struct Other {
     int last;
     unsigned long long bar[kMaxFW][kMaxStages];
     unsigned long long fin_bar[2];       // the split-K combine's two streaming rounds
+    unsigned long long app_bar;          // the new rows are in new_packed (one arrival per row)
 };
 
 // f32 -> f16 hi + lo for two values at once: hi = rn(x), lo = rn(x - hi).
@@ -153,7 +156,10 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     }
     const uint32_t bar0 = base + (uint32_t)offsetof(Other, bar) + (uint32_t)(warp * kMaxStages) * 8u;
     if (lane < kMaxStages) mbar_init(bar0 + lane * 8u, 1);
+    const uint32_t app_bar = base + (uint32_t)offsetof(Other, app_bar);
     if (tid < 2) mbar_init(base + (uint32_t)offsetof(Other, fin_bar) + tid * 8u, 1);
+    if (tid == 2) mbar_init(app_bar, 2);
+    if (tid == 3) o.last = 1;  // the slice combine's waits have not run out
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     __syncthreads();
 
@@ -165,7 +171,9 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     const int L = meta.chunk_len;
     const int n_chunks = (n_pos + L - 1) / L;
     const int local = item - meta.item_start[s];
-    const int kv = local / n_chunks, chunk = local - kv * n_chunks;
+    // The kv heads of a chunk are neighbours (they read the same pages of the cache at the same time), the last chunk
+    // comes first: its CTAs, which also store the new rows, are the first to run.
+    const int kv = local % a.n_kv, chunk = n_chunks - 1 - local / a.n_kv;
     const int p0 = chunk * L, p1 = min(p0 + L, n_pos);
     const int n_tiles = (p1 - p0 + kTile - 1) / kTile;
     const size_t seq_rows = (size_t)meta.seq_id[s] * a.seq_stride_rows;
@@ -206,16 +214,7 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
             }
         }
     };
-    auto wait_tile = [&](int st, uint32_t parity) {
-        const uint32_t bar = bar0 + (uint32_t)st * 8u;
-        int polls = 0;
-        while (!mbar_try_wait(bar, parity)) {
-            if (++polls > kWaitPolls) {  // never expected; leave a mark and go on rather than hang
-                if (lane == 0) raise_error(err_flag, 1);
-                break;
-            }
-        }
-    };
+    auto wait_tile = [&](int st, uint32_t parity) { wait_bar(bar0 + (uint32_t)st * 8u, parity, lane, err_flag); };
 
     // ---- constant tables first: with programmatic dependent launch this overlaps the previous
     // kernel's tail.  q, the newest row and the split-K scratch are read after the wait.
@@ -243,84 +242,23 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
             *reinterpret_cast<__half2 *>(lut_ptr + e * 256 + 128 + lane * 4) = __floats2half2_rn(lo - hf.x, hi - hf.y);
         }
     }
+    __syncthreads();  // tables and barriers are ready
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    // the counter set of the next launch: whatever the launch before the previous one left there goes now
-    if (blockIdx.x == 0 && a.counters_other)
-        for (int i = tid; i < a.other_n; i += blockDim.x) a.counters_other[i] = 0;
-    // q first: its loads are in flight before the tile copies below fill the memory system's queues
-    constexpr int kQPer = (NREP * kHd + kFT - 1) / kFT;
-    float q_reg[kQPer];
-    {
-        const float *q = a.q + ((size_t)meta.slot[s] * a.n_head + (size_t)kv * NREP) * a.q_stride;
-#pragma unroll
-        for (int u = 0; u < kQPer; u++) {
-            const int i = tid + u * kFT;
-            q_reg[u] = i < NREP * kHd ? __ldg(q + (size_t)(i >> 8) * a.q_stride + (i & 255)) : 0.f;
-        }
-    }
-
-    // ---- fused append: the CTA that scans the last chunk of this kv head stores the head's new K
-    // and V rows first, exactly as the append kernel would (src/forward.rs:259-277: rope on K,
-    // then f32 -> f16 by the reference's own rounding rule).
-    if (a.new_k != nullptr && chunk == n_chunks - 1) {
-        __syncthreads();  // the rope row is in shared memory
-        if (warp < 2) {
-            const float *src = (warp == 0 ? a.new_k : a.new_v) + ((size_t)meta.slot[s] * a.n_kv + kv) * kHd;
-            float *sx = o.new_row[warp];
-            reinterpret_cast<float4 *>(sx)[lane] = reinterpret_cast<const float4 *>(src)[lane];
-            reinterpret_cast<float4 *>(sx)[lane + 32] = reinterpret_cast<const float4 *>(src)[lane + 32];
-            __syncwarp();
-            if (warp == 0 && a.k_norm_w) {  // per-head RMSNorm of the new k row, bit-exact (src/forward.rs:244-245)
-                float sc = 0.f;
-                if (lane == 0) sc = rms_scale_ref(sx, kHd, a.eps);
-                sc = __shfl_sync(0xffffffffu, sc, 0);
-                for (int i = lane; i < kHd; i += 32) sx[i] = __fmul_rn(__fmul_rn(sx[i], sc), a.k_norm_w[i]);
-                __syncwarp();
-            }
-            if (warp == 0 && !a.no_rope) {
-                const int half = a.n_rot >> 1;
-                for (int j = lane; j < half; j += 32) {
-                    float x0 = sx[j], x1 = sx[j + half];
-                    rope_pair(x0, x1, o.rope_row[j]);
-                    sx[j] = x0;
-                    sx[j + half] = x1;
-                }
-                __syncwarp();
-            }
-            const size_t row = seq_rows + (size_t)(n_pos - 1) * a.n_kv + kv;
-            uint8_t *dst = warp == 0 ? a.k_rows_w + row * kRowK : a.v_rows_w + row * kRowV;
-            const int eb = warp == 0 ? KB : VB;
-            if (eb == 2) {
-                uint32_t w[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    w[i] = (uint32_t)f32_to_half_ref(sx[lane * 8 + 2 * i]) | ((uint32_t)f32_to_half_ref(sx[lane * 8 + 2 * i + 1]) << 16);
-                reinterpret_cast<uint4 *>(dst)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
-            } else if (eb == 4) {  // f32 rows are stored as they are (src/forward.rs:279-285)
-                reinterpret_cast<float4 *>(dst)[lane] = reinterpret_cast<const float4 *>(sx)[lane];
-                reinterpret_cast<float4 *>(dst)[lane + 32] = reinterpret_cast<const float4 *>(sx)[lane + 32];
-            } else {  // planar K row: norm, unit vector, Givens rotation, nearest centroid, pack (src/kvquant.rs:397-412)
-                float n = 0.f;
-                if (lane == 0) n = serial_norm(sx, kHd);
-                n = __shfl_sync(0xffffffffu, n, 0);
-                const float inv = (n > 1e-12f) ? __fdiv_rn(1.0f, n) : 0.0f;
-                uint64_t packed = 0;
-#pragma unroll
-                for (int pr = 0; pr < 4; pr++) {
-                    const int i = lane * 4 + pr;  // pair index: coordinates 2i, 2i+1
-                    float r0, r1;
-                    givens_fwd(__fmul_rn(sx[2 * i], inv), __fmul_rn(sx[2 * i + 1], inv), o.givens[2 * i], o.givens[2 * i + 1], r0, r1);
-                    constexpr int kB = kPlanarK ? kBits : 4;
-                    packed |= (uint64_t)nearest_centroid_fast<kB>(r0, o.book) << (kB * (2 * pr));
-                    packed |= (uint64_t)nearest_centroid_fast<kB>(r1, o.book) << (kB * (2 * pr + 1));
-                }
-                store_group8<(kPlanarK ? kBits : 4)>(dst, lane, packed);
-                if (lane == 0) a.k_norms_w[row] = n;
-            }
-            __threadfence();
-            asm volatile("fence.proxy.async;\n" ::: "memory");  // generic-proxy stores before the TMA reads below
-        }
-        __syncthreads();
+    // ---- q and the new rows first: their loads are in flight before the tile copies fill the memory system's queues.
+    // Warp w < NREP prepares head w; the last two warps of the CTA that scans a kv head's last chunk (never among
+    // those) store the head's new K and V rows at the same time.
+    static_assert(NREP <= kFW - 2 && kFW >= 8, "the appending warps prepare no q head; eight warps fill the columns");
+    const bool appender = a.new_k != nullptr && chunk == n_chunks - 1;
+    const int half_rot = a.no_rope ? 0 : a.n_rot >> 1;
+    const int role = appender ? warp - (kFW - 2) : -1;  // 0 = K, 1 = V
+    QHead qhd;
+    float4 new_lo, new_hi;
+    if (warp < NREP) {
+        qhd.load(a.q + ((size_t)meta.slot[s] * a.n_head + (size_t)kv * NREP + warp) * a.q_stride, lane, half_rot);
+    } else if (role >= 0) {
+        const float4 *src = reinterpret_cast<const float4 *>((role == 0 ? a.new_k : a.new_v) + ((size_t)meta.slot[s] * a.n_kv + kv) * kHd);
+        new_lo = src[lane];
+        new_hi = src[lane + 32];
     }
     // fill the ring now so that the copies fly during the rest of the set-up
     if constexpr (kSplit) {
@@ -333,86 +271,99 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
             if (warp + st * kFW < n_tiles) issue_tile(warp + st * kFW, st);
     }
 
-    // ---- q: rope, scale, split into f16 hi/lo, laid out as B fragments ---------------------
-    {
-        float *sq = o.sq;  // [NREP][256]
+    // ---- q: RMSNorm, rope, scale, split into f16 hi/lo, laid out as B fragments ---------------------
+    // 1/sqrt(hd) * log2(e): the scores come out in the exp2 domain.
+    // k-step ks covers coordinates 16 ks .. 16 ks + 15; lane (g, t) holds head g's values at
+    // 16 ks + 2t, +1 (b0) and 16 ks + 2t + 8, +9 (b1): the coordinates 8 l .. 8 l + 7 of lane l are b0 or b1 of k-step l / 2.
+    // Planar K: q is Givens-rotated into the stored rows' basis (src/forward.rs:304), the table's alpha is
+    // undone in the scale, and k-step ks = c*8 + w*2 + bp covers coordinates (2t+c)*32 + w*8 + bp*4 + 0..3
+    // (the order in which the packed bytes of a row come out of the table): t = l / 8, c = l / 4 % 2, w = l % 4, bp = 0 and 1.
+    if (warp < 8) {
+        uint32_t hi[4] = {0u, 0u, 0u, 0u}, lo[4] = {0u, 0u, 0u, 0u};
+        if (warp < NREP) {
+            const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / (kPlanarK ? lut_alpha : 1.0f);
+            qhd.finish(lane, half_rot, a.q_norm_w ? o.qw : nullptr, a.eps, o.rope_row);
 #pragma unroll
-        for (int u = 0; u < kQPer; u++) {
-            const int i = tid + u * kFT;
-            if (i < NREP * kHd) sq[i] = q_reg[u];
+            for (int i = 0; i < 4; i++) {
+                float x0 = qhd.x[2 * i], x1 = qhd.x[2 * i + 1];
+                if constexpr (kPlanarK) givens_fwd(qhd.x[2 * i], qhd.x[2 * i + 1], o.givens[8 * lane + 2 * i], o.givens[8 * lane + 2 * i + 1], x0, x1);
+                split_pair(x0 * qscale, x1 * qscale, hi[i], lo[i]);
+            }
         }
-        __syncthreads();
-        if (a.q_norm_w) {  // per-head RMSNorm of q (src/forward.rs:242-243); q is not stored, so a tree sum will do
-            if (warp < NREP) {
-                float ss = 0.f;
+        if constexpr (kPlanarK) {
+            const int ks0 = ((lane >> 2) & 1) * 8 + (lane & 3) * 2, ln = warp * 4 + (lane >> 3);
 #pragma unroll
-                for (int j = 0; j < kHd / 32; j++) {
-                    const float x = sq[warp * kHd + lane + 32 * j];
-                    ss = fmaf(x, x, ss);
-                }
+            for (int bp = 0; bp < 2; bp++) {
+                o.q_hi_frag[ks0 + bp][ln] = make_uint2(hi[2 * bp], hi[2 * bp + 1]);
+                o.q_lo_frag[ks0 + bp][ln] = make_uint2(lo[2 * bp], lo[2 * bp + 1]);
+            }
+        } else {
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-                if (lane == 0) o.M[warp] = 1.0f / sqrtf(ss / (float)kHd + a.eps);
+            for (int tt = 0; tt < 4; tt++) {
+                reinterpret_cast<uint32_t *>(&o.q_hi_frag[lane >> 1][warp * 4 + tt])[lane & 1] = hi[tt];
+                reinterpret_cast<uint32_t *>(&o.q_lo_frag[lane >> 1][warp * 4 + tt])[lane & 1] = lo[tt];
             }
-            __syncthreads();
-            for (int i = tid; i < NREP * kHd; i += kFT) sq[i] = sq[i] * o.M[i >> 8] * o.qw[i & 255];
-            __syncthreads();
-        }  // also: the rope row is complete
-        if (!a.no_rope) {
-            const int half = a.n_rot >> 1;
-            for (int i = tid; i < NREP * half; i += kFT) {
-                const int r = i / half, j = i - r * half;
-                float x0 = sq[r * kHd + j], x1 = sq[r * kHd + j + half];
-                rope_pair(x0, x1, o.rope_row[j]);
-                sq[r * kHd + j] = x0;
-                sq[r * kHd + j + half] = x1;
-            }
-            __syncthreads();
         }
-        // 1/sqrt(hd) * log2(e): the scores come out in the exp2 domain.
-        // k-step ks covers coordinates 16 ks .. 16 ks + 15; lane (g, t) holds head g's values at
-        // 16 ks + 2t, +1 (b0) and 16 ks + 2t + 8, +9 (b1).
-        // Planar K: q is Givens-rotated into the stored rows' basis (src/forward.rs:304), the table's alpha is
-        // undone in the scale, and k-step ks = c*8 + w*2 + bp covers coordinates (2t+c)*32 + w*8 + bp*4 + 0..3
-        // (the order in which the packed bytes of a row come out of the table).
-        const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / (kPlanarK ? lut_alpha : 1.0f);
-        for (int i = tid; i < 16 * 32; i += kFT) {
-            const int ks = i >> 5, ln = i & 31, gg = ln >> 2, tt = ln & 3;
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
-            if constexpr (kPlanarK) {
-                const int c = ks >> 3, w = (ks >> 1) & 3, bp = ks & 1;
-                const int d0 = (2 * tt + c) * 32 + w * 8 + bp * 4;
-                if (gg < NREP) {
-                    givens_fwd(sq[gg * kHd + d0], sq[gg * kHd + d0 + 1], o.givens[d0], o.givens[d0 + 1], x[0], x[1]);
-                    givens_fwd(sq[gg * kHd + d0 + 2], sq[gg * kHd + d0 + 3], o.givens[d0 + 2], o.givens[d0 + 3], x[2], x[3]);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) x[e] *= qscale;
-                }
-            } else {
-                const int d0 = 16 * ks + 2 * tt;
-                if (gg < NREP) {
-                    x[0] = sq[gg * kHd + d0] * qscale;
-                    x[1] = sq[gg * kHd + d0 + 1] * qscale;
-                    x[2] = sq[gg * kHd + d0 + 8] * qscale;
-                    x[3] = sq[gg * kHd + d0 + 9] * qscale;
-                }
-            }
-            __half h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                h[e] = __float2half_rn(x[e]);
-                l[e] = __float2half_rn(x[e] - __half2float(h[e]));
-            }
-            auto pack = [](__half lo, __half hi) { return (uint32_t)__half_as_ushort(lo) | ((uint32_t)__half_as_ushort(hi) << 16); };
-            o.q_hi_frag[ks][ln] = make_uint2(pack(h[0], h[1]), pack(h[2], h[3]));
-            o.q_lo_frag[ks][ln] = make_uint2(pack(l[0], l[1]), pack(l[2], l[3]));
-        }
-        __syncthreads();
     }
+    // ---- fused append: exactly what the append kernel would store (src/forward.rs:259-285).  The rows also stay in
+    // shared memory, where the warp that holds the chunk's last tile puts them over what the copies brought: nothing
+    // waits for a round trip through global memory.
+    if (!appender) {
+        __syncthreads();
+    } else if (role < 0) {
+        asm volatile("bar.arrive 3, %0;\n" ::"n"(kFT) : "memory");
+        asm volatile("bar.sync 2, %0;\n" ::"n"(kFT) : "memory");  // does not wait for the appending warps' rows
+    } else {
+        asm volatile("bar.arrive 2, %0;\n" ::"n"(kFT) : "memory");
+        float *sx = o.new_row[role];
+        prepare_new_row(a, role, lane, new_lo, new_hi, sx, o.rope_row);
+        const size_t row = seq_rows + (size_t)(n_pos - 1) * a.n_kv + kv;
+        uint8_t *dst = role == 0 ? a.k_rows_w + row * kRowK : a.v_rows_w + row * kRowV;
+        uint8_t *keep = o.new_packed[role];
+        const int eb = role == 0 ? KB : VB;
+        if (eb == 2) {  // the reference's own f32 -> f16 rounding rule
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                w[i] = (uint32_t)f32_to_half_ref(sx[lane * 8 + 2 * i]) | ((uint32_t)f32_to_half_ref(sx[lane * 8 + 2 * i + 1]) << 16);
+            reinterpret_cast<uint4 *>(keep)[lane] = reinterpret_cast<uint4 *>(dst)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
+        } else if (eb == 4) {  // f32 rows are stored as they are (src/forward.rs:279-285)
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                reinterpret_cast<float4 *>(keep)[lane + 32 * i] = reinterpret_cast<float4 *>(dst)[lane + 32 * i] =
+                    reinterpret_cast<const float4 *>(sx)[lane + 32 * i];
+        } else {  // planar K row: norm, unit vector, Givens rotation, nearest centroid, pack
+            constexpr int kB = kPlanarK ? kBits : 4;
+            uint64_t packed;
+            const float n = quantize_new_row<kB>(sx, lane, o.givens, o.book, packed);
+            store_group8<kB>(keep, lane, packed);
+            store_group8<kB>(dst, lane, packed);
+            if (lane == 0) a.k_norms_w[row] = o.new_norm = n;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(app_bar);
+        asm volatile("bar.sync 3, %0;\n" ::"n"(kFT) : "memory");  // every q fragment is written
+    }
+    // The new K or V row over the chunk's last tile, in shared memory.
+    auto patch_half = [&](uint32_t addr, int which) {
+        if (which == 0) wait_bar(app_bar, 0, lane, err_flag);
+        const uint32_t r = (uint32_t)(n_pos - 1) % kTile;
+        const int row_bytes = which == 0 ? kRowK : kRowV;
+        for (int i = lane; i < row_bytes / 16; i += 32) {
+            // (3-bit rows lie densely, without a swizzle)
+            const uint32_t at = row_bytes % 128 == 0 ? (uint32_t)(i >> 3) * kSlabBytes + r * 128u + (((uint32_t)(i & 7) ^ (r & 7u)) << 4)
+                                                     : r * (uint32_t)row_bytes + (uint32_t)i * 16u;
+            const uint4 v = reinterpret_cast<const uint4 *>(o.new_packed[which])[i];
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr + at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+        }
+        if (kPlanarK && which == 0 && lane == 0)
+            asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(addr + (uint32_t)kSlabBytes + (r * (uint32_t)a.n_kv + (uint32_t)kv) * 4u), "f"(o.new_norm) : "memory");
+        __syncwarp();
+    };
     const uint32_t qh_addr = base + (uint32_t)offsetof(Other, q_hi_frag) + (uint32_t)lane * 8u;
     const uint32_t ql_addr = base + (uint32_t)offsetof(Other, q_lo_frag) + (uint32_t)lane * 8u;
     auto q_frag = [&](uint32_t addr0, int ks, uint32_t &x, uint32_t &y) {
-        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(x), "=r"(y) : "r"(addr0 + (uint32_t)ks * 256u));
+        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(x), "=r"(y) : "r"(addr0 + (uint32_t)(ks * kFragRow * 8)));
     };
 
     float acc[16][4];
@@ -666,11 +617,14 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
         if (warp < kScanW)
             for (int tile = warp; tile < n_tiles; tile += kScanW) {
                 const uint32_t st_addr = stage_of(0);
+                const bool newest = appender && tile == n_tiles - 1;
                 wait_tile(0, parity);
+                if (newest) patch_half(st_addr, 0);
                 compute_scores(tile, st_addr);
                 __syncwarp();
                 if (tile + kScanW < n_tiles) issue_half(tile + kScanW, 0);
                 wait_tile(1, parity);
+                if (newest) patch_half(st_addr + kHalfK, 1);
                 compute_out(tile, st_addr + kHalfK);
                 __syncwarp();
                 if (tile + kScanW < n_tiles) issue_half(tile + kScanW, 1);
@@ -682,6 +636,10 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
         uint32_t parity = 0;
         for (int tile = warp; tile < n_tiles; tile += kFW) {
             wait_tile(st, parity);
+            if (appender && tile == n_tiles - 1) {
+                patch_half(stage_of(st), 0);
+                patch_half(stage_of(st) + kHalfK, 1);
+            }
             compute_scores(tile, stage_of(st));
             compute_out(tile, stage_of(st) + kHalfK);
             __syncwarp();  // every lane has read the stage: lane 0 may refill it
@@ -704,21 +662,31 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
         o.l_w[warp][2 * t + 1] = l1;
     }
     __syncthreads();  // every warp has consumed its last stage
+    // every lane finds the maxima of its own two heads; the sums are one warp's work beside it
+    float Ma = -CUDART_INF_F, Mb = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < kFW; w++) {
+        Ma = fmaxf(Ma, o.m_w[w][2 * t]);
+        Mb = fmaxf(Mb, o.m_w[w][2 * t + 1]);
+    }
     if (tid < 8) {
         float M = -CUDART_INF_F;
+#pragma unroll
         for (int w = 0; w < kFW; w++) M = fmaxf(M, o.m_w[w][tid]);
         float Ls = 0.f;
+#pragma unroll
         for (int w = 0; w < kFW; w++)
-            if (o.m_w[w][tid] > -CUDART_INF_F) Ls += o.l_w[w][tid] * exp2f(o.m_w[w][tid] - M);
+            if (o.m_w[w][tid] > -CUDART_INF_F) Ls += o.l_w[w][tid] * fast_exp2(o.m_w[w][tid] - M);
         o.M[tid] = M;
         o.L[tid] = Ls;
     }
-    __syncthreads();
     float *area = reinterpret_cast<float *>(smem_raw + (ring0 - base));  // [kFW][NREP][kHeadStride]
+    constexpr int kMergeFloats = (kFW * NREP * kHeadStride + 3) & ~3;
+    static_assert((size_t)kMergeFloats * 4 + kCombineBytes <= (size_t)kScanW * kStageBytes, "the combine's scratch does not fit behind the merge area");
     {
         const float unscale = 1.0f / kWScale;
-        const float f0 = (M0 > -CUDART_INF_F) ? exp2f(M0 - o.M[2 * t]) * unscale : 0.f;
-        const float f1 = (M1 > -CUDART_INF_F) ? exp2f(M1 - o.M[2 * t + 1]) * unscale : 0.f;
+        const float f0 = (M0 > -CUDART_INF_F) ? fast_exp2(M0 - Ma) * unscale : 0.f;
+        const float f1 = (M1 > -CUDART_INF_F) ? fast_exp2(M1 - Mb) * unscale : 0.f;
         float *w0 = area + ((size_t)warp * NREP + 2 * t) * kHeadStride + g;
         float *w1 = w0 + kHeadStride;
 #pragma unroll
@@ -743,6 +711,12 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
 #pragma unroll
             for (int w = 0; w < kFW; w++) sums[r] += area[((size_t)w * NREP + r) * kHeadStride + tid];
     }
+    const int first_item = meta.item_start[s] + kv * n_chunks;
+    if (a.dist && n_chunks > 1) {  // (the ring behind the merge area is free: every tile has been consumed)
+        float *red = reinterpret_cast<float *>(smem_raw + (ring0 - base)) + kMergeFloats;
+        combine_slice<NREP>(a, meta.slot[s], kv, chunk, n_chunks, first_item, sums, o.M, o.L, red, &o.last, false, nullptr, err_flag);
+        return;
+    }
     __syncthreads();
     float *s_acc = area;  // [NREP][256]
     if (tid < kHd)
@@ -756,8 +730,7 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     fs.bar = base + (uint32_t)offsetof(Other, fin_bar);
     fs.ptr = smem_raw + (fs.addr - base);
     fs.err_flag = err_flag;
-    const int first_item = meta.item_start[s] + kv * n_chunks;
-    finish_item<NREP, true>(a, meta.slot[s], s, kv, item, n_chunks, first_item, s_acc, o.M, o.L, &o.last, false, nullptr, fs);
+    finish_item<NREP, true>(a, meta.slot[s], s, kv, first_item + chunk, n_chunks, first_item, s_acc, o.M, o.L, &o.last, false, nullptr, fs);
 }
 
 template <int KB, int VB, int NREP, bool QSPLIT>

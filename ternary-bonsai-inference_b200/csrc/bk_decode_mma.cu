@@ -107,10 +107,13 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 }
 
 struct Other {                          // bookkeeping block, lives outside the lookup table
+    alignas(16) uint2 q_frag[2][16 * 32];  // q as B fragments, hi and lo parts: [k-step * 32 + lane]
+    alignas(16) float new_row[2][kHd];   // the newest token's k and v of this kv head (fused append)
+    alignas(16) uint8_t new_packed[2][128];  // the same as they are stored
+    float new_norm[2];
     float givens[kHd];                   // (cos, sin) pairs
     float2 rope_row[kHd / 2];            // (cos, sin) of the q position
     float qw[kHd];                       // q RMSNorm weight (layer form of the step)
-    float new_row[2][kHd];               // the newest token's k and v of this kv head (fused append)
     float book[2][16];                   // unscaled centroids, one copy per appending warp
     float m_w[kMW][8], l_w[kMW][8];
     float M[8], L[8];
@@ -118,8 +121,9 @@ struct Other {                          // bookkeeping block, lives outside the 
     int next_tile;                       // the chunk's tile counter
     unsigned long long bar[kMW][kMaxStages];  // one mbarrier per warp and stage
     unsigned long long fin_bar[2];            // the split-K combine's two streaming rounds
+    unsigned long long app_bar;               // the new rows are in new_packed (one arrival per row)
 };
-constexpr uint32_t kOtherBytes = 7168;
+constexpr uint32_t kOtherBytes = 15360;
 static_assert(sizeof(Other) <= kOtherBytes, "Other does not fit");
 
 // Table lookup of packed byte K (0..3) of word x: lane_base holds the table's shared address in
@@ -182,7 +186,10 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     const uint32_t lane_base = lut_addr | (uint32_t)(lane << 2);
     const uint32_t bar0 = other_addr + (uint32_t)offsetof(Other, bar) + (uint32_t)(warp * kMaxStages) * 8u;
     if (lane < kMaxStages) mbar_init(bar0 + lane * 8u, 1);
+    const uint32_t app_bar = other_addr + (uint32_t)offsetof(Other, app_bar);
     if (tid < 2) mbar_init(other_addr + (uint32_t)offsetof(Other, fin_bar) + tid * 8u, 1);
+    if (tid == 2) mbar_init(app_bar, 2);
+    if (tid == 3) o.last = 1;  // the slice combine's waits have not run out
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 
     // ---- which item ------------------------------------------------------------------------
@@ -190,16 +197,16 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     int s = 0;
     while (s + 1 < meta.n_seqs && meta.item_start[s + 1] <= item) s++;
     const int n_pos = meta.n_pos[s];
-    const int L = meta.chunk_len;  // a multiple of 128 positions
+    const int L = meta.chunk_len;  // a multiple of the tile
     const int n_chunks = (n_pos + L - 1) / L;
     const int local = item - meta.item_start[s];
-    const int kv = local / n_chunks, chunk = local - kv * n_chunks;
+    // The kv heads of a chunk are neighbours (they read the same pages of the cache at the same time), the last chunk
+    // comes first: its CTAs, which also store the new rows, are the first to run.
+    const int kv = local % a.n_kv, chunk = n_chunks - 1 - local / a.n_kv;
     const int p0 = chunk * L, p1 = min(p0 + L, n_pos);
     const int tile0 = p0 / kTile;                              // first tile of the chunk (sequence-wide index)
     const bool appender = a.new_k != nullptr && chunk == n_chunks - 1;
-    // The tile that holds the new token's row is not drawn from the pool: warp 0 of the appending
-    // CTA takes it once that row is stored.
-    const int n_tiles = (p1 - p0 + kTile - 1) / kTile, n_pool = n_tiles - (appender ? 1 : 0);
+    const int n_tiles = (p1 - p0 + kTile - 1) / kTile;
     const size_t seq_rows = (size_t)meta.seq_id[s] * a.seq_stride_rows;
     const bool dyn = (a.dyn & 1) != 0;
 
@@ -255,200 +262,148 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
         if (tid == 0) o.next_tile = kMW * n_stages;  // the first n_stages tiles of every warp are fixed
         constexpr int kIdxMask = (1 << BITS) - 1;
         const float c_lo = a.book[lane & kIdxMask] * lut_alpha;  // the low lanes hold the scaled centroids
-        // the lookup table: entry e -> half2(alpha*c[low nibble], alpha*c[high nibble]), one copy per lane
-        for (int e = warp; e < 256; e += kMW) {
+        // The lookup table: entry e -> half2(alpha*c[low nibble], alpha*c[high nibble]), one copy per lane; PRECISE
+        // (short contexts: the table's f16 centroids, good to 1e-4, are not averaged out over enough positions): what
+        // their rounding left over goes into the upper half of the slot and every product gets a second term.
+        // Eight lanes write an entry with one 16-byte store each (1.4 us of the prologue with a word per lane).
+#pragma unroll 2
+        for (int e = warp * 4 + (lane >> 3); e < 256; e += kMW * 4) {
             const float lo = __shfl_sync(0xffffffffu, c_lo, e & kIdxMask), hi = __shfl_sync(0xffffffffu, c_lo, (e >> 4) & kIdxMask);
             const __half2 h = __floats2half2_rn(lo, hi);
-            *reinterpret_cast<__half2 *>(lut_ptr + e * 256 + lane * 4) = h;
+            const uint32_t u = *reinterpret_cast<const uint32_t *>(&h);
+            *reinterpret_cast<uint4 *>(lut_ptr + e * 256 + (lane & 7) * 16) = make_uint4(u, u, u, u);
+            if constexpr (PRECISE) {
+                const float2 hf = __half22float2(h);
+                const __half2 rem = __floats2half2_rn(lo - hf.x, hi - hf.y);
+                const uint32_t w = *reinterpret_cast<const uint32_t *>(&rem);
+                *reinterpret_cast<uint4 *>(lut_ptr + e * 256 + 128 + (lane & 7) * 16) = make_uint4(w, w, w, w);
+            }
         }
     }
     __syncthreads();  // tables and barriers are ready; from here to the end of the scan the warps run on their own
     BK_STAMP(0);
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     BK_STAMP(1);
-    // the counter set of the next launch: whatever the launch before the previous one left there goes now
-    if (blockIdx.x == 0 && a.counters_other)
-        for (int i = tid; i < a.other_n; i += blockDim.x) a.counters_other[i] = 0;
-
-
-    // ---- q first: its loads are in flight before the tile copies fill the memory system's queues
-    constexpr int kQPer = (NREP * kHd + kMT - 1) / kMT;
-    float q_reg[kQPer];
-    {
-        const float *q = a.q + ((size_t)meta.slot[s] * a.n_head + (size_t)kv * NREP) * a.q_stride;
-#pragma unroll
-        for (int u = 0; u < kQPer; u++) {
-            const int i = tid + u * kMT;
-            q_reg[u] = i < NREP * kHd ? __ldg(q + (size_t)(i >> 8) * a.q_stride + (i & 255)) : 0.f;
-        }
+    // ---- q and the new rows first: their loads are in flight before the tile copies fill the memory system's queues.
+    // Warp w < NREP prepares head w; the last two warps of the CTA that scans a kv head's last chunk (never among
+    // those: NREP <= 6) store the head's new K and V rows at the same time.
+    static_assert(NREP <= kMW - 2, "the appending warps prepare no q head");
+    const int half = a.no_rope ? 0 : a.n_rot >> 1;
+    const int role = appender ? warp - (kMW - 2) : -1;  // 0 = K, 1 = V
+    QHead qhd;
+    float4 new_lo, new_hi;
+    if (warp < NREP) {
+        qhd.load(a.q + ((size_t)meta.slot[s] * a.n_head + (size_t)kv * NREP + warp) * a.q_stride, lane, half);
+    } else if (role >= 0) {
+        const float4 *src = reinterpret_cast<const float4 *>((role == 0 ? a.new_k : a.new_v) + ((size_t)meta.slot[s] * a.n_kv + kv) * kHd);
+        new_lo = src[lane];
+        new_hi = src[lane + 32];
     }
     // Fixed shares (the default: the result then does not depend on timing).  Warp w takes tiles w, w + 8, ...;
-    // in the appending CTA warps 0 and 1 start late (they store the new rows first), so there the other six
-    // warps share the first kHeadStart rounds among themselves.
-    constexpr int kHeadStart = 4;
+    // in the appending CTA the last two warps start late (they store the new rows first, about a tile's time), so there
+    // the other six share the first kHeadStart rounds among themselves.
+    constexpr int kHeadStart = 1, kOthers = kMW - 2;
     auto fixed_tile = [&](int i) -> int {
         if (!appender) return warp + kMW * i;
-        if (warp < 2) return (kMW - 2) * kHeadStart + kMW * i + warp;
-        return i < kHeadStart ? (kMW - 2) * i + (warp - 2) : (kMW - 2) * kHeadStart + kMW * (i - kHeadStart) + warp;
+        if (warp >= kOthers) return kOthers * kHeadStart + kMW * i + warp - kOthers;
+        return i < kHeadStart ? kOthers * i + warp : kOthers * kHeadStart + 2 + kMW * (i - kHeadStart) + warp;
     };
     // ---- fill the ring
     int in_stage[kMaxStages];  // which tile each stage holds, -1 = none
 #pragma unroll
     for (int st = 0; st < kMaxStages; st++) {
         const int lt = dyn ? warp + st * kMW : fixed_tile(st);
-        in_stage[st] = (st < n_stages && lt < n_pool) ? lt : -1;
+        in_stage[st] = (st < n_stages && lt < n_tiles) ? lt : -1;
         if (in_stage[st] >= 0) issue_tile(lt, st);
     }
     int i_next = n_stages;
     // ---- q: per-head RMSNorm (layer form), rope, Givens rotation, scale, split into f16 hi/lo, written in the
-    // MMA's B-fragment layout and then fetched by every lane into registers.  The scratch for this is the
-    // unused upper half of the table's 256-byte slots (the table itself fills only the lower halves):
-    // slot h, word x is at table + 256 h + 128 + 4 x.  sq[i] takes slots 0..47, the fragments slots 64..127.
-    uint32_t qh[16][2], ql[QSPLIT ? 16 : 1][2];
+    // MMA's B-fragment layout and then fetched by every lane into registers.
+    // 1/sqrt(hd) * log2(e) / alpha: the scores come out in the exp2 domain, alpha undone.
+    // k-step ks = c*8 + w*2 + bp covers coordinates (2t+c)*32 + w*8 + bp*4 + 0..3 of head g: lane l's coordinates
+    // 8 l .. 8 l + 7 are t = l / 8, c = l / 4 % 2, w = l % 4, bp = 0 and 1.
     {
-        auto sq = [&](int i) -> float & { return *reinterpret_cast<float *>(lut_ptr + (i >> 5) * 256 + 128 + (i & 31) * 4); };
-        auto frag = [&](int lo_part, int j) -> uint2 & {  // j = k-step * 32 + lane
-            return *reinterpret_cast<uint2 *>(lut_ptr + (64 + 32 * lo_part + (j >> 4)) * 256 + 128 + (j & 15) * 8);
-        };
+        const int ks0 = ((lane >> 2) & 1) * 8 + (lane & 3) * 2, ln = warp * 4 + (lane >> 3);
+        if (warp < NREP) {
+            const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / lut_alpha;
+            qhd.finish(lane, half, a.q_norm_w ? o.qw : nullptr, a.eps, o.rope_row);
 #pragma unroll
-        for (int u = 0; u < kQPer; u++) {
-            const int i = tid + u * kMT;
-            if (i < NREP * kHd) sq(i) = q_reg[u];
-        }
-        __syncthreads();
-        if (a.q_norm_w) {  // per-head RMSNorm of q (src/forward.rs:242-243); q is not stored, so a tree sum will do
-            if (warp < NREP) {
-                float ss = 0.f;
+            for (int bp = 0; bp < 2; bp++) {
+                const int d0 = 8 * lane + 4 * bp;
+                float x[4];
+                givens_fwd(qhd.x[4 * bp], qhd.x[4 * bp + 1], o.givens[d0], o.givens[d0 + 1], x[0], x[1]);
+                givens_fwd(qhd.x[4 * bp + 2], qhd.x[4 * bp + 3], o.givens[d0 + 2], o.givens[d0 + 3], x[2], x[3]);
+                __half h[4], l[4];
 #pragma unroll
-                for (int j = 0; j < kHd / 32; j++) {
-                    const float x = sq(warp * kHd + lane + 32 * j);
-                    ss = fmaf(x, x, ss);
+                for (int e = 0; e < 4; e++) {
+                    x[e] *= qscale;
+                    h[e] = __float2half_rn(x[e]);
+                    l[e] = __float2half_rn(x[e] - __half2float(h[e]));
                 }
+                o.q_frag[0][(ks0 + bp) * 32 + ln] = make_uint2(pack_h2(h[0], h[1]), pack_h2(h[2], h[3]));
+                o.q_frag[1][(ks0 + bp) * 32 + ln] = make_uint2(pack_h2(l[0], l[1]), pack_h2(l[2], l[3]));
+            }
+        } else {  // the unused columns
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-                if (lane == 0) o.M[warp] = 1.0f / sqrtf(ss / (float)kHd + a.eps);
-            }
-            __syncthreads();
-            for (int i = tid; i < NREP * kHd; i += kMT) sq(i) = sq(i) * o.M[i >> 8] * o.qw[i & 255];
-            __syncthreads();
-        }
-        if (!a.no_rope) {
-            const int half = a.n_rot >> 1;
-            for (int i = tid; i < NREP * half; i += kMT) {
-                const int r = i / half, j = i - r * half;
-                float x0 = sq(r * kHd + j), x1 = sq(r * kHd + j + half);
-                rope_pair(x0, x1, o.rope_row[j]);
-                sq(r * kHd + j) = x0;
-                sq(r * kHd + j + half) = x1;
-            }
-            __syncthreads();
-        }
-        // 1/sqrt(hd) * log2(e) / alpha: the scores come out in the exp2 domain, alpha undone.
-        // k-step ks = c*8 + w*2 + bp covers coordinates (2t+c)*32 + w*8 + bp*4 + 0..3 of head g.
-        const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / lut_alpha;
-        for (int i = tid; i < 16 * 32; i += kMT) {
-            const int ks = i >> 5, ln = i & 31, gg = ln >> 2, tt = ln & 3;
-            const int c = ks >> 3, w = (ks >> 1) & 3, bp = ks & 1;
-            const int d0 = (2 * tt + c) * 32 + w * 8 + bp * 4;
-            float x[4] = {0.f, 0.f, 0.f, 0.f};
-            if (gg < NREP) {
-                givens_fwd(sq(gg * kHd + d0), sq(gg * kHd + d0 + 1), o.givens[d0], o.givens[d0 + 1], x[0], x[1]);
-                givens_fwd(sq(gg * kHd + d0 + 2), sq(gg * kHd + d0 + 3), o.givens[d0 + 2], o.givens[d0 + 3], x[2], x[3]);
-            }
-            __half h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                x[e] *= qscale;
-                h[e] = __float2half_rn(x[e]);
-                l[e] = __float2half_rn(x[e] - __half2float(h[e]));
-            }
-            frag(0, i) = make_uint2(pack_h2(h[0], h[1]), pack_h2(h[2], h[3]));
-            frag(1, i) = make_uint2(pack_h2(l[0], l[1]), pack_h2(l[2], l[3]));
-        }
-        __syncthreads();
-#pragma unroll
-        for (int ks = 0; ks < 16; ks++) {
-            const uint2 v = frag(0, ks * 32 + lane);
-            qh[ks][0] = v.x;
-            qh[ks][1] = v.y;
-            if constexpr (QSPLIT) {
-                const uint2 u = frag(1, ks * 32 + lane);
-                ql[ks][0] = u.x;
-                ql[ks][1] = u.y;
-            }
+            for (int bp = 0; bp < 2; bp++) o.q_frag[0][(ks0 + bp) * 32 + ln] = o.q_frag[1][(ks0 + bp) * 32 + ln] = make_uint2(0u, 0u);
         }
     }
-    if constexpr (PRECISE) {
-        // Short contexts: the table's f16 centroids (good to 1e-4) are not averaged out over enough positions, so
-        // what their rounding left over goes into the upper halves of the table slots (free again now that every
-        // warp has its q fragments) and every product gets a second term.
+    // ---- fused append: exactly what the append kernel would store (src/forward.rs:259-285; the rope row of the new
+    // token is the q position's).  The rows also stay in shared memory, where the warp that holds the chunk's last
+    // tile puts them over what the copy brought: nothing waits for a round trip through global memory.
+    if (!appender) {
         __syncthreads();
-        constexpr int kIdxMask = (1 << BITS) - 1;
-        const float c_lo = a.book[lane & kIdxMask] * lut_alpha;
-        for (int e = warp; e < 256; e += kMW) {
-            const float lo = __shfl_sync(0xffffffffu, c_lo, e & kIdxMask), hi = __shfl_sync(0xffffffffu, c_lo, (e >> 4) & kIdxMask);
-            const float2 hf = __half22float2(__floats2half2_rn(lo, hi));
-            *reinterpret_cast<__half2 *>(lut_ptr + e * 256 + 128 + lane * 4) = __floats2half2_rn(lo - hf.x, hi - hf.y);
+    } else if (role < 0) {
+        asm volatile("bar.arrive 3, 256;\n" ::: "memory");
+        asm volatile("bar.sync 2, 256;\n" ::: "memory");  // does not wait for the appending warps' rows
+    } else {
+        asm volatile("bar.arrive 2, 256;\n" ::: "memory");
+        float *sx = o.new_row[role];
+        prepare_new_row(a, role, lane, new_lo, new_hi, sx, o.rope_row);
+        uint64_t packed;
+        const float n = quantize_new_row<BITS>(sx, lane, o.givens, o.book[role], packed);
+        store_group8<BITS>(o.new_packed[role], lane, packed);
+        if (lane == 0) o.new_norm[role] = n;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(app_bar);
+        const size_t row = seq_rows + (size_t)(n_pos - 1) * a.n_kv + kv;
+        store_group8<BITS>((role == 0 ? a.k_rows_w : a.v_rows_w) + row * kRowBytes, lane, packed);
+        if (lane == 0) (role == 0 ? a.k_norms_w : a.v_norms_w)[row] = n;
+        asm volatile("bar.sync 3, 256;\n" ::: "memory");  // every q fragment is written
+    }
+    static_assert(kMT == 256, "barriers 2 and 3 count 256 threads");
+    uint32_t qh[16][2], ql[QSPLIT ? 16 : 1][2];
+#pragma unroll
+    for (int ks = 0; ks < 16; ks++) {
+        const uint2 v = o.q_frag[0][ks * 32 + lane];
+        qh[ks][0] = v.x;
+        qh[ks][1] = v.y;
+        if constexpr (QSPLIT) {
+            const uint2 u = o.q_frag[1][ks * 32 + lane];
+            ql[ks][0] = u.x;
+            ql[ks][1] = u.y;
         }
-        __syncthreads();
     }
     BK_STAMP(2);
-    // ---- fused append: warps 0 and 1 of the CTA that scans the last chunk of this kv head store the
-    // head's new K and V rows, exactly as the append kernel would (src/forward.rs:259-285; the rope
-    // row of the new token is the q position's).  Only the chunk's last tile sees those rows; it is
-    // issued by warp 0 after both rows are stored and fenced.
-    bool inject = false;
-    if (appender && warp < 2) {
-        const float *src = (warp == 0 ? a.new_k : a.new_v) + ((size_t)meta.slot[s] * a.n_kv + kv) * kHd;
-        float *sx = o.new_row[warp];
-        const float *book = o.book[warp];
-        reinterpret_cast<float4 *>(sx)[lane] = reinterpret_cast<const float4 *>(src)[lane];
-        reinterpret_cast<float4 *>(sx)[lane + 32] = reinterpret_cast<const float4 *>(src)[lane + 32];
+    // The new rows over the chunk's last tile, in shared memory.
+    auto patch_tile = [&](uint32_t st_addr) {
+        wait_bar(app_bar, 0, lane, err_flag);
+        const uint32_t r = (uint32_t)(n_pos - 1) % kTile, half_sel = (uint32_t)lane >> 3, ch = (uint32_t)lane & 7u;
+        if (lane < 16 && ch < (uint32_t)(kRowBytes / 16)) {
+            const uint32_t pos = BITS == 4 ? ch ^ (r & 7u) : BITS == 2 ? ch ^ ((r >> 1) & 3u) : ch;  // the tile's swizzle
+            const uint4 v = *reinterpret_cast<const uint4 *>(&o.new_packed[half_sel][ch * 16]);
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(st_addr + half_sel * kTileBytes + r * kRowBytes + (pos << 4)), "r"(v.x), "r"(v.y),
+                         "r"(v.z), "r"(v.w)
+                         : "memory");
+        } else if (lane == 16 || lane == 17) {
+            const uint32_t which = (uint32_t)lane - 16u;
+            asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(st_addr + 2 * kTileBytes + which * norm_pad + (r * (uint32_t)a.n_kv + (uint32_t)kv) * 4u),
+                         "f"(o.new_norm[which])
+                         : "memory");
+        }
+        asm volatile("fence.proxy.async;\n" ::: "memory");  // (a later copy may refill the stage)
         __syncwarp();
-        if (warp == 0 && a.k_norm_w) {  // per-head RMSNorm of the new k row, bit-exact (src/forward.rs:244-245)
-            float sc = 0.f;
-            if (lane == 0) sc = rms_scale_ref(sx, kHd, a.eps);
-            sc = __shfl_sync(0xffffffffu, sc, 0);
-            for (int i = lane; i < kHd; i += 32) sx[i] = __fmul_rn(__fmul_rn(sx[i], sc), a.k_norm_w[i]);
-            __syncwarp();
-        }
-        if (warp == 0 && !a.no_rope) {
-            const int half = a.n_rot >> 1;
-            for (int j = lane; j < half; j += 32) {
-                float x0 = sx[j], x1 = sx[j + half];
-                rope_pair(x0, x1, o.rope_row[j]);
-                sx[j] = x0;
-                sx[j + half] = x1;
-            }
-            __syncwarp();
-        }
-        float n = 0.f;
-        if (lane == 0) n = serial_norm(sx, kHd);
-        n = __shfl_sync(0xffffffffu, n, 0);
-        const float inv = (n > 1e-12f) ? __fdiv_rn(1.0f, n) : 0.0f;
-        uint64_t packed = 0;
-#pragma unroll
-        for (int pr = 0; pr < 4; pr++) {
-            const int i = lane * 4 + pr;  // pair index: coordinates 2i, 2i+1
-            float r0, r1;
-            givens_fwd(__fmul_rn(sx[2 * i], inv), __fmul_rn(sx[2 * i + 1], inv), o.givens[2 * i], o.givens[2 * i + 1], r0, r1);
-            packed |= (uint64_t)nearest_centroid_fast<BITS>(r0, book) << (BITS * (2 * pr));
-            packed |= (uint64_t)nearest_centroid_fast<BITS>(r1, book) << (BITS * (2 * pr + 1));
-        }
-        const size_t row = seq_rows + (size_t)(n_pos - 1) * a.n_kv + kv;
-        store_group8<BITS>((warp == 0 ? a.k_rows_w : a.v_rows_w) + row * kRowBytes, lane, packed);
-        if (lane == 0) (warp == 0 ? a.k_norms_w : a.v_norms_w)[row] = n;
-        __threadfence();
-        asm volatile("fence.proxy.async;\n" ::: "memory");  // generic-proxy stores before the TMA reads of the last tile
-        __syncwarp();
-        if (warp == 1) {
-            asm volatile("bar.arrive 1, 64;\n" ::: "memory");
-        } else {
-            asm volatile("bar.sync 1, 64;\n" ::: "memory");      // the V row of warp 1 is stored too
-            asm volatile("fence.proxy.async;\n" ::: "memory");
-            inject = true;
-        }
-    }
+    };
     BK_STAMP(3);
 
     float acc[16][4];
@@ -707,11 +662,6 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
 
     // ---- scan: the stages are used round robin; a freed stage takes the tile drawn one step earlier
     {
-        if (inject && in_stage[0] < 0) {  // a chunk so short that warp 0 holds nothing yet
-            in_stage[0] = n_tiles - 1;
-            issue_tile(n_tiles - 1, 0);
-            inject = false;
-        }
         const uint32_t ctr_addr = other_addr + (uint32_t)offsetof(Other, next_tile);
         int drawn = 0;
         auto draw = [&]() {
@@ -737,19 +687,20 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
 #ifdef BK_PHASE
                 if (!(a.dyn & 2))  // tuning builds: dyn bit 1 = stream the tiles without computing on them
 #endif
-                compute_tile(lt, stage_of(st));
+                {
+                    const uint32_t st_addr = stage_of(st);
+                    if (appender && lt == n_tiles - 1) patch_tile(st_addr);
+                    compute_tile(lt, st_addr);
+                }
                 __syncwarp();  // every lane has read the stage: lane 0 may refill it
                 int nu;
-                if (inject) {  // warp 0 of the appending CTA: the rows are stored, take their tile now
-                    nu = n_tiles - 1;
-                    inject = false;
-                } else if (dyn) {
+                if (dyn) {
                     nu = __shfl_sync(0xffffffffu, drawn, 0);
-                    if (nu < n_pool) draw();  // the draw after this one
+                    if (nu < n_tiles) draw();  // the draw after this one
                     else nu = -1;
                 } else {
                     nu = fixed_tile(i_next++);
-                    if (nu >= n_pool) nu = -1;
+                    if (nu >= n_tiles) nu = -1;
                 }
                 if (nu >= 0) issue_tile(nu, st);
                 else n_held--;
@@ -778,22 +729,32 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
         o.l_w[warp][2 * t + 1] = l1;
     }
     __syncthreads();  // every warp is also done with the lookup table
+    // every lane finds the maxima of its own two heads; the sums are one warp's work beside it
+    float Ma = -CUDART_INF_F, Mb = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < kMW; w++) {
+        Ma = fmaxf(Ma, o.m_w[w][2 * t]);
+        Mb = fmaxf(Mb, o.m_w[w][2 * t + 1]);
+    }
     if (tid < 8) {
         float M = -CUDART_INF_F;
+#pragma unroll
         for (int w = 0; w < kMW; w++) M = fmaxf(M, o.m_w[w][tid]);
         float Ls = 0.f;
+#pragma unroll
         for (int w = 0; w < kMW; w++)
-            if (o.m_w[w][tid] > -CUDART_INF_F) Ls += o.l_w[w][tid] * exp2f(o.m_w[w][tid] - M);
+            if (o.m_w[w][tid] > -CUDART_INF_F) Ls += o.l_w[w][tid] * fast_exp2(o.m_w[w][tid] - M);
         o.M[tid] = M;
         o.L[tid] = Ls;
     }
-    __syncthreads();
     float *area = reinterpret_cast<float *>(lut_ptr);  // [kMW][NREP][kHeadStride], reuses the table
-    static_assert((size_t)kMW * 6 * kHeadStride * sizeof(float) <= kLutBytes, "merge area does not fit the table");
+    // (NREP <= 6: the combine's scratch follows the merge area in the ring behind the table, whose stages are drained)
+    constexpr uint32_t kMergeBytes = (kMW * NREP * kHeadStride * 4 + 15) & ~15;
+    static_assert(kMergeBytes <= kLutBytes, "merge area does not fit the table");
     {
         const float unscale = 1.0f / (kWScale * lut_alpha);
-        const float f0 = (M0 > -CUDART_INF_F) ? exp2f(M0 - o.M[2 * t]) * unscale : 0.f;
-        const float f1 = (M1 > -CUDART_INF_F) ? exp2f(M1 - o.M[2 * t + 1]) * unscale : 0.f;
+        const float f0 = (M0 > -CUDART_INF_F) ? fast_exp2(M0 - Ma) * unscale : 0.f;
+        const float f1 = (M1 > -CUDART_INF_F) ? fast_exp2(M1 - Mb) * unscale : 0.f;
         float *w0 = area + ((size_t)warp * NREP + 2 * t) * kHeadStride + g * 33;
         float *w1 = w0 + kHeadStride;
 #pragma unroll
@@ -819,6 +780,14 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
             for (int w = 0; w < kMW; w++) sums[r] += area[((size_t)w * NREP + r) * kHeadStride + idx];
         }
     }
+    BK_STAMP(5);
+    const int first_item = meta.item_start[s] + kv * n_chunks;
+    if (a.dist && n_chunks > 1) {  // the ring before the table and behind it is free: every tile has been consumed
+        float *red = reinterpret_cast<float *>(lut_ptr + kMergeBytes);
+        combine_slice<NREP>(a, meta.slot[s], kv, chunk, n_chunks, first_item, sums, o.M, o.L, red, &o.last, true, o.givens, err_flag);
+        BK_STAMP(9);
+        return;
+    }
     __syncthreads();
     float *s_acc = area;  // [NREP][256]
 #pragma unroll
@@ -833,9 +802,7 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     fs.bar = other_addr + (uint32_t)offsetof(Other, fin_bar);
     fs.ptr = smem_raw + (fs.addr - base);
     fs.err_flag = err_flag;
-    BK_STAMP(5);
-    const int first_item = meta.item_start[s] + kv * n_chunks;
-    finish_item<NREP, true>(a, meta.slot[s], s, kv, item, n_chunks, first_item, s_acc, o.M, o.L, &o.last, true, o.givens, fs);
+    finish_item<NREP, true>(a, meta.slot[s], s, kv, first_item + chunk, n_chunks, first_item, s_acc, o.M, o.L, &o.last, true, o.givens, fs);
     BK_STAMP(9);
 }
 

@@ -114,6 +114,32 @@ __device__ __forceinline__ float serial_norm(const float *x, int n) {
     return __fsqrt_rn(acc);
 }
 
+// The sequential sum of 256 squares of both rules below, of a 16-byte aligned row in shared memory: the next 32 values
+// are on their way while the chain of additions works on the last 32 (1.0 -> 0.6 us; the chain alone is 0.5).
+__device__ __forceinline__ float serial_sumsq256(const float *row) {
+    const float4 *x = reinterpret_cast<const float4 *>(row);
+    float4 cur[8], nxt[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) cur[i] = x[i];
+    float acc = 0.0f;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (b < 7) nxt[i] = x[8 * (b + 1) + i];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            acc = __fadd_rn(acc, __fmul_rn(cur[i].x, cur[i].x));
+            acc = __fadd_rn(acc, __fmul_rn(cur[i].y, cur[i].y));
+            acc = __fadd_rn(acc, __fmul_rn(cur[i].z, cur[i].z));
+            acc = __fadd_rn(acc, __fmul_rn(cur[i].w, cur[i].w));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) cur[i] = nxt[i];
+    }
+    return acc;
+}
+
 // src/kernels.rs:112-116 (rms_norm_rows): sequential f32 sum of squares, then
 // 1 / sqrt(ss / n + eps); the row is then (x * scale) * w, two roundings, left to right (:118).
 __device__ __forceinline__ float rms_scale_ref(const float *x, int n, float eps) {

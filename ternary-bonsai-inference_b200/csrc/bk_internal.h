@@ -23,12 +23,12 @@ constexpr int kScratchStride = kHd + 4; // floats per partial in the split-K scr
 constexpr int kMmaMinPos = 2048;       // 4-, 3- and 2-bit caches: launches with a shorter sequence carry the table's rounding remainders
 constexpr int kRowMinPos = 128;        // sequences shorter than this take the generic f32 decode kernel (speed only)
 constexpr int kMaxWorld = 8;            // ranks a context-split mailbox can connect
-// The arrival counters of the split-K scratch, one per (sequence in the launch, kv head) pair i (i < 512),
-// in three sets of kCtrSet: set 0 for the generic kernel, whose last arriver puts its counter back to zero;
-// sets 1 and 2 for the tensor-core kernels, which alternate between them from launch to launch: a launch
-// counts in one set and clears what the launch before the previous one left in the other, so that no CTA
-// has to stay behind to reset anything.
-constexpr int kCtrSet = 512, kCtrTotal = 3 * kCtrSet;
+// Arrival counters of the split-K scratch, one per (sequence in the launch, kv head) pair; the last arriver puts its counter back to zero.
+constexpr int kCounters = 512;
+// Floats per work item and q head in the boxes of the slice combine (bk_decode_common.cuh): a chunk's 256 values cut into
+// slices, and an (m, l) pair per slice.
+constexpr int kBoxFloats = 384;
+constexpr int kFactorCap = 256;        // chunks whose rescale factors the combine caches in shared memory
 constexpr int kDescSlots = 8;          // launches of bk_append_batch that may be in flight
 constexpr int kDescCap = 4096;         // tokens one bk_append_batch call may carry
 
@@ -91,8 +91,8 @@ struct bk_ctx {
     // split-K scratch of the decode kernel: partial results and arrival counters
     float *d_partials = nullptr;
     unsigned *d_counters = nullptr;
-    int ctr_set = 0;               // which of the two tensor-core counter sets the next launch counts in
-    int ctr_dirty[2] = {0, 0};     // entries of each set that a launch has left non-zero
+    float *d_boxes = nullptr;      // slice combine of the tensor-core kernels: kBoxFloats x kMaxRep per SM, empty between launches
+    size_t box_bytes = 0;
     // Set by a kernel whose bounded wait ran out (the code says which wait).  The word lives in pinned host
     // memory that the device writes directly, so every host-side wait for the stream can look at it for free.
     int *d_err = nullptr;          // device view
@@ -246,11 +246,9 @@ struct DecodeArgs {
     //         fixed shares (off by default: with it the last bits of a result depend on timing)
     //   dist  every CTA of the launch is resident at once (items <= SMs): the split-K combine is
     //         done in slices by all CTAs of a kv head instead of by the last one to arrive
-    //   counters_other / other_n  the counter set the next launch will count in, and how many of its
-    //         entries an earlier launch has left non-zero: CTA 0 clears them
+    //   boxes where the chunks' results travel then
     int dyn, dist;
-    unsigned *counters_other;
-    int other_n;
+    float *boxes;
 };
 bk_status launch_decode(bk_ctx *ctx, const DecodeArgs &a, const DecodeMeta &m);
 

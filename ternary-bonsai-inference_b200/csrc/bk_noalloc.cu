@@ -35,7 +35,7 @@ namespace bk {
 namespace {
 
 constexpr int kStaticItems = 512;     // work items one call may create
-constexpr int kStaticCounters = kCtrTotal; // three counters per (sequence-in-call, kv head) pair, up to 512 pairs
+constexpr int kStaticCounters = kCounters; // a counter per (sequence-in-call, kv head) pair, up to 512 pairs
 constexpr int kStaticSeqs = kMaxSeqsPerLaunch;
 
 // The scratch itself.  In host code these names are only handles for the runtime: the device
