@@ -711,6 +711,36 @@ def test_fused_step_on_long_f16_cache(bk, gpu_ctx, oracle):
     cache.close()
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [("f16", MODE_F16, 0, False), ("f32", MODE_F32, 0, False), ("planar4", MODE_PLANAR, 4, True),
+                                              ("planar3", MODE_PLANAR, 3, True), ("planar2", MODE_PLANAR, 2, True), ("planar4k", MODE_PLANAR, 4, False)])
+@pytest.mark.parametrize("n_head,n_kv", [(6, 1), (8, 2), (24, 4)])
+def test_chunks_of_one_launch_meet_without_counters(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv):
+    """The split-K combine sends slices between the chunks of a launch: one chunk, two, a few, one per SM; new rows on
+    the first and the last row of a tile; q at an address that is no multiple of 16.  A second launch over the same
+    rows gives the same bits (every word that travelled was taken and the space is empty again)."""
+    rng = np.random.default_rng(7)
+    for n0 in (1, 31, 32, 96, 128, 159, 192, 300, 1000, 4800):
+        k = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
+        v = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
+        q = rng.standard_normal((n_head, HD)).astype(np.float32)
+        cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n0 + 8, n_head=n_head, n_kv=n_kv)
+        cache.append(0, k[:n0], v[:n0])
+        ref = oracle.cache(mode, bits, vq, n_head=n_head, n_kv=n_kv)
+        for p in range(n0):
+            ref.append(0, k[p], v[p], p)
+        want = ref.step(0, q, k[n0], v[n0], n0, threads=8)
+        got = bk.full_attention_step(cache, 0, q, k[n0], v[n0], n0)
+        assert_close(got, want, f"{tag} {n0}")
+        compare_dumps(cache.dump_kv(0, pos0=n0 - 1), {key: val[n0 - 1:] for key, val in ref.dump(0).items()})
+        shifted = gpu_ctx.to_device(np.concatenate([np.zeros(1, np.float32), q.ravel()]))
+        out = gpu_ctx.alloc(q.nbytes)
+        for _ in range(3):
+            cache.decode_device(0, shifted.offset(4), out.ptr)
+            again = out.download(q.shape, np.float32)
+            assert np.array_equal(again.view(np.uint32), got.reshape(q.shape).view(np.uint32)), f"{tag} {n0}"
+        cache.close()
+
+
 ROW_KERNEL_MODES = [("f32", MODE_F32, 0, False), ("planar4k", MODE_PLANAR, 4, False), ("planar3k", MODE_PLANAR, 3, False),
                     ("planar2", MODE_PLANAR, 2, True)]   # (planar2: the 4-bit kernel with 2-bit rows widened to nibbles)
 
