@@ -764,6 +764,7 @@ void fill_decode_args(const bk_cache *c, int layer, int partial, DecodeArgs *out
     a.givens = ctx->d_givens;
     a.bits = c->cfg.mode.kind == BK_MODE_PLANAR ? c->cfg.mode.bits : 0;
     a.book = a.bits ? ctx->d_codebooks + (a.bits - 1) * kBookStride : nullptr;
+    for (int i = 0; i < 16; i++) a.book16[i] = c->cfg.mode.bits >= 1 && c->cfg.mode.bits <= 4 && i < (1 << c->cfg.mode.bits) ? ctx->h_codebooks[(c->cfg.mode.bits - 1) * kBookStride + i] : 0.f;
     a.n_head = c->cfg.n_head;
     a.n_kv = c->cfg.n_kv;
     a.k_kind = c->k_kind;

@@ -161,7 +161,6 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     if (tid == 2) mbar_init(app_bar, 2);
     if (tid == 3) o.last = 1;  // the slice combine's waits have not run out
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    __syncthreads();
 
     // ---- which item ------------------------------------------------------------------------
     const int item = blockIdx.x;
@@ -228,18 +227,21 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     if constexpr (kPlanarK) {
         for (int i = tid; i < kHd; i += kFT) o.givens[i] = a.givens[i];
         constexpr int kIdxMask = (1 << (kPlanarK ? kBits : 1)) - 1;
-        if (tid < 16) o.book[tid] = tid <= kIdxMask ? a.book[tid] : 0.f;
+        if (tid < 16) o.book[tid] = a.book16[tid];
         // the lookup table: entry e -> half2(alpha * c[low nibble], alpha * c[high nibble]), one copy per lane
         uint8_t *lut_ptr = smem_raw + (lut_addr - base);
-        const float c_lo = a.book[lane & kIdxMask] * lut_alpha;
-        for (int e = warp; e < 256; e += kFW) {
+        const float c_lo = a.book16[lane & kIdxMask] * lut_alpha;
+        // (eight lanes write an entry, 16 bytes each).  The upper half of the slot: what the rounding to f16 left over
+        // (the V rows of this mode are raw activations, so the scores need more than the table's 11 bits; see
+        // compute_scores).
+        for (int e = warp * 4 + (lane >> 3); e < 256; e += kFW * 4) {
             const float lo = __shfl_sync(0xffffffffu, c_lo, e & kIdxMask), hi = __shfl_sync(0xffffffffu, c_lo, (e >> 4) & kIdxMask);
             const __half2 hv = __floats2half2_rn(lo, hi);
             const float2 hf = __half22float2(hv);
-            *reinterpret_cast<__half2 *>(lut_ptr + e * 256 + lane * 4) = hv;
-            // the upper half of the slot: what the rounding to f16 left over (the V rows of this mode are raw
-            // activations, so the scores need more than the table's 11 bits; see compute_scores)
-            *reinterpret_cast<__half2 *>(lut_ptr + e * 256 + 128 + lane * 4) = __floats2half2_rn(lo - hf.x, hi - hf.y);
+            const __half2 rv = __floats2half2_rn(lo - hf.x, hi - hf.y);
+            const uint32_t u = *reinterpret_cast<const uint32_t *>(&hv), w = *reinterpret_cast<const uint32_t *>(&rv);
+            *reinterpret_cast<uint4 *>(lut_ptr + e * 256 + (lane & 7) * 16) = make_uint4(u, u, u, u);
+            *reinterpret_cast<uint4 *>(lut_ptr + e * 256 + 128 + (lane & 7) * 16) = make_uint4(w, w, w, w);
         }
     }
     __syncthreads();  // tables and barriers are ready

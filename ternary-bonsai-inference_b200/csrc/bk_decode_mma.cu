@@ -250,18 +250,16 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     // it overlaps the tail of the previous kernel in the stream.  Everything a previous kernel may
     // have written (q, the newest cache row, the split-K scratch) is read after the wait below.
     {
-        for (int i = tid; i < kHd; i += kMT) o.givens[i] = a.givens[i];
-        if (!a.no_rope) {
-            const int half = a.n_rot >> 1;
-            const float2 *cs = a.rope + (size_t)meta.q_pos[s] * half;
-            for (int i = tid; i < half; i += kMT) o.rope_row[i] = cs[i];
-        }
-        if (a.q_norm_w)
-            for (int i = tid; i < kHd; i += kMT) o.qw[i] = a.q_norm_w[i];
-        if (tid < 2 * 16) o.book[tid >> 4][tid & 15] = (tid & 15) < (1 << BITS) ? a.book[tid & 15] : 0.f;
-        if (tid == 0) o.next_tile = kMW * n_stages;  // the first n_stages tiles of every warp are fixed
+        // (the loads of the small tables fly while the lookup table is built; the centroids come with the parameters)
+        static_assert(kMT == kHd, "a thread per coordinate");
+        const int half = a.no_rope ? 0 : a.n_rot >> 1;
+        const float g_reg = a.givens[tid];
+        const float2 r_reg = tid < half ? a.rope[(size_t)meta.q_pos[s] * half + tid] : make_float2(0.f, 0.f);
+        const float w_reg = a.q_norm_w ? a.q_norm_w[tid] : 0.f;
         constexpr int kIdxMask = (1 << BITS) - 1;
-        const float c_lo = a.book[lane & kIdxMask] * lut_alpha;  // the low lanes hold the scaled centroids
+        const float c_lo = a.book16[lane & kIdxMask] * lut_alpha;  // the low lanes hold the scaled centroids
+        if (tid < 2 * 16) o.book[tid >> 4][tid & 15] = a.book16[tid & 15];
+        if (tid == 0) o.next_tile = kMW * n_stages;  // the first n_stages tiles of every warp are fixed
         // The lookup table: entry e -> half2(alpha*c[low nibble], alpha*c[high nibble]), one copy per lane; PRECISE
         // (short contexts: the table's f16 centroids, good to 1e-4, are not averaged out over enough positions): what
         // their rounding left over goes into the upper half of the slot and every product gets a second term.
@@ -279,6 +277,9 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
                 *reinterpret_cast<uint4 *>(lut_ptr + e * 256 + 128 + (lane & 7) * 16) = make_uint4(w, w, w, w);
             }
         }
+        o.givens[tid] = g_reg;
+        if (tid < half) o.rope_row[tid] = r_reg;
+        o.qw[tid] = w_reg;
     }
     __syncthreads();  // tables and barriers are ready; from here to the end of the scan the warps run on their own
     BK_STAMP(0);

@@ -207,6 +207,7 @@ struct DecodeArgs {
     const float2 *rope;
     int n_rot;
     const float *givens, *book;
+    float book16[16];                // widths up to 4: the codebook again, for set-up code that should not wait for a load
     int bits, n_head, n_kv, k_kind, v_kind;
     size_t k_row_bytes, v_row_bytes;
     float *partials;
