@@ -371,8 +371,8 @@ BK_API size_t bk_kvq_packed_len(int32_t hd, int32_t bits);
 BK_API bk_status bk_kvq_codebook(int32_t hd, int32_t bits, float *out_host);
 /* givens_table(d) (src/kvquant.rs:131-145): ceil(hd/2) (cos, sin) pairs. */
 BK_API bk_status bk_kvq_givens(int32_t hd, float *out_host);
-/* No counterpart in the reference: the table behind the bulk append's nearest-centroid search for head
- * dimension 256 and widths 1..4, for checking that search against the reference's scan
+/* No counterpart in the reference: the decision thresholds behind the bulk append's nearest-centroid search for head
+ * dimension 256 and widths 1..4, for checking them against the reference's scan
  * (src/kvquant.rs:357-370) without a GPU.  512 cells of width 2^-10 over [-0.25, 0.25): out_host[2k] = how
  * many decision thresholds lie in cells below k, out_host[2k + 1] = the bits of the one threshold inside
  * cell k (+inf if none).  nearest(v) = out[2k] + (v >= threshold) with k = clamp(floor((v + 0.25) * 1024)),

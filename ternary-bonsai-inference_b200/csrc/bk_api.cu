@@ -20,10 +20,9 @@ namespace bk {
 // Scale alpha in [1, 2) that minimises the worst relative error of f16(alpha * c) / alpha over a
 // codebook: the centroids are only 2^bits distinct values, so a good alpha makes all of them
 // round almost exactly and the tensor-core path loses nothing to the f16 table.
-// Host side of nearest_centroid_thr() (bk_device.cuh): the 512 (count, threshold) cells of one ascending
-// codebook of n <= 16 centroids.  Everything is computed with the kernels' own single-precision operations
-// (this file is built without floating-point contraction).  Returns false if a cell would hold two thresholds.
-static bool build_threshold_cells(const float *book, int n, uint2 *tab) {
+// The decision thresholds of one ascending codebook of n centroids: thr[i] is the smallest float for which the reference's
+// scan moves from centroid i to i + 1.  false: a centroid never wins.
+static bool find_thresholds(const float *book, int n, float *thr) {
     auto key = [](float f) -> int64_t {  // floats in ascending order as integers
         int32_t b;
         memcpy(&b, &f, 4);
@@ -35,14 +34,6 @@ static bool build_threshold_cells(const float *book, int n, uint2 *tab) {
         memcpy(&f, &b, 4);
         return f;
     };
-    auto cell_of = [](float v) -> int {
-        volatile float t = v + 0.25f;
-        volatile float u = t * 1024.0f;
-        const int c = (int)floorf(u);
-        return c < 0 ? 0 : (c > 511 ? 511 : c);
-    };
-    float thr[16];
-    int thr_cell[16];
     for (int i = 0; i + 1 < n; i++) {
         const float c0 = book[i], c1 = book[i + 1];
         auto beats = [&](float v) {  // does the scan move from centroid i to i + 1 at v?
@@ -57,6 +48,45 @@ static bool build_threshold_cells(const float *book, int n, uint2 *tab) {
             else lo = mid;
         }
         thr[i] = unkey(hi);
+    }
+    return true;
+}
+
+// Host side of nearest_centroid_lanes() (bk_device.cuh).  false: two thresholds fall into one cell.
+static bool build_lane_cells(const float *book, int n, LaneCells *out) {
+    float thr[16], far = 0.05f;
+    if (!find_thresholds(book, n, thr)) return false;
+    for (int i = 0; i + 1 < n; i++) far = std::max(far, fabsf(thr[i]) * 1.03125f);
+    out->scale = 0.5f / far;
+    int cell_of[16];
+    for (int i = 0; i + 1 < n; i++) {
+        const float u = std::min(1.0f, std::max(0.0f, fmaf(thr[i], out->scale, 0.5f)));
+        cell_of[i] = (int)floor((double)u * (double)kLaneCells);  // (an exact product)
+        if (i > 0 && cell_of[i] <= cell_of[i - 1]) return false;
+    }
+    for (int k = 0; k < 32; k++) {
+        out->cell[k] = LaneCell{0, INFINITY};
+        for (int i = 0; i + 1 < n; i++) {
+            if (cell_of[i] < k) out->cell[k].below++;
+            else if (cell_of[i] == k) out->cell[k].thr = thr[i];
+        }
+    }
+    return true;
+}
+
+// The same thresholds in 512 cells of width 2^-10 over [-0.25, 0.25) (bk_kvq_threshold_cells), for programs that look the
+// index up in memory.
+static bool build_threshold_cells(const float *book, int n, uint2 *tab) {
+    auto cell_of = [](float v) -> int {
+        volatile float t = v + 0.25f;
+        volatile float u = t * 1024.0f;
+        const int c = (int)floorf(u);
+        return c < 0 ? 0 : (c > 511 ? 511 : c);
+    };
+    float thr[16];
+    int thr_cell[16];
+    if (!find_thresholds(book, n, thr)) return false;
+    for (int i = 0; i + 1 < n; i++) {
         thr_cell[i] = cell_of(thr[i]);
         if (i > 0 && thr_cell[i] <= thr_cell[i - 1]) return false;  // two thresholds in one cell (or out of order)
     }
@@ -273,17 +303,16 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
         ctx->dist_combine = !(e6 && e6[0] == '0');
     }
     if ((e = cudaMalloc(&ctx->d_givens, sizeof(ctx->h_givens))) != cudaSuccess) return bail(e, "cudaMalloc givens");
-    {   // the threshold cells of the widths 1..4 (the append kernel's nearest-centroid search)
-        std::vector<uint2> tabs(4 * 512);
+    {   // the threshold cells of the widths 1..4 (nearest-centroid search of the bulk append and the quantizer)
+        LaneCells cells[4] = {};
         for (int b = 1; b <= 4; b++)
-            if (!build_threshold_cells(ctx->h_codebooks + (b - 1) * kBookStride, 1 << b, tabs.data() + (b - 1) * 512)) {
+            if (!build_lane_cells(ctx->h_codebooks + (b - 1) * kBookStride, 1 << b, &cells[b - 1])) {
                 fail(nullptr, BK_ERR_UNSUPPORTED, "codebook thresholds do not fit the cell table");
                 bk_ctx_destroy(ctx);
                 return BK_ERR_UNSUPPORTED;
             }
-        if ((e = cudaMalloc(&ctx->d_cell_tabs, tabs.size() * sizeof(uint2))) != cudaSuccess) return bail(e, "cudaMalloc cell tables");
-        if ((e = cudaMemcpy(ctx->d_cell_tabs, tabs.data(), tabs.size() * sizeof(uint2), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(e, "cudaMemcpy cell tables");
+        if ((e = cudaMalloc(&ctx->d_lane_cells, sizeof(cells))) != cudaSuccess) return bail(e, "cudaMalloc cell tables");
+        if ((e = cudaMemcpy(ctx->d_lane_cells, cells, sizeof(cells), cudaMemcpyHostToDevice)) != cudaSuccess) return bail(e, "cudaMemcpy cell tables");
     }
     if ((e = cudaMalloc(&ctx->d_codebooks, sizeof(ctx->h_codebooks))) != cudaSuccess)
         return bail(e, "cudaMalloc codebooks");
@@ -328,7 +357,7 @@ void bk_ctx_destroy(bk_ctx *ctx) {
     ctx->ropes.clear();
     if (ctx->d_givens) cudaFree(ctx->d_givens);
     if (ctx->d_codebooks) cudaFree(ctx->d_codebooks);
-    if (ctx->d_cell_tabs) cudaFree(ctx->d_cell_tabs);
+    if (ctx->d_lane_cells) cudaFree(ctx->d_lane_cells);
     if (ctx->d_partials) cudaFree(ctx->d_partials);
     if (ctx->d_counters) cudaFree(ctx->d_counters);
     if (ctx->d_boxes) cudaFree(ctx->d_boxes);
@@ -625,7 +654,7 @@ static AppendArgs base_append_args(const bk_cache *c, const float *k, const floa
     a.rope = c->rope->d;
     a.givens = c->ctx->d_givens;
     a.book = c->cfg.mode.kind == BK_MODE_PLANAR ? c->ctx->d_codebooks + (c->cfg.mode.bits - 1) * kBookStride : nullptr;
-    a.cell_tab = (c->cfg.mode.kind == BK_MODE_PLANAR && c->cfg.mode.bits <= 4) ? c->ctx->d_cell_tabs + (c->cfg.mode.bits - 1) * 512 : nullptr;
+    a.cells = (c->cfg.mode.kind == BK_MODE_PLANAR && c->cfg.mode.bits <= 4) ? c->ctx->d_lane_cells + (c->cfg.mode.bits - 1) : nullptr;
     a.seq_stride_rows = (size_t)c->cfg.n_ctx * c->cfg.n_kv;
     a.n_kv = c->cfg.n_kv;
     a.n_rot = c->cfg.n_rot;

@@ -8,8 +8,8 @@
 //      the (cos, sin) row of the token's position from the host-built rope table;
 //   2. planar rows: one warp adds the 256 squares of all 32 vectors, a vector per lane, each lane
 //      in order (the reference's f32 sum is sequential, so each chain is; 32 run side by side);
-//   3. the warps scale, Givens-rotate, find the nearest centroid (one read of a host-built cell table of the
-//      decision thresholds, or a binary search and a neighbour check: the same index as the reference's
+//   3. the warps scale, Givens-rotate, find the nearest centroid (two shuffles from a host-built cell table of
+//      the decision thresholds, or a binary search and a neighbour check: the same index as the reference's
 //      linear scan) and write `bits` bytes per lane;
 //      f32/f16 rows leave as 128-bit stores.
 // Traffic per token is the algorithmic minimum: 2*n_kv*1 KiB in, rows + norms out.
@@ -68,18 +68,16 @@ __device__ __forceinline__ void store_planar_row(const float *sx, int lane, floa
     store_group8<BITS>(row, group, packed);
 }
 
-// The same with the one-read centroid search (codebooks of up to 16 centroids; nearest_centroid_thr in bk_device.cuh).  The bulk
-// kernel is bound by its instructions, so nothing is decided per coordinate: a finite norm bounds every rotated
-// value by 1.5 (a norm is no smaller than any of its coordinates, or it is at most 1e-12 and inv is 0), and then the cell is
-// the low bits of 2^23 + 1024 (v + 0.25), rounded down.  Vectors with an infinite or NaN norm take the scan.
-// (A call of 4096 tokens into a 4-bit cache, with one decode step after it: 35.6 -> 33.9 us.)
+// The same for codebooks of up to 16 centroids (nearest_centroid_lanes in bk_device.cuh).  The bulk kernel is bound by its
+// instructions, so nothing is decided per coordinate: a finite norm bounds every rotated value by 1.5 (a norm is no
+// smaller than any of its coordinates, or it is at most 1e-12 and inv is 0).  Vectors with an infinite or NaN norm take the
+// scan.  A lane takes eight consecutive coordinates (two 128-bit reads, each with two lanes on a bank) and keeps their
+// rotations in registers.
 template <int BITS>
-__device__ __forceinline__ void store_planar_row_thr(const float *sx, int lane, float n, float inv, const float *givens,
-                                                     const float *sbook, uint32_t tab, uint8_t *row) {
-    float x[8];
-    const int group = load_group_of_8(sx, lane, x);  // coordinates 8 group .. 8 group + 7
-    const float4 g0 = reinterpret_cast<const float4 *>(givens)[2 * group], g1 = reinterpret_cast<const float4 *>(givens)[2 * group + 1];
-    const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+__device__ __forceinline__ void store_planar_row_lanes(const float *sx, int lane, float n, float inv, const float (&gv)[8], float scale,
+                                                       LaneCell my, const float *book, uint8_t *row) {
+    const float4 xa = reinterpret_cast<const float4 *>(sx)[2 * lane], xb = reinterpret_cast<const float4 *>(sx)[2 * lane + 1];
+    const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
     float v[8];
 #pragma unroll
     for (int pr = 0; pr < 4; pr++) {
@@ -89,18 +87,12 @@ __device__ __forceinline__ void store_planar_row_thr(const float *sx, int lane, 
     uint32_t packed = 0;  // 8 indices of at most 4 bits
     if (n < CUDART_INF_F) {
 #pragma unroll
-        for (int i = 7; i >= 0; i--) {
-            const float u = fminf(fmaxf(__fadd_rn(v[i], 0.25f), 0.0f), 511.0f / 1024.0f);
-            const uint32_t cell = __float_as_uint(__fmaf_rd(u, 1024.0f, 8388608.0f)) - 0x4b000000u;
-            uint32_t cnt, thr;
-            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(cnt), "=r"(thr) : "r"(tab + 8u * cell));
-            packed = (packed << BITS) + cnt + (v[i] >= __uint_as_float(thr) ? 1u : 0u);
-        }
+        for (int i = 7; i >= 0; i--) packed = (packed << BITS) + nearest_centroid_lanes(v[i], scale, my.below, my.thr);
     } else {
 #pragma unroll
-        for (int i = 7; i >= 0; i--) packed = (packed << BITS) + nearest_centroid(v[i], sbook, 1 << BITS);
+        for (int i = 7; i >= 0; i--) packed = (packed << BITS) + nearest_centroid(v[i], book, 1 << BITS);
     }
-    store_group8<BITS>(row, group, (uint64_t)packed);
+    store_group8<BITS>(row, lane, (uint64_t)packed);
 }
 
 __device__ __forceinline__ void store_f32_row(const float *sx, int lane, uint8_t *row) {
@@ -136,7 +128,6 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
     float *sbook = smem + kVecs * kVecPad;  // centroids
     float *sgiv = sbook + 256;              // Givens table
     float *snorm = sgiv + kHd;              // the 32 norms, and what a vector is scaled by
-    [[maybe_unused]] uint2 *tab = reinterpret_cast<uint2 *>(snorm + 64);    // the 512 cells of the one-read centroid search
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kv = a.n_kv, per_tok = 2 * n_kv;
     const int n_vec = a.n_tokens * per_tok, v0 = blockIdx.x * kVecs;
@@ -145,11 +136,9 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
     auto tok_of = [&](int vec) { return tok_shift >= 0 ? vec >> tok_shift : vec / per_tok; };
     const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
 
-    if (BITS > 0) {
+    if (BITS > 4) {
         for (int i = threadIdx.x; i < (1 << BITS); i += kThreads) sbook[i] = a.book[i];
         for (int i = threadIdx.x; i < kHd; i += kThreads) sgiv[i] = a.givens[i];
-        if constexpr (BITS >= 1 && BITS <= 4)  // built once per context on the host
-            for (int i = threadIdx.x; i < 256; i += kThreads) reinterpret_cast<uint4 *>(tab)[i] = __ldg(reinterpret_cast<const uint4 *>(a.cell_tab) + i);
     }
     // k and v may come from the previous kernel in the stream: with programmatic dependent launch
     // only the table copies above run ahead of it.  Nothing after this kernel depends on more
@@ -211,6 +200,17 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
         }
     }
     __syncthreads();
+    // widths up to 4: this lane's threshold cell (built once per context on the host) and rotations; not before pass 1, whose
+    // loads want the registers
+    [[maybe_unused]] LaneCell my = {0u, 0.f};
+    [[maybe_unused]] float scale = 0.f, gv[8] = {};
+    if constexpr (BITS >= 1 && BITS <= 4) {
+        my = a.cells->cell[lane];
+        scale = a.cells->scale;
+        const float4 g0 = __ldg(reinterpret_cast<const float4 *>(a.givens) + 2 * lane), g1 = __ldg(reinterpret_cast<const float4 *>(a.givens) + 2 * lane + 1);
+        gv[0] = g0.x; gv[1] = g0.y; gv[2] = g0.z; gv[3] = g0.w;
+        gv[4] = g1.x; gv[5] = g1.y; gv[6] = g1.z; gv[7] = g1.w;
+    }
     // ---- pass 2: 32 sequential sums side by side ----------------------------------------------------
     if (planar && warp == 0 && lane < kVecs && v0 + lane < n_vec) {
         const float4 *x4 = reinterpret_cast<const float4 *>(smem + lane * kVecPad);
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
             if constexpr (BITS > 0) {
                 const float n = snorm[lv];
                 if (lane == 0) (is_v ? a.v_norms : a.k_norms)[r] = n;
-                if constexpr (BITS <= 4) store_planar_row_thr<BITS>(sx, lane, n, snorm[32 + lv], sgiv, sbook, (uint32_t)__cvta_generic_to_shared(tab), row);
+                if constexpr (BITS <= 4) store_planar_row_lanes<BITS>(sx, lane, n, snorm[32 + lv], gv, scale, my, a.book, row);
                 else store_planar_row<BITS>(sx, lane, snorm[32 + lv], sgiv, sbook, row);
             }
         }
@@ -272,7 +272,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     const size_t n_vec = (size_t)a.n_tokens * 2 * a.n_kv;
     const bool bulk = n_vec > (size_t)8 * 2 * ctx->n_sms;  // more than two small CTAs per SM: go for throughput
     const int vecs = bulk ? 32 : 8;
-    const size_t smem = (size_t)(vecs * kVecPad + 256 + kHd + 64) * sizeof(float) + 512 * sizeof(uint2);
+    const size_t smem = (size_t)(vecs * kVecPad + 256 + kHd + 64) * sizeof(float);
     const unsigned grid = (unsigned)((n_vec + vecs - 1) / vecs);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);

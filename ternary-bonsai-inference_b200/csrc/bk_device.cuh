@@ -9,6 +9,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "bk_internal.h"
+
 namespace bk {
 
 // src/gguf.rs:914-944.  Round-to-nearest-even on the 13 dropped bits, except that the
@@ -90,22 +92,21 @@ __device__ __forceinline__ uint32_t nearest_centroid_fast(float v, const float *
     return (uint32_t)((d1 < d0) ? hi : lo);
 }
 
-// The same index once more, for codebooks of up to 16 centroids, from ONE 8-byte read.  Along the ascending codebook the scan's answer is the number of
-// thresholds T_i <= v, where T_i is the smallest float for which centroid i + 1 beats centroid i in the scan's
-// own arithmetic (|v - c_{i+1}| < |v - c_i|, both differences rounded to f32; the predicate is monotone in v
-// because f32 subtraction is).  The host finds every T_i by bisection over the floats, with the same rounded
-// operations, and lays them out in 512 cells of width 2^-10 over [-0.25, 0.25) (clamped): cell k holds how many
-// thresholds lie in lower cells and the one threshold inside it (+inf if none; the host checks that no cell
-// holds two).  tab[cell] = (count, threshold bits).  Non-finite and huge v take the scan.
-template <int BITS>
-__device__ __forceinline__ uint32_t nearest_centroid_thr(float v, const float *book, const uint2 *tab) {
-    static_assert(BITS <= 4, "the cell table covers codebooks of up to 16 centroids");
-    if (!(fabsf(v) < 4.0f)) return nearest_centroid(v, book, 1 << BITS);
-    const int cell = min(max(__float2int_rd(__fmul_rn(__fadd_rn(v, 0.25f), 1024.0f)), 0), 511);
-    const uint2 e = tab[cell];
-    return e.x + (v >= __uint_as_float(e.y) ? 1u : 0u);
+// The same index once more, for codebooks of up to 16 centroids, from a table that a warp holds in registers.  Along the
+// ascending codebook the scan's answer is the number of thresholds T_i <= v, where T_i is the smallest float for which
+// centroid i + 1 beats centroid i in the scan's own arithmetic (|v - c_{i+1}| < |v - c_i|, both differences rounded to
+// f32; the predicate is monotone in v because f32 subtraction is).  The host finds every T_i by bisection over the floats,
+// with the same rounded operations, and lays them out in 32 cells of cell(v) = floor(kLaneCells * clamp(v * scale + 1/2)):
+// cell is monotone in v, so a threshold in a lower cell is below v and one in a higher cell above it, and cell k needs to
+// hold only how many thresholds lie in lower cells and the one inside it (+inf if none; the host checks that no cell holds
+// two).  Lane k of the warp keeps cell k, two shuffles fetch it: no bank conflicts, which 32 random reads of a table in
+// shared memory had (3.5 wavefronts for each half warp).  v must be finite; every lane of the warp calls.
+__device__ __forceinline__ uint32_t nearest_centroid_lanes(float v, float scale, uint32_t below, float thr) {
+    const float u = __saturatef(__fmaf_rn(v, scale, 0.5f));
+    const int cell = (int)(__float_as_uint(__fmaf_rd(u, kLaneCells, 8388608.0f)) & 31u);
+    const float t = __shfl_sync(0xffffffffu, thr, cell);
+    return __shfl_sync(0xffffffffu, below, cell) + (v >= t ? 1u : 0u);
 }
-
 // src/kvquant.rs:398: sequential f32 sum of squares then sqrt; 256 dependent adds by design.
 __device__ __forceinline__ float serial_norm(const float *x, int n) {
     float acc = 0.0f;

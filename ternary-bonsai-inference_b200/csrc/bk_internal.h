@@ -41,6 +41,18 @@ void host_rope_rows(int64_t pos0, int64_t n_pos, int n_rot, float freq_base, flo
 // Which of the four position ids (t, h, w, e -> 0..3) pair j takes: src/rope.rs:37-49.
 int host_rope_band(int j, const int32_t sections[4]);
 
+// Nearest-centroid search of the widths up to 4: see nearest_centroid_lanes() in bk_device.cuh.
+constexpr float kLaneCells = 31.999998f;  // the float below 32: the cell of clamp(...) = 1 is 31
+struct LaneCell {
+    uint32_t below;  // thresholds in lower cells
+    float thr;       // the one in this cell
+};
+struct LaneCells {   // one width, in device memory
+    LaneCell cell[32];
+    float scale;
+    float pad[3];
+};
+
 struct RopeTable {
     int n_rot = 0;
     float freq_base = 0.f;
@@ -67,7 +79,7 @@ struct bk_ctx {
     uint64_t launches = 0;
     float *d_givens = nullptr;     // 128 (cos, sin) pairs
     float *d_codebooks = nullptr;  // 8 books, book of width b at (b-1)*kBookStride
-    uint2 *d_cell_tabs = nullptr;  // widths 1..4: 512 (index, threshold) cells each, table of width b at (b-1)*512 (bk_device.cuh)
+    bk::LaneCells *d_lane_cells = nullptr;  // widths 1..4: threshold cells of the nearest-centroid search (bk_device.cuh), width b at b - 1
     float h_givens[bk::kHd];
     float h_codebooks[bk::kMaxBits * bk::kBookStride];
     float lut_alpha[bk::kMaxBits + 1] = {};  // per width: scale applied to centroids before f16 rounding
@@ -177,7 +189,7 @@ struct AppendArgs {
     const float2 *rope;        // [rope_n_pos][n_rot/2]
     const float *givens;
     const float *book;         // codebook of this width (null unless planar)
-    const uint2 *cell_tab;     // widths 1..4: the 512 cells of nearest_centroid_thr() (null otherwise)
+    const LaneCells *cells;    // widths 1..4: the cells of nearest_centroid_lanes() (null otherwise)
     const int4 *desc;          // per token (seq, row, rope_pos, 0); nullptr = contiguous single sequence
     size_t seq_stride_rows;    // rows (pos*n_kv units) between sequences of one layer
     int n_tokens, n_kv, n_rot, bits;

@@ -1,6 +1,8 @@
 // GPU versions of the kvquant.rs / rope.rs / gguf.rs entry points, used for parity checks of
 // the encode/decode format outside a cache.  Each mirrors one reference function and follows
 // its f32 operation order, so results equal the reference CPU path bit for bit.
+#include <math_constants.h>
+
 #include "bk_device.cuh"
 #include "bk_internal.h"
 
@@ -10,16 +12,19 @@ namespace {
 
 // PlanarQuant::quantize, src/kvquant.rs:397-412.  One warp per vector.
 template <int BITS>
-__global__ void quantize_kernel(int n_vec, const float *x, const float *givens, const float *book, const uint2 *cell_tab,
+__global__ void quantize_kernel(int n_vec, const float *x, const float *givens, const float *book, const LaneCells *cells,
                                 uint8_t *packed, float *norms) {
     __shared__ __align__(16) float sx[4][kHd];
     __shared__ float sbook[256];
-    __shared__ __align__(16) uint2 tab[BITS <= 4 ? 512 : 1];  // the cells of the one-read centroid search (up to 16 centroids)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int vec = blockIdx.x * 4 + warp;
     for (int i = threadIdx.x; i < (1 << BITS); i += blockDim.x) sbook[i] = book[i];
-    if constexpr (BITS <= 4)
-        for (int i = threadIdx.x; i < 512; i += blockDim.x) tab[i] = cell_tab[i];
+    [[maybe_unused]] LaneCell my = {0u, 0.f};
+    [[maybe_unused]] float scale = 0.f;
+    if constexpr (BITS <= 4) {
+        my = cells->cell[lane];
+        scale = cells->scale;
+    }
     if (vec < n_vec) {
         const float4 *src = reinterpret_cast<const float4 *>(x + (size_t)vec * kHd);
         reinterpret_cast<float4 *>(sx[warp])[lane] = src[lane];
@@ -39,9 +44,10 @@ __global__ void quantize_kernel(int n_vec, const float *x, const float *givens, 
         float r0, r1;
         givens_fwd(__fmul_rn(sx[warp][2 * i], inv), __fmul_rn(sx[warp][2 * i + 1], inv), givens[2 * i],
                    givens[2 * i + 1], r0, r1);
-        if constexpr (BITS <= 4) {  // the search the bulk append uses
-            word |= (uint64_t)nearest_centroid_thr<BITS>(r0, sbook, tab) << (BITS * (2 * pr));
-            word |= (uint64_t)nearest_centroid_thr<BITS>(r1, sbook, tab) << (BITS * (2 * pr + 1));
+        const uint64_t sh = BITS * (2 * pr);
+        if (BITS <= 4 && n < CUDART_INF_F) {  // the search the bulk append uses (a finite norm: finite coordinates)
+            word |= (uint64_t)nearest_centroid_lanes(r0, scale, my.below, my.thr) << sh;
+            word |= (uint64_t)nearest_centroid_lanes(r1, scale, my.below, my.thr) << (sh + BITS);
         } else {
             word |= (uint64_t)nearest_centroid_fast<BITS>(r0, sbook) << (BITS * (2 * pr));
             word |= (uint64_t)nearest_centroid_fast<BITS>(r1, sbook) << (BITS * (2 * pr + 1));
@@ -134,7 +140,7 @@ bk_status launch_quantize(bk_ctx *ctx, int bits, int n_vec, const float *x, uint
     const float *book = ctx->d_codebooks + (bits - 1) * kBookStride;
     if (!dispatch_bits(bits, [&]<int B>() {
             quantize_kernel<B><<<(n_vec + 3) / 4, 128, 0, ctx->stream>>>(n_vec, x, ctx->d_givens, book,
-                                                                         B <= 4 ? ctx->d_cell_tabs + (B - 1) * 512 : nullptr, packed, norms);
+                                                                         B <= 4 ? ctx->d_lane_cells + (B - 1) : nullptr, packed, norms);
         }))
         return fail(ctx, BK_ERR_INVALID, "bits must be 1..8");
     BK_LAUNCH_DONE(ctx);
