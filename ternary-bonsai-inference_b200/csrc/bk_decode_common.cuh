@@ -144,7 +144,7 @@ __device__ __forceinline__ void exchange_slice(const DecodeArgs &a, int n_rep, i
 // One warp prepares one q head: lane l holds coordinates 8 l .. 8 l + 7.  load() issues every load (the rope partners
 // among them, whatever n_rot), so that tile copies can be issued behind them; finish() applies RMSNorm
 // (src/forward.rs:242-243; q is not stored, so a tree sum will do) and rope.  A warp per head needs no barrier between
-// the steps: q was ready 2.5 us after the dependency wait with the CTA's threads spread over all heads, 1.2 us now.
+// the steps: q was ready 2.5 us after the dependency wait with the CTA's threads spread over all heads, 1.8 us now.
 struct QHead {
     float x[8], y[8];  // the lane's coordinates and their rope partners
     __device__ __forceinline__ void load(const float *row, int lane, int half) {
@@ -258,8 +258,8 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, int lane
 // no sender ever stores.  A word therefore validates itself: the owner of a slice reads it until it is not empty,
 // uses it and empties it again.  No counter, no fence between data and flag, no set-up from launch to launch: one
 // trip through L2 instead of three (stores, ticket, loads of the triples).  What bounds this stage is that trip and
-// the barriers around it; per launch (planar4, 9000 rows) publish + arrive + combine took 4.6 us with a ticket
-// counter and take 1.9 us.
+// the barriers around it; from the last chunk's sums to the end of the launch 4.0 to 4.7 us with a ticket
+// counter, 3.3 us now (planar4 9000 rows, f16 8192 rows).
 //
 // Boxes of a (sequence, kv head) start at first_item * NREP * kBoxFloats:
 //     values  [slice][chunk][NREP][D]     relative to the chunk's maximum, not normalised

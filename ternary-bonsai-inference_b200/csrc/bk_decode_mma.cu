@@ -263,7 +263,7 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
         // The lookup table: entry e -> half2(alpha*c[low nibble], alpha*c[high nibble]), one copy per lane; PRECISE
         // (short contexts: the table's f16 centroids, good to 1e-4, are not averaged out over enough positions): what
         // their rounding left over goes into the upper half of the slot and every product gets a second term.
-        // Eight lanes write an entry with one 16-byte store each (1.4 us of the prologue with a word per lane).
+        // Eight lanes write an entry with one 16-byte store each (with a word per lane the prologue of a CTA took 1.4 us instead of 1.0).
 #pragma unroll 2
         for (int e = warp * 4 + (lane >> 3); e < 256; e += kMW * 4) {
             const float lo = __shfl_sync(0xffffffffu, c_lo, e & kIdxMask), hi = __shfl_sync(0xffffffffu, c_lo, (e >> 4) & kIdxMask);

@@ -11,13 +11,14 @@
 // cudaMalloc/cudaFree, not the host heap, not a tensor library.
 //
 // What it costs: every GPU that loads this library reserves kStaticItems partial results
-// (about 4.3 MB) plus 1024 counters for as long as the process lives, whether or not the entry
+// (about 4.3 MB) plus 512 counters for as long as the process lives, whether or not the entry
 // point is ever called.  One call handles at most 64 sequences (more are rejected, not split); the
 // work of a call is cut into at most kStaticItems (sequence, kv head, chunk) items, with coarser
 // chunks than bk_decode_attn would use if need be, so the two agree within the parity tolerance
 // rather than bit for bit.
 //
-// All calls on a device share the one array.  It keeps whatever the previous call left in it;
+// All calls on a device share the one array (launches whose CTAs are all resident at once meet in the context's boxes
+// instead, which were made with the context).  It keeps whatever the previous call left in it;
 // the only part that must start from zero, the arrival counters, is cleared at the start of
 // every call.  Two calls whose kernels overlap on the GPU (different contexts or streams, or
 // mixed with nothing else - the normal entry points use their own per-context scratch) race on
