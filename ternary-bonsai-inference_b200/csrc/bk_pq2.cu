@@ -121,43 +121,54 @@ __global__ void __launch_bounds__(kPqGroupThreads * kPqMaxGroups) pq2_matvec_ker
     // block's max |x|; the block's 2^(e - 24 - 6) (the products carry 4^3) multiplies its f16 scale.
     // Element jj of a block (32 t + 16 r + 4 q + m: word 2t + r of the block, byte q, slot m) lands in
     // byte q of the word [col][block][t][m][r]; a lane's 8 words of a block are 32 contiguous bytes.
-    for (int unit = warp_all; unit < NT * nb; unit += n_warps) {
-        const int tok = unit / nb, b = unit - tok * nb;
-        const float *xr = a.x + (size_t)tok * a.ne0;
-        const bool real = tok < a.n_tok;  // columns past n_tok are zeros
-        float xv[4], am = 0.f;
+    // A lane makes one word of every digit: word [t][m][r] = its number, so its four elements are 4 apart.
+    const int my_m = (lane >> 1) & 3, my_elem = 32 * (lane >> 3) + 16 * (lane & 1) + my_m;
+    // The loads of a warp's next two units go out together: rows of 5120 or 6144 numbers are 40 or 48 blocks for 32 warps, so
+    // with one at a time every CTA waited for L2 twice.
+    for (int unit0 = warp_all; unit0 < NT * nb; unit0 += 2 * n_warps) {
+        float xs[2][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int j = b * kPqQK + lane + 32 * i;
-            xv[i] = (real && j < a.ne0) ? xr[j] : 0.f;
-            am = fmaxf(am, fabsf(xv[i]));
-        }
-        for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-        int e = 0;
-        if (am > 0.f && am < CUDART_INF_F) frexpf(am, &e);  // am = f * 2^e, f in [0.5, 1)
-        const float s = ldexpf(1.0f, kPqFrac - e);
-        int ds[4] = {0, 0, 0, 0};
+        for (int h = 0; h < 2; h++) {
+            const int unit = unit0 + h * n_warps, tok = unit / nb, b = unit - tok * nb;
+            const float *xr = a.x + (size_t)tok * a.ne0;
+            const bool real = unit < NT * nb && tok < a.n_tok;  // columns past n_tok are zeros
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int jj = lane + 32 * i;
-            const int tt = jj >> 5, r = (jj >> 4) & 1, q = (jj >> 2) & 3, m = jj & 3;
-            int B = __float2int_rn(xv[i] * s) << (2 * (3 - m));  // |x s| < 2^24
-            uint8_t *dst = sm + off_x + ((((size_t)(4 * tok) * nb + b) * 4 + tt) * 8 + m * 2 + r) * 4 + q;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                const int dg = (int)(int8_t)(B & 0xff);
-                B = (B - dg) >> 8;
-                dst[(size_t)d * nb * 128] = (uint8_t)dg;
-                ds[d] += dg << (2 * m);
+            for (int i = 0; i < 4; i++) {  // byte i of the lane's word
+                const int j = b * kPqQK + my_elem + 4 * i;
+                xs[h][i] = (real && j < a.ne0) ? xr[j] : 0.f;
             }
         }
 #pragma unroll
-        for (int d = 0; d < 4; d++) {
-            int v = ds[d];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) dsum[b * 8 + 4 * tok + d] = v;
+        for (int h = 0; h < 2; h++) {
+            const int unit = unit0 + h * n_warps, tok = unit / nb, b = unit - tok * nb;
+            if (unit >= NT * nb) break;
+            const float (&xv)[4] = xs[h];
+            float am = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) am = fmaxf(am, fabsf(xv[i]));
+            am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));  // (neither NaN nor negative: the bits are in order)
+            int e = 0;
+            if (am > 0.f && am < CUDART_INF_F) frexpf(am, &e);  // am = f * 2^e, f in [0.5, 1)
+            const float s = ldexpf(1.0f, kPqFrac - e);
+            // All four digits of a number at once: adding 128 to every byte with carries and taking it off again without them
+            // leaves the balanced digits; then a 4 x 4 transpose of the bytes.
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t B = (uint32_t)__float2int_rn(xv[i] * s) << (2 * (3 - my_m));  // |x s| < 2^24
+                u[i] = (B + 0x80808080u) ^ 0x80808080u;
+            }
+            const uint32_t t0 = __byte_perm(u[0], u[1], 0x5140), t1 = __byte_perm(u[2], u[3], 0x5140);
+            const uint32_t t2 = __byte_perm(u[0], u[1], 0x7362), t3 = __byte_perm(u[2], u[3], 0x7362);
+            const uint32_t w[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632)};
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                *reinterpret_cast<uint32_t *>(sm + off_x + ((size_t)(4 * tok + d) * nb + b) * 128 + lane * 4) = w[d];
+                const int v = __reduce_add_sync(0xffffffffu, __dp4a((int)w[d], 0x01010101, 0) * (1 << (2 * my_m)));
+                if (lane == 0) dsum[b * 8 + 4 * tok + d] = v;
+            }
+            if (lane == 0) bscale[tok * nb + b] = ldexpf(1.0f, e - kPqFrac - 6);
         }
-        if (lane == 0) bscale[tok * nb + b] = ldexpf(1.0f, e - kPqFrac - 6);
     }
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
