@@ -106,12 +106,7 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
     float x[8];
     const int group = load_group_of_8(sx, lane, x);
     uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t lo = f32_to_half_ref(x[2 * i]);
-        const uint32_t hi = f32_to_half_ref(x[2 * i + 1]);
-        w[i] = lo | (hi << 16);
-    }
+    pack8_half_ref(x, w);
     reinterpret_cast<uint4 *>(row)[group] = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
@@ -250,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
         uint8_t *row = (is_v ? a.v_rows + r * a.v_row_bytes : a.k_rows + r * a.k_row_bytes);
         if (kind == ROW_F32) {
             store_f32_row(sx, lane, row);
-        } else if (kind == ROW_F16) {
+        } else if (BITS == 0 && kind == ROW_F16) {  // (f16 rows never lie beside planar ones)
             store_f16_row(sx, lane, row);
         } else {
             if constexpr (BITS > 0) {

@@ -216,6 +216,27 @@ def test_append_special_vectors(bk, gpu_ctx, oracle):
 
 
 @pytest.mark.parametrize("n", [7, 400])
+def test_append_halfs_of_any_magnitude(bk, gpu_ctx, oracle, n):
+    """f16 rows around the edges of the rounding that the hardware shares with the reference (zero, 2^-14, 2^16), subnormal halfs, infinities
+    and NaN, one such value among seven ordinary ones, in the small and the bulk form of the append: bit for bit."""
+    rng = np.random.default_rng(n)
+    k, v = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    edges = [np.float32(e) for b in (2.0 ** -14, 2.0 ** -15, 2.0 ** -24, 2.0 ** -25, 65504.0, 65520.0, 65536.0, 1.0)
+             for e in (np.nextafter(np.float32(b), np.float32(0)), b, np.nextafter(np.float32(b), np.float32(np.inf)))]
+    edges = np.array(edges + [0.0, 1e-30, 1e-42, np.inf, np.nan, 3e38], np.float32)
+    at = np.arange(v.size // 8) * 8 + rng.integers(0, 8, v.size // 8)
+    at = at[rng.random(at.size) < 0.5]
+    v.reshape(-1)[at] = rng.choice(edges, at.size) * rng.choice(np.array([1, -1], np.float32), at.size)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode("f16"), n_layers=1, n_ctx=n)
+    ref = oracle.cache(MODE_F16, 0, False)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    cache.append(0, k, v)
+    compare_dumps(cache.dump_kv(0), ref.dump(0))
+    cache.close()
+
+
+@pytest.mark.parametrize("n", [7, 400])
 @pytest.mark.parametrize("bits", [2, 3, 4])
 def test_append_vectors_of_any_magnitude(bk, gpu_ctx, oracle, bits, n):
     """Rows from 1e-25 to 1e25 (norms that vanish or overflow), one-hot rows, and rows with infinities and NaN, in the
