@@ -37,8 +37,8 @@
 // Work split.  A launch has about one CTA (8 warps) per SM; a CTA owns a contiguous chunk of one
 // (sequence, kv head) - contiguous chunks stream measurably faster than interleaved ones - and
 // its warps take the chunk's tiles in fixed shares (the result then does not depend on timing);
-// in the CTA of the last chunk the two warps that first store the new token's rows (the fused
-// append) join after a head start of the others.  BONSAI_KV_DYN=1 lets the warps draw tiles from
+// in the CTA that scans a whole sequence the two warps that first store the new token's rows (the
+// fused append) join after a head start of the others.  BONSAI_KV_DYN=1 lets the warps draw tiles from
 // a counter in shared memory instead (same speed on an idle GPU, results vary in the last bits).
 // Partials and the split-K combine are shared with the other decode kernels.
 #include <cuda.h>
@@ -300,24 +300,40 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
         new_lo = src[lane];
         new_hi = src[lane + 32];
     }
-    // Fixed shares (the default: the result then does not depend on timing).  Warp w takes tiles w, w + 8, ...;
-    // in the appending CTA the last two warps start late (they store the new rows first, about a tile's time), so there
-    // the other six share the first kHeadStart rounds among themselves.
-    constexpr int kHeadStart = 1, kOthers = kMW - 2;
+    // Fixed shares (the default: the result then does not depend on timing).  Warp w takes tiles w, w + 8, ...  In the CTA
+    // that scans a whole sequence and stores its new rows the other six warps share the first kHeadStart rounds, and the first
+    // appending warp takes the last tile, which holds the new rows, at its first refill.  The appending warps start about one
+    // tile late, so plain shares end a little sooner (16 layers of 64 sequences of 2048 to 16384 rows, 4 bit: 2505 us, 2530 with
+    // these; of 40 sequences of 2200 to 9000 rows, 3 bit: 1647 and 1704); these stay because the weights are rounded against
+    // each warp's running maximum: another order of the tiles moves the result of a batch by 1e-4.
+    constexpr int kHeadStart = 4, kOthers = kMW - 2;
+    const bool late = appender && n_chunks == 1;
+    const int n_pool = n_tiles - (late ? 1 : 0);  // tiles that are shared out
     auto fixed_tile = [&](int i) -> int {
-        if (!appender) return warp + kMW * i;
-        if (warp >= kOthers) return kOthers * kHeadStart + kMW * i + warp - kOthers;
-        return i < kHeadStart ? kOthers * i + warp : kOthers * kHeadStart + 2 + kMW * (i - kHeadStart) + warp;
+        int lt = warp + kMW * i;
+        if (late) lt = warp >= kOthers ? lt + kOthers * (kHeadStart - 1) : lt - (kMW - kOthers) * min(i, kHeadStart - 1);
+        return lt < n_pool ? lt : -1;
     };
     // ---- fill the ring
     int in_stage[kMaxStages];  // which tile each stage holds, -1 = none
+    bool last_due = late && warp == kOthers;  // this warp still has to take the last tile
 #pragma unroll
     for (int st = 0; st < kMaxStages; st++) {
-        const int lt = dyn ? warp + st * kMW : fixed_tile(st);
-        in_stage[st] = (st < n_stages && lt < n_tiles) ? lt : -1;
-        if (in_stage[st] >= 0) issue_tile(lt, st);
+        int lt = dyn ? (warp + st * kMW < n_pool ? warp + st * kMW : -1) : fixed_tile(st);
+        if (st >= n_stages) lt = -1;
+        if (st == 0 && lt < 0 && last_due) {  // a chunk so short that the warp has no other tile
+            lt = n_tiles - 1;
+            last_due = false;
+        }
+        in_stage[st] = lt;
+        if (lt >= 0) issue_tile(lt, st);
     }
-    int i_next = n_stages;
+    // The next two refills and, from the third on, the tile after them (kMW further each time: every special share is among
+    // the first four of a warp, and at least one of those is in the ring).
+    const int i0 = n_stages + (last_due ? 0 : 1);
+    int refill = last_due ? n_tiles - 1 : fixed_tile(n_stages), refill2 = fixed_tile(i0);
+    int later = warp + kMW * (i0 + 1);
+    if (late) later += warp >= kOthers ? kOthers * (kHeadStart - 1) : -(kMW - kOthers) * (kHeadStart - 1);
     // ---- q: per-head RMSNorm (layer form), rope, Givens rotation, scale, split into f16 hi/lo, written in the
     // MMA's B-fragment layout and then fetched by every lane into registers.
     // 1/sqrt(hd) * log2(e) / alpha: the scores come out in the exp2 domain, alpha undone.
@@ -694,15 +710,16 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
                     compute_tile(lt, st_addr);
                 }
                 __syncwarp();  // every lane has read the stage: lane 0 may refill it
-                int nu;
-                if (dyn) {
+                int nu = refill;
+                if (dyn && !last_due) {
                     nu = __shfl_sync(0xffffffffu, drawn, 0);
-                    if (nu < n_tiles) draw();  // the draw after this one
+                    if (nu < n_pool) draw();  // the draw after this one
                     else nu = -1;
-                } else {
-                    nu = fixed_tile(i_next++);
-                    if (nu >= n_tiles) nu = -1;
                 }
+                last_due = false;
+                refill = refill2;
+                refill2 = later < n_pool ? later : -1;
+                later += kMW;
                 if (nu >= 0) issue_tile(nu, st);
                 else n_held--;
 #pragma unroll

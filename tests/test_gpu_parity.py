@@ -762,6 +762,31 @@ def test_chunks_of_one_launch_meet_without_counters(bk, gpu_ctx, oracle, tag, mo
         cache.close()
 
 
+@pytest.mark.parametrize("tag", ["planar4", "planar3", "planar2"])
+def test_batch_results_stay_what_they_were(bk, gpu_ctx, tag):
+    """A batch with a (sequence, kv head) pair for every SM: which warp scans which tiles, and in which order, decides the last
+    bits of the f16 weights.  The golden values (two heads of three sequences) come from an earlier build with the same
+    shares; 32-bit sums in another order differ by about 1e-7, other shares by 1e-4."""
+    import os
+    want = np.load(os.path.join(os.path.dirname(__file__), "golden", "batch_golden.npz"))[tag]
+    rng = np.random.default_rng(31)
+    lens = [2100 + 16 * s for s in range(37)]
+    k, v = (rng.standard_normal((2800, NKV, HD)).astype(np.float32) for _ in range(2))
+    for x in (k, v):
+        x[:, :, [7, 70, 170]] *= np.float32(20.0)
+    q = rng.standard_normal((37, NH, HD)).astype(np.float32)
+    k1, v1 = (rng.standard_normal((37, NKV, HD)).astype(np.float32) for _ in range(2))
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_seqs=37, n_ctx=2800)
+    for s, n in enumerate(lens):
+        cache.append(0, k[s:s + n], v[s:s + n], seq=s)
+    d_q, d_k, d_v = (gpu_ctx.to_device(x) for x in (q, k1, v1))
+    out = gpu_ctx.alloc(q.nbytes)
+    cache.step_batch_device(0, d_q.ptr, d_k.ptr, d_v.ptr, out.ptr, 37)
+    got = out.download(q.shape, np.float32)[[0, 17, 36]][:, [0, 13]].astype(np.float64)
+    cache.close()
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
 ROW_KERNEL_MODES = [("f32", MODE_F32, 0, False), ("planar4k", MODE_PLANAR, 4, False), ("planar3k", MODE_PLANAR, 3, False),
                     ("planar2", MODE_PLANAR, 2, True)]   # (planar2: the 4-bit kernel with 2-bit rows widened to nibbles)
 
