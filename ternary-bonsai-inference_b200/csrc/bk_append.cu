@@ -106,7 +106,8 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
     float x[8];
     const int group = load_group_of_8(sx, lane, x);
     uint32_t w[4];
-    pack8_half_ref(x, w);
+#pragma unroll
+    for (int i = 0; i < 4; i++) w[i] = pack_half2_ref(x[2 * i], x[2 * i + 1]);
     reinterpret_cast<uint4 *>(row)[group] = make_uint4(w[0], w[1], w[2], w[3]);
 }
 

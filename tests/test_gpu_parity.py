@@ -236,6 +236,43 @@ def test_append_halfs_of_any_magnitude(bk, gpu_ctx, oracle, n):
     cache.close()
 
 
+@pytest.mark.parametrize("std", [3e-2, 1e-4, 1e-6, 1e-8])
+def test_append_small_halfs(bk, gpu_ctx, oracle, std):
+    """f16 rows of every scale at which some, most or all of the halfs are subnormal, bit for bit."""
+    rng = np.random.default_rng(int(-np.log10(std)))
+    n = 400
+    k, v = (rng.standard_normal((n, NKV, HD)).astype(np.float32) * np.float32(std) for _ in range(2))
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode("f16"), n_layers=1, n_ctx=n)
+    ref = oracle.cache(MODE_F16, 0, False)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    cache.append(0, k, v)
+    compare_dumps(cache.dump_kv(0), ref.dump(0))
+    cache.close()
+
+
+def test_append_time_does_not_depend_on_the_rows_scale(bk, gpu_ctx):
+    """A bulk append of f16 rows takes as long for small rows (subnormal halfs among them) as for rows of unit variance."""
+    n, layers = 4096, 16
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode("f16"), n_layers=layers, n_ctx=n)
+    x = np.random.default_rng(3).standard_normal((n, NKV, HD)).astype(np.float32)
+    best = {}
+    for std in (1.0, 0.1, 0.01, 1e-4):
+        d = gpu_ctx.to_device(x * np.float32(std))
+        for _ in range(6):
+            cache.reset()
+            gpu_ctx.synchronize()
+            start, stop = gpu_ctx.event(), gpu_ctx.event()
+            start.record()
+            for il in range(layers):
+                cache.append_device(il, d.ptr, d.ptr, n_tokens=n)
+            stop.record()
+            best[std] = min(best.get(std, 1e9), start.elapsed_ms(stop))
+        d.free()
+    cache.close()
+    assert max(best.values()) <= 1.2 * best[1.0], best
+
+
 @pytest.mark.parametrize("n", [7, 400])
 @pytest.mark.parametrize("bits", [2, 3, 4])
 def test_append_vectors_of_any_magnitude(bk, gpu_ctx, oracle, bits, n):
