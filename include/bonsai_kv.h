@@ -14,6 +14,15 @@
  *  - A bk_ctx owns one CUDA stream and is NOT thread-safe: one in-order stream
  *    per context, as the reference decodes on one thread.  Use one context per
  *    host thread / per GPU.
+ *  - A decode launch whose CTAs wait for one another needs all of them on the GPU
+ *    at once.  Launches of a context that is alone on its device (in this
+ *    process) work like that; while other contexts live on the device they take
+ *    a form that waits for nobody and is slower by a few microseconds, so the
+ *    last bits of a result may differ between the two.  A captured launch keeps
+ *    the form it was captured in: capture again after a second context has been
+ *    made on the device.  (BONSAI_KV_DIST=1, read when a context is created, keeps
+ *    the first form for a program whose contexts never decode at the same time;
+ *    0 takes the second one always.)
  *  - Pointers named *_dev are device pointers valid on the context's device and
  *    the call is asynchronous on the context's stream.  Pointers named *_host
  *    are host pointers and the call returns after the result is in host memory.

@@ -87,7 +87,9 @@ struct bk_ctx {
     bool force_generic = false;            // BONSAI_KV_GENERIC=1: never take the tensor-core path
     bool qsplit = true;                    // q as f16 hi + lo in the tensor-core path (BONSAI_KV_QSPLIT=0: hi only)
     int mma_min_rows = 0;                  // BONSAI_KV_MMA_MIN: rows from which the row kernel (f16, f32, K-only) is taken; 0 = built-in
-    int dyn_tiles = 0; bool dist_combine = true;  // BONSAI_KV_DYN=0 / BONSAI_KV_DIST=0 switch them off
+    int dyn_tiles = 0;                     // BONSAI_KV_DYN
+    int dist_combine = -1;                 // slice form of the split-K combine: never (BONSAI_KV_DIST=0), always (1), by the rule (-1)
+    bool counted = false;                  // among the live contexts of its device (bk_api.cu)
     // staging for the *_host entry points (grown on demand)
     void *h_stage = nullptr;
     size_t h_stage_bytes = 0;
@@ -257,8 +259,9 @@ struct DecodeArgs {
     // Set by launch_decode_group for the tensor-core kernels:
     //   dyn   bit 0: the warps of a CTA draw their tiles from a counter in shared memory instead of taking
     //         fixed shares (off by default: with it the last bits of a result depend on timing)
-    //   dist  every CTA of the launch is resident at once (items <= SMs): the split-K combine is
-    //         done in slices by all CTAs of a kv head instead of by the last one to arrive
+    //   dist  every CTA of the launch is resident at once (items <= SMs, and no other context of this process waits
+    //         for its own on this device): the split-K combine is done in slices by all CTAs of a kv head, which
+    //         wait for one another, instead of by the last one to arrive
     //   boxes where the chunks' results travel then
     int dyn, dist;
     float *boxes;

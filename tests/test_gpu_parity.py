@@ -799,6 +799,65 @@ def test_chunks_of_one_launch_meet_without_counters(bk, gpu_ctx, oracle, tag, mo
         cache.close()
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [("f16", MODE_F16, 0, False), ("f32", MODE_F32, 0, False), ("planar4", MODE_PLANAR, 4, True),
+                                              ("planar4k", MODE_PLANAR, 4, False)])
+@pytest.mark.parametrize("n_head,n_kv", [(6, 1), (4, 2), (24, 4)])
+def test_last_arriver_combine(bk, oracle, monkeypatch, tag, mode, bits, vq, n_head, n_kv):
+    """The split-K combine that waits for nobody (BONSAI_KV_DIST=0 forces it): two chunks, a few, more than one streaming
+    round of 32; the whole result, the layer form's gate and the partial triple; a second launch gives the same bits."""
+    monkeypatch.setenv("BONSAI_KV_DIST", "0")
+    ctx = bk.Context(0)
+    rng = np.random.default_rng(11)
+    for n0 in (159, 1000, 4800 if n_kv > 1 else 15000):
+        k = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
+        v = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
+        q = rng.standard_normal((n_head, HD)).astype(np.float32)
+        cache = bk.AttnCache(ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n0 // 4 * 4 + 8, n_head=n_head, n_kv=n_kv)
+        cache.append(0, k[:n0], v[:n0])
+        ref = oracle.cache(mode, bits, vq, n_head=n_head, n_kv=n_kv)
+        for p in range(n0):
+            ref.append(0, k[p], v[p], p)
+        want = ref.step(0, q, k[n0], v[n0], n0, threads=8)
+        got = bk.full_attention_step(cache, 0, q, k[n0], v[n0], n0)
+        assert_close(got, want, f"{tag} {n0}")
+        assert np.array_equal(bits_of(cache.attend(0, q)[0]), bits_of(got.reshape(q.shape)))
+        part = cache.attend(0, q, partial=True)[0]
+        assert_close(part[:, :HD] / part[:, HD + 1:], want, f"{tag} {n0} partial")
+        cache.close()
+    ctx.close()
+
+
+def test_two_contexts_decode_at_the_same_time(bk, gpu_ctx):
+    """Two contexts on one GPU, launches that each take all SMs in flight on both streams at once: neither waits for a place that
+    the other holds (a combine that waits for all chunks of its launch would), and results equal what a launch that runs by
+    itself gives in the same form."""
+    rng = np.random.default_rng(5)
+    other = bk.Context(0)
+    tag, n, layers, steps = "f16", 1300, 4, 60
+    k, v = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((NH, HD)).astype(np.float32)
+    runs = []
+    for ctx in (gpu_ctx, other):
+        cache = bk.AttnCache(ctx, bk.parse_mode(tag), n_layers=layers, n_ctx=n)
+        for il in range(layers):
+            cache.append(il, k, v)
+        d_q, d_out = ctx.to_device(q), [ctx.alloc(q.nbytes) for _ in range(layers)]
+        cache.decode_device(0, d_q.ptr, d_out[0].ptr)
+        ctx.synchronize()
+        runs.append((ctx, cache, d_q, d_out, d_out[0].download(q.shape, np.float32)))
+    assert np.array_equal(bits_of(runs[0][4]), bits_of(runs[1][4]))
+    for _ in range(steps):
+        for il in range(layers):
+            for ctx, cache, d_q, d_out, _w in runs:
+                cache.decode_device(il, d_q.ptr, d_out[il].ptr)
+    for ctx, cache, d_q, d_out, want in runs:
+        ctx.synchronize()
+        for o in d_out:
+            assert np.array_equal(bits_of(o.download(q.shape, np.float32)), bits_of(want))
+        cache.close()
+    other.close()
+
+
 @pytest.mark.parametrize("tag", ["planar4", "planar3", "planar2"])
 def test_batch_results_stay_what_they_were(bk, gpu_ctx, tag):
     """A batch with a (sequence, kv head) pair for every SM: which warp scans which tiles, and in which order, decides the last

@@ -138,3 +138,10 @@ def test_exchange_of_several_layers_rows_in_one_call(bk, monkeypatch):
         lib.bk_mailbox_destroy(boxes[r][0])
     for c in part + [whole]:
         c.close()
+
+
+def test_exchange_of_slices(bk, monkeypatch):
+    """The same with the slice form of the split-K combine in rank 0's launches (next to another context they take the
+    last-arriver form unless told that the two never run together)."""
+    monkeypatch.setenv("BONSAI_KV_DIST", "1")
+    test_exchange_wait_gives_up_reports_and_recovers(bk, monkeypatch)
