@@ -38,8 +38,8 @@
  *  - Every wait inside a kernel is bounded.  A wait that runs out (a peer of the
  *    context split never sent its rows) sets an error word; every call that
  *    blocks the host (bk_synchronize, the *_host forms, downloads, snapshots,
- *    bk_event_elapsed_ms) then returns BK_ERR_CUDA with the reason, the step
- *    in flight is void, and the context stays usable.
+ *    bk_event_elapsed_ms) then returns BK_ERR_CUDA with the reason, everything
+ *    since the last such call is void, and the context stays usable.
  *  - Layouts follow the reference: token-major [pos][kv_head][...].
  */
 #ifndef BONSAI_KV_H

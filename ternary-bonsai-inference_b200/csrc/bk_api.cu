@@ -342,7 +342,7 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
     const size_t cnt_bytes = (size_t)kCounters * sizeof(unsigned);
     if ((e = cudaMalloc(&ctx->d_counters, cnt_bytes)) != cudaSuccess) return bail(e, "cudaMalloc counters");
     if ((e = cudaMemset(ctx->d_counters, 0, cnt_bytes)) != cudaSuccess) return bail(e, "clear counters");
-    ctx->box_bytes = (size_t)ctx->n_sms * kMaxRep * kBoxFloats * sizeof(float);
+    ctx->box_bytes = ((size_t)ctx->n_sms * kMaxRep * kBoxFloats + 4) * sizeof(float);  // (and the state word)
     if ((e = cudaMalloc(&ctx->d_boxes, ctx->box_bytes)) != cudaSuccess) return bail(e, "cudaMalloc boxes");
     if ((e = cudaMemset(ctx->d_boxes, 0xff, ctx->box_bytes)) != cudaSuccess) return bail(e, "empty boxes");
     if ((e = cudaMalloc(&ctx->d_pq2_x, kPq2ScratchBytes)) != cudaSuccess) return bail(e, "cudaMalloc pq2 scratch");
@@ -559,6 +559,7 @@ bk_status bk_cache_create(bk_ctx *ctx, const bk_cache_config *cfg, bk_cache **ou
         return st;
     }
     c->n_pos.assign((size_t)cfg->n_layers * cfg->n_seqs, 0);
+    if (const char *polls = getenv("BONSAI_KV_BOX_POLLS")) c->box_polls = std::max(0, atoi(polls));
     // tiles of 16 positions: f16, f32, and 4- or 3-bit K beside f32 V; tiles of 32: K and V both 4, 3 or 2 bit
     const bool row_tiles = (k_kind == ROW_F16 && v_kind == ROW_F16) || (k_kind == ROW_F32 && v_kind == ROW_F32) ||
                            (k_kind == ROW_PLANAR && (bits == 4 || bits == 3) && v_kind == ROW_F32);
@@ -836,6 +837,8 @@ void fill_decode_args(const bk_cache *c, int layer, int partial, DecodeArgs *out
     a.xch_spin = ctx->xch_polls;
     a.dyn = a.dist = 0;
     a.boxes = ctx->d_boxes;
+    a.box_state = ctx->box_state();
+    a.box_polls = c->box_polls;
     a.k_rows_w = c->k_rows(layer, 0);
     a.v_rows_w = c->v_rows(layer, 0);
     a.k_norms_w = c->k_norms(layer, 0);

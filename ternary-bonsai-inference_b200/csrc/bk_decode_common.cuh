@@ -20,8 +20,6 @@
 
 namespace bk {
 
-constexpr int kBoxPolls = 1 << 21;  // polls of box words before a thread of the slice combine gives up
-
 // Per-CTA time stamps for tuning builds (-DBK_PHASE): stamp i of CTA b lands in g_phase[b][i].
 #ifdef BK_PHASE
 static __device__ unsigned long long g_phase[1024][16];
@@ -261,6 +259,10 @@ __device__ __forceinline__ void wait_bar(uint32_t bar, uint32_t parity, int lane
 // the barriers around it; from the last chunk's sums to the end of the launch 4.0 to 4.7 us with a ticket
 // counter, 3.3 us now (planar4 9000 rows, f16 8192 rows).
 //
+// A wait that runs out leaves words behind that the next launch would take for its own, so it also marks the boxes as foul
+// (DecodeArgs::box_state).  While they are, launches that are already queued write nothing and raise the
+// error again; the host empties the boxes and takes the mark off when it reports the error.
+//
 // Boxes of a (sequence, kv head) start at first_item * NREP * kBoxFloats:
 //     values  [slice][chunk][NREP][D]     relative to the chunk's maximum, not normalised
 //     (m, l)  [slice][chunk][NREP][2]     a copy per slice, so that every word has one reader
@@ -282,6 +284,12 @@ constexpr bool boxes_fit() {
 }
 static_assert(boxes_fit(), "a box does not hold a chunk's values and (m, l) pairs, or a slice has no owner");
 
+// Are the boxes fit for use?  Read by one thread behind the dependency wait.
+__device__ __forceinline__ bool boxes_clean(const DecodeArgs &a) {
+    unsigned w;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(w) : "l"(a.box_state) : "memory");
+    return w == kEmptyWord;
+}
 __device__ __forceinline__ float box_word(float x) {  // kEmptyWord becomes the ordinary NaN
     return __float_as_uint(x) == kEmptyWord ? __uint_as_float(0x7fffffffu) : x;
 }
@@ -302,7 +310,7 @@ __device__ __forceinline__ bool box_full(float x) { return __float_as_uint(x) !=
 __device__ __forceinline__ bool box_full4(float4 v) { return box_full(v.x) && box_full(v.y) && box_full(v.z) && box_full(v.w); }
 
 // sums[r]: this chunk's value of coordinate tid (threads 0..255) of head r; s_M, s_L: its maxima and sums.  `red` is
-// free shared memory (16-byte aligned, kCombineBytes); *s_ok is 1 on entry.  Every thread of the CTA calls.
+// free shared memory (16-byte aligned, kCombineBytes); *s_ok is boxes_clean() on entry.  Every thread of the CTA calls.
 // A thread merges a few chunks of one 16-byte column on its own (its own reference, no exchange of maxima), the threads
 // that write the output merge the thread groups: one barrier between the loads and the output.
 constexpr uint32_t kCombineBytes = 12288;
@@ -343,7 +351,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     float M = -CUDART_INF_F, L = 0.f;
     if (grp < n_grp) {
-        int polls = 0;
+        int left = a.box_polls;
         for (int c0 = grp; c0 < n_chunks; c0 += kPre * n_grp) {
             float4 v[kPre];
             float2 x[kPre];
@@ -369,7 +377,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
                         full = false;
                     }
                 }
-            } while (!full && ++polls <= kBoxPolls);
+            } while (!full && --left > 0);
             float Mn = M;
 #pragma unroll
             for (int u = 0; u < kPre; u++) Mn = fmaxf(Mn, x[u].x);
@@ -390,9 +398,9 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
                     sum.w = fmaf(v[u].w, f, sum.w);
                 }
         }
-        if (polls > kBoxPolls) {  // never expected: leave a mark, write nothing
+        if (left <= 0) {  // never expected: leave marks, write nothing
             *s_ok = 0;
-            raise_error(err_flag, 6);
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(a.box_state), "r"(0u) : "memory");
         }
     }
     float2 *s_ml = reinterpret_cast<float2 *>(red);  // [n_grp][NREP]
@@ -404,7 +412,10 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
     float *s_Mg = s_sum + 1024, *s_Lg = s_Mg + 8, *snd = s_Lg + 8;  // context split: what this slice sends
     __syncthreads();
     BK_STAMP(7);
-    if (!*s_ok) return;
+    if (!*s_ok) {
+        if (tid == 0) raise_error(err_flag, 6);
+        return;
+    }
     // ---- merge the groups in a fixed order and write.  Whole warps, because a Givens pair is two neighbouring lanes.
     for (int i0 = tid & ~31; i0 < n_out; i0 += nthr) {
         const int i = i0 + (tid & 31), r_o = i < n_out ? i >> (lg + 2) : 0, d_o = i & (D - 1);

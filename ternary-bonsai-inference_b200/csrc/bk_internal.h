@@ -105,8 +105,9 @@ struct bk_ctx {
     // split-K scratch of the decode kernel: partial results and arrival counters
     float *d_partials = nullptr;
     unsigned *d_counters = nullptr;
-    float *d_boxes = nullptr;      // slice combine of the tensor-core kernels: kBoxFloats x kMaxRep per SM, empty between launches
-    size_t box_bytes = 0;
+    float *d_boxes = nullptr;      // slice combine of the tensor-core kernels: kBoxFloats x kMaxRep per SM, empty between launches, and
+    size_t box_bytes = 0;          // behind them the word that says whether they are (kEmptyWord: yes)
+    unsigned *box_state() const { return reinterpret_cast<unsigned *>(d_boxes + (size_t)n_sms * bk::kMaxRep * bk::kBoxFloats); }
     // Set by a kernel whose bounded wait ran out (the code says which wait).  The word lives in pinned host
     // memory that the device writes directly, so every host-side wait for the stream can look at it for free.
     int *d_err = nullptr;          // device view
@@ -129,6 +130,7 @@ struct bk_cache {
     uint8_t *d_k = nullptr, *d_v = nullptr;   // [layer][seq][n_ctx][n_kv][row_bytes]
     float *d_kn = nullptr, *d_vn = nullptr;   // [layer][seq][n_ctx][n_kv], planar sides only
     std::vector<int32_t> n_pos;               // [layer][seq]
+    int box_polls = 1 << 21;                  // looks at the words of the slice combine before a wait gives up (BONSAI_KV_BOX_POLLS)
     std::shared_ptr<bk::RopeTable> rope;
     size_t device_bytes = 0;
     alignas(64) unsigned char tmap_k[128], tmap_v[128];  // CUtensorMap objects (4/3-bit planar and f16 K+V caches): boxes of 16 positions
@@ -179,7 +181,7 @@ bk_status cuda_fail(bk_ctx *ctx, cudaError_t e, const char *what);
 // Staging of at least `bytes` on the device and, unless the call moves its data through the host pipe, in pinned memory.
 bk_status ensure_stage(bk_ctx *ctx, size_t bytes, bool host = true);
 // Wait for the context's stream, then look at the error word the kernels raise when a bounded wait runs
-// out: BK_ERR_CUDA (and the word and the split-K counters cleared) if one did.
+// out: BK_ERR_CUDA (and the word and the split-K counters cleared, the boxes emptied) if one did.
 bk_status sync_and_check(bk_ctx *ctx);
 
 // ---- kernel launchers (bk_append.cu, bk_decode.cu, bk_kvq.cu) --------------
@@ -262,9 +264,12 @@ struct DecodeArgs {
     //   dist  every CTA of the launch is resident at once (items <= SMs, and no other context of this process waits
     //         for its own on this device): the split-K combine is done in slices by all CTAs of a kv head, which
     //         wait for one another, instead of by the last one to arrive
-    //   boxes where the chunks' results travel then
+    //   boxes where the chunks' results travel then; box_state: kEmptyWord unless an earlier launch gave up a wait and left
+    //         words in them; box_polls: looks before a wait gives up
     int dyn, dist;
     float *boxes;
+    unsigned *box_state;
+    int box_polls;
 };
 bk_status launch_decode(bk_ctx *ctx, const DecodeArgs &a, const DecodeMeta &m);
 

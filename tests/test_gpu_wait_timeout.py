@@ -145,3 +145,52 @@ def test_exchange_of_slices(bk, monkeypatch):
     last-arriver form unless told that the two never run together)."""
     monkeypatch.setenv("BONSAI_KV_DIST", "1")
     test_exchange_wait_gives_up_reports_and_recovers(bk, monkeypatch)
+
+
+@pytest.mark.parametrize("tag", ["f16", "planar4"])
+def test_combine_wait_gives_up_and_nothing_stale_is_handed_out(bk, monkeypatch, tag):
+    """The wait of the split-K combine runs out (a limit of no polls, read when a cache is made): the error is reported once;
+    launches that were already queued behind it, with the ordinary limit, neither take the words that it left behind as
+    results nor write anything; after the report the same launches give what a context that saw no error gives."""
+    monkeypatch.setenv("BONSAI_KV_DIST", "1")   # (whatever other contexts the session holds)
+    abi = bk._abi
+    rng = np.random.default_rng(29)
+    n = 2500
+    k, v = (rng.standard_normal((n, NKV, HD), dtype=np.float32) for _ in range(2))
+    q = rng.standard_normal((2, NH, HD), dtype=np.float32)
+    mode = bk.parse_mode(tag)
+
+    def make(ctx):
+        c = bk.AttnCache(ctx, mode, n_layers=1, n_ctx=n)
+        c.append(0, k, v)
+        return c
+    ctx = bk.Context(0)
+    cache = make(ctx)
+    want = cache.attend(0, q[1])[0]
+    cache.close()
+    ctx.close()
+
+    ctx = bk.Context(0)
+    monkeypatch.setenv("BONSAI_KV_BOX_POLLS", "0")
+    hasty = make(ctx)
+    monkeypatch.delenv("BONSAI_KV_BOX_POLLS")
+    cache = make(ctx)
+    ones = np.ones((NH, HD), np.float32)
+    d_q, d_out = [ctx.to_device(x) for x in q], [ctx.to_device(ones) for _ in range(3)]
+    for _ in range(2):
+        hasty.decode_device(0, d_q[0].ptr, d_out[0].ptr)
+        cache.decode_device(0, d_q[1].ptr, d_out[1].ptr)
+        cache.decode_device(0, d_q[1].ptr, d_out[2].ptr)
+        assert ctx.lib.bk_synchronize(ctx.h) == abi.BK_ERR_CUDA
+        msg = ctx.lib.bk_last_error(ctx.h)
+        assert b"bounded wait" in msg and b"code 6" in msg, msg
+        assert ctx.lib.bk_synchronize(ctx.h) == abi.BK_OK       # reported once, then clear
+        for o in d_out:
+            assert np.array_equal(o.download((NH, HD), np.float32), ones)
+        cache.decode_device(0, d_q[1].ptr, d_out[1].ptr)
+        got = d_out[1].download((NH, HD), np.float32)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        d_out[1].upload(ones)
+    for c in (hasty, cache):
+        c.close()
+    ctx.close()
