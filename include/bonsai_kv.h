@@ -382,11 +382,16 @@ BK_API bk_status bk_kvq_codebook(int32_t hd, int32_t bits, float *out_host);
 BK_API bk_status bk_kvq_givens(int32_t hd, float *out_host);
 /* No counterpart in the reference: the decision thresholds behind the bulk append's nearest-centroid search for head
  * dimension 256 and widths 1..4, for checking them against the reference's scan
- * (src/kvquant.rs:357-370) without a GPU.  512 cells of width 2^-10 over [-0.25, 0.25): out_host[2k] = how
+ * (src/kvquant.rs:357-370) without a GPU, for programs that look the index up in memory.  512 cells of width 2^-10 over [-0.25, 0.25): out_host[2k] = how
  * many decision thresholds lie in cells below k, out_host[2k + 1] = the bits of the one threshold inside
  * cell k (+inf if none).  nearest(v) = out[2k] + (v >= threshold) with k = clamp(floor((v + 0.25) * 1024)),
- * all in f32.  Host only. */
+ * all in f32.  Host only; the kernels hold the same thresholds in the cells of bk_kvq_lane_cells. */
 BK_API bk_status bk_kvq_threshold_cells(int32_t bits, uint32_t *out_host);
+/* No counterpart in the reference: the table that the append and quantize kernels read, for checking it without a GPU.  32 cells:
+ * out_host[2k] = how many thresholds lie in cells below k, out_host[2k + 1] = the bits of the one in cell k (+inf if none);
+ * out_host[64] = the bits of `scale`.  nearest(v) = out[2k] + (v >= threshold) with k = floor(31.999998f * clamp(fma(v, scale, 0.5f),
+ * 0, 1)), the product not rounded.  Host only. */
+BK_API bk_status bk_kvq_lane_cells(int32_t bits, uint32_t *out_host);
 /* PlanarQuant::quantize (src/kvquant.rs:397-412) for n_vec vectors of hd floats. */
 BK_API bk_status bk_kvq_quantize(bk_ctx *ctx, int32_t hd, int32_t bits, int32_t n_vec,
                                  const float *x_host, uint8_t *packed_host, float *norms_host);

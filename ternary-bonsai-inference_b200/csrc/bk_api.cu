@@ -2,6 +2,7 @@
 // Declarations and the reference interface each entry point replaces are in
 // include/bonsai_kv.h.
 #include <math.h>
+#include <stddef.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1486,6 +1487,17 @@ bk_status bk_kvq_threshold_cells(int32_t bits, uint32_t *out) {
     static_assert(sizeof(uint2) == 2 * sizeof(uint32_t), "cell layout");
     if (!build_threshold_cells(book, 1 << bits, reinterpret_cast<uint2 *>(out)))
         return fail(nullptr, BK_ERR_UNSUPPORTED, "codebook thresholds do not fit the cell table");
+    return BK_OK;
+}
+
+bk_status bk_kvq_lane_cells(int32_t bits, uint32_t *out) {
+    if (!out || bits < 1 || bits > 4) return fail(nullptr, BK_ERR_INVALID, "bk_kvq_lane_cells: bits must be 1..4");
+    float book[256];
+    host_codebook(kHd, bits, book);
+    LaneCells cells = {};
+    if (!build_lane_cells(book, 1 << bits, &cells)) return fail(nullptr, BK_ERR_UNSUPPORTED, "codebook thresholds do not fit the cell table");
+    static_assert(offsetof(LaneCells, scale) == 64 * sizeof(uint32_t), "cell layout");
+    memcpy(out, &cells, 65 * sizeof(uint32_t));
     return BK_OK;
 }
 

@@ -88,10 +88,10 @@ def test_setup_tables_equal_the_oracle(bk, oracle, bits):
 
 @pytest.mark.parametrize("bits", [1, 2, 3, 4])
 def test_threshold_cells_give_the_reference_scan(bk, oracle, bits):
-    """The bulk append finds the nearest centroid with one table read and one comparison.  The table is built
-    on the host; here it is checked against the reference's scan (src/kvquant.rs:357-370: ascending, strict
-    '<', f32 differences) on the values where the two could part: centroids, exact midpoints, the decision
-    thresholds themselves, cell edges, each with their neighbouring floats, and a dense random sample."""
+    """The decision thresholds in 512 cells, for programs that find the nearest centroid with one table read and one
+    comparison, against the reference's scan (src/kvquant.rs:357-370: ascending, strict '<', f32 differences) on the
+    values where the two could part: centroids, exact midpoints, the decision thresholds themselves, cell edges, each with
+    their neighbouring floats, and a dense random sample.  (The kernels' own table: the next test.)"""
     lib = bk._abi.load()
     cells = np.zeros((512, 2), np.uint32)
     assert lib.bk_kvq_threshold_cells(bits, cells.ctypes.data) == 0
@@ -124,6 +124,38 @@ def test_threshold_cells_give_the_reference_scan(bk, oracle, bits):
     want = np.argmin(np.abs(v[:, None] - book[None, :]), axis=1)       # f32 differences; first minimum = lowest index
     cell = np.clip(np.floor((v + np.float32(0.25)) * np.float32(1024)).astype(np.int64), 0, 511)
     got = count[cell] + (v >= thr[cell])
+    bad = np.flatnonzero(got != want)
+    assert bad.size == 0, (v[bad[:5]], got[bad[:5]], want[bad[:5]])
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+def test_lane_cells_give_the_reference_scan(bk, oracle, bits):
+    """The table that the append and quantize kernels read: 32 cells of floor(31.999998 clamp(v scale + 1/2)), the sum rounded
+    once to f32.  Checked against the reference's scan on centroids, midpoints, thresholds and cell edges, each with their
+    neighbouring floats, and on a dense random sample."""
+    lib = bk._abi.load()
+    words = np.zeros(65, np.uint32)
+    assert lib.bk_kvq_lane_cells(bits, words.ctypes.data) == 0
+    below, thr, scale = words[0:64:2].astype(np.int64), words[1:64:2].copy().view(np.float32), words[64:].view(np.float32)[0]
+    book = oracle.codebook(256, bits).astype(np.float32)
+    assert int(np.isfinite(thr).sum()) == (1 << bits) - 1 and np.all(np.diff(below) >= 0) and scale > 0
+    edges = [(np.float64(c) / np.float64(np.float32(31.999998)) - 0.5) / np.float64(scale) for c in range(33)]
+    at = np.array([*book, *(0.5 * (book[:-1].astype(np.float64) + book[1:])), *thr[np.isfinite(thr)], *edges, 0.0, 0.25, -0.25], np.float32)
+    probes = [at]
+    for towards in (np.float32(-np.inf), np.float32(np.inf)):
+        x = at
+        for _ in range(6):
+            x = np.nextafter(x, towards)
+            probes.append(x)
+    rng = np.random.default_rng(bits)
+    probes += [(rng.standard_normal(300000) / 16).astype(np.float32), rng.uniform(-0.3, 0.3, 300000).astype(np.float32),
+               np.array([1.5, -1.5, -0.0, 1e-30, -1e-30, 1e-45], np.float32)]   # (rotated unit vectors stay below 1.5)
+    v = np.concatenate(probes)
+    want = np.argmin(np.abs(v[:, None].astype(np.float32) - book[None, :]), axis=1)
+    u = np.clip((v.astype(np.longdouble) * np.longdouble(scale) + np.longdouble(0.5)).astype(np.float32), np.float32(0), np.float32(1))
+    cell = np.floor(u.astype(np.float64) * np.float64(np.float32(31.999998))).astype(np.int64)   # (24 + 24 bits: exact)
+    assert cell.min() == 0 and cell.max() == 31
+    got = below[cell] + (v >= thr[cell])
     bad = np.flatnonzero(got != want)
     assert bad.size == 0, (v[bad[:5]], got[bad[:5]], want[bad[:5]])
 
