@@ -362,6 +362,8 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
         const char *e8 = getenv("BONSAI_KV_MMA_MIN");
         if (e8 && atoi(e8) > 0) ctx->mma_min_rows = atoi(e8);
     }
+    // the fills and uploads above went to the legacy stream, which the context's own stream does not wait for
+    if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return bail(e, "cudaStreamSynchronize");
     count_context(ctx, 1);
     *out = ctx;
     return BK_OK;
