@@ -773,11 +773,12 @@ def test_fused_step_on_long_f16_cache(bk, gpu_ctx, oracle):
                                               ("planar3", MODE_PLANAR, 3, True), ("planar2", MODE_PLANAR, 2, True), ("planar4k", MODE_PLANAR, 4, False)])
 @pytest.mark.parametrize("n_head,n_kv", [(6, 1), (8, 2), (24, 4)])
 def test_chunks_of_one_launch_meet_without_counters(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv):
-    """The split-K combine sends slices between the chunks of a launch: one chunk, two, a few, one per SM; new rows on
-    the first and the last row of a tile; q at an address that is no multiple of 16.  A second launch over the same
-    rows gives the same bits (every word that travelled was taken and the space is empty again)."""
+    """The split-K combine sends slices between the chunks of a launch: two chunks, a few, up to 76 (one per SM:
+    test_a_chunk_per_sm); new rows on the first and the last row of a tile; q at an address that is no multiple of 16.
+    Fewer than 128 rows take the generic kernel.  A second launch over the same rows gives the same bits (every word that
+    travelled was taken and the space is empty again)."""
     rng = np.random.default_rng(7)
-    for n0 in (1, 31, 32, 96, 128, 159, 192, 300, 1000, 4800):
+    for n0 in (1, 31, 32, 96, 127, 128, 159, 160, 191, 192, 300, 1000, 4800):
         k = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
         v = rng.standard_normal((n0 + 1, n_kv, HD)).astype(np.float32)
         q = rng.standard_normal((n_head, HD)).astype(np.float32)
@@ -856,6 +857,60 @@ def test_two_contexts_decode_at_the_same_time(bk, gpu_ctx):
             assert np.array_equal(bits_of(o.download(q.shape, np.float32)), bits_of(want))
         cache.close()
     other.close()
+
+
+@pytest.mark.parametrize("tag,mode,bits,vq,n", [("f16", MODE_F16, 0, False, 4730), ("f32", MODE_F32, 0, False, 14200),
+                                                ("planar4", MODE_PLANAR, 4, True, 14200)])
+def test_a_chunk_per_sm(bk, gpu_ctx, oracle, tag, mode, bits, vq, n):
+    """One kv head on the whole chip: as many chunks as SMs meet in one combine (148 of 32 or 96 rows); whole and partial results."""
+    rng = np.random.default_rng(n)
+    k, v = (rng.standard_normal((n + 1, 1, HD)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((6, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n // 4 * 4 + 8, n_head=6, n_kv=1)
+    cache.append(0, k[:n], v[:n])
+    ref = oracle.cache(mode, bits, vq, n_head=6, n_kv=1)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    want = ref.step(0, q, k[n], v[n], n, threads=8)
+    assert_close(bk.full_attention_step(cache, 0, q, k[n], v[n], n), want, tag)
+    part = cache.attend(0, q, partial=True)[0]
+    assert_close(part[:, :HD] / part[:, HD + 1:], want, f"{tag} partial")
+    cache.close()
+
+
+@pytest.mark.parametrize("tag,mode,bits,vq", [("f16", MODE_F16, 0, False), ("planar4", MODE_PLANAR, 4, True)])
+def test_split_and_whole_sequences_in_one_launch(bk, gpu_ctx, oracle, tag, mode, bits, vq):
+    """A batch whose short sequences are one chunk each and whose long ones are many, new rows included; the partial triples of the
+    same batch, merged with an empty part, give the same."""
+    rng = np.random.default_rng(4)
+    lens = [131, 4100, 260, 9000]
+    nmax = max(lens)
+    k, v = synth_kv(rng, nmax + 1)
+    q = rng.standard_normal((len(lens), NH, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_seqs=len(lens), n_ctx=nmax + 8)
+    want = []
+    ref = oracle.cache(mode, bits, vq)
+    for s, n in sorted(enumerate(lens), key=lambda x: x[1]):
+        cache.append(0, k[:n - 1], v[:n - 1], seq=s)
+        for p in range(ref.n_pos(0), n):
+            ref.append(0, k[p], v[p], p)
+        want.append((s, ref.attend(0, q[s], n - 1, n, threads=8)))
+    d_q, d_k, d_v = (gpu_ctx.to_device(x) for x in (q, k[[n - 1 for n in lens]], v[[n - 1 for n in lens]]))
+    out = gpu_ctx.alloc(q.nbytes)
+    launches = gpu_ctx.launch_count
+    cache.step_batch_device(0, d_q.ptr, d_k.ptr, d_v.ptr, out.ptr, len(lens))
+    assert gpu_ctx.launch_count - launches == 1
+    got = out.download(q.shape, np.float32)
+    parts = cache.attend(0, q, n_seqs=len(lens), partial=True)
+    empty = np.zeros_like(parts)
+    empty[..., HD] = -np.inf
+    d_parts, d_merged = gpu_ctx.to_device(np.stack([parts, empty])), gpu_ctx.alloc(q.nbytes)
+    gpu_ctx.check(gpu_ctx.lib.bk_lse_merge(gpu_ctx.h, 2, len(lens) * NH, HD, d_parts.ptr, d_merged.ptr))
+    merged = d_merged.download(q.shape, np.float32)
+    for s, w in want:
+        assert_close(got[s], w, f"{tag} {lens[s]}")
+        assert_close(merged[s], w, f"{tag} {lens[s]} merged")
+    cache.close()
 
 
 @pytest.mark.parametrize("tag", ["planar4", "planar3", "planar2"])

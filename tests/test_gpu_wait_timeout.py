@@ -147,6 +147,55 @@ def test_exchange_of_slices(bk, monkeypatch):
     test_exchange_wait_gives_up_reports_and_recovers(bk, monkeypatch)
 
 
+def test_exchange_of_more_chunks_than_one_round(bk, oracle, monkeypatch):
+    """A rank whose slices come from as many chunks as SMs (one kv head, 32 rows each), more than a thread of the slice combine takes
+    in one round when slices lie on the mailbox's grid of eight coordinates."""
+    monkeypatch.setenv("BONSAI_KV_XCH_POLLS", "3000")
+    monkeypatch.setenv("BONSAI_KV_DIST", "1")
+    from oracle_lib import MODE_F16
+    abi = bk._abi
+    ctx = [bk.Context(0), bk.Context(0)]
+    lib = ctx[0].lib
+    rng = np.random.default_rng(37)
+    n = [4731, 700]
+    total = sum(n)
+    k, v = (rng.standard_normal((total, 1, HD), dtype=np.float32) for _ in range(2))
+    q = rng.standard_normal((6, HD), dtype=np.float32)
+    ref = oracle.cache(MODE_F16, 0, False, n_head=6, n_kv=1)
+    for p in range(total):
+        ref.append(0, k[p], v[p], p)
+    want = ref.attend(0, q, total - 1, total, threads=8)
+    part = [bk.AttnCache(ctx[r], bk.parse_mode("f16"), n_layers=1, n_ctx=n[r], n_head=6, n_kv=1, rope_positions=total) for r in range(2)]
+    part[0].append(0, k[:n[0]], v[:n[0]], pos=0)
+    part[1].append(0, k[n[0]:], v[n[0]:], pos=n[0])
+    boxes = []
+    for r in range(2):
+        handle = (C.c_ubyte * 64)()
+        mb = C.c_void_p()
+        ctx[r].check(lib.bk_mailbox_create(ctx[r].h, 2, r, 6, HD, C.byref(mb), handle))
+        boxes.append((mb, bytes(handle)))
+    blob = (C.c_ubyte * 128).from_buffer_copy(boxes[0][1] + boxes[1][1])
+    for r in range(2):
+        ctx[r].check(lib.bk_mailbox_open_peers(boxes[r][0], blob))
+    d_q = [ctx[r].to_device(q) for r in range(2)]
+    d_out = [ctx[r].alloc(q.nbytes) for r in range(2)]
+
+    def call(r):
+        ctx[r].check(lib.bk_decode_attn_split(part[r].h, 0, 0, n[r], total - 1, d_q[r].ptr, d_out[r].ptr, boxes[r][0], 1))
+        return lib.bk_synchronize(ctx[r].h)
+
+    assert call(1) == abi.BK_ERR_CUDA                      # rank 1 alone: sends, then gives up on rank 0
+    assert call(0) == abi.BK_OK
+    got = d_out[0].download(q.shape, np.float32)
+    assert float(np.max(np.abs(got - want))) <= 1e-5
+    for r in range(2):
+        lib.bk_mailbox_destroy(boxes[r][0])
+    for c in part:
+        c.close()
+    for c in ctx:
+        c.close()
+
+
 @pytest.mark.parametrize("tag", ["f16", "planar4"])
 def test_combine_wait_gives_up_and_nothing_stale_is_handed_out(bk, monkeypatch, tag):
     """The wait of the split-K combine runs out (a limit of no polls, read when a cache is made): the error is reported once;
