@@ -306,9 +306,12 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     // appending warp takes the last tile, which holds the new rows, at its first refill.  The appending warps start about one
     // tile late, so plain shares end a little sooner (16 layers of 64 sequences of 2048 to 16384 rows, 4 bit: 2505 us, 2530 with
     // these; of 40 sequences of 2200 to 9000 rows, 3 bit: 1647 and 1704); these stay because the weights are rounded against
-    // each warp's running maximum: another order of the tiles moves the result of a batch by 1e-4.
+    // each warp's running maximum: another order of the tiles moves the result of a batch by 1e-4.  2-bit rows take plain
+    // shares: the schedule of their scan is touchy, and with these in the loop split launches lose 2 % (16 layers at 90000 rows
+    // 590 us, 604 with them; of 4- and 3-bit launches at most 1 %).
     constexpr int kHeadStart = 4, kOthers = kMW - 2;
-    const bool late = appender && n_chunks == 1;
+    constexpr bool kShares = BITS != 2;
+    const bool late = kShares && appender && n_chunks == 1;
     const int n_pool = n_tiles - (late ? 1 : 0);  // tiles that are shared out
     auto fixed_tile = [&](int i) -> int {
         int lt = warp + kMW * i;
@@ -331,9 +334,9 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     }
     // The next two refills and, from the third on, the tile after them (kMW further each time: every special share is among
     // the first four of a warp, and at least one of those is in the ring).
+    [[maybe_unused]] int i_next = n_stages;  // plain shares need no more than this
     const int i0 = n_stages + (last_due ? 0 : 1);
-    int refill = last_due ? n_tiles - 1 : fixed_tile(n_stages), refill2 = fixed_tile(i0);
-    int later = warp + kMW * (i0 + 1);
+    [[maybe_unused]] int refill = last_due ? n_tiles - 1 : fixed_tile(n_stages), refill2 = fixed_tile(i0), later = warp + kMW * (i0 + 1);
     if (late) later += warp >= kOthers ? kOthers * (kHeadStart - 1) : -(kMW - kOthers) * (kHeadStart - 1);
     if (tid == kMT - 1) o.last = clean;
     // ---- q: per-head RMSNorm (layer form), rope, Givens rotation, scale, split into f16 hi/lo, written in the
@@ -712,16 +715,23 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
                     compute_tile(lt, st_addr);
                 }
                 __syncwarp();  // every lane has read the stage: lane 0 may refill it
-                int nu = refill;
+                int nu;
                 if (dyn && !last_due) {
                     nu = __shfl_sync(0xffffffffu, drawn, 0);
                     if (nu < n_pool) draw();  // the draw after this one
                     else nu = -1;
+                } else if constexpr (kShares) {
+                    nu = refill;
+                } else {
+                    nu = warp + kMW * i_next++;
+                    if (nu >= n_tiles) nu = -1;
                 }
-                last_due = false;
-                refill = refill2;
-                refill2 = later < n_pool ? later : -1;
-                later += kMW;
+                if constexpr (kShares) {
+                    last_due = false;
+                    refill = refill2;
+                    refill2 = later < n_pool ? later : -1;
+                    later += kMW;
+                }
                 if (nu >= 0) issue_tile(nu, st);
                 else n_held--;
 #pragma unroll

@@ -913,7 +913,7 @@ def test_split_and_whole_sequences_in_one_launch(bk, gpu_ctx, oracle, tag, mode,
     cache.close()
 
 
-@pytest.mark.parametrize("tag", ["planar4", "planar3", "planar2"])
+@pytest.mark.parametrize("tag", ["planar4", "planar3"])
 def test_batch_results_stay_what_they_were(bk, gpu_ctx, tag):
     """A batch with a (sequence, kv head) pair for every SM: which warp scans which tiles, and in which order, decides the last
     bits of the f16 weights.  The golden values (two heads of three sequences) come from an earlier build with the same
