@@ -908,10 +908,14 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
         // Fewer pairs than SMs: one wave.  The balanced chunk length, grown until the items fit the SMs, so
         // that all CTAs are resident together (which the slice form of the split-K combine needs) and no
         // second, nearly empty wave doubles the launch.
-        // Short contexts: chunks of at least 96 rows over quantized V (a launch of 36 to 68 CTAs leaves room for the next
-        // launch's set-up; 511 rows 9.8 us, with 32-row chunks 10.2), of 32 rows otherwise (511 rows of f16 7.4 us, with
-        // 96-row chunks 7.6).  Where V is f32 six warps scan tiles of 16 rows, and a chunk above 96 rows is a multiple of
-        // that round (4096 rows: 192-row chunks 13.1 us, 128-row chunks 14.0).
+        // Short contexts: chunks of at least 96 rows over quantized V, of 32 rows otherwise.  Microseconds a layer of a 16-layer
+        // step, 32 / 96 rows: planar4, 24 heads on 4: 200 rows 10.5 / 10.9, 511 10.5 / 10.5, 1024 10.8 / 10.0, 1500 10.6 / 10.1; 6 on
+        // 1: 2600 rows 10.7 / 9.2, 6000 10.3 / 9.4.  f16, 24 on 4: 511 rows 7.8 / 8.0, 1024 8.2 / 8.1; 6 on 1: 511 rows
+        // 7.5 / 7.5, 4096 8.8 / 8.2 (64 rows: 7.1 and 8.3).  f32, 24 on 4: 350 rows 9.1 / 9.5, 1500 9.8 / 9.5; 8 on 2: 2040
+        // rows 10.5 / 9.2.  (For f16 and f32 neither is better over the whole range.)
+        // Where V is f32 six warps scan tiles of 16 rows, and a chunk above 96 rows is a multiple of that round: f32, 24 on 4: 4096 rows
+        // 14.0 without, 13.3 with; 8 on 2: 9000 rows 14.7 / 13.3; planar4k, 8 on 2: 9000 rows 12.4 / 11.9, 24 on 4: 9000
+        // rows 14.8 / 15.2; elsewhere the same.
         const bool v_planar = a.v_kind == ROW_PLANAR, v_f32 = a.v_kind == ROW_F32;
         const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms / n_kv);
         L = (total + target_items - 1) / target_items;
