@@ -927,7 +927,7 @@ def main():
                      "peak_kind": f"of {peak_kind}",
                      # not measured by this run: dram__bytes_read.sum + dram__bytes_write.sum of one launch of this
                      # kernel at this workload, copied from an ncu capture (mean of the captured launches)
-                     "traffic": {("planar4", 131072): 142.5e6, ("f16", 32768): 138.3e6}.get((args.mode, args.ctx)),
+                     "traffic": {("planar4", 131072): 142.5e6, ("f16", 32768): 138.5e6}.get((args.mode, args.ctx)),
                      "traffic_source": "ncu capture of one layer of this workload (copied constant, see the profile summaries)",
                      "algorithmic_bytes_per_launch": alg, "avg_launch_ms": dec_ms_avg,
                      "avg_launch_ms_source": "timed region / (steps x layers): one decode launch per layer, overlapped by "
