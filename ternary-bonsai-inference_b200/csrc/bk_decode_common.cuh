@@ -284,7 +284,7 @@ constexpr bool boxes_fit() {
 }
 static_assert(boxes_fit(), "a box does not hold a chunk's values and (m, l) pairs, or a slice has no owner");
 
-// Are the boxes fit for use?  Read by one thread behind the dependency wait.
+// Are the boxes fit for use?  Read by one thread of a CTA beside its first boxes.
 __device__ __forceinline__ bool boxes_clean(const DecodeArgs &a) {
     unsigned w;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(w) : "l"(a.box_state) : "memory");
@@ -310,7 +310,7 @@ __device__ __forceinline__ bool box_full(float x) { return __float_as_uint(x) !=
 __device__ __forceinline__ bool box_full4(float4 v) { return box_full(v.x) && box_full(v.y) && box_full(v.z) && box_full(v.w); }
 
 // sums[r]: this chunk's value of coordinate tid (threads 0..255) of head r; s_M, s_L: its maxima and sums.  `red` is
-// free shared memory (16-byte aligned, kCombineBytes); *s_ok is boxes_clean() on entry.  Every thread of the CTA calls.
+// free shared memory (16-byte aligned, kCombineBytes); *s_ok is 1 on entry.  Every thread of the CTA calls.
 // A thread merges a few chunks of one 16-byte column on its own (its own reference, no exchange of maxima), the threads
 // that write the output merge the thread groups: one barrier between the loads and the output.
 constexpr uint32_t kCombineBytes = 12288;
@@ -322,6 +322,8 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
     const int lg = slice_lg(n_chunks, a.xch_peer != nullptr), D4 = 1 << lg, D = 4 * D4, n_slices = kHd / 4 >> lg;
     float *const boxes = a.boxes + (size_t)first_item * NREP * kBoxFloats;
     float *const ml = boxes + (size_t)n_slices * n_chunks * NREP * D;
+    bool clean = true;
+    if (tid == nthr - 1) clean = boxes_clean(a);
     // ---- send
     if (tid < kHd) {
         const int sl = tid >> (lg + 2);
@@ -403,6 +405,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
             asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(a.box_state), "r"(0u) : "memory");
         }
     }
+    if (!clean) *s_ok = 0;
     float2 *s_ml = reinterpret_cast<float2 *>(red);  // [n_grp][NREP]
     float *s_sum = red + 2 * 256;                     // [n_grp][NREP][D]
     if (grp < n_grp) {

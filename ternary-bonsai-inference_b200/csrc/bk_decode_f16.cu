@@ -159,6 +159,7 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     const uint32_t app_bar = base + (uint32_t)offsetof(Other, app_bar);
     if (tid < 2) mbar_init(base + (uint32_t)offsetof(Other, fin_bar) + tid * 8u, 1);
     if (tid == 2) mbar_init(app_bar, 2);
+    if (tid == 3) o.last = 1;  // the slice combine's waits have not run out
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 
     // ---- which item ------------------------------------------------------------------------
@@ -252,8 +253,6 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
     const bool appender = a.new_k != nullptr && chunk == n_chunks - 1;
     const int half_rot = a.no_rope ? 0 : a.n_rot >> 1;
     const int role = appender ? warp - (kFW - 2) : -1;  // 0 = K, 1 = V
-    bool clean = true;
-    if (a.dist && tid == kFT - 1) clean = boxes_clean(a);
     QHead qhd;
     float4 new_lo, new_hi;
     if (warp < NREP) {
@@ -274,7 +273,6 @@ decode_f16_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t s
             if (warp + st * kFW < n_tiles) issue_tile(warp + st * kFW, st);
     }
 
-    if (tid == kFT - 1) o.last = clean;
     // ---- q: RMSNorm, rope, scale, split into f16 hi/lo, laid out as B fragments ---------------------
     // 1/sqrt(hd) * log2(e): the scores come out in the exp2 domain.
     // k-step ks covers coordinates 16 ks .. 16 ks + 15; lane (g, t) holds head g's values at

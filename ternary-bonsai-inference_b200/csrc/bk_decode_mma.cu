@@ -189,6 +189,7 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     const uint32_t app_bar = other_addr + (uint32_t)offsetof(Other, app_bar);
     if (tid < 2) mbar_init(other_addr + (uint32_t)offsetof(Other, fin_bar) + tid * 8u, 1);
     if (tid == 2) mbar_init(app_bar, 2);
+    if (tid == 3) o.last = 1;  // the slice combine's waits have not run out
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 
     // ---- which item ------------------------------------------------------------------------
@@ -290,8 +291,6 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     static_assert(NREP <= kMW - 2, "the appending warps prepare no q head");
     const int half = a.no_rope ? 0 : a.n_rot >> 1;
     const int role = appender ? warp - (kMW - 2) : -1;  // 0 = K, 1 = V
-    bool clean = true;
-    if (a.dist && tid == kMT - 1) clean = boxes_clean(a);
     QHead qhd;
     float4 new_lo, new_hi;
     if (warp < NREP) {
@@ -338,7 +337,6 @@ decode_p4_mma_kernel(DecodeArgs a, DecodeMeta meta, float lut_alpha, uint32_t sm
     const int i0 = n_stages + (last_due ? 0 : 1);
     [[maybe_unused]] int refill = last_due ? n_tiles - 1 : fixed_tile(n_stages), refill2 = fixed_tile(i0), later = warp + kMW * (i0 + 1);
     if (late) later += warp >= kOthers ? kOthers * (kHeadStart - 1) : -(kMW - kOthers) * (kHeadStart - 1);
-    if (tid == kMT - 1) o.last = clean;
     // ---- q: per-head RMSNorm (layer form), rope, Givens rotation, scale, split into f16 hi/lo, written in the
     // MMA's B-fragment layout and then fetched by every lane into registers.
     // 1/sqrt(hd) * log2(e) / alpha: the scores come out in the exp2 domain, alpha undone.
