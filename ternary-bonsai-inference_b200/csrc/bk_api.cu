@@ -350,6 +350,9 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
     const size_t run_bytes = (size_t)ctx->n_sms * kPrefillRunFloats * sizeof(float);
     if ((e = cudaMalloc(&ctx->d_prefill_runs, run_bytes + ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc prefill sums");
     if ((e = cudaMemset((char *)ctx->d_prefill_runs + run_bytes, 0, ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "clear prefill sums");
+    const size_t prefill_floats = (size_t)2 * std::min(ctx->n_sms, kPrefillStretches) * kPrefillPartFloats;
+    if ((e = cudaMalloc((void **)&ctx->d_prefill, prefill_floats * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc prefill scratch");
+    ctx->d_prefill_floats = prefill_floats;
     {
         void *herr = nullptr, *derr = nullptr;
         if ((e = cudaHostAlloc(&herr, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) return bail(e, "cudaHostAlloc error word");
@@ -1493,6 +1496,14 @@ bk_status bk_kvq_threshold_cells(int32_t bits, uint32_t *out) {
     static_assert(sizeof(uint2) == 2 * sizeof(uint32_t), "cell layout");
     if (!build_threshold_cells(book, 1 << bits, reinterpret_cast<uint2 *>(out)))
         return fail(nullptr, BK_ERR_UNSUPPORTED, "codebook thresholds do not fit the cell table");
+    return BK_OK;
+}
+
+bk_status bk_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces, int32_t *n_pieces) {
+    if (!n_pieces || (capacity > 0 && !pieces) || n_sms < 1 || pos0 < 0 || n_tokens < 1 || n_kv < 1 || n_head % n_kv != 0 || n_head / n_kv < 1 ||
+        n_head / n_kv > 128)
+        return fail(nullptr, BK_ERR_INVALID, "bk_prefill_plan: bad argument");
+    *n_pieces = prefill_plan(n_sms, pos0, n_tokens, n_head, n_kv, capacity, pieces);
     return BK_OK;
 }
 

@@ -64,6 +64,10 @@ struct RopeTable {
 
 // A CTA's f32 sums in the prefill attention: 128 query rows of 256 coordinates.
 constexpr size_t kPrefillRunFloats = 128 * 256;
+// The prefill attention's work is cut into a stretch per SM and these into pieces; a piece of a cut item - there are two a stretch at most - has a
+// place in the scratch, 128 query rows of (O, m, l).
+constexpr int kPrefillStretches = 160, kPrefillParts = 2 * kPrefillStretches, kPrefillPieces = 768;
+constexpr size_t kPrefillPartFloats = 128 * (256 + 2);
 
 struct HostPipe;  // pinned slots and copy threads of bulk host transfers (bk_hostpipe.cpp)
 void host_pipe_destroy(HostPipe *p);
@@ -97,7 +101,7 @@ struct bk_ctx {
     size_t d_stage_bytes = 0;
     float *d_layer = nullptr;              // normed q and k rows of the layer step (generic decode path)
     size_t d_layer_floats = 0;
-    float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention's context chunks
+    float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention (the mma.sync form may grow it)
     size_t d_prefill_floats = 0;
     float *d_prefill_runs = nullptr;       // prefill attention: kPrefillRunFloats per SM, then an int per SM (taken or not)
     bk::HostPipe *pipe = nullptr;          // made by the first bulk host transfer
@@ -329,6 +333,7 @@ bool prefill_mma_supported(const DecodeArgs &a);
 bk_status launch_prefill_mma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha);
 // The same on tcgen05 tensor cores with the accumulators in tensor memory (bk_prefill_umma.cu).
 bool prefill_umma_supported(const DecodeArgs &a);  // planar4 / planar3 / f16 caches
+int prefill_plan(int n_sms, int pos0, int n_tokens, int n_head, int n_kv, int capacity, int32_t *pieces);  // see bk_prefill_plan
 bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha);
 bk_status launch_lse_merge(bk_ctx *ctx, int n_parts, int n_rows, int hd, const float *parts, float *out);
 

@@ -2,27 +2,27 @@
 // 5th-generation tensor cores: the same work split and operands as bk_prefill.cu (which documents them and
 // stays as the mma.sync form), with both contractions issued as tcgen05.mma and the accumulators in tensor memory.
 //
-// One CTA = 128 query rows (M = 128) of one kv head over one context chunk, tile by tile of 32 positions.  What
-// bounds it: for 4-bit and f32 rows six 128 x 32 x 256 products per tile (hi.hi, hi.lo, lo.hi twice), 1536 clocks of
-// the tensor cores, and about as much traffic of shared memory; so nothing may wait for anything else, and shared
-// memory has to be spared.  Thirteen warps in three roles, coupled by mbarriers only:
+// One CTA = 128 query rows (M = 128) of one kv head over a piece of the context they see, tile by tile of 32 positions.  What
+// bounds it: for 4-bit and f32 rows six 128 x 32 x 256 products per tile (hi.hi, hi.lo, lo.hi twice), 1800 clocks of the tensor cores as
+// issued; softmax warps and producers each take 2000 to 2600 of a tile's 2800 clocks, and shared memory is about as busy; so nothing may
+// wait for anything else.  Thirteen warps in three roles, coupled by mbarriers only:
 //   * warps 4-11 (producers) turn packed rows into f16 operand tiles (for 4 bit with the rounding remainders, for
-//     f32 rows hi + lo parts) in a ring of four slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
-//     16-byte pieces of a row go out in an order that depends on its lane, or the eight lanes of a row would meet on
-//     two of eight bank groups.  f16 rows are operands as stored and are dropped in by the TMA engine.
+//     f32 rows hi + lo parts) in a ring of five slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
+//     16-byte pieces of a packed row go out in an order that depends on its lane, or the eight lanes of a row would meet on
+//     two of eight bank groups; of f32 rows a warp takes one at a time.  f16 rows are operands as stored and are dropped in by the TMA engine.
 //   * warp 12 issues the products: S(t + 1) = Q . K^T goes ahead of O += P(t) . V, so the tensor cores work on S(t + 1)
 //     under the softmax of tile t.  The small terms of S have columns of their own: the accumulator truncates, and does
 //     so at the size of what it holds.
 //   * warps 0-3 (thread = query row = tensor-memory lane) read S, scale by ||k||, apply the causal limit, move the
-//     running reference R of s + log2 ||v|| LAZILY (only when the row maximum exceeds R by more than 8: the weights
-//     p = 2^(t - R) * 64 then stay below 2^14 in f16; their row of O is then rescaled in place) and write the
-//     weights as f16 hi + lo.
-// Tensor memory (all 512 columns): O 256 | half of q_hi 64 | S 2 x (32 + 32) | P (hi, lo) 2 x 32.  A product with N = 32 costs as
-// much as one with N = 64 (32 clocks), so q_hi meets k_hi and k_lo side by side; P and as much of q_hi as there are columns for
+//     running reference of s + log2 ||v|| LAZILY (only when the row maximum has run ahead; their row of O is then rescaled in place) and
+//     write the weights 2^(s - ref) ||v|| as f16 hi + lo.
+// Tensor memory (all 512 columns): O 256 | q_hi 128 | S 2 x (32 + 32), where the weights (hi, lo) take the place of the scores.  A product
+// with N = 32 costs as much as one with N = 64 (32 clocks), so q_hi meets k_hi and k_lo side by side; P and q_hi
 // are A operands from tensor memory, which spares shared memory 4 KiB a product.
-// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.3 -> 5.9 ms, a 777-token f32 prompt in
-// one block 741 -> 309 us.  Before, one role after the other per tile with every MMA operand moved to uniform registers.  Without
-// the runs of collect_o 5.5 ms and 287 us.
+// Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.3 ms with one role after the other per tile, 5.95 with the
+// roles and (query block, kv head, chunk) items of one length each, 4.95 in pieces (plan_pieces), 4.70 with less around the tiles of a piece
+// (q's preparation 5.6 -> 3.3 us, the first tile and the epilogue 2 us each), 4.50 when a producer's first use of a row no longer stood
+// right behind its load, 4.46 with all of q_hi in tensor memory; a 777-token f32 prompt in one block 741, 320, 302, 288, 255 us.
 // Every mbarrier wait is bounded: one that runs out raises the context's error flag, the others of the CTA stop
 // waiting, and the kernel runs on to its end, where the tensor memory is always released.
 #include <cuda_fp16.h>
@@ -44,8 +44,9 @@ namespace {
 constexpr int kSoftWarps = 4, kProdWarps = 8, kMmaWarp = kSoftWarps + kProdWarps, kUWarps = kMmaWarp + 1, kUT = kUWarps * 32;
 constexpr int kRows = 128;  // query rows per CTA = tensor-memory lanes
 constexpr int kTK = 32;     // positions per tile
-constexpr float kPScale = 64.0f, kPScaleLog2 = 6.0f;
-constexpr float kLazy = 8.0f;  // the reference moves when a row maximum exceeds it by more than this (log2 units)
+// Weights are 2^(s - ref) ||v||, with the reference kBelow under a row's maximum of s + log2 ||v|| when it moves, which it does when the maximum
+// has run kLazy further ahead: they stay below 2^14.
+constexpr float kBelow = 6.0f, kLazy = 8.0f;
 constexpr size_t kRunFloats = kPrefillRunFloats;  // a CTA's sums of the runs done, [4 coordinates][row][4]
 static_assert(kRunFloats == (size_t)kRows * kHd, "a place per row and coordinate");
 
@@ -53,24 +54,23 @@ constexpr uint32_t kQSlab = kRows * 128, kQTile = 4 * kQSlab;  // 16 KiB per 64-
 constexpr uint32_t kKVSlab = kTK * 128, kKVTile = 4 * kKVSlab;  // 4 KiB, 16 KiB
 // Operand slots.  Four: K(t) then takes the place of K(t - 2), whose S products were issued when the softmax had read tile
 // t - 4, so the norms of four tiles can be kept.
-constexpr int kSlots = 4, kNormTiles = 4;
+constexpr int kSlots = 5, kNormTiles = 4;
 constexpr uint32_t kSlotBytes = 2 * kKVTile;  // hi and lo tile
 // offsets from the 1024-byte aligned base
-constexpr uint32_t oQlo = 0, oQhi2 = kQTile, oSlots = oQhi2 + kQTile / 2, oSmall = oSlots + kSlots * kSlotBytes;
+constexpr uint32_t oQlo = 0, oSlots = kQTile, oSmall = oSlots + kSlots * kSlotBytes;
 struct SmallU {
     float givens[kHd];
-    float kn[kNormTiles][kTK], lv[kNormTiles][kTK];  // ||k|| and log2 ||v|| of a tile's positions
+    alignas(16) float kn[kNormTiles][kTK], vn[kNormTiles][kTK], lv[kNormTiles][kTK];  // ||k||, ||v|| and log2 ||v|| of a tile's positions
     unsigned long long full[kSlots], empty[kSlots];  // operand slots
     unsigned long long norms[kNormTiles];            // kn, lv of a tile written
     unsigned long long s_full[2], p_full[2], o_done[2], drain;
-    float mul[kRows];  // what a row's sums are multiplied by at the end
     uint32_t tmem_slot;
     int gave_up;
     int run_slot;
 };
 constexpr uint32_t kUmmaSmem = oSmall + 3072;
 static_assert(sizeof(SmallU) <= 3072 && kUmmaSmem <= 227 * 1024, "shared memory of a CTA");
-constexpr uint32_t kTmemCols = 512, kColO = 0, kColQ = 256, kColS = 320, kColP = 448;
+constexpr uint32_t kTmemCols = 512, kColO = 0, kColQ = 256, kColS = 384;
 
 __device__ __forceinline__ uint32_t sw_off(int rows, int row, int chunk) {  // as tile_off in bk_prefill.cu
     return (uint32_t)((chunk >> 3) * rows * 128 + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
@@ -89,7 +89,7 @@ __device__ __forceinline__ uint32_t expand16u(uint32_t y) {  // eight 2-bit indi
     y = (y | (y << 2)) & 0x33333333u;
     return y;
 }
-// The first `rot` (0..3) of four words go to the end: the piece order of a lane, see dequant_store_shfl.
+// The first `rot` (0..3) of four words go to the end: the piece order of a lane, see dequant_store.
 __device__ __forceinline__ void rotate4(uint32_t (&w)[4], int rot) {
     if (rot & 1) {
         const uint32_t t = w[0];
@@ -100,12 +100,46 @@ __device__ __forceinline__ void rotate4(uint32_t (&w)[4], int rot) {
         w[0] = w[2], w[1] = w[3], w[2] = t0, w[3] = t1;
     }
 }
+// Eight nibbles of up to 7 -> eight f16 centroids, two a word, by byte permutes: a permute picks four bytes out of eight by four nibbles,
+// so the table is kept as its low bytes and its high bytes.  No shared memory is involved, whose bandwidth the kernel has to spare.
+struct Planes {
+    uint32_t lo[2], hi[2];
+    __device__ __forceinline__ void build(uint32_t tab) {  // lane i holds entry i
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t a = __byte_perm(__shfl_sync(0xffffffffu, tab, 4 * k), __shfl_sync(0xffffffffu, tab, 4 * k + 1), 0x5410);
+            const uint32_t b = __byte_perm(__shfl_sync(0xffffffffu, tab, 4 * k + 2), __shfl_sync(0xffffffffu, tab, 4 * k + 3), 0x5410);
+            lo[k] = __byte_perm(a, b, 0x6420);
+            hi[k] = __byte_perm(a, b, 0x7531);
+        }
+    }
+    __device__ __forceinline__ void look_up(uint32_t x, uint32_t (&h)[4]) const {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const uint32_t sel = x >> (16 * q), bl = __byte_perm(lo[0], lo[1], sel), bh = __byte_perm(hi[0], hi[1], sel);
+            h[2 * q] = __byte_perm(bl, bh, 0x5140);
+            h[2 * q + 1] = __byte_perm(bl, bh, 0x7362);
+        }
+    }
+};
+
 // 32 coordinates (four words of eight nibbles, rotated by `rot`) -> 32 halfs as four 16-byte chunks of a tile row.
 // The eight lanes of a row store chunks 4 c + ((j + c / 2) & 3) together, one per bank group (4 c + j would put them on two).
-// The table sits in registers: lane i holds (hi | lo << 16) of centroid i & 15, one shuffle looks both parts of an index
-// up, and no shared-memory bank is involved.  (A shuffle takes the low five bits of the lane number; the fifth, the next index's, does not matter.)
-template <bool LO>
-__device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint32_t tab, uint8_t *tile_hi, uint8_t *tile_lo, int rows,
+__device__ __forceinline__ void dequant_store(const uint32_t (&w)[4], const Planes &tab, uint8_t *tile_hi, uint8_t *, int rows, int row_hi, int,
+                                              int chunk0, int rot) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        uint32_t h[4];
+        tab.look_up(w[j], h);
+        const int chunk = chunk0 + ((j + rot) & 3);
+        *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, row_hi, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+}
+
+// The same for tables with remainders, which take 37 instructions a word by permutes: the table sits in registers, lane i holds
+// (hi | lo << 16) of centroid i & 15, one shuffle looks both parts of an index up.  (A shuffle takes the low five bits of the lane number;
+// the fifth, the next index's, does not matter.)
+__device__ __forceinline__ void dequant_store(const uint32_t (&w)[4], uint32_t tab, uint8_t *tile_hi, uint8_t *tile_lo, int rows,
                                                    int row_hi, int row_lo, int chunk0, int rot) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -119,13 +153,53 @@ __device__ __forceinline__ void dequant_store_shfl(const uint32_t (&w)[4], uint3
         }
         const int chunk = chunk0 + ((j + rot) & 3);
         *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, row_hi, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
-        if (LO) *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, chunk)) = make_uint4(l[0], l[1], l[2], l[3]);
+        *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, chunk)) = make_uint4(l[0], l[1], l[2], l[3]);
     }
+}
+
+// An item is a (query block, kv head), the last block first.  A launch has a CTA per piece: some tiles of an item, a whole item (part < 0) or a
+// part of one, which then leaves (O, m, l) of its query rows in a place of the scratch.
+struct Piece {
+    int item;
+    uint16_t at, end;  // tiles
+    int16_t part;
+};
+struct PieceList {
+    int n;  // 0: every item whole
+    Piece p[kPrefillPieces];
+};
+struct ItemParts {  // of every item: its first place in the scratch (they lie side by side) and how many
+    int16_t first[kPrefillPieces], n[kPrefillPieces];
+};
+static_assert((size_t)kRows * (kHd + 2) == kPrefillPartFloats, "scratch of a piece: [row][coordinate], then [row](m, l)");
+
+// Two f32 operations in one instruction (the softmax warps are bound by what they issue).
+__device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t first(uint64_t x) { return (uint32_t)x; }
+__device__ __forceinline__ uint32_t second(uint64_t x) { return (uint32_t)(x >> 32); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
 }
 
 struct PrefillUArgs {
     DecodeArgs d;
-    int seq, pos0, n_tokens, tq, n_blocks, n_chunks;
+    int seq, pos0, n_tokens, tq, n_blocks;
     float lut_alpha;
     float *scratch;
     float *runs;      // a place of kRunFloats per resident CTA, and which of them are taken
@@ -136,7 +210,7 @@ struct PrefillUArgs {
 
 template <int BITS, int NREP, bool VF32 = false>
 __global__ void __launch_bounds__(kUT, 1)
-prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
+prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_constant__ PieceList list, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
     extern __shared__ __align__(1024) uint8_t sm[];
     const DecodeArgs &a = pa.d;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm), small = base + oSmall;
@@ -161,32 +235,16 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
 
     constexpr int kRun = kLoTiles ? 16 : 20;  // tiles that O collects, at most, before it is added up in f32 (see collect_o)
 
-    // ---- which item (as in the mma.sync kernel) ---------------------------------------------
-    const int item = blockIdx.x;
-    // the blocks late in the prompt see the most rows: they go first
-    const int chunk = item % pa.n_chunks, kv = (item / pa.n_chunks) % a.n_kv, blk = pa.n_blocks - 1 - item / (pa.n_chunks * a.n_kv);
+    // ---- which piece ------------------------------------------------------------------------
+    const int item = list.n ? list.p[blockIdx.x].item : blockIdx.x;
+    const int kv = item % a.n_kv, blk = pa.n_blocks - 1 - item / a.n_kv;
     const int tok0 = blk * pa.tq, n_tok = min(pa.tq, pa.n_tokens - tok0), n_rows = n_tok * NREP;
-    const int vis = pa.pos0 + tok0 + n_tok;
-    const int L = ((vis + pa.n_chunks - 1) / pa.n_chunks + kTK - 1) / kTK * kTK;
-    const int c0 = chunk * L, c1 = min(c0 + L, vis);
-    const int n_tiles = c1 > c0 ? (c1 - c0 + kTK - 1) / kTK : 0;
+    const int vis = pa.pos0 + tok0 + n_tok, at = list.n ? list.p[blockIdx.x].at : 0, t_end = list.n ? list.p[blockIdx.x].end : (vis + kTK - 1) / kTK;
+    const int part = list.n ? list.p[blockIdx.x].part : -1;
+    const int c0 = at * kTK, c1 = min(t_end * kTK, vis), n_tiles = t_end - at;
     const int n_runs = (n_tiles + kRun - 1) / kRun, run_len = n_runs > 1 ? (n_tiles + n_runs - 1) / n_runs : kRun;
 
-    // ---- the query rows start travelling: every row's round trip at once -----------------------------------
     const int half = a.n_rot >> 1;
-    {
-        const float *q0 = a.q + ((size_t)tok0 * a.n_head + kv * NREP) * kHd;
-        auto row_src = [&](int r) { return q0 + ((size_t)(r / NREP) * a.n_head + r % NREP) * kHd; };
-        if (((uintptr_t)a.q & 15) == 0) {
-            for (int i = tid; i < n_rows * (kHd / 4); i += kUT)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + oSlots + 16u * i), "l"(row_src(i / (kHd / 4)) + 4 * (i % (kHd / 4)))
-                             : "memory");
-        } else {
-            for (int i = tid; i < n_rows * kHd; i += kUT)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(base + oSlots + 4u * i), "l"(row_src(i / kHd) + i % kHd) : "memory");
-        }
-    }
-
     // ---- tables, barriers, tensor memory ----------------------------------------------------
     for (int i = tid; i < kHd; i += kUT) ss.givens[i] = a.givens[i];
     auto bar_at = [&](size_t off, int i) { return small + (uint32_t)off + 8u * (uint32_t)i; };
@@ -225,12 +283,26 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) tmem_alloc(small + (uint32_t)offsetof(SmallU, tmem_slot), kTmemCols);
+    // Nothing above was another kernel's.  The query rows start travelling: every row's round trip at once.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    {
+        const float *q0 = a.q + ((size_t)tok0 * a.n_head + kv * NREP) * kHd;
+        auto row_src = [&](int r) { return q0 + ((size_t)(r / NREP) * a.n_head + r % NREP) * kHd; };
+        if (((uintptr_t)a.q & 15) == 0) {
+            for (int i = tid; i < n_rows * (kHd / 4); i += kUT)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(base + oSlots + 16u * i), "l"(row_src(i / (kHd / 4)) + 4 * (i % (kHd / 4)))
+                             : "memory");
+        } else {
+            for (int i = tid; i < n_rows * kHd; i += kUT)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(base + oSlots + 4u * i), "l"(row_src(i / kHd) + i % kHd) : "memory");
+        }
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, ss.tmem_slot, 0);
     auto run_sums = [&]() { return reinterpret_cast<float4 *>(pa.runs + (size_t)ss.run_slot * kRunFloats); };
-    float *run_mul = reinterpret_cast<float *>(sm + oQlo);  // [row], where q_lo was: the runs' factor at the end
+    float *run_mul = reinterpret_cast<float *>(sm + oQlo), *row_mul = run_mul + kRows;  // where q_lo was: the runs' and the rows' factors at the end
     const uint32_t my_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's 32 lanes
 
     // bounded wait; after one has run out (never expected) the others of the CTA do not start to wait
@@ -257,14 +329,15 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     };
     uint32_t pk[4], pv[4];  // packed K of one tile and packed V of the tile before, on their way
     float pn = 0.f;
-    // f32 rows: the thread's 128 bytes, its four 16-byte operand pieces in the lane's order
+    // f32 rows: a warp takes four rows of the tile, a lane 32 bytes of each, which become a 16-byte operand piece.  (Eight lanes a row with 128 bytes
+    // each, as for packed rows, made every load touch 32 lines: 4096 of a tile's 3970 clocks.)
     [[maybe_unused]] float4 fk[kF32 ? 8 : 1], fv[kVRows32 ? 8 : 1];
     auto fetch_f32 = [&](float4 *dst, const uint8_t *rows, int tile) {
-        const float4 *src = reinterpret_cast<const float4 *>(rows + row_of(tile, my_row) * 1024) + 8 * my_c;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            dst[2 * j] = __ldg(src + 2 * ((j + rot) & 3));
-            dst[2 * j + 1] = __ldg(src + 2 * ((j + rot) & 3) + 1);
+            const float4 *src = reinterpret_cast<const float4 *>(rows + row_of(tile, (pt >> 5) * 4 + j) * 1024) + 2 * lane;
+            dst[2 * j] = __ldg(src);
+            dst[2 * j + 1] = __ldg(src + 1);
         }
     };
     auto fetch_packed = [&](uint32_t (&w)[4], const uint8_t *rows, int tile) {
@@ -293,50 +366,72 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         else if constexpr (!kF16) fetch_packed(pv, a.v_rows, tile);
     };
 
-    // ---- q rows -> q_hi and q_lo: rope, Givens, scale, f16 hi/lo; a warp takes a row, the 32 bytes of a lane are coordinates
-    // 8 lane .. + 7; the half of q_hi for tensor memory goes where the row was ---------------------------------------
+    if (producer) {  // the first K tile travels too (and of packed rows the first V tile)
+        if constexpr (!kF32) fetch_k(0);
+        if constexpr (!kVRows32) fetch_v(0);
+    }
+
+    // ---- q rows -> q_hi and q_lo: rope, Givens, scale, f16 hi/lo; a warp takes every kUWarps-th row.  Its rows' rope entries, a pair of
+    // coordinates per lane, travel with the rows (up to 32 pairs; wider rotations read the others where they need them).  Then the 32 bytes
+    // of a lane are coordinates 8 lane .. + 7; the half of q_hi for tensor memory goes where the row was.  (Pairs of lanes that exchange
+    // their coordinates of the rotated quarter cost twice the instructions, which is what this takes: 5.5 us.)
+    constexpr int kMyRows = (kRows + kUWarps - 1) / kUWarps;
+    auto rope_row = [&](int r) { return a.rope + (size_t)(pa.pos0 + tok0 + r / NREP) * half; };
+    float2 cs[kMyRows];
+#pragma unroll
+    for (int i = 0; i < kMyRows; i++) {
+        const int r = warp + i * kUWarps;
+        if (r < n_rows && lane < half) cs[i] = __ldg(rope_row(r) + lane);
+    }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     {
         const float qscale = rsqrtf((float)kHd) * 1.4426950408889634f / pa.lut_alpha;
-        // the rope entries of the warp's next two rows travel (up to 32 per row; wider rotations read the rest where they need it)
-        auto rope_row = [&](int r) { return a.rope + (size_t)(pa.pos0 + tok0 + r / NREP) * half; };
-        auto rope_of = [&](int r) { return r < n_rows && lane < half ? __ldg(rope_row(r) + lane) : make_float2(1.f, 0.f); };
-        float2 c0r = rope_of(warp), c1r = rope_of(warp + kUWarps);
-        for (int r = warp; r < kRows; r += kUWarps) {
+#pragma unroll
+        for (int i = 0; i < kMyRows; i++) {
+            const int r = warp + i * kUWarps;
             float *row = reinterpret_cast<float *>(sm + oSlots) + r * kHd;
-            uint32_t hw[4] = {}, lw[4] = {};
-            const float2 c2r = rope_of(r + 2 * kUWarps);
-            if (r < n_rows) {
-                for (int j = lane; j < half; j += 32) {
-                    float x0 = row[j], x1 = row[j + half];
-                    rope_pair(x0, x1, j < 32 ? c0r : __ldg(rope_row(r) + j));
+            if (r < n_rows && lane < half) {
+                float x0 = row[lane], x1 = row[lane + half];
+                rope_pair(x0, x1, cs[i]);
+                row[lane] = x0;
+                row[lane + half] = x1;
+                for (int j = lane + 32; j < half; j += 32) {
+                    x0 = row[j], x1 = row[j + half];
+                    rope_pair(x0, x1, __ldg(rope_row(r) + j));
                     row[j] = x0;
                     row[j + half] = x1;
                 }
-                __syncwarp();
+            }
+        }
+        float gv[8];
+        if constexpr (!kRaw) {
+            const float4 g0 = reinterpret_cast<const float4 *>(ss.givens)[2 * lane], g1 = reinterpret_cast<const float4 *>(ss.givens)[2 * lane + 1];
+            gv[0] = g0.x, gv[1] = g0.y, gv[2] = g0.z, gv[3] = g0.w, gv[4] = g1.x, gv[5] = g1.y, gv[6] = g1.z, gv[7] = g1.w;
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int r = warp; r < kRows; r += kUWarps) {
+            uint4 *row = reinterpret_cast<uint4 *>(sm + oSlots + r * (kHd * 4));
+            uint32_t hw[4] = {}, lw[4] = {};
+            if (r < n_rows) {
                 const float4 x0 = reinterpret_cast<const float4 *>(row)[2 * lane], x1 = reinterpret_cast<const float4 *>(row)[2 * lane + 1];
                 const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
                 for (int p = 0; p < 4; p++) {
                     float o0 = x[2 * p], o1 = x[2 * p + 1];
-                    if constexpr (!kRaw) {
-                        const int d = 8 * lane + 2 * p;
-                        givens_fwd(x[2 * p], x[2 * p + 1], ss.givens[d], ss.givens[d + 1], o0, o1);
-                    }
+                    if constexpr (!kRaw) givens_fwd(x[2 * p], x[2 * p + 1], gv[2 * p], gv[2 * p + 1], o0, o1);
                     o0 *= qscale;
                     o1 *= qscale;
-                    const __half h0 = __float2half_rn(o0), h1 = __float2half_rn(o1);
-                    const __half l0 = __float2half_rn(o0 - __half2float(h0)), l1 = __float2half_rn(o1 - __half2float(h1));
-                    hw[p] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
-                    lw[p] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
+                    const __half2 h = __floats2half2_rn(o0, o1);
+                    const float2 hf = __half22float2(h);
+                    const __half2 l = __floats2half2_rn(o0 - hf.x, o1 - hf.y);
+                    hw[p] = *reinterpret_cast<const uint32_t *>(&h);
+                    lw[p] = *reinterpret_cast<const uint32_t *>(&l);
                 }
                 __syncwarp();
             }
-            c0r = c1r;
-            c1r = c2r;
-            uint4 *hi = lane < 16 ? reinterpret_cast<uint4 *>(row) + (lane ^ (r & 7)) : reinterpret_cast<uint4 *>(sm + oQhi2 + sw_off(kRows, r, lane - 16));
-            *hi = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            row[lane ^ (r & 7)] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
             *reinterpret_cast<uint4 *>(sm + oQlo + sw_off(kRows, r, lane)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
     }
@@ -345,7 +440,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     const int my_q = (warp & 3) * 32 + lane;  // query row of a softmax thread
     if (warp < kSoftWarps) {
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < 4; b++) {
             uint32_t r[32];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
@@ -361,7 +456,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     __syncthreads();
     tc_fence_after_sync();
 
-    float R = -CUDART_INF_F, lsum = 0.f;  // a query row's running reference and sum
+    float ref = -CUDART_INF_F, lsum = 0.f;  // a query row's running reference and sum
     if (warp == kMmaWarp) {
         // ---- the products -----------------------------------------------------------------------------------
         constexpr int kKRows = kLoTiles ? 64 : 32;  // a K slab holds k_hi in rows 0-31 and k_lo in rows 32-63
@@ -372,19 +467,17 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             if (++slot == kSlots) slot = 0, use ^= 1u;
         };
         auto issue_s = [&](int tile) -> bool {
-            if (!__all_sync(0xffffffffu, wait(bar_full + 8 * slot, use))) return false;
+            bool go = wait(bar_full + 8 * slot, use);
+            if (tile >= 2) go = go && wait(bar_o + 8 * (tile & 1), (uint32_t)((tile - 2) >> 1) & 1u);  // P(tile - 2), in the same columns, has been used
+            if (!__all_sync(0xffffffffu, go)) return false;
             tc_fence_after_sync();
             // columns 0-31: q_hi k_hi; 32-63: the small terms
             const uint32_t d = tmem + kColS + (uint32_t)(tile & 1) * 64u, kb = base + oSlots + slot * kSlotBytes;
             const uint64_t kd = umma_smem_desc(kb, 16, 1024, kUmmaSwizzle128), ql = umma_smem_desc(base + oQlo, 16, 1024, kUmmaSwizzle128);
-            const uint64_t qh2 = umma_smem_desc(base + oQhi2, 16, 1024, kUmmaSwizzle128);
             if (elect_one()) {  // (the address field of a descriptor counts 16-byte units)
 #pragma unroll
-                for (int ks = 0; ks < 8; ks++)
+                for (int ks = 0; ks < 16; ks++)
                     umma_f16_ts(d, tmem + kColQ + 8 * ks, kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s2, ks > 0);
-#pragma unroll
-                for (int ks = 8; ks < 16; ks++)
-                    umma_f16_ss(d, qh2 + ((((ks >> 2) - 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s2, true);
 #pragma unroll
                 for (int ks = 0; ks < 16; ks++)
                     umma_f16_ss(d + 32, ql + (((ks >> 2) * kQSlab + (ks & 3) * 32) >> 4), kd + (((ks >> 2) * kKSlab + (ks & 3) * 32) >> 4), idesc_s,
@@ -399,14 +492,13 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         bool ok = n_tiles == 0 || issue_s(0);
         int run_start = 0;
         for (int tile = 0; ok && tile < n_tiles; tile++) {
-            // (S(tile + 1) goes where S(tile - 1) was, which the softmax had read when P(tile - 1) was awaited)
             if (tile + 1 < n_tiles && !issue_s(tile + 1)) break;
             ok = wait(bar_full + 8 * slot, use);
             ok = ok && wait(bar_p + 8 * (tile & 1), (uint32_t)(tile >> 1) & 1u);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
-            const uint32_t p = tmem + kColP + (uint32_t)(tile & 1) * 32u, vb = base + oSlots + slot * kSlotBytes;
+            const uint32_t p = tmem + kColS + (uint32_t)(tile & 1) * 64u, vb = base + oSlots + slot * kSlotBytes;
             const uint64_t vd = umma_smem_desc(vb, kKVSlab, 1024, kUmmaSwizzle128);
             if (elect_one()) {
 #pragma unroll
@@ -481,25 +573,37 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             const float cent = kRaw ? 0.f : a.book[lane & ((1 << (kRaw ? 4 : BITS)) - 1)] * pa.lut_alpha;
             const __half cent_hi = __float2half_rn(cent);
             const uint32_t tab = (uint32_t)__half_as_ushort(cent_hi) | ((uint32_t)__half_as_ushort(__float2half_rn(cent - __half2float(cent_hi))) << 16);
-            // split the fetched floats into f16 hi + lo and store both as four 16-byte chunks of a tile row; rows at or past
-            // the chunk's end are stored as zeros (they may hold anything, and 0 * Inf would poison the accumulators)
-            auto split_store = [&](const float4 *f, uint8_t *tile_hi, uint8_t *tile_lo, int rows, int row_lo, bool live) {
+            // tables without remainders (8 entries at most) by permutes, others by shuffles
+            auto make_table = [&]() {
+                if constexpr (kRaw || kLoTiles) {
+                    return tab;
+                } else {
+                    Planes p;
+                    p.build(tab);
+                    return p;
+                }
+            };
+            const auto table = make_table();
+            // split the fetched floats into f16 hi + lo and store both as a 16-byte chunk of a tile row each; rows at or past
+            // the piece's end are stored as zeros (they may hold anything, and 0 * Inf would poison the accumulators)
+            auto split_store = [&](const float4 *f, int tile, uint8_t *tile_hi, uint8_t *tile_lo, int rows, int lo_rows) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
+                    const int r = (pt >> 5) * 4 + j;
                     const float x[8] = {f[2 * j].x, f[2 * j].y, f[2 * j].z, f[2 * j].w, f[2 * j + 1].x, f[2 * j + 1].y, f[2 * j + 1].z, f[2 * j + 1].w};
-                    uint32_t h[4], l[4];
+                    uint32_t h[4] = {}, l[4] = {};
+                    if (c0 + tile * kTK + r < c1) {
 #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float x0 = live ? x[2 * e] : 0.f, x1 = live ? x[2 * e + 1] : 0.f;
-                        const __half2 hv = __floats2half2_rn(x0, x1);
-                        const float2 hf = __half22float2(hv);
-                        const __half2 lv = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
-                        h[e] = *reinterpret_cast<const uint32_t *>(&hv);
-                        l[e] = *reinterpret_cast<const uint32_t *>(&lv);
+                        for (int e = 0; e < 4; e++) {
+                            const __half2 hv = __floats2half2_rn(x[2 * e], x[2 * e + 1]);
+                            const float2 hf = __half22float2(hv);
+                            const __half2 lv = __floats2half2_rn(x[2 * e] - hf.x, x[2 * e + 1] - hf.y);
+                            h[e] = *reinterpret_cast<const uint32_t *>(&hv);
+                            l[e] = *reinterpret_cast<const uint32_t *>(&lv);
+                        }
                     }
-                    const int ch = 4 * my_c + ((j + rot) & 3);
-                    *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, my_row, ch)) = make_uint4(h[0], h[1], h[2], h[3]);
-                    *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, row_lo, ch)) = make_uint4(l[0], l[1], l[2], l[3]);
+                    *reinterpret_cast<uint4 *>(tile_hi + sw_off(rows, r, lane)) = make_uint4(h[0], h[1], h[2], h[3]);
+                    *reinterpret_cast<uint4 *>(tile_lo + sw_off(rows, r + lo_rows, lane)) = make_uint4(l[0], l[1], l[2], l[3]);
                 }
             };
             auto widen = [&](uint32_t (&w)[4]) {
@@ -524,18 +628,33 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                 if (lane == 0) mbar_arrive(bar_full + 8 * slot);
                 next_slot();
             };
-            auto live = [&](int tile) { return c0 + tile * kTK + my_row < c1; };
+            // (What is done with a fetched row begins here: left to itself the compiler puts the first of it right behind the loads.)
+            auto arrived = [&](uint32_t (&w)[4]) { asm volatile("" : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3])); };
+            auto arrived_f32 = [&](float4 *f) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) asm volatile("" : "+f"(f[j].x), "+f"(f[j].y), "+f"(f[j].z), "+f"(f[j].w));
+            };
             auto put_k = [&](int tile) -> bool {
                 if (!__all_sync(0xffffffffu, slot_free())) return false;  // one answer for the warp, also when a wait runs out
+                if constexpr (kF32) {
+                    arrived_f32(fk);
+                } else {
+                    arrived(pk);
+                    asm volatile("" : "+f"(pn));
+                }
                 uint8_t *dst = sm + oSlots + slot * kSlotBytes;
                 if constexpr (kF32) {
-                    split_store(fk, dst, dst, 64, my_row + 32, live(tile));
+                    split_store(fk, tile, dst, dst, 64, 32);
                 } else {
                     widen(pk);
-                    dequant_store_shfl<kLoTiles>(pk, tab, dst, dst, kLoTiles ? 64 : 32, my_row, my_row + 32, 4 * my_c, rot);
+                    dequant_store(pk, table, dst, dst, kLoTiles ? 64 : 32, my_row, my_row + 32, 4 * my_c, rot);
                     if (pt < 2 * kTK) {
                         if (pt < kTK) ss.kn[tile % kNormTiles][pt] = pn;
-                        else ss.lv[tile % kNormTiles][pt - kTK] = VF32 ? 0.f : fast_log2(fmaxf(pn, 1e-30f));
+                        else if constexpr (!VF32) {
+                            pn = fmaxf(pn, 1e-30f);
+                            ss.vn[tile % kNormTiles][pt - kTK] = fminf(pn, 3.4028235e38f);  // (finite: it meets weights of 0)
+                            ss.lv[tile % kNormTiles][pt - kTK] = fast_log2(pn);
+                        }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_norms + 8 * (tile % kNormTiles));
                     }
@@ -546,19 +665,22 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
             };
             auto put_v = [&](int tile) -> bool {
                 if (!__all_sync(0xffffffffu, slot_free())) return false;  // one answer for the warp, also when a wait runs out
+                if constexpr (kVRows32) arrived_f32(fv);
+                else arrived(pv);
                 uint8_t *dst = sm + oSlots + slot * kSlotBytes;
                 if constexpr (kVRows32) {
-                    split_store(fv, dst, dst + kKVTile, kTK, my_row, live(tile));
+                    split_store(fv, tile, dst, dst + kKVTile, kTK, 0);
                 } else {
                     widen(pv);
-                    dequant_store_shfl<kLoTiles>(pv, tab, dst, dst + kKVTile, kTK, my_row, my_row, 4 * my_c, rot);
+                    dequant_store(pv, table, dst, dst + kKVTile, kTK, my_row, my_row, 4 * my_c, rot);
                 }
                 put_done();
                 if (tile + 1 < n_tiles) fetch_v(tile + 1);
                 return true;
             };
-            if (n_tiles > 0) fetch_k(0), fetch_v(0);
-            bool ok = n_tiles == 0 || put_k(0);
+            if constexpr (kF32) fetch_k(0);
+            if constexpr (kVRows32) fetch_v(0);
+            bool ok = put_k(0);
             for (int tile = 0; ok && tile < n_tiles; tile++) {
                 if (tile + 1 < n_tiles) ok = put_k(tile + 1);
                 ok = ok && put_v(tile);
@@ -567,7 +689,7 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     } else {
         // ---- softmax: thread = query row ------------------------------------------------------------------------
         const int lim = my_q < n_rows ? pa.pos0 + tok0 + my_q / NREP + 1 : 0;
-        float run_R = -CUDART_INF_F;  // the reference of the sums of the runs done
+        float run_ref = -CUDART_INF_F;  // the reference of the sums of the runs done
         int run_start = 0;
         // O collects a run of tiles, joins the sums of the runs before, rounded to nearest, and starts again: its adds truncate at the
         // size of what it holds, so its error grows with the tiles it collects.  Against float64, channels with x20 outliers: 777
@@ -575,59 +697,95 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
         // of 512 2.0e-6 (3.5e-6, 2.2e-6); V of one sign, 4608 tokens, 2.8e-6 (7.9e-6).  Without lo tiles a run may be longer: fewer
         // products.  The sums stay in L2; a launch pays 5 us for the first and the last pass over them and 4 for each between: the
         // 4608 tokens 6.2 -> 6.7 ms (four layers), 777 tokens 287 -> 309 us.  The same by shorter chunks: 7.1 ms and 341 us.
-        auto collect_o = [&](bool first) {
-            const float f = run_R > -CUDART_INF_F ? fast_exp2(run_R - R) : 0.f;
-            for (int b = 0; b < 8; b++) {
-                float4 *at = run_sums() + (8 * b) * kRows + my_q;
-                float4 old[8];
+        // The sums so far come in a block of 32 coordinates ahead of their use, the first before the run's last product is awaited (one block
+        // after the other, each with its trip to L2, made 4 us of it).
+        auto collect_o = [&](bool first, auto &&run_done) -> bool {
+            float4 old[2][8];
+            auto fetch = [&](int b, float4 (&dst)[8]) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) old[j] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(at + j * kRows);
+                for (int j = 0; j < 8; j++) dst[j] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
+            };
+            fetch(0, old[0]);
+            if (!run_done()) return false;
+            const float f = run_ref > -CUDART_INF_F ? fast_exp2(run_ref - ref) : 0.f;
+#pragma unroll 2
+            for (int b = 0; b < 8; b++) {
+                if (b < 7) fetch(b + 1, old[(b + 1) & 1]);
                 uint32_t o[32];
                 tmem_ld32(my_tmem + kColO + 32 * b, o);
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    __stcg(at + j * kRows, make_float4(fmaf(old[j].x, f, __uint_as_float(o[4 * j])), fmaf(old[j].y, f, __uint_as_float(o[4 * j + 1])),
-                                                       fmaf(old[j].z, f, __uint_as_float(o[4 * j + 2])), fmaf(old[j].w, f, __uint_as_float(o[4 * j + 3]))));
+                for (int j = 0; j < 8; j++) {
+                    const float4 x = old[b & 1][j];
+                    __stcg(run_sums() + (8 * b + j) * kRows + my_q,
+                           make_float4(fmaf(x.x, f, __uint_as_float(o[4 * j])), fmaf(x.y, f, __uint_as_float(o[4 * j + 1])),
+                                       fmaf(x.z, f, __uint_as_float(o[4 * j + 2])), fmaf(x.w, f, __uint_as_float(o[4 * j + 3]))));
+                }
             }
-            run_R = R;
+            run_ref = ref;
+            return true;
         };
         for (int tile = 0; tile < n_tiles; tile++) {
             const uint32_t buf = (uint32_t)tile & 1u, par = (uint32_t)(tile >> 1) & 1u;
             if (tile == run_start && tile > 0) {  // (the next product, which starts O again, waits for this tile's weights)
-                if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
-                tc_fence_after_sync();
-                collect_o(tile == run_len);
+                const bool ok = collect_o(tile == run_len, [&]() {
+                    if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) return false;
+                    tc_fence_after_sync();
+                    return true;
+                });
+                if (!ok) break;
             }
             bool ok = wait(bar_s + 8 * buf, par);
             if constexpr (!kRaw) ok = ok && wait(bar_norms + 8 * (tile % kNormTiles), (uint32_t)(tile / kNormTiles) & 1u);
-            if (tile >= 2) ok = ok && wait(bar_o + 8 * buf, par ^ 1u);  // P of two tiles ago has been used
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after_sync();
             uint32_t sr[32], t[32];
             tmem_ld32(my_tmem + kColS + 64 * buf, sr);
             tmem_ld32(my_tmem + kColS + 64 * buf + 32, t);
-            const float *kn = ss.kn[tile % kNormTiles], *lv = ss.lv[tile % kNormTiles];
+            // Two positions at a time: scores less the reference to sv, the same + log2 ||v|| to tv (one array for raw V rows).  The
+            // reference goes in with the first product: a score of about 64 as an f32 number would be off by 2^-18.
+            uint64_t sv[16], tv_[kVPlanar ? 16 : 1];
+            auto tv = [&](int i) -> uint64_t & { return kVPlanar ? tv_[kVPlanar ? i : 0] : sv[i]; };
+            const ulonglong2 *kn2 = reinterpret_cast<const ulonglong2 *>(ss.kn[tile % kNormTiles]), *lv2 = reinterpret_cast<const ulonglong2 *>(ss.lv[tile % kNormTiles]);
+            const float base_ref = ref > -CUDART_INF_F ? ref : 0.f;
+            const uint64_t nref = pair(__float_as_uint(-base_ref), __float_as_uint(-base_ref));
             float mx = -CUDART_INF_F;
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                float s = __uint_as_float(sr[j]) + __uint_as_float(t[j]);
-                if constexpr (!kRaw) s *= kn[j];
-                sr[j] = __float_as_uint(s);
-                t[j] = __float_as_uint(kVPlanar ? s + lv[j] : s);
+            for (int i = 0; i < 16; i += 2) {
+                const uint64_t main[2] = {pair(sr[2 * i], sr[2 * i + 1]), pair(sr[2 * i + 2], sr[2 * i + 3])};
+                const uint64_t small[2] = {pair(t[2 * i], t[2 * i + 1]), pair(t[2 * i + 2], t[2 * i + 3])};
+                if constexpr (kRaw) {
+                    sv[i] = add2(add2(main[0], nref), small[0]);
+                    sv[i + 1] = add2(add2(main[1], nref), small[1]);
+                } else {
+                    const ulonglong2 k2 = kn2[i / 2];
+                    sv[i] = fma2(small[0], k2.x, fma2(main[0], k2.x, nref));
+                    sv[i + 1] = fma2(small[1], k2.y, fma2(main[1], k2.y, nref));
+                }
+                if constexpr (kVPlanar) {
+                    const ulonglong2 l2 = lv2[i / 2];
+                    tv_[i] = add2(sv[i], l2.x);
+                    tv_[i + 1] = add2(sv[i + 1], l2.y);
+                }
             }
             const int n_ok = min(c1, lim) - (c0 + tile * kTK);  // positions of the tile that this row sees
             if (!__all_sync(0xffffffffu, n_ok >= kTK)) {
 #pragma unroll
-                for (int j = 0; j < 32; j++)
-                    if (j >= n_ok) sr[j] = t[j] = __float_as_uint(-CUDART_INF_F);
+                for (int i = 0; i < 16; i++) {
+                    const uint32_t none = __float_as_uint(-CUDART_INF_F);
+                    sv[i] = pair(2 * i < n_ok ? first(sv[i]) : none, 2 * i + 1 < n_ok ? second(sv[i]) : none);
+                    if constexpr (kVPlanar) tv_[i] = pair(2 * i < n_ok ? first(tv_[i]) : none, 2 * i + 1 < n_ok ? second(tv_[i]) : none);
+                }
             }
 #pragma unroll
-            for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(t[j]));
+            for (int i = 0; i < 16; i++) mx = fmaxf(mx, fmaxf(__uint_as_float(first(tv(i))), __uint_as_float(second(tv(i)))));
             // lazy reference: move it only when this row's maximum ran ahead by more than kLazy
-            const bool move = mx > -CUDART_INF_F && (R == -CUDART_INF_F || mx > R + kLazy);
+            const bool move = mx > -CUDART_INF_F && (ref == -CUDART_INF_F || mx > kBelow + kLazy);
             if (__any_sync(0xffffffffu, move)) {  // tensor-memory traffic is warp-collective
-                const float newR = move ? mx : R;
-                const float f = (move && R > -CUDART_INF_F) ? fast_exp2(R - newR) : (move ? 0.f : 1.f);
+                const float new_ref = move ? base_ref + (mx - kBelow) : ref, by = move ? (mx < CUDART_INF_F ? new_ref - base_ref : CUDART_NAN_F) : 0.f;
+                const float f = move ? (ref > -CUDART_INF_F ? fast_exp2(-by) : 0.f) : 1.f;
+                const uint64_t nby = pair(__float_as_uint(-by), __float_as_uint(-by));
+#pragma unroll
+                for (int i = 0; i < 16; i++) sv[i] = add2(sv[i], nby);
                 lsum *= f;
                 if (tile != run_start) {  // (the first product of a run does not add to O)
                     if (!__all_sync(0xffffffffu, wait(bar_o + 8 * (buf ^ 1u), (uint32_t)((tile - 1) >> 1) & 1u))) break;
@@ -640,93 +798,102 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
                         tmem_st16(my_tmem + kColO + 16 * b, o);
                     }
                 }
-                R = newR;
+                ref = new_ref;
             }
-            const float ref = (R > -CUDART_INF_F ? R : 0.f) - kPScaleLog2;
-            // weights, two positions a column: for each K-step of 16 positions eight columns of hi parts and eight of lo parts;
-            // lsum carries their scale
+            // weights p ||v||, two positions a column: for each K-step of 16 positions eight columns of hi parts and eight of lo parts.
+            // (p = 2^(s - ref) stays below 2^114: the norms are taken as 1e-30 at least.)
+            const ulonglong2 *vn2 = reinterpret_cast<const ulonglong2 *>(ss.vn[tile % kNormTiles]);
+            uint64_t l2 = 0;
 #pragma unroll
             for (int kk = 0; kk < 2; kk++) {
                 uint32_t pw[16];
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int j = 16 * kk + 2 * e;
-                    const float w0 = fast_exp2(__uint_as_float(t[j]) - ref), w1 = fast_exp2(__uint_as_float(t[j + 1]) - ref);
-                    if constexpr (kVPlanar) {
-                        lsum += fast_exp2(__uint_as_float(sr[j]) - ref);
-                        lsum += fast_exp2(__uint_as_float(sr[j + 1]) - ref);
-                    } else {
-                        lsum += w0;
-                        lsum += w1;
+                for (int e = 0; e < 8; e += 2) {
+                    ulonglong2 v2;
+                    if constexpr (kVPlanar) v2 = vn2[4 * kk + e / 2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const uint64_t x = sv[8 * kk + e + u];
+                        const float p0 = fast_exp2(__uint_as_float(first(x))), p1 = fast_exp2(__uint_as_float(second(x)));
+                        const uint64_t p = pair(__float_as_uint(p0), __float_as_uint(p1));
+                        l2 = add2(l2, p);
+                        uint64_t w = p;
+                        if constexpr (kVPlanar) w = mul2(p, u ? v2.y : v2.x);
+                        const float w0 = __uint_as_float(first(w)), w1 = __uint_as_float(second(w));
+                        const __half2 h = __floats2half2_rn(w0, w1);
+                        const float2 hf = __half22float2(h);
+                        const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
+                        pw[e + u] = *reinterpret_cast<const uint32_t *>(&h);
+                        pw[8 + e + u] = *reinterpret_cast<const uint32_t *>(&l);
                     }
-                    const __half2 h = __floats2half2_rn(w0, w1);
-                    const float2 hf = __half22float2(h);
-                    const __half2 l = __floats2half2_rn(w0 - hf.x, w1 - hf.y);
-                    pw[e] = *reinterpret_cast<const uint32_t *>(&h);
-                    pw[8 + e] = *reinterpret_cast<const uint32_t *>(&l);
                 }
-                tmem_st16(my_tmem + kColP + 32 * buf + 16 * kk, pw);
+                tmem_st16(my_tmem + kColS + 64 * buf + 16 * kk, pw);  // (where this row's S was, which is in registers)
             }
+            lsum += __uint_as_float(first(l2)) + __uint_as_float(second(l2));
             if (tile == run_start) run_start += run_len;
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p + 8 * buf);
         }
-        const float unscale = 1.0f / (kPScale * (kVPlanar ? pa.lut_alpha : 1.0f));  // (raw V rows carry no table scale)
-        lsum *= 1.0f / kPScale;
-        if (n_runs > 1) run_mul[my_q] = run_R > -CUDART_INF_F ? fast_exp2(run_R - R) : 0.f;
-        ss.mul[my_q] = pa.n_chunks == 1 ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
-        if (pa.n_chunks > 1 && my_q < n_rows) {
-            float *dst = pa.scratch + (((size_t)(tok0 + my_q / NREP) * a.n_head + kv * NREP + my_q % NREP) * pa.n_chunks + chunk) * (kHd + 2);
-            dst[kHd] = R;
-            dst[kHd + 1] = lsum;
+        const float unscale = 1.0f / (kVPlanar ? pa.lut_alpha : 1.0f);  // (raw V rows carry no table scale)
+        if (n_runs > 1) run_mul[my_q] = run_ref > -CUDART_INF_F ? fast_exp2(run_ref - ref) : 0.f;
+        row_mul[my_q] = part < 0 ? (lsum > 0.f ? unscale / lsum : 0.f) : unscale;
+        if (part >= 0 && my_q < n_rows) {
+            float *dst = pa.scratch + (size_t)part * kPrefillPartFloats + kRows * kHd + 2 * my_q;
+            dst[0] = ref;
+            dst[1] = lsum;
         }
     }
     tc_fence_before_sync();
     __syncthreads();  // (the issuing warp has seen all its products complete)
     tc_fence_after_sync();
 
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     // ---- epilogue: warps 0-11, 32 query rows x 32 columns at a time through a padded shared-memory block, so that the
-    // global stores of a warp cover one row's 128 bytes instead of 32 rows' 8 bytes
+    // global stores of a warp cover four rows' 128 bytes instead of 32 rows' 16 bytes
     if (warp < kMmaWarp) {
-        const bool whole = pa.n_chunks == 1;
-        const float mul = ss.mul[my_q], rmul = n_runs > 1 ? run_mul[my_q] : 0.f;
-        float *stg = reinterpret_cast<float *>(sm + oSlots) + warp * (32 * 33);
-        const int wrow0 = (warp & 3) * 32;
+        const bool whole = part < 0, vec = !whole || ((uintptr_t)a.out & 15) == 0;
+        const float mul = row_mul[my_q], rmul = n_runs > 1 ? run_mul[my_q] : 0.f;
+        constexpr int kPad = 36;
+        float *stg = reinterpret_cast<float *>(sm + oSlots) + warp * (32 * kPad);
+        const int row0 = (warp & 3) * 32 + (lane >> 3), ch = lane & 7;
         for (int b = warp >> 2; b < 8; b += 3) {
-            uint32_t o[32];
-            tmem_ld32(my_tmem + kColO + 32 * b, o);
+            float4 old[8];
             if (n_runs > 1) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float4 x = __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
-                    o[4 * j] = __float_as_uint(fmaf(x.x, rmul, __uint_as_float(o[4 * j])));
-                    o[4 * j + 1] = __float_as_uint(fmaf(x.y, rmul, __uint_as_float(o[4 * j + 1])));
-                    o[4 * j + 2] = __float_as_uint(fmaf(x.z, rmul, __uint_as_float(o[4 * j + 2])));
-                    o[4 * j + 3] = __float_as_uint(fmaf(x.w, rmul, __uint_as_float(o[4 * j + 3])));
-                }
+                for (int j = 0; j < 8; j++) old[j] = __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
             }
+            uint32_t o[32];
+            tmem_ld32(my_tmem + kColO + 32 * b, o);
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                const int d = 32 * b + j;
-                float o0 = n_tiles > 0 ? __uint_as_float(o[j]) * mul : 0.f, o1 = n_tiles > 0 ? __uint_as_float(o[j + 1]) * mul : 0.f;
+            for (int j = 0; j < 8; j++) {
+                float4 x = make_float4(__uint_as_float(o[4 * j]), __uint_as_float(o[4 * j + 1]), __uint_as_float(o[4 * j + 2]), __uint_as_float(o[4 * j + 3]));
+                if (n_runs > 1)
+                    x = make_float4(fmaf(old[j].x, rmul, x.x), fmaf(old[j].y, rmul, x.y), fmaf(old[j].z, rmul, x.z), fmaf(old[j].w, rmul, x.w));
+                x = make_float4(x.x * mul, x.y * mul, x.z * mul, x.w * mul);
                 if (whole && kVPlanar) {
-                    float r0, r1;
-                    givens_inv(o0, o1, ss.givens[d], ss.givens[d + 1], r0, r1);
-                    o0 = r0;
-                    o1 = r1;
+                    const float4 g = *reinterpret_cast<const float4 *>(ss.givens + 32 * b + 4 * j);
+                    float4 y;
+                    givens_inv(x.x, x.y, g.x, g.y, y.x, y.y);
+                    givens_inv(x.z, x.w, g.z, g.w, y.z, y.w);
+                    x = y;
                 }
-                stg[lane * 33 + j] = o0;
-                stg[lane * 33 + j + 1] = o1;
+                *reinterpret_cast<float4 *>(stg + lane * kPad + 4 * j) = x;
             }
             __syncwarp();
-            for (int rr = 0; rr < 32; rr++) {
-                const int q = wrow0 + rr;
-                if (q >= n_rows) break;
-                const size_t orow = (size_t)(tok0 + q / NREP) * a.n_head + kv * NREP + q % NREP;
-                float *drow = whole ? a.out + orow * kHd : pa.scratch + (orow * pa.n_chunks + chunk) * (kHd + 2);
-                drow[32 * b + lane] = stg[rr * 33 + lane];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int q = row0 + 4 * i;
+                if (q >= n_rows) continue;
+                const float4 x = *reinterpret_cast<const float4 *>(stg + ((lane >> 3) + 4 * i) * kPad + 4 * ch);
+                float *dst = (whole ? a.out + ((size_t)(tok0 + q / NREP) * a.n_head + kv * NREP + q % NREP) * kHd
+                                    : pa.scratch + (size_t)part * kPrefillPartFloats + (size_t)q * kHd) + 32 * b + 4 * ch;
+                if (vec) {
+                    *reinterpret_cast<float4 *>(dst) = x;
+                } else {
+                    dst[0] = x.x, dst[1] = x.y, dst[2] = x.z, dst[3] = x.w;
+                }
             }
             __syncwarp();
         }
@@ -740,60 +907,75 @@ prefill_umma_kernel(PrefillUArgs pa, const __grid_constant__ CUtensorMap tm_k, c
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-// Merge the chunks' triples, rotate back, write: a warp per output row, so that the references and sums of up to 64 chunks
-// are one or two loads and the rows' loads do not wait for them.  A chunk that the row does not see counts as zeros whatever it holds.
-constexpr int kMergeWarps = 8;
-__global__ void __launch_bounds__(kMergeWarps * 32) prefill_umma_merge_kernel(const float *scratch, const float *givens, int n_chunks, int n_out, float *out) {
-    const int row = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= n_out) return;
-    const float *basep = scratch + (size_t)row * n_chunks * (kHd + 2);
-    float m[2], f[2], l[2];
+// Merge the pieces of the items that are cut, rotate back, write: a warp per output row, so that the references and sums of all pieces
+// are a few loads side by side and the rows' loads do not wait for them.  A piece that the row does not see counts as zeros whatever it holds.
+constexpr int kMergeWarps = 8, kPerLane = (kPrefillParts + 31) / 32;
+__global__ void __launch_bounds__(kMergeWarps * 32) prefill_umma_merge_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_constant__ ItemParts parts,
+                                                                              const float *givens) {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const int n_head = pa.d.n_head, n_rep = n_head / pa.d.n_kv, row = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int tok = row / n_head, head = row - tok * n_head, blk = tok / pa.tq, my_q = (tok - blk * pa.tq) * n_rep + head % n_rep;
+    if (tok >= pa.n_tokens) return;
+    const int item = (pa.n_blocks - 1 - blk) * pa.d.n_kv + head / n_rep, n = parts.n[item];
+    if (n == 0) return;  // whole: written where it was computed
+    const float *base = pa.scratch + (size_t)parts.first[item] * kPrefillPartFloats;
+    float f[kPerLane], l[kPerLane], M = -CUDART_INF_F, Ls = 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int c = lane + 32 * h;
-        m[h] = c < n_chunks ? basep[(size_t)c * (kHd + 2) + kHd] : -CUDART_INF_F;
-        l[h] = c < n_chunks ? basep[(size_t)c * (kHd + 2) + kHd + 1] : 0.f;
+    for (int h = 0; h < kPerLane; h++) {
+        const int i = lane + 32 * h;
+        const float2 ml = i < n ? *reinterpret_cast<const float2 *>(base + i * kPrefillPartFloats + kRows * kHd + 2 * my_q) : make_float2(-CUDART_INF_F, 0.f);
+        f[h] = ml.x;
+        l[h] = ml.y;
+        M = fmaxf(M, f[h]);
     }
-    float M = fmaxf(m[0], m[1]);
     for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    float Ls = 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        f[h] = m[h] > -CUDART_INF_F ? exp2f(m[h] - M) : 0.f;
+    for (int h = 0; h < kPerLane; h++) {
+        f[h] = f[h] > -CUDART_INF_F ? exp2f(f[h] - M) : 0.f;
         if (f[h] > 0.f) Ls = fmaf(l[h], f[h], Ls);
     }
     for (int o = 16; o > 0; o >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, o);
-    float2 acc[4] = {};  // coordinates 2 lane, 2 lane + 1 of each quarter
+    float4 acc[2] = {};  // coordinates 4 lane .. + 3 of each half
+#pragma unroll
+    for (int h = 0; h < kPerLane; h++)
 #pragma unroll 4
-    for (int c = 0; c < n_chunks; c++) {
-        const float2 *p = reinterpret_cast<const float2 *>(basep + (size_t)c * (kHd + 2)) + lane;
-        const float fc = __shfl_sync(0xffffffffu, c < 32 ? f[0] : f[1], c & 31);
+        for (int i = 32 * h; i < min(n, 32 * h + 32); i++) {
+            const float4 *p = reinterpret_cast<const float4 *>(base + i * kPrefillPartFloats + my_q * kHd) + lane;
+            const float fc = __shfl_sync(0xffffffffu, f[h], i & 31);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float2 v = p[32 * i];
-            acc[i].x = fmaf(fc > 0.f ? v.x : 0.f, fc, acc[i].x);
-            acc[i].y = fmaf(fc > 0.f ? v.y : 0.f, fc, acc[i].y);
+            for (int j = 0; j < 2; j++) {
+                const float4 v = p[32 * j];
+                acc[j].x = fmaf(fc > 0.f ? v.x : 0.f, fc, acc[j].x);
+                acc[j].y = fmaf(fc > 0.f ? v.y : 0.f, fc, acc[j].y);
+                acc[j].z = fmaf(fc > 0.f ? v.z : 0.f, fc, acc[j].z);
+                acc[j].w = fmaf(fc > 0.f ? v.w : 0.f, fc, acc[j].w);
+            }
         }
-    }
     const float inv = Ls > 0.f ? 1.0f / Ls : 0.f;
+    const bool vec = ((uintptr_t)pa.d.out & 15) == 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int d = 64 * i + 2 * lane;
-        float o0 = acc[i].x * inv, o1 = acc[i].y * inv;
+    for (int j = 0; j < 2; j++) {
+        const int d = 128 * j + 4 * lane;
+        float4 o = make_float4(acc[j].x * inv, acc[j].y * inv, acc[j].z * inv, acc[j].w * inv);
         if (givens) {  // planar V only
-            float r0, r1;
-            givens_inv(o0, o1, givens[d], givens[d + 1], r0, r1);
-            o0 = r0;
-            o1 = r1;
+            const float4 g = *reinterpret_cast<const float4 *>(givens + d);
+            float4 r;
+            givens_inv(o.x, o.y, g.x, g.y, r.x, r.y);
+            givens_inv(o.z, o.w, g.z, g.w, r.z, r.w);
+            o = r;
         }
-        float *dst = out + (size_t)row * kHd + d;  // (the caller's alignment is only that of a float)
-        dst[0] = o0;
-        dst[1] = o1;
+        float *dst = pa.d.out + (size_t)row * kHd + d;
+        if (vec) {
+            *reinterpret_cast<float4 *>(dst) = o;
+        } else {  // (the caller's alignment is only that of a float)
+            dst[0] = o.x, dst[1] = o.y, dst[2] = o.z, dst[3] = o.w;
+        }
     }
 }
 
 template <int BITS, int NREP, bool VF32 = false>
-bk_status launch_umma_one(bk_ctx *ctx, const PrefillUArgs &pa) {
+bk_status launch_umma_one(bk_ctx *ctx, const PrefillUArgs &pa, const PieceList &list, const ItemParts &parts) {
     static std::atomic<bool> configured[64] = {};  // per device; racing first calls set the same attribute
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64) return fail(ctx, BK_ERR_UNSUPPORTED, "prefill: device index above 63");
@@ -801,16 +983,28 @@ bk_status launch_umma_one(bk_ctx *ctx, const PrefillUArgs &pa) {
         BK_CUDA(ctx, cudaFuncSetAttribute(prefill_umma_kernel<BITS, NREP, VF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmem));
         configured[dev].store(true);
     }
-    const int grid = pa.n_blocks * pa.d.n_kv * pa.n_chunks;
     if (!pa.d.h_tmap_k || !pa.d.h_tmap_v) return fail(ctx, BK_ERR_INVALID, "prefill: the cache has no tensor maps");
-    prefill_umma_kernel<BITS, NREP, VF32><<<grid, kUT, kUmmaSmem, ctx->stream>>>(pa, *static_cast<const CUtensorMap *>(pa.d.h_tmap_k),
-                                                                          *static_cast<const CUtensorMap *>(pa.d.h_tmap_v));
+    const int n_items = pa.n_blocks * pa.d.n_kv;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(list.n ? list.n : n_items));
+    cfg.blockDim = dim3(kUT);
+    cfg.dynamicSmemBytes = kUmmaSmem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see griddepcontrol.* in the kernels
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, prefill_umma_kernel<BITS, NREP, VF32>, pa, list, *static_cast<const CUtensorMap *>(pa.d.h_tmap_k),
+                                    *static_cast<const CUtensorMap *>(pa.d.h_tmap_v)));
     ctx->launches++;
     BK_CUDA(ctx, cudaGetLastError());
-    if (pa.n_chunks > 1) {
+    if (list.n > n_items) {
         const int n_out = pa.n_tokens * pa.d.n_head;
-        prefill_umma_merge_kernel<<<(n_out + kMergeWarps - 1) / kMergeWarps, kMergeWarps * 32, 0, ctx->stream>>>(
-            pa.scratch, (BITS == 16 || BITS == 32 || VF32) ? nullptr : pa.d.givens, pa.n_chunks, n_out, pa.d.out);
+        cfg.gridDim = dim3((unsigned)((n_out + kMergeWarps - 1) / kMergeWarps));
+        cfg.blockDim = dim3(kMergeWarps * 32);
+        cfg.dynamicSmemBytes = 0;
+        BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, prefill_umma_merge_kernel, pa, parts, (BITS == 16 || BITS == 32 || VF32) ? (const float *)nullptr : pa.d.givens));
         ctx->launches++;
         BK_CUDA(ctx, cudaGetLastError());
     }
@@ -828,29 +1022,89 @@ bool prefill_umma_supported(const DecodeArgs &a) {
     return (planar || f16 || f32 || k_only) && a.h_tmap_k && a.h_tmap_v && (n_rep == 1 || n_rep == 2 || n_rep == 4 || n_rep == 6);
 }
 
-// Into how many chunks the context is cut: the count with the least estimated time.  A CTA has an SM to itself and costs
-// kFixed tiles' worth of set-up, q preparation and epilogue beside its tiles; what a launch then takes is bounded both by full rounds of its
-// longest item and by its work spread evenly plus one longest item (items are handed out longest first).  Merging costs a
-// launch and one read of every chunk's rows.
-static int plan_chunks(int n_sms, int pos0, int n_tokens, int tq, int n_kv, int n_head) {
-    constexpr double kFixed = 6.0, kMergeLaunch = 3.0, kMergeRow = 1.0 / 2048;
-    const int n_blocks = (n_tokens + tq - 1) / tq, vis = pos0 + n_tokens;
-    // no more than about four items per SM, which also bounds the scratch
-    const int most = std::max(1, std::min({64, vis / 256, (4 * n_sms + n_blocks * n_kv - 1) / (n_blocks * n_kv)}));
-    const double mean_vis = pos0 + 0.5 * (n_tokens + tq);
-    double best = 0.0;
-    int chunks = 1;
-    for (int c = 1; c <= most; c++) {
-        const double longest = kFixed + (double)((vis + c * kTK - 1) / (c * kTK)), items = (double)n_blocks * n_kv * c;
-        const double mean = kFixed + std::max(1.0, mean_vis / (c * kTK));
-        const double t = std::min(std::ceil(items / n_sms) * longest, items * mean / n_sms + longest) +
-                         (c > 1 ? kMergeLaunch + kMergeRow * c * n_tokens * n_head / 24 : 0.0);
-        if (c == 1 || t < best) {
-            best = t;
-            chunks = c;
+// How the items are cut into pieces.  All tiles of all items side by side are one line, which is cut into a stretch per SM so that the longest
+// stretch is as short as possible; every piece costs kFixed tiles' worth of set-up, q preparation, filling and draining of the pipeline, and
+// results beside its tiles, and cutting at all costs a launch that merges.  The first CTAs get the longest piece of each stretch,
+// the others follow in order of length: as the SMs come free, the SM with the shortest piece first, each finds about what its stretch had left.
+// With more than kPrefillItems items (four and more an SM) whole ones, longest first, are spread evenly enough.
+constexpr int kPrefillItems = kPrefillPieces - kPrefillStretches;
+static void plan_pieces(int n_sms, int pos0, int n_tokens, int tq, int n_kv, PieceList &list, ItemParts &parts) {
+    constexpr int kFixed = 7, kMerge = 3, kLeast = 4;  // (a piece has kLeast tiles or the rest of its item)
+    const int most = std::min(n_sms, kPrefillStretches), n_blocks = (n_tokens + tq - 1) / tq, n_items = n_blocks * n_kv;
+    list.n = 0;
+    if (n_items > kPrefillItems || (int64_t)pos0 + n_tokens > UINT16_MAX * kTK) return;
+    auto tiles_of = [&](int item) { return (std::min((n_blocks - item / n_kv) * tq, n_tokens) + pos0 + kTK - 1) / kTK; };
+    int n = 0, n_stretches = 0, start[kPrefillStretches + 1];  // pieces in the order of the line, and where the stretches start
+    Piece piece[kPrefillPieces];
+    // into stretches of at most `budget`; false if there are not enough
+    auto cut = [&](int budget) {
+        n = n_stretches = 0;
+        int left = 0;  // of the current stretch
+        for (int item = 0, all = 0; item < n_items; item++) {
+            if (item % n_kv == 0) all = tiles_of(item);
+            for (int at = 0; at < all;) {
+                if (left < kFixed + std::min(all - at, kLeast)) {
+                    if (n_stretches == most) return false;
+                    start[n_stretches++] = n;
+                    left = budget;
+                }
+                int take = std::min(all - at, left - kFixed);
+                if (all - at - take > 0 && all - at - take < kLeast) take = std::max(kLeast, all - at - kLeast);  // no short rest
+                left -= kFixed + take;
+                piece[n++] = Piece{item, (uint16_t)at, (uint16_t)(at + take), -1};
+                at += take;
+            }
         }
+        start[n_stretches] = n;
+        return true;
+    };
+    int total = 0;
+    for (int b = 0; b < n_blocks; b++) total += n_kv * (kFixed + tiles_of(b * n_kv));
+    const int longest = kFixed + tiles_of(0);
+    int lo = std::max(kFixed + kLeast, (total + most - 1) / most), hi = lo + kFixed;
+    if (n_items <= most && longest <= lo + kMerge) return;
+    while (!cut(hi)) lo = hi + 1, hi += std::max(1, hi / 8);
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (cut(mid)) hi = mid;
+        else lo = mid + 1;
     }
-    return chunks;
+    if (n_items <= most && longest <= hi + kMerge) return;  // an item per CTA
+    cut(hi);
+    // places in the scratch
+    int places = 0;
+    for (int i = 0; i < n_items; i++) parts.n[i] = 0;
+    for (int i = 0; i < n; i++) {
+        Piece &p = piece[i];
+        if (p.at == 0 && p.end == tiles_of(p.item)) continue;
+        if (parts.n[p.item]++ == 0) parts.first[p.item] = (int16_t)places;
+        p.part = (int16_t)places++;
+    }
+    // order of the CTAs
+    auto length = [](const Piece &p) { return p.end - p.at; };
+    for (int c = 0; c < n_stretches; c++) {
+        int best = start[c];
+        for (int i = start[c] + 1; i < start[c + 1]; i++)
+            if (length(piece[i]) > length(piece[best])) best = i;
+        list.p[c] = piece[best];
+        piece[best].item = -1;
+    }
+    list.n = n_stretches;
+    for (int i = 0; i < n; i++)
+        if (piece[i].item >= 0) list.p[list.n++] = piece[i];
+    std::stable_sort(list.p + n_stretches, list.p + n, [&](const Piece &x, const Piece &y) { return length(x) > length(y); });
+}
+
+int prefill_plan(int n_sms, int pos0, int n_tokens, int n_head, int n_kv, int capacity, int32_t *pieces) {
+    PieceList list;
+    ItemParts parts;
+    plan_pieces(n_sms, pos0, n_tokens, kRows / (n_head / n_kv), n_kv, list, parts);
+    for (int i = 0; i < std::min(list.n, capacity); i++) {
+        const Piece &p = list.p[i];
+        const int32_t words[4] = {p.item, p.at, p.end, p.part};
+        std::copy(words, words + 4, pieces + 4 * i);
+    }
+    return list.n;
 }
 
 bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha) {
@@ -865,30 +1119,20 @@ bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos
     pa.n_blocks = (n_tokens + pa.tq - 1) / pa.tq;
     pa.lut_alpha = alpha;
     pa.err_flag = ctx->d_err;
-    const int chunks = plan_chunks(ctx->n_sms, pos0, n_tokens, pa.tq, a.n_kv, a.n_head);
-    pa.n_chunks = chunks;
     pa.runs = ctx->d_prefill_runs;
     pa.runs_taken = reinterpret_cast<int *>(ctx->d_prefill_runs + ctx->n_sms * kRunFloats);
     pa.n_runs = ctx->n_sms;
-    if (chunks > 1) {
-        const size_t need = (size_t)n_tokens * a.n_head * chunks * (kHd + 2);
-        if (ctx->d_prefill_floats < need) {
-            BK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (ctx->d_prefill) cudaFree(ctx->d_prefill);
-            ctx->d_prefill = nullptr;
-            ctx->d_prefill_floats = 0;
-            BK_CUDA(ctx, cudaMalloc((void **)&ctx->d_prefill, need * sizeof(float)));
-            ctx->d_prefill_floats = need;
-        }
-        pa.scratch = ctx->d_prefill;
-    }
+    pa.scratch = ctx->d_prefill;
+    PieceList list;
+    ItemParts parts;
+    plan_pieces(ctx->n_sms, pos0, n_tokens, pa.tq, a.n_kv, list, parts);
 #define BK_PU_CASE(R)                                                                            \
     case R:                                                                                      \
-        if (a.k_kind == ROW_F16) return launch_umma_one<16, R>(ctx, pa);                         \
-        if (a.k_kind == ROW_F32) return launch_umma_one<32, R>(ctx, pa);                         \
-        if (a.v_kind == ROW_F32) return a.bits == 3 ? launch_umma_one<3, R, true>(ctx, pa) : launch_umma_one<4, R, true>(ctx, pa); \
-        if (a.bits == 2) return launch_umma_one<2, R>(ctx, pa);                                  \
-        return a.bits == 3 ? launch_umma_one<3, R>(ctx, pa) : launch_umma_one<4, R>(ctx, pa);
+        if (a.k_kind == ROW_F16) return launch_umma_one<16, R>(ctx, pa, list, parts);                         \
+        if (a.k_kind == ROW_F32) return launch_umma_one<32, R>(ctx, pa, list, parts);                         \
+        if (a.v_kind == ROW_F32) return a.bits == 3 ? launch_umma_one<3, R, true>(ctx, pa, list, parts) : launch_umma_one<4, R, true>(ctx, pa, list, parts); \
+        if (a.bits == 2) return launch_umma_one<2, R>(ctx, pa, list, parts);                                  \
+        return a.bits == 3 ? launch_umma_one<3, R>(ctx, pa, list, parts) : launch_umma_one<4, R>(ctx, pa, list, parts);
     switch (n_rep) {
         BK_PU_CASE(1)
         BK_PU_CASE(2)

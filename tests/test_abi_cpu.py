@@ -160,6 +160,37 @@ def test_lane_cells_give_the_reference_scan(bk, oracle, bits):
     assert bad.size == 0, (v[bad[:5]], got[bad[:5]], want[bad[:5]])
 
 
+@pytest.mark.parametrize("n_head,n_kv", [(24, 4), (6, 1), (4, 4), (8, 4), (8, 8)])
+def test_prefill_plan_covers_every_tile_once(bk, n_head, n_kv):
+    """The pieces of a prompt block: every tile that an item sees in exactly one of them, a place of the scratch (two a processor, up to 160
+    processors) for every piece of a cut item, one item's places side by side in the order of its tiles."""
+    lib = bk._abi.load()
+    tq = 128 // (n_head // n_kv)
+    rng = np.random.default_rng(n_head + n_kv)
+    shapes = [(0, 4), (0, 512), (0, 777), (4096, 512), (262000, 100), (20000, 5), (0, 3100), (0, 3400), (0, 9000), (2097000, 300)]
+    shapes += [(int(rng.integers(0, 9000)) * (i % 3 > 0), int(rng.integers(4, 2000))) for i in range(60)]
+    for n_sms in (148, 1, 2, 200):
+        for pos0, n_tok in shapes:
+            words, n = np.full((768, 4), -7, np.int32), C.c_int32(-1)
+            assert lib.bk_prefill_plan(n_sms, pos0, n_tok, n_head, n_kv, 768, words.ctypes.data, C.addressof(n)) == 0
+            if n.value == 0:
+                continue
+            blocks = -(-n_tok // tq)
+            assert blocks * n_kv <= n.value <= 768
+            words = words[:n.value]
+            parts = words[words[:, 3] >= 0, 3]
+            assert len(set(parts)) == len(parts) and (len(parts) == 0 or parts.max() < 2 * min(n_sms, 160))
+            words = words[np.lexsort((words[:, 1], words[:, 0]))]
+            assert np.array_equal(np.unique(words[:, 0]), np.arange(blocks * n_kv))
+            for item in range(blocks * n_kv):
+                w = words[words[:, 0] == item]
+                tiles = -(-(pos0 + min((blocks - item // n_kv) * tq, n_tok)) // 32)
+                assert w[0, 1] == 0 and w[-1, 2] == tiles and np.array_equal(w[1:, 1], w[:-1, 2]) and (w[:, 2] > w[:, 1]).all()
+                assert np.array_equal(w[:, 3], w[0, 3] + np.arange(len(w))) and (w[0, 3] >= 0 or len(w) == 1)
+    assert lib.bk_prefill_plan(0, 0, 4, 24, 4, 0, None, C.addressof(n)) == bk._abi.BK_ERR_INVALID
+    assert lib.bk_prefill_plan(148, 0, 4, 24, 5, 0, None, C.addressof(n)) == bk._abi.BK_ERR_INVALID
+
+
 def test_default_config_is_qwen35(bk):
     cfg = bk._abi.CacheConfig()
     bk._abi.load().bk_default_config(C.byref(cfg))

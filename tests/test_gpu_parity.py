@@ -1423,6 +1423,45 @@ def test_prefill_other_group_sizes_and_long_context(bk, gpu_ctx, oracle):
     assert_close(got, want, "long")
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [MODES[0], MODES[1], MODES[2]])
+@pytest.mark.parametrize("n_head,n_kv,n0,n_tok", [(6, 1, 9000, 5), (24, 4, 2000, 300), (24, 4, 0, 900), (4, 4, 1000, 130)])
+def test_prefill_in_pieces(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv, n0, n_tok):
+    """One item cut into a piece per SM, items in one and in two pieces side by side, items of few tiles.  Tokens at both ends of the blocks
+    against the oracle; the same call again gives the same bits, also after a call that is cut otherwise."""
+    rng = np.random.default_rng(n0 + n_tok)
+    n = n0 + n_tok
+    k, v = rng.standard_normal((2, n, n_kv, HD)).astype(np.float32)
+    q = rng.standard_normal((n_tok, n_head, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n, n_head=n_head, n_kv=n_kv)
+    cache.append(0, k, v)
+    ref = oracle.cache(mode, bits, vq, n_head=n_head, n_kv=n_kv)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got = cache.prefill_attend(0, q, n0)
+    for i in sorted({0, 1, min(20, n_tok - 1), min(21, n_tok - 1), n_tok // 2, n_tok - 2, n_tok - 1}):
+        assert_close(got[i], ref.attend(0, q[i], n0 + i, n0 + i + 1, threads=8), f"{tag} token {i}")
+    cache.prefill_attend(0, q[:4], n0)
+    assert np.array_equal(cache.prefill_attend(0, q, n0), got)
+    cache.close()
+
+
+def test_prefill_of_more_items_than_are_cut(bk, gpu_ctx, oracle):
+    """A prompt block of so many items that they go out whole: 153 blocks of 21 tokens."""
+    rng = np.random.default_rng(3)
+    n = 3200
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode("planar4"), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    ref = oracle.cache(MODE_PLANAR, 4, True)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got = cache.prefill_attend(0, q, 0)
+    for i in (0, 20, 21, 1599, 3191, n - 1):
+        assert_close(got[i], ref.attend(0, q[i], i, i + 1, threads=8), f"token {i}")
+    cache.close()
+
+
 def test_prefill_step_appends_then_attends(bk, gpu_ctx, oracle):
     """bk_prefill_step from the empty cache in blocks: rows bit-exact, outputs within the bar,
     and refusals for tokens that are not in the cache."""
