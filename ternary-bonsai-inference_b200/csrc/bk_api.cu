@@ -867,7 +867,7 @@ bk_status check_decode_entry(const bk_cache *c, int layer, int slot, const int32
 }
 
 // One launch for up to kMaxSeqsPerLaunch sequences of one class.  Chunk length: generic kernel
-// about 4 CTAs per SM over the whole launch, at least 64 positions each; tensor-core kernel one
+// one wave or 2 to 4 CTAs per SM over the whole launch, at least 64 positions each; tensor-core kernel one
 // CTA per SM in one wave (chunks in units of 32 positions), or whole sequences when there are
 // at least as many (sequence, kv head) pairs as SMs; never more than max_items work items (the
 // capacity of the split-K scratch behind a.partials).
@@ -925,8 +925,14 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
         L = std::max<int64_t>(v_planar ? 96 : gran, (L + gran - 1) / gran * gran);
         if (v_f32 && L > 96) L = (L + 95) / 96 * 96;
         while (items_for(L) > ctx->n_sms && L < max_np) L += gran;
+    } else if (a.k_kind == ROW_PLANAR && (int64_t)nb * n_kv * 2 <= ctx->n_sms) {
+        // Generic kernel on planar rows, one CTA of all registers per SM: one wave, as above.  With more pairs about two such CTAs'
+        // time for an SM: 8 bit, 64 sequences of 500 to 3000 rows 164 us a layer (188 with four), 24 such sequences 93 (99).
+        L = (total * n_kv + ctx->n_sms - 1) / ctx->n_sms;
+        L = std::max<int64_t>(gran, (L + 15) / 16 * 16);
+        while (items_for(L) > ctx->n_sms && L < max_np) L += 16;
     } else {
-        const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms * 4 / n_kv);  // about four CTAs per SM
+        const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms * (a.k_kind == ROW_PLANAR ? 2 : 4) / n_kv);  // about two or four CTAs per SM
         L = (total + target_items - 1) / target_items;
         L = std::max<int64_t>(gran, (L + gran - 1) / gran * gran);
     }

@@ -479,6 +479,43 @@ def test_decode_ragged_lengths(bk, gpu_ctx, oracle, n_pos):
         assert_close(got, want, f"{tag} n_pos={n_pos}")
 
 
+@pytest.mark.parametrize("n_head,n_kv", [(24, 4), (4, 4), (16, 2), (8, 2), (4, 2)])
+@pytest.mark.parametrize("tag,bits,vq", [("planar8", 8, True), ("planar5", 5, True), ("planar1", 1, True), ("planar8k", 8, False), ("planar2k", 2, False)])
+def test_generic_planar_decode_in_groups_of_four(bk, gpu_ctx, oracle, tag, bits, vq, n_head, n_kv):
+    """Ragged groups of four rows, chunks with idle warps, several chunks, several rounds of a warp's ring, with every number of heads per kv head."""
+    rng = np.random.default_rng(bits + n_head)
+    lens = [1, 2, 3, 5, 47, 49, 64, 66, 190, 1001, 5003]
+    k, v = rng.standard_normal((2, max(lens), n_kv, HD)).astype(np.float32)
+    q = rng.standard_normal((n_head, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=max(lens), n_head=n_head, n_kv=n_kv)
+    cache.append(0, k, v)
+    ref = oracle.cache(MODE_PLANAR, bits, vq, n_head=n_head, n_kv=n_kv)
+    for p in range(max(lens)):
+        ref.append(0, k[p], v[p], p)
+    for n in lens:
+        got, want = cache.attend(0, q, n_pos=[n], q_pos=[n - 1])[0], ref.attend(0, q, n - 1, n, threads=8)
+        # both add up in f32, each 2e-7 to 6e-7 (2-norm) from the 64-bit result at these lengths; a coordinate may be a dozen times that off
+        assert np.max(np.abs(got - want)) <= 1e-5 * np.max(np.abs(want)), n
+    cache.close()
+
+
+def test_generic_decode_keeps_infinities_where_they_are(bk, gpu_ctx, oracle):
+    """K-only rows: an infinite V coordinate in the last row, of which copies stand in for the rows a group lacks."""
+    rng = np.random.default_rng(5)
+    n = 5
+    k, v = rng.standard_normal((2, n, NKV, HD)).astype(np.float32)
+    q = rng.standard_normal((NH, HD)).astype(np.float32)
+    v[n - 1, 1, 7] = np.inf
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode("planar8k"), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    ref = oracle.cache(MODE_PLANAR, 8, False)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got, want = cache.attend(0, q)[0].reshape(NH, HD), ref.attend(0, q, n - 1, n).reshape(NH, HD)
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.isposinf(want).any() and not np.isnan(got).any()
+    cache.close()
+
+
 def test_decode_long_context_split_k(bk, gpu_ctx, oracle):
     """Enough positions for many chunks per kv head (the partials + last-arriver combine)."""
     for tag, mode, bits, vq in [MODES[2], MODES[1]]:
