@@ -3,11 +3,11 @@
 // kv_store.comp, kv_store_f16.comp and kv_store_q.comp and follows the reference CPU path
 // bit for bit (src/forward.rs:259-285, src/kvquant.rs:397-412, src/rope.rs:61-69).
 //
-// A CTA stages 32 vectors of 256 floats ((K|V, kv head) of consecutive tokens):
+// A CTA stages 8 or 32 vectors of 256 floats ((K|V, kv head) of consecutive tokens):
 //   1. coalesced float4 loads into shared memory; K vectors rotate pairs (j, j + n_rot/2) with
 //      the (cos, sin) row of the token's position from the host-built rope table;
-//   2. planar rows: one warp adds the 256 squares of all 32 vectors, a vector per lane, each lane
-//      in order (the reference's f32 sum is sequential, so each chain is; 32 run side by side);
+//   2. planar rows: one warp adds the 256 squares of all vectors, a vector per lane, each lane
+//      in order (the reference's f32 sum is sequential, so each chain is; they run side by side);
 //   3. the warps scale, Givens-rotate, find the nearest centroid (two shuffles from a host-built cell table of
 //      the decision thresholds, or a binary search and a neighbour check: the same index as the reference's
 //      linear scan) and write `bits` bytes per lane;
@@ -28,6 +28,17 @@ constexpr int kVecPad = kHd + 4;  // floats per staged vector; +4 keeps float4 a
                                   // per-lane 128-bit reads of the norm pass conflict-free
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
+
+// Two f32 products in one instruction, each rounded as __fmul_rn does.
+__device__ __forceinline__ float2 mul_pair(float x, float y, float a, float b) {
+    uint64_t p, q;
+    float2 r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(p) : "f"(x), "f"(y));
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(q) : "f"(a), "f"(b));
+    asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(p) : "l"(q));
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
 
 // Eight consecutive coordinates of a staged vector for every lane without bank conflicts: two 128-bit reads
 // in the staging layout (coordinates 4 l .. 4 l + 3 and 128 + 4 l .. + 3), then lanes 2m and 2m + 1 swap
@@ -81,8 +92,12 @@ __device__ __forceinline__ void store_planar_row_lanes(const float *sx, int lane
     float v[8];
 #pragma unroll
     for (int pr = 0; pr < 4; pr++) {
-        const float a = __fmul_rn(x[2 * pr], inv), b = __fmul_rn(x[2 * pr + 1], inv);
-        givens_fwd(a, b, gv[2 * pr], gv[2 * pr + 1], v[2 * pr], v[2 * pr + 1]);
+        // givens_fwd of the scaled pair, its six products as three
+        const float2 ab = mul_pair(x[2 * pr], x[2 * pr + 1], inv, inv);
+        const float c = gv[2 * pr], sn = gv[2 * pr + 1];
+        const float2 by_c = mul_pair(ab.x, ab.y, c, c), by_s = mul_pair(ab.x, ab.y, sn, sn);
+        v[2 * pr] = __fsub_rn(by_c.x, by_s.y);
+        v[2 * pr + 1] = __fadd_rn(by_s.x, by_c.y);
     }
     uint32_t packed = 0;  // 8 indices of at most 4 bits
     if (n < CUDART_INF_F) {
@@ -111,25 +126,29 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
     reinterpret_cast<uint4 *>(row)[group] = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// A CTA takes 32 consecutive vectors of the launch (vector = token * 2*n_kv + j; j < n_kv: K head
-// j, else V head j - n_kv).  Pass 1: each warp stages 8 vectors with float4 loads and ropes the K
-// ones.  Pass 2: warp 0 adds the squares of all 32 vectors, one vector per lane, each lane in
+// A warp takes one K or V head of kVecs / 8 consecutive tokens, the next warp the next head (j < n_kv: K head j, else V head
+// j - n_kv), so what depends on the head is worked out once a warp.  Pass 1: the warp stages its vectors with float4 loads and
+// ropes the K ones.  Pass 2: warp 0 adds the squares of all 32 vectors, one vector per lane, each lane in
 // order (the reference's f32 sum is sequential, so the chain is; 32 chains run side by side).
-// Pass 3: each warp scales, rotates, finds the nearest centroids of and stores its 8 vectors.
-// kVecs = 32 for bulk calls (throughput: every lane of the norm pass works), 8 for small calls
-// (latency: one vector per warp).
+// Pass 3: each warp scales, rotates, finds the nearest centroids of and stores its vectors.
+// kVecs = 32 for bulk calls of planar rows (throughput: every lane of the norm pass works), 8 for small calls
+// (latency: one vector per warp) and for f32 and f16 rows, which have no norm: many small CTAs load while others store.
+// Registers: four CTAs of 64 an SM; five of 48 spill.  Us a layer of back-to-back calls of 2048 / 4096 tokens: planar4 12.6 / 20.4 with
+// the head worked out per vector, one product at a time and five CTAs, 12.4 / 19.5 without these two, 10.7 / 18.3 with four CTAs; f32
+// 10.3 / 17.7 in CTAs of 32 vectors, 8.2 / 13.5 of 8; f16 11.1 / 17.3 and 8.5 / 14.1.  (Planar rows 16 a CTA: 12.0 / 19.1.)
 template <int BITS, int kVecs>
-__global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(AppendArgs a) {
+__global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : 4) append_kernel(AppendArgs a) {
     extern __shared__ __align__(16) float smem[];
     float *sbook = smem + kVecs * kVecPad;  // centroids
     float *sgiv = sbook + 256;              // Givens table
     float *snorm = sgiv + kHd;              // the 32 norms, and what a vector is scaled by
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kv = a.n_kv, per_tok = 2 * n_kv;
-    const int n_vec = a.n_tokens * per_tok, v0 = blockIdx.x * kVecs;
-    // vector -> (token, K|V head): a shift and a mask when 2 * n_kv is a power of two (it is for qwen35)
-    const int tok_shift = (per_tok & (per_tok - 1)) == 0 ? __ffs(per_tok) - 1 : -1;
-    auto tok_of = [&](int vec) { return tok_shift >= 0 ? vec >> tok_shift : vec / per_tok; };
+    constexpr int kPerWarp = kVecs / kWarps;
+    const int unit = blockIdx.x * kWarps + warp, t0 = unit / per_tok * kPerWarp, j = unit % per_tok;
+    const int n_here = min(kPerWarp, a.n_tokens - t0);  // (0 or less past the last token)
+    const bool is_v = j >= n_kv;
+    const int kv = is_v ? j - n_kv : j;
     const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
 
     if (BITS > 4) {
@@ -142,40 +161,39 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
-    // ---- pass 1: stage (and rope).  A warp owns vectors warp, warp + 8, ...; all of their global
-    // loads (rows and rope entries) are issued before any is used, so the pass costs one round trip.
-    constexpr int kPerWarp = kVecs / kWarps;
+    // ---- pass 1: stage (and rope).  All of a warp's global loads (rows and rope entries) are issued before any is used, so the
+    // pass costs one round trip.
     float4 ra[kPerWarp], rb[kPerWarp];
     float2 rcs[kPerWarp];
     const int half = a.n_rot >> 1;
+    const float4 *src4 = reinterpret_cast<const float4 *>(is_v ? a.v : a.k) + ((size_t)t0 * n_kv + kv) * (kHd / 4) + lane;
 #pragma unroll
     for (int u = 0; u < kPerWarp; u++) {
-        const int vec = v0 + warp + u * kWarps;
         ra[u] = rb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
         rcs[u] = make_float2(1.f, 0.f);
-        if (vec < n_vec) {
-            const int tok = tok_of(vec), j = vec - tok * per_tok;
-            const bool is_v = j >= n_kv;
-            const int kv = is_v ? j - n_kv : j;
-            const float4 *src4 = reinterpret_cast<const float4 *>((is_v ? a.v : a.k) + ((size_t)tok * n_kv + kv) * kHd);
-            ra[u] = __ldg(src4 + lane);
-            rb[u] = __ldg(src4 + lane + 32);
+        if (u < n_here) {
+            ra[u] = __ldg(src4 + (size_t)u * n_kv * (kHd / 4));
+            rb[u] = __ldg(src4 + (size_t)u * n_kv * (kHd / 4) + 32);
             if (!is_v && lane < half) {  // n_rot <= 64: one rope entry per lane
-                const int pos = a.desc ? a.desc[tok].z : a.pos0 + tok;
+                const int pos = a.desc ? a.desc[t0 + u].z : a.pos0 + t0 + u;
                 rcs[u] = __ldg(a.rope + (size_t)pos * half + lane);
             }
         }
     }
+    float *const mine = smem + warp * (kPerWarp * kVecPad);  // the warp's vectors
 #pragma unroll
     for (int u = 0; u < kPerWarp; u++) {
-        const int lv = warp + u * kWarps, vec = v0 + lv;
-        if (vec >= n_vec) continue;
-        float *sx = smem + lv * kVecPad;
+        if (u >= n_here) break;
+        float *sx = mine + u * kVecPad;
         reinterpret_cast<float4 *>(sx)[lane] = ra[u];
         reinterpret_cast<float4 *>(sx)[lane + 32] = rb[u];
-        const bool is_v = (vec - tok_of(vec) * per_tok) >= n_kv;
-        if (!is_v) {
-            __syncwarp();
+    }
+    if (!is_v) {
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kPerWarp; u++) {
+            if (u >= n_here) break;
+            float *sx = mine + u * kVecPad;
             if (half <= 32) {
                 if (lane < half) {
                     float x0 = sx[lane], x1 = sx[lane + half];
@@ -184,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
                     sx[lane + half] = x1;
                 }
             } else {  // wider rotations: entries beyond the prefetched 32 come straight from the table
-                const int tok = tok_of(vec), pos = a.desc ? a.desc[tok].z : a.pos0 + tok;
+                const int pos = a.desc ? a.desc[t0 + u].z : a.pos0 + t0 + u;
                 const float2 *cs = a.rope + (size_t)pos * half;
                 for (int p = lane; p < half; p += 32) {
                     float x0 = sx[p], x1 = sx[p + half];
@@ -208,16 +226,17 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
         gv[4] = g1.x; gv[5] = g1.y; gv[6] = g1.z; gv[7] = g1.w;
     }
     // ---- pass 2: 32 sequential sums side by side ----------------------------------------------------
-    if (planar && warp == 0 && lane < kVecs && v0 + lane < n_vec) {
+    if (planar && warp == 0 && lane < kVecs) {  // (a place without a vector gives a number nobody reads)
         const float4 *x4 = reinterpret_cast<const float4 *>(smem + lane * kVecPad);
         float acc = 0.0f;
 #pragma unroll 8
         for (int i = 0; i < kHd / 4; i++) {
             const float4 x = x4[i];
-            acc = __fadd_rn(acc, __fmul_rn(x.x, x.x));
-            acc = __fadd_rn(acc, __fmul_rn(x.y, x.y));
-            acc = __fadd_rn(acc, __fmul_rn(x.z, x.z));
-            acc = __fadd_rn(acc, __fmul_rn(x.w, x.w));
+            const float2 lo = mul_pair(x.x, x.y, x.x, x.y), hi = mul_pair(x.z, x.w, x.z, x.w);
+            acc = __fadd_rn(acc, lo.x);
+            acc = __fadd_rn(acc, lo.y);
+            acc = __fadd_rn(acc, hi.x);
+            acc = __fadd_rn(acc, hi.y);
         }
         const float n = __fsqrt_rn(acc);
         snorm[lane] = n;
@@ -225,35 +244,32 @@ __global__ void __launch_bounds__(kThreads, kVecs == 32 ? 5 : 4) append_kernel(A
     }
     __syncthreads();
     // ---- pass 3: store --------------------------------------------------------------------------------
-    for (int lv = warp; lv < kVecs; lv += kWarps) {
-        const int vec = v0 + lv;
-        if (vec >= n_vec) break;
-        const int tok = tok_of(vec), j = vec - tok * per_tok;
-        const bool is_v = j >= n_kv;
-        const int kv = is_v ? j - n_kv : j;
-        size_t seq_rows = 0;
-        int row_idx;
+    const int kind = is_v ? a.v_kind : a.k_kind;
+    uint8_t *const rows = is_v ? a.v_rows : a.k_rows;
+    [[maybe_unused]] float *const norms = is_v ? a.v_norms : a.k_norms;
+    const size_t row_bytes = is_v ? a.v_row_bytes : a.k_row_bytes;
+#pragma unroll
+    for (int u = 0; u < kPerWarp; u++) {
+        if (u >= n_here) break;
+        size_t r;  // row of the cache's slab
         if (a.desc) {
-            const int4 d = a.desc[tok];
-            seq_rows = (size_t)d.x * a.seq_stride_rows;
-            row_idx = d.y;
+            const int4 d = a.desc[t0 + u];
+            r = (size_t)d.x * a.seq_stride_rows + (size_t)d.y * n_kv + kv;
         } else {
-            row_idx = a.row0 + tok;
+            r = (size_t)(a.row0 + t0 + u) * n_kv + kv;
         }
-        const float *sx = smem + lv * kVecPad;
-        const size_t r = seq_rows + (size_t)row_idx * n_kv + kv;
-        const int kind = is_v ? a.v_kind : a.k_kind;
-        uint8_t *row = (is_v ? a.v_rows + r * a.v_row_bytes : a.k_rows + r * a.k_row_bytes);
+        const float *sx = mine + u * kVecPad;
+        uint8_t *row = rows + r * row_bytes;
         if (kind == ROW_F32) {
             store_f32_row(sx, lane, row);
         } else if (BITS == 0 && kind == ROW_F16) {  // (f16 rows never lie beside planar ones)
             store_f16_row(sx, lane, row);
         } else {
             if constexpr (BITS > 0) {
-                const float n = snorm[lv];
-                if (lane == 0) (is_v ? a.v_norms : a.k_norms)[r] = n;
-                if constexpr (BITS <= 4) store_planar_row_lanes<BITS>(sx, lane, n, snorm[32 + lv], gv, scale, my, a.book, row);
-                else store_planar_row<BITS>(sx, lane, snorm[32 + lv], sgiv, sbook, row);
+                const float n = snorm[warp * kPerWarp + u], inv = snorm[32 + warp * kPerWarp + u];
+                if (lane == 0) norms[r] = n;
+                if constexpr (BITS <= 4) store_planar_row_lanes<BITS>(sx, lane, n, inv, gv, scale, my, a.book, row);
+                else store_planar_row<BITS>(sx, lane, inv, sgiv, sbook, row);
             }
         }
     }
@@ -266,10 +282,12 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     if (a.n_tokens <= 0) return BK_OK;
     const int threads = kThreads;
     const size_t n_vec = (size_t)a.n_tokens * 2 * a.n_kv;
+    const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
     const bool bulk = n_vec > (size_t)8 * 2 * ctx->n_sms;  // more than two small CTAs per SM: go for throughput
-    const int vecs = bulk ? 32 : 8;
+    const int vecs = bulk && planar ? 32 : 8;
     const size_t smem = (size_t)(vecs * kVecPad + 256 + kHd + 64) * sizeof(float);
-    const unsigned grid = (unsigned)((n_vec + vecs - 1) / vecs);
+    const int per_warp = vecs / kWarps;
+    const unsigned grid = (unsigned)(((size_t)(a.n_tokens + per_warp - 1) / per_warp * 2 * a.n_kv + kWarps - 1) / kWarps);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3((unsigned)threads);
@@ -281,8 +299,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaError_t err = cudaSuccess;
-    const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
-    // The bulk kernel wants five CTAs of 39 KiB per SM: ask for the largest shared-memory carve-out (once per
+    // A bulk call wants four CTAs of 36 KiB or eight of 11 KiB per SM: ask for the largest shared-memory carve-out (once per
     // kernel and process; a hint, so its result is not checked).
     auto launch_bulk = [&](auto *kernel) {
         static std::atomic<bool> hinted{false};
@@ -290,7 +307,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
         return cudaLaunchKernelEx(&cfg, kernel, a);
     };
     if (!planar) {
-        err = bulk ? launch_bulk(append_kernel<0, 32>) : cudaLaunchKernelEx(&cfg, append_kernel<0, 8>, a);
+        err = bulk ? launch_bulk(append_kernel<0, 8>) : cudaLaunchKernelEx(&cfg, append_kernel<0, 8>, a);
     } else {
         const bool ok = dispatch_bits(a.bits, [&]<int B>() {
             err = bulk ? launch_bulk(append_kernel<B, 32>) : cudaLaunchKernelEx(&cfg, append_kernel<B, 8>, a);
