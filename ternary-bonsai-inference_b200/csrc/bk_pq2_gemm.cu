@@ -22,9 +22,11 @@
 //     (one rounding) that is added up as scale * sum, as the reference's scalar path groups it (src/kernels.rs:633-650).
 //     Two pairs of accumulators alternate: the drain of one step runs under the MMAs of the other's next.  128 columns a
 //     pair are what the operand stages leave, hence at most 64 tokens a tile.
-// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 to 16 tokens 52 us (62 and 176 as
-// pairs of tokens; 4 tokens as pairs take 45, which is where the line lies), 64 tokens 69 (702), 128 tokens 97 (1410), 512
-// tokens 299 (5750), 1024 tokens 516.  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
+//   * The two digits that meet the same weights are one B operand of 2 N columns, into both sums of a pair at once: half as many
+//     products as one digit each, and up to 32 tokens each costs the same 32 clocks (512 tokens: 298 us a layer before, 281 so).
+// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 to 16 tokens 51 us (62 and 176 as
+// pairs of tokens; 4 tokens as pairs take 41, which is where the line lies), 64 tokens 67 (702), 128 tokens 93 (1410), 512
+// tokens 281 (5750).  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
 // 57, 86, 129, 287 and 574.  Error against float64, 2-norm: 7.4e-8 on normal data, 8.0e-8 with x20 outliers in x, 4.5e-8 without
 // a bias on products of one sign; 1.02e-7, 2.4e-7 and 5.0e-8 as pairs of tokens; 1.01e-7, 1.0e-7 and 6.5e-8 (bias -5e-8) in the
 // form before, which also lost blocks that lie 2^40 below the token's largest element.
@@ -56,15 +58,15 @@ constexpr uint32_t kGemmStageW = 2 * 2 * 128 * kGemmRowWords * 4;  // staged wei
 // Shared memory of the sums of the segments done, [row tile][token][row].
 __host__ __device__ constexpr uint32_t gemm_sum_bytes(int mt, int n) { return (uint32_t)(mt * n) * 512u; }
 constexpr int kGemmFrac = 27;                     // X = round(x * 2^(kGemmFrac - e))
-// tensor-memory columns: per owner a pair of sums (low | high), then per owner two A stages (weights | times -64)
-constexpr uint32_t kColsD = 128, kColHi = 64, kColA = 256, kColsA = 64;
+// tensor-memory columns: per owner one or two pairs of sums (low | high, N columns each), then per owner two A stages (weights | times -64)
+constexpr uint32_t kColsD = 128, kColA = 256, kColsA = 64;
 
 struct GemmArgs {
     const uint8_t *rows[kGemmMaxSegs];
     float *y[kGemmMaxSegs];
     int seg_rows[kGemmMaxSegs], seg_tile0[kGemmMaxSegs];
     int y_stride[kGemmMaxSegs];  // rows of a token in y (the range may be a part of them)
-    const uint8_t *xb;        // [token tile][block][digit][n][128 B, swizzled]
+    const uint8_t *xb;        // [token tile][block][digit 0 2 1 3][n][128 B, swizzled]
     const float *x_scale;     // [token tile][block][n]: 2^(e - kGemmFrac), NaN for a block with an infinity or a NaN in it
     int nb, row_bytes, n_tok, n_stages_b;
     int vec;                  // bit s: the rows of range s all start on 16-byte boundaries
@@ -116,7 +118,8 @@ __global__ void __launch_bounds__(256) pq2_split_x_kernel(const float *x, int ne
         }
     uint8_t *dst = xb + ((size_t)tile * nb + blk) * (size_t)n * 512 + (size_t)r * 128 + ((i ^ (r & 7)) << 4);
 #pragma unroll
-    for (int k = 0; k < 4; k++) *reinterpret_cast<uint4 *>(dst + (size_t)k * n * 128) = make_uint4(d[k][0], d[k][1], d[k][2], d[k][3]);
+    for (int k = 0; k < 4; k++)  // (in the order 0 2 1 3: what meets the same weights lies side by side)
+        *reinterpret_cast<uint4 *>(dst + (size_t)((k & 1) * 2 + (k >> 1)) * n * 128) = make_uint4(d[k][0], d[k][1], d[k][2], d[k][3]);
 }
 
 // A tensor-memory load without the wait.
@@ -180,12 +183,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
     extern __shared__ __align__(1024) uint8_t sm[];
     constexpr int N = 16 * NC, NH = 8 * NC;  // tokens of the tile, and of one warp
     constexpr uint32_t kBlockB = (uint32_t)N * 512u;
+    constexpr int kBufs = 4 * N <= (int)kColsD ? 2 : 1;  // pairs of sums an owner has room for: with two, a step's products need not wait for the step before to be drained
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
-    // barriers: B full [4] | B free [4] | A full [owner][2] | D full [2] | D free [2] | turn [2] | block scales | drain; then the
-    // tensor-memory address and a give-up flag
-    const uint32_t bar_bf = sbase, bar_be = sbase + 32, bar_af = sbase + 64, bar_df = sbase + 96, bar_de = sbase + 112, bar_turn = sbase + 128,
-                   bar_sc = sbase + 144, bar_drain = sbase + 152, slot = sbase + 160;
+    // barriers: B full [4] | B free [4] | A full [owner][2] | turn [2] | block scales | drain; then the tensor-memory address, a give-up flag,
+    // the order of the segments, D full [owner][2] | D free [owner][2]
+    const uint32_t bar_bf = sbase, bar_be = sbase + 32, bar_af = sbase + 64, bar_turn = sbase + 128, bar_sc = sbase + 144, bar_drain = sbase + 152,
+                   slot = sbase + 160, bar_df = sbase + 384, bar_de = sbase + 416;
+    static_assert(168 + 3 * kGemmMaxSegments <= 384, "the segments' order ends before the barriers behind it");
     volatile int *gave_up = reinterpret_cast<volatile int *>(sm + 164);
     const int nst = a.n_stages_b, nb = a.nb, n_seg = (nb + kGemmSegBlocks - 1) / kGemmSegBlocks;
     const uint32_t off_b = 1024u, off_w = off_b + (uint32_t)nst * kBlockB, off_t = off_w + kGemmStageW, off_s = off_t + gemm_sum_bytes(MT, N);
@@ -212,12 +217,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
             mbar_init(bar_bf + 8 * i, 1);
             mbar_init(bar_be + 8 * i, 1);
             mbar_init(bar_af + 8 * i, 8);
-        }
-        for (int i = 0; i < 2; i++) {
             mbar_init(bar_df + 8 * i, 1);
             mbar_init(bar_de + 8 * i, 8);
-            mbar_init(bar_turn + 8 * i, 8);
         }
+        for (int i = 0; i < 2; i++) mbar_init(bar_turn + 8 * i, 8);
         mbar_init(bar_sc, 1);
         mbar_init(bar_drain, 1);
         *gave_up = 0;
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
             for (int polls = 0; !mbar_try_wait(bar_bf + 8 * (c % nst), (uint32_t)(c / nst) & 1u) && polls < kWaitPolls; polls++) {}
         for (int polls = 0; !mbar_try_wait(bar_sc, 0) && polls < kWaitPolls; polls++) {}
     } else if (warp == kMmaWarp) {
-        const uint32_t idesc = umma_idesc_s8(128, N);
+        const uint32_t idesc = umma_idesc_s8(128, 2 * N);
         uint32_t st = 0, b_par = 0;
         bool ok = true;
         for (int q = 0; q < n_rounds && ok; q++)
@@ -293,20 +296,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
                 if (block_of(q, o) >= nb) continue;
                 if (MT == 1 || o == 0) ok = ok && wait_all(bar_bf + 8 * st, b_par);
                 ok = ok && wait_all(bar_af + 16 * o + 8 * (q & 1), (uint32_t)(q >> 1) & 1u);
-                if (q > 0) ok = ok && wait_all(bar_de + 8 * o, (uint32_t)(q - 1) & 1u);
+                const uint32_t buf = (uint32_t)q % kBufs, turn = (uint32_t)q / kBufs;
+                if (turn > 0) ok = ok && wait_all(bar_de + 16 * o + 8 * buf, (turn - 1) & 1u);
                 if (!ok) break;
                 tc_fence_after_sync();
-                const uint32_t d = tmem + o * kColsD, am = tmem + kColA + o * (2 * kColsA) + (q & 1) * kColsA;
+                const uint32_t d = tmem + o * kColsD + buf * (2 * N), am = tmem + kColA + o * (2 * kColsA) + (q & 1) * kColsA;
                 const uint64_t bd = umma_smem_desc(sbase + off_b + st * kBlockB, 16, 1024, kUmmaSwizzle128);
                 const bool last_use = MT == 1 || o == 1;
                 if (elect_one()) {
 #pragma unroll
-                    for (int dg = 0; dg < 4; dg++)  // digits 0 and 1: low sums, 2 and 3: high ones; the odd ones meet the weights times -64
+                    // digits 0 and 2 side by side into low and high sums, then 1 and 3, which meet the weights times -64: a product of
+                    // up to 64 columns takes the same 32 clocks
+                    for (int odd = 0; odd < 2; odd++)
 #pragma unroll
                         for (int k = 0; k < 4; k++)  // (the address field of a descriptor counts 16-byte units)
-                            umma_i8_ts(d + (dg >> 1) * kColHi, am + (dg & 1) * 32 + 8 * k, bd + (uint64_t)((dg * (N * 128) + k * 32) >> 4), idesc,
-                                       !((dg & 1) == 0 && k == 0));
-                    umma_commit(bar_df + 8 * o);
+                            umma_i8_ts(d, am + odd * 32 + 8 * k, bd + (uint64_t)((odd * (2 * N * 128) + k * 32) >> 4), idesc, odd + k > 0);
+                    umma_commit(bar_df + 16 * o + 8 * buf);
                     if (last_use) umma_commit(bar_be + 8 * st);
                 }
                 __syncwarp();
@@ -403,25 +408,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
         };
         bool ok = wait(bar_sc, 0);
         auto drain = [&](int t, int b, float sc) {
-            ok = ok && wait(bar_df + 8 * owner, (uint32_t)t & 1u);
+            const uint32_t buf = (uint32_t)t % kBufs;
+            ok = ok && wait(bar_df + 16 * owner + 8 * buf, ((uint32_t)t / kBufs) & 1u);
             __syncwarp();
             tc_fence_after_sync();
-            const uint32_t d = lane_base + (uint32_t)owner * kColsD + (uint32_t)half * NH;
+            const uint32_t d = lane_base + (uint32_t)owner * kColsD + buf * (2 * N) + (uint32_t)half * NH;
             const uint32_t xs = sbase + off_s + (uint32_t)(b * N + half * NH) * 4u;
             // eight tokens at a time, the next eight on their way meanwhile (sixteen at a time spill: 308 us for 512 tokens, 299 so)
             uint32_t lo[2][8], hi[2][8];
             tmem_ld8(d, lo[0]);
-            tmem_ld8(d + kColHi, hi[0]);
+            tmem_ld8(d + N, hi[0]);
 #pragma unroll
             for (int c = 0; c < NC; c++) {
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 if (c + 1 < NC) {
                     tmem_ld8(d + 8u * (c + 1), lo[(c + 1) & 1]);
-                    tmem_ld8(d + kColHi + 8u * (c + 1), hi[(c + 1) & 1]);
+                    tmem_ld8(d + N + 8u * (c + 1), hi[(c + 1) & 1]);
                 } else {
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_de + 8 * owner);
+                    if (lane == 0) mbar_arrive(bar_de + 16 * owner + 8 * buf);
                 }
 #pragma unroll
                 for (int c4 = 0; c4 < 2; c4++) {
