@@ -24,8 +24,8 @@
 //     pair are what the operand stages leave, hence at most 64 tokens a tile.
 //   * The two digits that meet the same weights are one B operand of 2 N columns, into both sums of a pair at once: half as many
 //     products as one digit each, and up to 32 tokens each costs the same 32 clocks (512 tokens: 298 us a layer before, 281 so).
-// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 to 16 tokens 51 us (62 and 176 as
-// pairs of tokens; 4 tokens as pairs take 41, which is where the line lies), 64 tokens 67 (702), 128 tokens 93 (1410), 512
+// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 tokens 40 us, 16 tokens 42 (62 and
+// 176 as pairs of tokens; 4 tokens as pairs take 41, which is where the line lies), 64 tokens 61 (702), 128 tokens 93 (1410), 512
 // tokens 281 (5750).  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
 // 57, 86, 129, 287 and 574.  Error against float64, 2-norm: 7.4e-8 on normal data, 8.0e-8 with x20 outliers in x, 4.5e-8 without
 // a bias on products of one sign; 1.02e-7, 2.4e-7 and 5.0e-8 as pairs of tokens; 1.01e-7, 1.0e-7 and 6.5e-8 (bias -5e-8) in the
@@ -55,8 +55,11 @@ constexpr int kGemmRowWords = 36;                 // words of a staged row: nine
 constexpr int kGemmMaxSegs = 4;
 constexpr int kGemmMaxSegments = 64;              // of four blocks in a row (the length limit leaves 36)
 constexpr uint32_t kGemmStageW = 2 * 2 * 128 * kGemmRowWords * 4;  // staged weights of the two owners
-// Shared memory of the sums of the segments done, [row tile][token][row].
-__host__ __device__ constexpr uint32_t gemm_sum_bytes(int mt, int n) { return (uint32_t)(mt * n) * 512u; }
+// Shared memory of the sums of the segments done, [row tile][token][row]; of a split tile every unit's, [unit of the CTA][token][row].
+__host__ __device__ constexpr uint32_t gemm_sum_bytes(int places, int n) { return (uint32_t)(places * n) * 512u; }
+// Pairs of units of a row of nb blocks, see the kernel.
+__host__ __device__ constexpr int gemm_pairs(int nb) { return (((nb + kGemmSegBlocks - 1) / kGemmSegBlocks + 1) / 2 + 1) / 2; }
+__host__ __device__ constexpr int gemm_places(int mt, int nb, int split) { return split > 1 ? 2 * ((gemm_pairs(nb) + split - 1) / split) : mt; }
 constexpr int kGemmFrac = 27;                     // X = round(x * 2^(kGemmFrac - e))
 // tensor-memory columns: per owner one or two pairs of sums (low | high, N columns each), then per owner two A stages (weights | times -64)
 constexpr uint32_t kColsD = 128, kColA = 256, kColsA = 64;
@@ -69,6 +72,7 @@ struct GemmArgs {
     const uint8_t *xb;        // [token tile][block][digit 0 2 1 3][n][128 B, swizzled]
     const float *x_scale;     // [token tile][block][n]: 2^(e - kGemmFrac), NaN for a block with an infinity or a NaN in it
     int nb, row_bytes, n_tok, n_stages_b;
+    int split;                // CTAs, a cluster, that share the blocks of a tile (one row tile a CTA); 1: none do
     int vec;                  // bit s: the rows of range s all start on 16-byte boundaries
     int *err_flag;
 };
@@ -178,7 +182,8 @@ __device__ __forceinline__ uint64_t int2_to_f2(uint32_t a, uint32_t b) { return 
 // its own sums and operand stages, so that the round trips of a step (operand stores, the MMAs, reading the sums back) are under
 // the other half's step: sixteen warps that share every step took 465 us for 512 tokens, two owners 340.
 // With two row tiles an owner has one of them; with one, the owners take every other unit of up to eight blocks.
-template <int MT, int NC>
+// SPLIT: a cluster of a.split CTAs shares a row tile's blocks.
+template <int MT, int NC, bool SPLIT>
 __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
     constexpr int N = 16 * NC, NH = 8 * NC;  // tokens of the tile, and of one warp
@@ -193,22 +198,33 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
     static_assert(168 + 3 * kGemmMaxSegments <= 384, "the segments' order ends before the barriers behind it");
     volatile int *gave_up = reinterpret_cast<volatile int *>(sm + 164);
     const int nst = a.n_stages_b, nb = a.nb, n_seg = (nb + kGemmSegBlocks - 1) / kGemmSegBlocks;
-    const uint32_t off_b = 1024u, off_w = off_b + (uint32_t)nst * kBlockB, off_t = off_w + kGemmStageW, off_s = off_t + gemm_sum_bytes(MT, N);
+    const uint32_t off_b = 1024u, off_w = off_b + (uint32_t)nst * kBlockB, off_t = off_w + kGemmStageW, off_s = off_t + gemm_sum_bytes(SPLIT ? gemm_places(MT, nb, a.split) : MT, N);
     // The segments form units of one or two, whose sums are kept apart; a pair of units has the same size as far as the row
     // goes.  Neither depends on the tiling.  The steps go in rounds of one per owner: round q is block q of both row tiles, or,
     // with one row tile, block q % 4 of the (q / 4)-th segment of the owner's units, which are every other one.
-    const int n_half = (n_seg + 1) / 2, n_pairs = (n_half + 1) / 2;
+    // A split tile's CTAs take every split-th pair each.
+    const int n_half = (n_seg + 1) / 2, n_pairs = (n_half + 1) / 2, split = SPLIT ? a.split : 1, rank = SPLIT ? blockIdx.x % split : 0;
+    int n_mine = n_half;  // the CTA's segments of one owner
+    if constexpr (SPLIT) {
+        n_mine = 0;
+        for (int p = rank; p < n_pairs; p += split) n_mine += (p + 1) * n_half / n_pairs - p * n_half / n_pairs;
+    }
     volatile uint8_t *seg_order = sm + 168, *unit_end = sm + 168 + 2 * kGemmMaxSegments;  // [owner][i]: i-th segment (one row tile); [segment]
     if (tid < n_half) {
         // pair p has the segments 2 f .. 2 f + 2 h - 1
         const int p = ((tid + 1) * n_pairs - 1) / n_half, f = p * n_half / n_pairs, h = (p + 1) * n_half / n_pairs - f;
+        int at = tid;
+        if constexpr (SPLIT) {
+            at -= f;
+            for (int p2 = rank; p2 < p; p2 += split) at += (p2 + 1) * n_half / n_pairs - p2 * n_half / n_pairs;
+        }
         for (int o = 0; o < 2; o++) {
             const int seg = 2 * f + o * h + tid - f;
-            seg_order[o * kGemmMaxSegments + tid] = (uint8_t)seg;
+            if (!SPLIT || p % split == rank) seg_order[o * kGemmMaxSegments + at] = (uint8_t)seg;
             unit_end[seg] = tid - f == h - 1 || seg == n_seg - 1;
         }
     }
-    const int n_rounds = MT == 2 ? nb : n_half * kGemmSegBlocks;
+    const int n_rounds = MT == 2 ? nb : n_mine * kGemmSegBlocks;
     auto segment = [&](int i, int owner) { return MT == 2 ? i : (int)seg_order[owner * kGemmMaxSegments + i]; };
     auto block_of = [&](int q, int owner) { return MT == 2 ? q : segment(q >> 2, owner) * kGemmSegBlocks + (q & 3); };
 
@@ -247,7 +263,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
     };
     auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, wait(bar, parity)); };  // one answer for the warp
 
-    const int row_tile = blockIdx.x, tok_tile = blockIdx.y;
+    const int row_tile = SPLIT ? blockIdx.x / split : blockIdx.x, tok_tile = blockIdx.y;
     int sg = 0;
 #pragma unroll
     for (int i = 1; i < kGemmMaxSegs; i++) sg += (row_tile >= a.seg_tile0[i]) ? 1 : 0;
@@ -325,7 +341,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
         const int owner = warp >> 3, quad = warp & 3, half = (warp >> 2) & 1, r = quad * 32 + lane;  // tensor-memory lane = row of the tile
         const int trow0 = row0 + (MT == 2 ? owner * 128 : 0);                                        // first row of the owner's tile
         auto seg_of = [&](int k) { return segment(k, owner); };
-        const int n_local = MT == 2 ? n_seg : (seg_of(n_half - 1) < n_seg ? n_half : n_half - 1);    // segments of the owner
+        const int n_local = MT == 2 ? n_seg : (seg_of(n_mine - 1) < n_seg ? n_mine : n_mine - 1);    // segments of the owner
         uint32_t *wst = reinterpret_cast<uint32_t *>(sm + off_w) + owner * (2 * 128 * kGemmRowWords);  // [2][128][kGemmRowWords]
         // The two warps of a quadrant stage its 32 rows, a segment of four blocks at a time.  Rows on 16-byte boundaries (their
         // length is then a multiple of eight blocks): the nine 16-byte pieces around the blocks, which start at the segment's
@@ -446,7 +462,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
         // A unit's sums join the ones before it in shared memory, in the order of the units, and leave for y after the last: one running
         // f32 sum over all blocks would round at the size of the whole result forty times.  With one row tile the owners take turns.
         float *tot = reinterpret_cast<float *>(sm + off_t) + (size_t)((MT == 2 ? owner * N : 0) + half * NH) * 128 + r;
+        // Of a split tile every unit's sums stay apart until all are there.
         auto flush = [&](int unit, bool last) {
+            if constexpr (SPLIT) {
+                float *own = reinterpret_cast<float *>(sm + off_t) + (size_t)(unit * N + half * NH) * 128 + r;
+#pragma unroll
+                for (int j = 0; j < NH / 2; j++) {
+                    const F2 v = split2(acc[j]);
+                    own[2 * j * 128] = v.x, own[(2 * j + 1) * 128] = v.y;
+                    acc[j] = 0;
+                }
+                return;
+            }
             if (MT == 1 && unit > 0) {
                 ok = ok && wait(bar_turn + 8 * (1 - owner), (uint32_t)((unit - 1) >> 1) & 1u);
                 __syncwarp();
@@ -504,56 +531,82 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
     tc_fence_before_sync();
     __syncthreads();  // (every product and every copy has come to its end)
     if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
+    if constexpr (SPLIT) {
+        // The units' sums join in the order of the units, as flush() does it, every CTA for its share of the tokens.
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");  // as in flush()
+        const int r = tid & 127, row = row0 + r, left = a.n_tok - tok_tile * N;
+        const int n_units = 2 * n_pairs;  // (none is empty where there are two pairs or more)
+        if (tid < 512)
+            for (int j = rank + split * (tid >> 7); j < N && j < left; j += split * 4) {
+                float sum = 0.f;
+                for (int u = 0; u < n_units; u++) {
+                    const int p = u >> 1;
+                    const uint32_t own = sbase + off_t + (uint32_t)(((p / split * 2 + (u & 1)) * N + j) * 128 + r) * 4u;
+                    uint32_t at;
+                    float v;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(own), "r"(p % split));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+                    sum = u ? v + sum : v;
+                }
+                if (row < seg_rows) a.y[sg][(size_t)(tok_tile * N + j) * a.y_stride[sg] + row] = sum;
+            }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // nobody leaves while its sums are read
+    }
 }
 
-template <int MT, int NC>
-bk_status launch_gemm(bk_ctx *ctx, const GemmArgs &a, dim3 grid, size_t smem) {
+template <int MT, int NC, bool SPLIT>
+bk_status launch_gemm(bk_ctx *ctx, const GemmArgs &a, dim3 grid, size_t smem) {  // grid: tiles; their CTAs beside one another
     static std::atomic<bool> opted_in[64] = {};
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64) return fail(ctx, BK_ERR_UNSUPPORTED, "pq2 matmul: device index above 63");
     if (!opted_in[dev].load()) {
-        BK_CUDA(ctx, cudaFuncSetAttribute(pq2_gemm_kernel<MT, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        BK_CUDA(ctx, cudaFuncSetAttribute(pq2_gemm_kernel<MT, NC, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         opted_in[dev].store(true);
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
+    cfg.gridDim = dim3(grid.x * a.split, grid.y);
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)a.split;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, pq2_gemm_kernel<MT, NC>, a));
+    cfg.numAttrs = SPLIT ? 2 : 1;
+    BK_CUDA(ctx, cudaLaunchKernelEx(&cfg, pq2_gemm_kernel<MT, NC, SPLIT>, a));
     ctx->launches++;
     BK_CUDA(ctx, cudaGetLastError());
     return BK_OK;
 }
 
-template <int MT>
+template <int MT, bool SPLIT = false>
 bk_status launch_gemm_nc(bk_ctx *ctx, int nc, const GemmArgs &a, dim3 grid, size_t smem) {
     switch (nc) {
-        case 1: return launch_gemm<MT, 1>(ctx, a, grid, smem);
-        case 2: return launch_gemm<MT, 2>(ctx, a, grid, smem);
-        case 3: return launch_gemm<MT, 3>(ctx, a, grid, smem);
-        default: return launch_gemm<MT, 4>(ctx, a, grid, smem);
+        case 1: return launch_gemm<MT, 1, SPLIT>(ctx, a, grid, smem);
+        case 2: return launch_gemm<MT, 2, SPLIT>(ctx, a, grid, smem);
+        case 3: return launch_gemm<MT, 3, SPLIT>(ctx, a, grid, smem);
+        default: return launch_gemm<MT, 4, SPLIT>(ctx, a, grid, smem);
     }
 }
 
 }  // namespace
 
-static size_t gemm_smem(int mt, int n, int nb, int stages) {
-    return 1024 + (size_t)stages * n * 512 + kGemmStageW + gemm_sum_bytes(mt, n) + (size_t)nb * n * sizeof(float);
+static size_t gemm_smem(int mt, int n, int nb, int stages, int split) {
+    return 1024 + (size_t)stages * n * 512 + kGemmStageW + gemm_sum_bytes(gemm_places(mt, nb, split), n) + (size_t)nb * n * sizeof(float);
 }
-static int gemm_stages(int mt, int n, int nb) {  // of B that shared memory has room for: four at most, two at least or the tile is not used
+static int gemm_stages(int mt, int n, int nb, int split = 1) {  // of B that shared memory has room for: four at most, two at least or the tile is not used
     int stages = 4;
-    while (stages > 0 && gemm_smem(mt, n, nb, stages) > 227 * 1024) stages--;
+    while (stages > 0 && gemm_smem(mt, n, nb, stages, split) > 227 * 1024) stages--;
     return stages;
 }
 
 struct GemmPlan {
     int mt = 1, nc = 1;
+    int split = 1;           // CTAs that share the blocks of a tile, with one row tile a CTA
     int64_t main_tiles = 0;  // how many of the launch's tiles of 128 mt rows; the rows of the others go to a second launch with one row tile per CTA
 };
 // Row tiles per CTA and token-tile width for a product: what has the least estimated time.  Work goes out in rounds of one CTA per SM.  A step
@@ -572,13 +625,21 @@ static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n
         const int64_t tok_tiles = (n_tok + n - 1) / n;
         const double round[3] = {0.0, (700.0 + 11.0 * n) * nb + 6000.0, (480.0 + 12.0 * n) * 2 * nb + 6000.0};
         auto rounds = [&](int64_t row_tiles) { return (double)((row_tiles * tok_tiles + n_sms - 1) / n_sms); };
-        auto take = [&](int mt, int64_t main_tiles, double cost) {
+        auto take = [&](int mt, int64_t main_tiles, double cost, int split = 1) {
             if (cost >= best) return;
             best = cost;
-            plan = GemmPlan{mt, nc, main_tiles};
+            plan = GemmPlan{mt, nc, split, main_tiles};
         };
         for (int mt = 1; mt <= 2; mt++)
             if (gemm_stages(mt, n, nb) >= 2) take(mt, tiles[mt], rounds(tiles[mt]) * round[mt]);
+        // Where the tiles leave SMs without work, clusters of up to eight share a tile's pairs of units: the output projection of up to 64
+        // tokens is 40 tiles of three pairs, 27 us on
+        // 40 SMs and 16 us on 120 for 16 tokens, 32 and 25 for 64.  A cluster costs about 3000 clocks beside its steps.
+        const int n_pairs = gemm_pairs(nb), room = (int)std::min<int64_t>(std::min(n_pairs, 8), n_sms / std::max<int64_t>(1, tiles[1] * tok_tiles));
+        for (int split = 2; split <= room; split++) {
+            const int most = (n_pairs + split - 1) / split;  // pairs of the busiest CTA
+            if (gemm_stages(1, n, nb, split) >= 2) take(1, tiles[1], (700.0 + 11.0 * n) * nb * most / n_pairs + 9000.0, split);
+        }
         const int64_t whole = tiles[2] * tok_tiles / n_sms, main_tiles = whole * n_sms / tok_tiles;
         if (whole > 0 && main_tiles < tiles[2] && gemm_stages(2, n, nb) >= 2)
             take(2, main_tiles, (double)whole * round[2] + rounds(2 * (tiles[2] - main_tiles)) * round[1]);
@@ -658,10 +719,12 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
     for (int h = 0; h < 2; h++) {
         if (tiles[h] == 0) continue;
         GemmArgs &g = part[h];
-        g.n_stages_b = gemm_stages(part_mt[h], n, a.nb);
-        const size_t smem = gemm_smem(part_mt[h], n, a.nb, g.n_stages_b);
+        g.split = h == 0 ? plan.split : 1;
+        g.n_stages_b = gemm_stages(part_mt[h], n, a.nb, g.split);
+        const size_t smem = gemm_smem(part_mt[h], n, a.nb, g.n_stages_b, g.split);
         const dim3 grid((unsigned)tiles[h], (unsigned)tok_tiles);
-        const bk_status st = part_mt[h] == 1 ? launch_gemm_nc<1>(ctx, plan.nc, g, grid, smem) : launch_gemm_nc<2>(ctx, plan.nc, g, grid, smem);
+        const bk_status st = g.split > 1          ? launch_gemm_nc<1, true>(ctx, plan.nc, g, grid, smem)
+                             : part_mt[h] == 1 ? launch_gemm_nc<1>(ctx, plan.nc, g, grid, smem) : launch_gemm_nc<2>(ctx, plan.nc, g, grid, smem);
         if (st != BK_OK) return st;
     }
     return BK_OK;

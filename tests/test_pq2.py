@@ -318,6 +318,21 @@ def test_gpu_pq2_tiling_does_not_show(bk, gpu_ctx, nb):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nb", [16, 17, 33, 36, 48, 49, 129])
+def test_gpu_pq2_clusters_on_a_tile_do_not_show(bk, gpu_ctx, nb):
+    """Few row tiles and few tokens: clusters of 2 to 8 share a tile's units (none with 16 blocks, which are one pair).  The same bits as among
+    so many tokens that nothing is shared, for tiles of 16 to 64 tokens and rows that do not fill their tile."""
+    ne0, n_rows, n_all = nb * 128 - 40, 1000, 1024
+    payload, _, _, x = synth(bk, nb, n_rows, ne0, n_all)
+    t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
+    want = t.matmul_n(x, n_all)
+    for n_tok in (5, 17, 33, 64):
+        assert np.array_equal(t.matmul_n(x[:n_tok], n_tok), want[:n_tok]), n_tok
+    assert np.array_equal(t.matmul_n(x[:9], 9, base_row=130, n_rows=150), want[:9, 130:280])
+    t.free()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n_tok", [5, 17, 200])
 def test_gpu_pq2_multi_token_block_equals_separate_calls(bk, gpu_ctx, n_tok):
     """Ranges of odd row counts, one of them off a 16-byte boundary, in one launch: bit for bit the separate calls."""
