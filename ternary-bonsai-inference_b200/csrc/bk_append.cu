@@ -4,7 +4,7 @@
 // bit for bit (src/forward.rs:259-285, src/kvquant.rs:397-412, src/rope.rs:61-69).
 //
 // A CTA stages 8 or 32 vectors of 256 floats ((K|V, kv head) of consecutive tokens):
-//   1. coalesced float4 loads into shared memory; K vectors rotate pairs (j, j + n_rot/2) with
+//   1. coalesced 16-byte copies (cp.async) into shared memory; K vectors rotate pairs (j, j + n_rot/2) with
 //      the (cos, sin) row of the token's position from the host-built rope table;
 //   2. planar rows: one warp adds the 256 squares of all vectors, a vector per lane, each lane
 //      in order (the reference's f32 sum is sequential, so each chain is; they run side by side);
@@ -127,21 +127,22 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
 }
 
 // A warp takes one K or V head of kVecs / 8 consecutive tokens, the next warp the next head (j < n_kv: K head j, else V head
-// j - n_kv), so what depends on the head is worked out once a warp.  Pass 1: the warp stages its vectors with float4 loads and
+// j - n_kv), so what depends on the head is worked out once a warp.  Pass 1: the warp stages its vectors and
 // ropes the K ones.  Pass 2: warp 0 adds the squares of all 32 vectors, one vector per lane, each lane in
 // order (the reference's f32 sum is sequential, so the chain is; 32 chains run side by side).
 // Pass 3: each warp scales, rotates, finds the nearest centroids of and stores its vectors.
 // kVecs = 32 for bulk calls of planar rows (throughput: every lane of the norm pass works), 8 for small calls
 // (latency: one vector per warp) and for f32 and f16 rows, which have no norm: many small CTAs load while others store.
-// Registers: four CTAs of 64 an SM; five of 48 spill.  Us a layer of back-to-back calls of 2048 / 4096 tokens: planar4 12.6 / 20.4 with
-// the head worked out per vector, one product at a time and five CTAs, 12.4 / 19.5 without these two, 10.7 / 18.3 with four CTAs; f32
-// 10.3 / 17.7 in CTAs of 32 vectors, 8.2 / 13.5 of 8; f16 11.1 / 17.3 and 8.5 / 14.1.  (Planar rows 16 a CTA: 12.0 / 19.1.)
+// Us a layer of back-to-back calls of 2048 / 4096 tokens: planar4 12.6 / 20.4 with the head worked out per vector, products one at a time and
+// five CTAs an SM, 10.3 / 17.8 without that and four CTAs, 9.9 / 16.8 with the rows staged by cp.async instead of through registers (five
+// CTAs 11.5 / 17.8, six spill: 14.3 / 21.7); f32 10.3 / 17.7 in CTAs of 32 vectors, 7.8 / 13.5 of 8, 7.4 / 12.1 by cp.async; f16 11.1 / 17.3, 7.9 /
+// 14.1 and 7.4 / 11.8.
 template <int BITS, int kVecs>
 __global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : 4) append_kernel(AppendArgs a) {
     extern __shared__ __align__(16) float smem[];
-    float *sbook = smem + kVecs * kVecPad;  // centroids
-    float *sgiv = sbook + 256;              // Givens table
-    float *snorm = sgiv + kHd;              // the 32 norms, and what a vector is scaled by
+    float *snorm = smem + kVecs * kVecPad;          // the norms, and what a vector is scaled by
+    [[maybe_unused]] float *sbook = snorm + 64;     // centroids (widths above 4)
+    [[maybe_unused]] float *sgiv = sbook + 256;     // Givens table
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kv = a.n_kv, per_tok = 2 * n_kv;
     constexpr int kPerWarp = kVecs / kWarps;
@@ -161,33 +162,29 @@ __global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : 4) append_kernel(App
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
-    // ---- pass 1: stage (and rope).  All of a warp's global loads (rows and rope entries) are issued before any is used, so the
+    // ---- pass 1: stage (and rope).  All of a warp's copies and loads (rows and rope entries) are issued before any is waited for, so the
     // pass costs one round trip.
-    float4 ra[kPerWarp], rb[kPerWarp];
     float2 rcs[kPerWarp];
     const int half = a.n_rot >> 1;
+    float *const mine = smem + warp * (kPerWarp * kVecPad);  // the warp's vectors
+    const uint32_t mine_at = (uint32_t)__cvta_generic_to_shared(mine) + lane * 16;
     const float4 *src4 = reinterpret_cast<const float4 *>(is_v ? a.v : a.k) + ((size_t)t0 * n_kv + kv) * (kHd / 4) + lane;
 #pragma unroll
     for (int u = 0; u < kPerWarp; u++) {
-        ra[u] = rb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
         rcs[u] = make_float2(1.f, 0.f);
         if (u < n_here) {
-            ra[u] = __ldg(src4 + (size_t)u * n_kv * (kHd / 4));
-            rb[u] = __ldg(src4 + (size_t)u * n_kv * (kHd / 4) + 32);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(mine_at + u * (kVecPad * 4) + h * 512),
+                             "l"(src4 + (size_t)u * n_kv * (kHd / 4) + h * 32)
+                             : "memory");
             if (!is_v && lane < half) {  // n_rot <= 64: one rope entry per lane
                 const int pos = a.desc ? a.desc[t0 + u].z : a.pos0 + t0 + u;
                 rcs[u] = __ldg(a.rope + (size_t)pos * half + lane);
             }
         }
     }
-    float *const mine = smem + warp * (kPerWarp * kVecPad);  // the warp's vectors
-#pragma unroll
-    for (int u = 0; u < kPerWarp; u++) {
-        if (u >= n_here) break;
-        float *sx = mine + u * kVecPad;
-        reinterpret_cast<float4 *>(sx)[lane] = ra[u];
-        reinterpret_cast<float4 *>(sx)[lane + 32] = rb[u];
-    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     if (!is_v) {
         __syncwarp();
 #pragma unroll
@@ -285,7 +282,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
     const bool bulk = n_vec > (size_t)8 * 2 * ctx->n_sms;  // more than two small CTAs per SM: go for throughput
     const int vecs = bulk && planar ? 32 : 8;
-    const size_t smem = (size_t)(vecs * kVecPad + 256 + kHd + 64) * sizeof(float);
+    const size_t smem = (size_t)(vecs * kVecPad + 64 + (a.bits > 4 ? 256 + kHd : 0)) * sizeof(float);
     const int per_warp = vecs / kWarps;
     const unsigned grid = (unsigned)(((size_t)(a.n_tokens + per_warp - 1) / per_warp * 2 * a.n_kv + kWarps - 1) / kWarps);
     cudaLaunchConfig_t cfg = {};
@@ -299,7 +296,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaError_t err = cudaSuccess;
-    // A bulk call wants four CTAs of 36 KiB or eight of 11 KiB per SM: ask for the largest shared-memory carve-out (once per
+    // A bulk call wants four CTAs of 34 KiB or eight of 9 KiB per SM: ask for the largest shared-memory carve-out (once per
     // kernel and process; a hint, so its result is not checked).
     auto launch_bulk = [&](auto *kernel) {
         static std::atomic<bool> hinted{false};
