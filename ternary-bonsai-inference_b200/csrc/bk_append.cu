@@ -3,7 +3,7 @@
 // kv_store.comp, kv_store_f16.comp and kv_store_q.comp and follows the reference CPU path
 // bit for bit (src/forward.rs:259-285, src/kvquant.rs:397-412, src/rope.rs:61-69).
 //
-// A CTA stages 8 or 32 vectors of 256 floats ((K|V, kv head) of consecutive tokens):
+// A CTA stages 8 or 16 vectors of 256 floats ((K|V, kv head) of consecutive tokens):
 //   1. coalesced 16-byte copies (cp.async) into shared memory; K vectors rotate pairs (j, j + n_rot/2) with
 //      the (cos, sin) row of the token's position from the host-built rope table;
 //   2. planar rows: one warp adds the 256 squares of all vectors, a vector per lane, each lane
@@ -128,17 +128,17 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
 
 // A warp takes one K or V head of kVecs / 8 consecutive tokens, the next warp the next head (j < n_kv: K head j, else V head
 // j - n_kv), so what depends on the head is worked out once a warp.  Pass 1: the warp stages its vectors and
-// ropes the K ones.  Pass 2: warp 0 adds the squares of all 32 vectors, one vector per lane, each lane in
-// order (the reference's f32 sum is sequential, so the chain is; 32 chains run side by side).
+// ropes the K ones.  Pass 2: warp 0 adds the squares of the CTA's vectors, one vector per lane, each lane in
+// order (the reference's f32 sum is sequential, so the chain is; they run side by side).
 // Pass 3: each warp scales, rotates, finds the nearest centroids of and stores its vectors.
-// kVecs = 32 for bulk calls of planar rows (throughput: every lane of the norm pass works), 8 for small calls
-// (latency: one vector per warp) and for f32 and f16 rows, which have no norm: many small CTAs load while others store.
-// Us a layer of back-to-back calls of 2048 / 4096 tokens: planar4 12.6 / 20.4 with the head worked out per vector, products one at a time and
-// five CTAs an SM, 10.3 / 17.8 without that and four CTAs, 9.9 / 16.8 with the rows staged by cp.async instead of through registers (five
-// CTAs 11.5 / 17.8, six spill: 14.3 / 21.7); f32 10.3 / 17.7 in CTAs of 32 vectors, 7.8 / 13.5 of 8, 7.4 / 12.1 by cp.async; f16 11.1 / 17.3, 7.9 /
-// 14.1 and 7.4 / 11.8.
+// kVecs = 16 for bulk calls of planar rows (half of the lanes of the norm pass work, and five CTAs an SM are at different passes), 8 for
+// smaller calls (latency: one vector per warp) and for f32 and f16 rows, which have no norm: many small CTAs load while others store.
+// Us a layer of back-to-back calls of 2048 / 4096 / 8192 tokens: planar4 12.6 / 20.4 / 33.9 with 32 vectors a CTA, the head worked out per
+// vector, products one at a time and five CTAs an SM, 10.3 / 17.8 / 32.2 without that and four CTAs, 9.9 / 16.8 / 29.6 with the rows staged by
+// cp.async instead of through registers, 9.8 / 15.9 / 27.4 with 16 vectors (six CTAs an SM spill); f32 10.3 / 17.7 / 29.7 in CTAs of 32
+// vectors, 7.8 / 13.5 / 25.0 of 8, 7.4 / 12.1 / 21.9 by cp.async; f16 11.1 / 17.3 / 29.5, 7.9 / 14.1 / 25.9 and 7.4 / 11.8 / 21.6.
 template <int BITS, int kVecs>
-__global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : 4) append_kernel(AppendArgs a) {
+__global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : kVecs == 16 ? 5 : 4) append_kernel(AppendArgs a) {
     extern __shared__ __align__(16) float smem[];
     float *snorm = smem + kVecs * kVecPad;          // the norms, and what a vector is scaled by
     [[maybe_unused]] float *sbook = snorm + 64;     // centroids (widths above 4)
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, BITS == 0 ? 8 : 4) append_kernel(App
         gv[0] = g0.x; gv[1] = g0.y; gv[2] = g0.z; gv[3] = g0.w;
         gv[4] = g1.x; gv[5] = g1.y; gv[6] = g1.z; gv[7] = g1.w;
     }
-    // ---- pass 2: 32 sequential sums side by side ----------------------------------------------------
+    // ---- pass 2: sequential sums side by side ----------------------------------------------------
     if (planar && warp == 0 && lane < kVecs) {  // (a place without a vector gives a number nobody reads)
         const float4 *x4 = reinterpret_cast<const float4 *>(smem + lane * kVecPad);
         float acc = 0.0f;
@@ -280,8 +280,10 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     const int threads = kThreads;
     const size_t n_vec = (size_t)a.n_tokens * 2 * a.n_kv;
     const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
-    const bool bulk = n_vec > (size_t)8 * 2 * ctx->n_sms;  // more than two small CTAs per SM: go for throughput
-    const int vecs = bulk && planar ? 32 : 8;
+    // More than ten small CTAs per SM: go for throughput.  Append and decode, us a layer, 8 / 16 vectors a CTA: planar4, 512 tokens 14.6 / 16.5,
+    // 1184 tokens 17.7 / 19.1, 1500 tokens 20.1 / 20.4, 2048 tokens 22.6 / 21.0; K only, 1500 tokens 19.4 / 18.7.  (32 vectors: 18.9 at 512.)
+    const bool bulk = n_vec > (size_t)8 * 10 * ctx->n_sms;
+    const int vecs = bulk && planar ? 16 : 8;
     const size_t smem = (size_t)(vecs * kVecPad + 64 + (a.bits > 4 ? 256 + kHd : 0)) * sizeof(float);
     const int per_warp = vecs / kWarps;
     const unsigned grid = (unsigned)(((size_t)(a.n_tokens + per_warp - 1) / per_warp * 2 * a.n_kv + kWarps - 1) / kWarps);
@@ -296,7 +298,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaError_t err = cudaSuccess;
-    // A bulk call wants four CTAs of 34 KiB or eight of 9 KiB per SM: ask for the largest shared-memory carve-out (once per
+    // A bulk call wants five CTAs of 17 KiB or eight of 9 KiB per SM: ask for the largest shared-memory carve-out (once per
     // kernel and process; a hint, so its result is not checked).
     auto launch_bulk = [&](auto *kernel) {
         static std::atomic<bool> hinted{false};
@@ -307,7 +309,7 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
         err = bulk ? launch_bulk(append_kernel<0, 8>) : cudaLaunchKernelEx(&cfg, append_kernel<0, 8>, a);
     } else {
         const bool ok = dispatch_bits(a.bits, [&]<int B>() {
-            err = bulk ? launch_bulk(append_kernel<B, 32>) : cudaLaunchKernelEx(&cfg, append_kernel<B, 8>, a);
+            err = bulk ? launch_bulk(append_kernel<B, 16>) : cudaLaunchKernelEx(&cfg, append_kernel<B, 8>, a);
         });
         if (!ok) return fail(ctx, BK_ERR_INVALID, "append: bits must be 1..8");
     }

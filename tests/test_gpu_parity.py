@@ -169,10 +169,11 @@ def test_append_bytes_bit_exact(bk, gpu_ctx, oracle, tag, mode, bits, vq):
 @pytest.mark.parametrize("n_head,n_kv", [(6, 1), (6, 3), (8, 8)])
 @pytest.mark.parametrize("tag,mode,bits,vq", [MODES[0], MODES[1], MODES[2], MODES[4], MODES[5]])
 def test_bulk_append_of_ragged_token_counts(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv):
-    """Warps with one to four tokens of a head, warps without any, numbers of heads that are no power of two: rows bit-exact."""
+    """Calls on both sides of the line between small and bulk calls; warps with one or two tokens of a head, warps without any, numbers of heads
+    that are no power of two: rows bit-exact."""
     rng = np.random.default_rng(n_kv)
-    n0 = 2400 // (2 * n_kv)  # from here on a call is a bulk call (two small CTAs an SM are 2368 vectors)
-    for n in (n0 + 1, n0 + 2, n0 + 3):
+    n0 = 8 * 10 * 148 // (2 * n_kv)  # ten small CTAs an SM
+    for n in (n0 - 1, n0 + 1, n0 + 2):
         k, v = rng.standard_normal((2, n, n_kv, HD)).astype(np.float32)
         cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n, n_head=n_head, n_kv=n_kv)
         cache.append(0, k, v)
