@@ -925,19 +925,27 @@ bk_status launch_decode_group(bk_ctx *ctx, const DecodeArgs &a, const DecodeEntr
         L = std::max<int64_t>(v_planar ? 96 : gran, (L + gran - 1) / gran * gran);
         if (v_f32 && L > 96) L = (L + 95) / 96 * 96;
         while (items_for(L) > ctx->n_sms && L < max_np) L += gran;
-    } else if (a.k_kind == ROW_PLANAR && (int64_t)nb * n_kv * 2 <= ctx->n_sms) {
-        // Generic kernel on planar rows, one CTA of all registers per SM: one wave, as above.  With more pairs about two such CTAs'
-        // time for an SM: 8 bit, 64 sequences of 500 to 3000 rows 164 us a layer (188 with four), 24 such sequences 93 (99).
-        // Up to three rounds of the CTA's warps go in one chunk: 8 bit, 60 rows 19.1 us a layer in two chunks, 15.5 in
-        // one, 100 rows 19.1 and 16.9, 120 rows 19.1 and 17.5; beyond, a chunk is 64 rows or more.
-        const int64_t round = a.v_kind == ROW_PLANAR && a.n_head / n_kv <= 6 ? 48 : 32;
-        L = (total * n_kv + ctx->n_sms - 1) / ctx->n_sms;
-        L = max_np <= 3 * round ? 3 * round : std::max<int64_t>(gran, (L + 15) / 16 * 16);
-        while (items_for(L) > ctx->n_sms && L < max_np) L += 16;
     } else {
-        const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms * (a.k_kind == ROW_PLANAR ? 2 : 4) / n_kv);  // about two or four CTAs per SM
-        L = (total + target_items - 1) / target_items;
-        L = std::max<int64_t>(gran, (L + gran - 1) / gran * gran);
+        // Generic kernels.  A sequence of one chunk needs no merging through global memory, which costs more than two more rounds of a CTA's
+        // warps (48 planar rows, 32 beside f32 or for eight heads; or 128 rows of f32 and f16, a row per warp and step): 8 bit, 60 rows 19.1 us
+        // a layer in two chunks, 15.5 in one, 100 rows 19.1 and 16.9, 120 rows 19.1 and 17.5; f32, 60 rows 20.6 and 17.5, 100 rows 20.7 and 19.9; f16, 40
+        // sequences of 40 to 120 rows 56.8 and 39.1.
+        const bool planar = a.k_kind == ROW_PLANAR;
+        const int64_t whole = !planar ? 128 : a.v_kind == ROW_PLANAR && a.n_head / n_kv <= 6 ? 144 : 96;
+        if (max_np <= whole) {
+            L = whole;
+        } else if (planar && (int64_t)nb * n_kv * 2 <= ctx->n_sms) {
+            // planar rows, one CTA of all registers per SM: one wave, as above
+            L = (total * n_kv + ctx->n_sms - 1) / ctx->n_sms;
+            L = std::max<int64_t>(gran, (L + 15) / 16 * 16);
+            while (items_for(L) > ctx->n_sms && L < max_np) L += 16;
+        } else {
+            // About two such CTAs' time for an SM (8 bit, 64 sequences of 500 to 3000 rows 164 us a layer, 188 with four; 24 such sequences 93
+            // and 99), or four of the smaller ones for f32 and f16.
+            const int64_t target_items = std::max<int64_t>(1, (int64_t)ctx->n_sms * (planar ? 2 : 4) / n_kv);
+            L = (total + target_items - 1) / target_items;
+            L = std::max<int64_t>(gran, (L + gran - 1) / gran * gran);
+        }
     }
     while (items_for(L) > max_items) L *= 2;
     m.chunk_len = (int)L;

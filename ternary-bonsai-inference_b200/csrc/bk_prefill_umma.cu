@@ -52,8 +52,8 @@ static_assert(kRunFloats == (size_t)kRows * kHd, "a place per row and coordinate
 
 constexpr uint32_t kQSlab = kRows * 128, kQTile = 4 * kQSlab;  // 16 KiB per 64-coordinate slab, 64 KiB per tile
 constexpr uint32_t kKVSlab = kTK * 128, kKVTile = 4 * kKVSlab;  // 4 KiB, 16 KiB
-// Operand slots.  Four: K(t) then takes the place of K(t - 2), whose S products were issued when the softmax had read tile
-// t - 4, so the norms of four tiles can be kept.
+// Operand slots.  Five: K(t) then takes the place of V(t - 4), whose products came after the softmax of tile t - 4, so the norms of
+// four tiles are kept.
 constexpr int kSlots = 5, kNormTiles = 4;
 constexpr uint32_t kSlotBytes = 2 * kKVTile;  // hi and lo tile
 // offsets from the 1024-byte aligned base
