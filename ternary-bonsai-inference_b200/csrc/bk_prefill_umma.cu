@@ -933,7 +933,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) prefill_umma_merge_kernel(co
 #pragma unroll
     for (int h = 0; h < kPerLane; h++) {
         f[h] = f[h] > -CUDART_INF_F ? exp2f(f[h] - M) : 0.f;
-        if (f[h] > 0.f) Ls = fmaf(l[h], f[h], Ls);
+        if (l[h] != l[h]) f[h] = CUDART_NAN_F;  // NaN among the row's scores, whatever became of its reference: the row is NaN
+        if (f[h] != 0.f) Ls = fmaf(l[h], f[h], Ls);
     }
     for (int o = 16; o > 0; o >>= 1) Ls += __shfl_xor_sync(0xffffffffu, Ls, o);
     float4 acc[2] = {};  // coordinates 4 lane .. + 3 of each half

@@ -1500,6 +1500,33 @@ def test_prefill_in_pieces(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_k
     cache.close()
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [MODES[0], MODES[1], MODES[2], MODES[3], MODES[4]])
+@pytest.mark.parametrize("n", [90, 400, 1500])
+def test_prefill_of_values_that_are_not_numbers(bk, gpu_ctx, oracle, tag, mode, bits, vq, n):
+    """A NaN and an infinity in a query row, and a kv head whose K rows are all NaN, in prompts of whole and of cut items: what is NaN for the
+    oracle is NaN here, and nothing else is touched."""
+    rng = np.random.default_rng(n)
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    a, b = n // 2, n - 7
+    q[a, 1, 17], q[b, 7, 100] = np.nan, np.inf
+    k[:, 2] = np.nan
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    ref = oracle.cache(mode, bits, vq)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got = cache.prefill_attend(0, q, 0)
+    cache.close()
+    nan = np.zeros((n, NH), bool)
+    nan[:, 12:18] = nan[a, 1] = nan[b, 7] = True
+    assert np.array_equal(np.isnan(got), np.repeat(nan[..., None], HD, 2))
+    for i in (0, a, b, n - 1):
+        want = ref.attend(0, q[i], i, i + 1, threads=8).reshape(NH, HD)
+        assert np.array_equal(np.isnan(want).all(1), nan[i]) and np.array_equal(np.isnan(want).any(1), nan[i])
+        assert_close(got[i][~nan[i]], want[~nan[i]], f"{tag} token {i}")
+
+
 def test_prefill_of_more_items_than_are_cut(bk, gpu_ctx, oracle):
     """A prompt block of so many items that they go out whole: 153 blocks of 21 tokens."""
     rng = np.random.default_rng(3)
