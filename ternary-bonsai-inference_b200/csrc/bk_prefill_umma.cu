@@ -47,6 +47,10 @@ constexpr int kTK = 32;     // positions per tile
 // Weights are 2^(s - ref) ||v||, with the reference kBelow under a row's maximum of s + log2 ||v|| when it moves, which it does when the maximum
 // has run kLazy further ahead: they stay below 2^14.
 constexpr float kBelow = 6.0f, kLazy = 8.0f;
+// A score is the sum of two terms that both meet ||k||, which is infinite for a K row of 1.8e19 and more: infinities of different signs would make
+// a NaN of minus infinity.  Such a norm counts as kMaxFloat, which leaves the score's sign as it is and its size above kInfinite, and what is above that
+// is infinite: scores of finite norms and of q's f16 parts end below 1e27.
+constexpr float kMaxFloat = 3.4028235e38f, kInfinite = 1e30f;
 constexpr size_t kRunFloats = kPrefillRunFloats;  // a CTA's sums of the runs done, [4 coordinates][row][4]
 static_assert(kRunFloats == (size_t)kRows * kHd, "a place per row and coordinate");
 
@@ -649,10 +653,10 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
                     widen(pk);
                     dequant_store(pk, table, dst, dst, kLoTiles ? 64 : 32, my_row, my_row + 32, 4 * my_c, rot);
                     if (pt < 2 * kTK) {
-                        if (pt < kTK) ss.kn[tile % kNormTiles][pt] = pn;
+                        if (pt < kTK) ss.kn[tile % kNormTiles][pt] = pn > kMaxFloat ? kMaxFloat : pn;  // (NaN stays)
                         else if constexpr (!VF32) {
                             pn = fmaxf(pn, 1e-30f);
-                            ss.vn[tile % kNormTiles][pt - kTK] = fminf(pn, 3.4028235e38f);  // (finite: it meets weights of 0)
+                            ss.vn[tile % kNormTiles][pt - kTK] = fminf(pn, kMaxFloat);  // (finite: it meets weights of 0)
                             ss.lv[tile % kNormTiles][pt - kTK] = fast_log2(pn);
                         }
                         __syncwarp();
@@ -781,7 +785,7 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
             // lazy reference: move it only when this row's maximum ran ahead by more than kLazy
             const bool move = mx > -CUDART_INF_F && (ref == -CUDART_INF_F || mx > kBelow + kLazy);
             if (__any_sync(0xffffffffu, move)) {  // tensor-memory traffic is warp-collective
-                const float new_ref = move ? base_ref + (mx - kBelow) : ref, by = move ? (mx < CUDART_INF_F ? new_ref - base_ref : CUDART_NAN_F) : 0.f;
+                const float new_ref = move ? base_ref + (mx - kBelow) : ref, by = move ? (mx < kInfinite ? new_ref - base_ref : CUDART_NAN_F) : 0.f;
                 const float f = move ? (ref > -CUDART_INF_F ? fast_exp2(-by) : 0.f) : 1.f;
                 const uint64_t nby = pair(__float_as_uint(-by), __float_as_uint(-by));
 #pragma unroll

@@ -1527,6 +1527,32 @@ def test_prefill_of_values_that_are_not_numbers(bk, gpu_ctx, oracle, tag, mode, 
         assert_close(got[i][~nan[i]], want[~nan[i]], f"{tag} token {i}")
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [MODES[2], MODES[3], ("planar2", MODE_PLANAR, 2, True), MODES[4], ("planar3k", MODE_PLANAR, 3, False)])
+def test_prefill_of_an_infinite_row(bk, gpu_ctx, oracle, tag, mode, bits, vq):
+    """K rows with an infinite norm: the queries that score minus infinity there do without them, the others are NaN."""
+    rng = np.random.default_rng(bits)
+    n, at = 200, (90, 131)
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    k[at[0], 1] *= np.float32(1e30)
+    k[at[1], 3, 9] = -np.inf
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    ref = oracle.cache(mode, bits, vq)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got = cache.prefill_attend(0, q, 0)
+    cache.close()
+    seen = 0
+    for i in (0, at[0] - 1, *range(at[0], n, 6)):
+        want = ref.attend(0, q[i], i, i + 1, threads=8).reshape(NH, HD)
+        nan = np.isnan(want).any(1)
+        seen += nan.sum()
+        assert np.array_equal(np.isnan(got[i]).any(1), nan), i
+        assert_close(got[i][~nan], want[~nan], f"{tag} token {i}")
+    assert 40 < seen < 160  # (20 tokens, 12 heads, about half)
+
+
 def test_prefill_of_more_items_than_are_cut(bk, gpu_ctx, oracle):
     """A prompt block of so many items that they go out whole: 153 blocks of 21 tokens."""
     rng = np.random.default_rng(3)
