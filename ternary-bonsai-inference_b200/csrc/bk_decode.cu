@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(kThreads) decode_kernel(DecodeArgs a, DecodeMe
         float M = -CUDART_INF_F;
         for (int w = 0; w < kWarps; w++) M = fmaxf(M, s_m[w][tid]);
         float Lsum = 0.f;
-        for (int w = 0; w < kWarps; w++)
-            if (s_m[w][tid] > -CUDART_INF_F) Lsum += s_l[w][tid] * exp2f(s_m[w][tid] - M);
+        for (int w = 0; w < kWarps; w++)  // (without a maximum: no row, or none but NaN, which the sum tells)
+            Lsum += s_l[w][tid] * (s_m[w][tid] > -CUDART_INF_F ? exp2f(s_m[w][tid] - M) : 0.f);
         s_M[tid] = M;
         s_L[tid] = Lsum;
     }

@@ -466,7 +466,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
                     po[kHd + 1] = Ls;
                 }
             } else {
-                o = Ls > 0.f ? o / Ls : 0.f;
+                o = Ls == 0.f ? 0.f : o / Ls;  // (a sum that is NaN makes a result that is)
                 // src/forward.rs:379-382 with src/kernels.rs:162: out *= 1 / (1 + exp(-gate))
                 if (gate) o *= 1.0f / (1.0f + expf(-(i == tid ? gate0 : __ldg(gate + (size_t)r_o * a.gate_stride + d_o))));
                 a.out[((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kHd + d0 + d_o] = o;
@@ -778,7 +778,7 @@ __device__ __forceinline__ void finish_item(const DecodeArgs &a, int slot, int s
 #pragma unroll
             for (int r = 0; r < NREP; r++) {
                 const float Ls = s_L[r];
-                float o = Ls > 0.f ? s_acc[r * kHd + tid] / Ls : 0.f;
+                float o = Ls == 0.f ? 0.f : s_acc[r * kHd + tid] / Ls;  // (a sum that is NaN makes a result that is)
                 // src/forward.rs:379-382 with src/kernels.rs:162: out *= 1 / (1 + exp(-gate))
                 if (gate) o *= 1.0f / (1.0f + expf(-gv[r]));
                 out[r * kHd + tid] = o;

@@ -534,6 +534,34 @@ def test_generic_decode_keeps_infinities_where_they_are(bk, gpu_ctx, oracle):
     cache.close()
 
 
+@pytest.mark.parametrize("tag,mode,bits,vq", [("planar8", MODE_PLANAR, 8, True), ("planar5", MODE_PLANAR, 5, True), ("planar8k", MODE_PLANAR, 8, False),
+                                              MODES[2], MODES[0], MODES[1]])
+@pytest.mark.parametrize("n", [1, 3, 7, 60, 100, 300])
+def test_generic_decode_of_values_that_are_not_numbers(bk, gpu_ctx, oracle, tag, mode, bits, vq, n):
+    """A query head that is NaN, a K row that holds a NaN, one of infinite norm: what is NaN for the oracle is NaN here, whatever group of rows
+    or chunk it falls into, and the other heads are not touched."""
+    if n > 127 and bits < 5:
+        n = 127  # (longer ones go to other kernels)
+    rng = np.random.default_rng(n)
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((NH, HD)).astype(np.float32)
+    q[2, 30] = np.nan
+    k[n // 2, 1, 17] = np.nan
+    if bits:  # (f32 and f16 rows would hold values of which products overflow before they are added up)
+        k[n - 1, 3] *= np.float32(1e30)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    ref = oracle.cache(mode, bits, vq)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got, want = cache.attend(0, q)[0].reshape(NH, HD), ref.attend(0, q, n - 1, n).reshape(NH, HD)
+    cache.close()
+    nan = np.isnan(want).any(1)
+    assert nan[2] and nan[6:12].all() and not nan[12:18].any()
+    assert np.array_equal(np.isnan(got).any(1), nan)
+    assert_close(got[~nan], want[~nan], tag)
+
+
 def test_decode_long_context_split_k(bk, gpu_ctx, oracle):
     """Enough positions for many chunks per kv head (the partials + last-arriver combine)."""
     for tag, mode, bits, vq in [MODES[2], MODES[1]]:
