@@ -47,10 +47,10 @@ template <int KIND>
 __device__ __forceinline__ RawRow<KIND> load_row(const uint8_t *row, int lane) {
     RawRow<KIND> x;
     if constexpr (KIND == ROW_F32) {
-        x.a = __ldg(reinterpret_cast<const float4 *>(row) + lane);
-        x.b = __ldg(reinterpret_cast<const float4 *>(row) + 32 + lane);
+        x.a = reinterpret_cast<const float4 *>(row)[lane];
+        x.b = reinterpret_cast<const float4 *>(row)[32 + lane];
     } else {
-        x.a = __ldg(reinterpret_cast<const uint4 *>(row) + lane);
+        x.a = reinterpret_cast<const uint4 *>(row)[lane];
     }
     return x;
 }

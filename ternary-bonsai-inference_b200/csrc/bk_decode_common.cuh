@@ -148,17 +148,17 @@ struct QHead {
     __device__ __forceinline__ void load(const float *row, int lane, int half) {
         const int d = 8 * lane;
         if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
-            const float4 u = __ldg(reinterpret_cast<const float4 *>(row + d)), v = __ldg(reinterpret_cast<const float4 *>(row + d) + 1);
+            const float4 u = reinterpret_cast<const float4 *>(row + d)[0], v = reinterpret_cast<const float4 *>(row + d)[1];
             x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
             x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
         } else {
 #pragma unroll
-            for (int e = 0; e < 8; e++) x[e] = __ldg(row + d + e);
+            for (int e = 0; e < 8; e++) x[e] = row[d + e];
         }
 #pragma unroll
         for (int e = 0; e < 8; e++) {
             y[e] = 0.f;
-            if (d + e < 2 * half) y[e] = __ldg(row + (d + e < half ? d + e + half : d + e - half));
+            if (d + e < 2 * half) y[e] = row[d + e < half ? d + e + half : d + e - half];
         }
     }
     __device__ __forceinline__ void finish(int lane, int half, const float *norm_w /* shared memory, or null */, float eps, const float2 *rope_row) {
@@ -349,7 +349,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
     // the gate of this thread's first output travels with the first loads
     const float *gate = (a.gate && !a.partial) ? a.gate + ((size_t)slot * a.n_head + (size_t)kv * NREP) * a.gate_stride + d0 : nullptr;
     float gate0 = 0.f;
-    if (gate && tid < n_out) gate0 = __ldg(gate + (size_t)(tid >> (lg + 2)) * a.gate_stride + (tid & (D - 1)));
+    if (gate && tid < n_out) gate0 = gate[(size_t)(tid >> (lg + 2)) * a.gate_stride + (tid & (D - 1))];
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     float M = -CUDART_INF_F, L = 0.f;
     if (grp < n_grp) {
@@ -468,7 +468,7 @@ __device__ __forceinline__ void combine_slice(const DecodeArgs &a, int slot, int
             } else {
                 o = Ls == 0.f ? 0.f : o / Ls;  // (a sum that is NaN makes a result that is)
                 // src/forward.rs:379-382 with src/kernels.rs:162: out *= 1 / (1 + exp(-gate))
-                if (gate) o *= 1.0f / (1.0f + expf(-(i == tid ? gate0 : __ldg(gate + (size_t)r_o * a.gate_stride + d_o))));
+                if (gate) o *= 1.0f / (1.0f + expf(-(i == tid ? gate0 : gate[(size_t)r_o * a.gate_stride + d_o])));
                 a.out[((size_t)slot * a.n_head + (size_t)kv * NREP + r_o) * kHd + d0 + d_o] = o;
             }
         }
@@ -520,7 +520,7 @@ __device__ __forceinline__ void finish_item(const DecodeArgs &a, int slot, int s
     float gv[NREP];
     auto load_gate = [&]() {
 #pragma unroll
-        for (int r = 0; r < NREP; r++) gv[r] = gate ? __ldg(gate + (size_t)r * a.gate_stride) : 0.f;
+        for (int r = 0; r < NREP; r++) gv[r] = gate ? gate[(size_t)r * a.gate_stride] : 0.f;
     };
     if (n_chunks <= 1) load_gate();
     if (n_chunks > 1) {

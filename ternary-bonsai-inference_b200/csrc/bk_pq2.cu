@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(kPqGroupThreads * kPqMaxGroups) pq2_matvec_ker
             }
             phase ^= 1u << sl;
         } else {  // a ragged last tile or an unaligned payload: ordinary 2-byte loads
-            const uint16_t *src = reinterpret_cast<const uint16_t *>(a.rows[sg] + (size_t)lt * tile_bytes);
+            const uint16_t *weights = reinterpret_cast<const uint16_t *>(a.rows[sg] + (size_t)lt * tile_bytes);
             uint16_t *dst = reinterpret_cast<uint16_t *>(sm + off_st + (size_t)st * a.stage_stride);
             const int n2 = rows_here * a.row_bytes / 2;
-            for (int i = tid; i < n2; i += kPqGroupThreads) dst[i] = __ldg(src + i);
+            for (int i = tid; i < n2; i += kPqGroupThreads) dst[i] = __ldg(weights + i);
             group_sync();
         }
 

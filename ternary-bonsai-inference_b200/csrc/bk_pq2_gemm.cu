@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) pq2_split_x_kernel(const float *x, int ne
         const float4 *p = reinterpret_cast<const float4 *>(x + (size_t)tok * ne0 + j0);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const float4 f = __ldg(p + k);
+            const float4 f = p[k];
             v[4 * k] = f.x, v[4 * k + 1] = f.y, v[4 * k + 2] = f.z, v[4 * k + 3] = f.w;
         }
     } else {

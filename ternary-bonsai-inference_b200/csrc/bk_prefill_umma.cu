@@ -340,20 +340,20 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float4 *src = reinterpret_cast<const float4 *>(rows + row_of(tile, (pt >> 5) * 4 + j) * 1024) + 2 * lane;
-            dst[2 * j] = __ldg(src);
-            dst[2 * j + 1] = __ldg(src + 1);
+            dst[2 * j] = src[0];
+            dst[2 * j + 1] = src[1];
         }
     };
     auto fetch_packed = [&](uint32_t (&w)[4], const uint8_t *rows, int tile) {
         const uint8_t *p = rows + row_of(tile, my_row) * kRowBytes;
         if constexpr (BITS == 4) {
-            const uint4 x = __ldg(reinterpret_cast<const uint4 *>(p) + my_c);
+            const uint4 x = reinterpret_cast<const uint4 *>(p)[my_c];
             w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
         } else if constexpr (BITS == 3) {
             const uint32_t *p3 = reinterpret_cast<const uint32_t *>(p) + 3 * my_c;
-            w[0] = __ldg(p3), w[1] = __ldg(p3 + 1), w[2] = __ldg(p3 + 2), w[3] = 0;
+            w[0] = p3[0], w[1] = p3[1], w[2] = p3[2], w[3] = 0;
         } else {  // 2 bit: 32 coordinates are 8 bytes
-            const uint2 x = __ldg(reinterpret_cast<const uint2 *>(p) + my_c);
+            const uint2 x = reinterpret_cast<const uint2 *>(p)[my_c];
             w[0] = x.x, w[1] = x.y, w[2] = w[3] = 0;
         }
     };
@@ -362,7 +362,7 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
             fetch_f32(fk, a.k_rows, tile);
         } else if constexpr (!kF16) {
             fetch_packed(pk, a.k_rows, tile);
-            if (pt < (VF32 ? kTK : 2 * kTK)) pn = __ldg((pt < kTK ? a.k_norms : a.v_norms) + row_of(tile, pt & (kTK - 1)));
+            if (pt < (VF32 ? kTK : 2 * kTK)) pn = (pt < kTK ? a.k_norms : a.v_norms)[row_of(tile, pt & (kTK - 1))];
         }
     };
     auto fetch_v = [&](int tile) {
@@ -549,7 +549,7 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
                     } else {
                         for (int r = 0; r < kTK; r++) {
                             uint4 x = make_uint4(0, 0, 0, 0);
-                            if (r < valid) x = __ldg(reinterpret_cast<const uint4 *>(rows + row_of(tile, r) * 512) + lane);
+                            if (r < valid) x = reinterpret_cast<const uint4 *>(rows + row_of(tile, r) * 512)[lane];
                             *reinterpret_cast<uint4 *>(sm + oSlots + slot * kSlotBytes + sw_off(kTK, r, lane)) = x;
                         }
                         fence_smem_to_async_proxy();

@@ -191,6 +191,21 @@ def test_prefill_plan_covers_every_tile_once(bk, n_head, n_kv):
     assert lib.bk_prefill_plan(148, 0, 4, 24, 5, 0, None, C.addressof(n)) == bk._abi.BK_ERR_INVALID
 
 
+def test_read_only_loads_are_of_constants():
+    """A kernel that is launched under the end of another one (it has a griddepcontrol.wait) may use the read-only path, which takes it for granted
+    that nobody writes the data while the kernel lives, only for tables and weights: its other inputs may still be on their way when it starts."""
+    csrc = os.path.join(ROOT, "ternary-bonsai-inference_b200", "csrc")
+    sources = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.endswith((".cu", ".cuh"))}
+    early = [f for f in sources if "griddepcontrol.wait" in sources[f] or f == "bk_decode_common.cuh"]
+    assert {"bk_append.cu", "bk_decode.cu", "bk_prefill_umma.cu"} <= set(early)
+    found = [(f, line.strip()) for f in early for line in sources[f].splitlines() if re.search(r"__ldg\(|global\.nc|__restrict__", line)]
+    assert len(found) > 3
+    for f, line in found:
+        for arg in re.split(r"__ldg\(", line)[1:]:
+            assert re.match(r"(reinterpret_cast<[^>]*>\()?(a\.rope|a\.givens|a\.book|a\.k_norm_w|rope_row|weights)\b", arg), (f, line)
+        assert "global.nc" not in line and "__restrict__" not in line, (f, line)
+
+
 def test_default_config_is_qwen35(bk):
     cfg = bk._abi.CacheConfig()
     bk._abi.load().bk_default_config(C.byref(cfg))
