@@ -16,7 +16,6 @@
 #include <math_constants.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "bk_decode_common.cuh"
 
@@ -604,13 +603,10 @@ bk_status launch_pdl(bk_ctx *ctx, Kernel *kernel, int threads, size_t smem, cons
 template <int VK, int BITS, int NREP>
 bk_status launch_planar(bk_ctx *ctx, const DecodeArgs &a, const DecodeMeta &m) {
     constexpr size_t smem = kPlanarSmem<VK, BITS, NREP>;
-    static std::atomic<bool> opted_in[64] = {};  // per device
-    const int dev = ctx->device;
-    if (dev < 0 || dev >= 64) return fail(ctx, BK_ERR_UNSUPPORTED, "decode: device index above 63");
-    if (!opted_in[dev].load()) {
-        BK_CUDA(ctx, cudaFuncSetAttribute(decode_planar_kernel<VK, BITS, NREP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        opted_in[dev].store(true);
-    }
+    static PerDevice opted_in;
+    BK_CUDA(ctx, opted_in.once(ctx->device, [] {
+        return cudaFuncSetAttribute(decode_planar_kernel<VK, BITS, NREP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanarSmem<VK, BITS, NREP>);
+    }));
     return launch_pdl(ctx, decode_planar_kernel<VK, BITS, NREP>, kPlanarWarps<VK, NREP> * 32, smem, a, m);
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <memory>
 #include <string>
 #include <vector>
@@ -70,6 +71,22 @@ constexpr size_t kPrefillRunFloats = 128 * 256;
 // place in the scratch, 128 query rows of (O, m, l).
 constexpr int kPrefillStretches = 160, kPrefillParts = 2 * kPrefillStretches, kPrefillPieces = 768;
 constexpr size_t kPrefillPartFloats = 128 * (256 + 2);
+
+// What a kernel needs once per device (an attribute of it): `set_up` runs where it has not succeeded yet.  Racing first calls run it twice, and
+// devices beyond the table run it with every launch.
+class PerDevice {
+    std::atomic<bool> done_[64] = {};
+
+  public:
+    template <typename F>
+    cudaError_t once(int device, F &&set_up) {
+        const bool known = device >= 0 && device < 64;
+        if (known && done_[device].load()) return cudaSuccess;
+        const cudaError_t e = set_up();
+        if (known && e == cudaSuccess) done_[device].store(true);
+        return e;
+    }
+};
 
 struct HostPipe;  // pinned slots and copy threads of bulk host transfers (bk_hostpipe.cpp)
 void host_pipe_destroy(HostPipe *p);

@@ -165,4 +165,12 @@ __attribute__((visibility("default"))) void fake_cache_free(bk_cache *c) {
     delete c;
 }
 __attribute__((visibility("default"))) int fake_n_pos(bk_cache *c, int l, int s) { return c->n_pos[c->slab(l, s)]; }
+// how often launches on these devices set a kernel up, when set-up number `fail_at` fails
+__attribute__((visibility("default"))) int fake_set_ups(const int *devices, int n, int fail_at, int *failed) {
+    bk::PerDevice per_device;
+    int runs = 0;
+    for (int i = 0; i < n; i++)
+        failed[i] = per_device.once(devices[i], [&] { return runs++ == fail_at ? cudaErrorInvalidValue : cudaSuccess; }) != cudaSuccess;
+    return runs;
+}
 }

@@ -150,3 +150,11 @@ def test_snapshot_without_memory_for_its_lists(fake, ctx):
             assert st == 0 and failed > 0
     for c in (a, b):
         fake.fake_cache_free(c)
+
+
+def test_kernels_are_set_up_once_per_device(fake):
+    """A kernel's attribute is set once on a device, again after a failure, and with every launch on devices beyond the table, which are not refused."""
+    devices = [0, 0, 63, 63, 0, 64, 64, 200]
+    failed = (C.c_int * len(devices))()
+    assert fake.fake_set_ups((C.c_int * len(devices))(*devices), len(devices), -1, failed) == 5 and not any(failed)
+    assert fake.fake_set_ups((C.c_int * len(devices))(*devices), len(devices), 0, failed) == 6 and list(failed) == [1] + [0] * 7
