@@ -372,14 +372,6 @@ BK_API bk_status bk_attn_oneshot_host(bk_ctx *ctx, const float *q_host, const fl
                                       const float *v_host, int32_t n_pos, int32_t nheads,
                                       int32_t kvheads, int32_t hd, float *out_host);
 
-/* No counterpart in the reference: how a prompt block of n_tokens at position pos0 would be spread over n_sms processors by bk_prefill_attn, for
- * checking it without a GPU.  A piece is four words of pieces_host: item = (blocks - 1 - block) * n_kv + kv head, with blocks of
- * 128 / (n_head / n_kv) tokens; first tile and end, in tiles of 32 rows; its place in the scratch, -1 for a whole item.  *n_pieces is how many
- * there are, in the order in which they are handed out; 0: every item whole, in the order of the items.  At most `capacity` are written.
- * Host only. */
-BK_API bk_status bk_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces_host,
-                                 int32_t *n_pieces);
-
 /* ---- kvquant.rs entry points (host in/out, computed on the GPU) ----------- */
 
 /* PlanarQuant::packed_len (src/kvquant.rs:348-350); 0 on bad arguments. */

@@ -81,7 +81,6 @@ SIGNATURES = {
     "bk_pq2_matvec_multi": (C.c_int, [_vp, _i32, _vp, _i64, _vp, _i32]),
     "bk_pq2_matvec_host": (C.c_int, [_vp, _vp, _sz, _i64, _i64, _i64, _vp, _i32, _vp]),
     "bk_attn_oneshot_host": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
-    "bk_prefill_plan": (C.c_int, [_i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp]),
     "bk_kvq_packed_len": (_sz, [_i32, _i32]),
     "bk_kvq_codebook": (C.c_int, [_i32, _i32, _vp]),
     "bk_kvq_givens": (C.c_int, [_i32, _vp]),

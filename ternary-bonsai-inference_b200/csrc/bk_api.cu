@@ -1516,14 +1516,6 @@ bk_status bk_kvq_threshold_cells(int32_t bits, uint32_t *out) {
     return BK_OK;
 }
 
-bk_status bk_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces, int32_t *n_pieces) {
-    if (!n_pieces || (capacity > 0 && !pieces) || n_sms < 1 || pos0 < 0 || n_tokens < 1 || n_kv < 1 || n_head % n_kv != 0 || n_head / n_kv < 1 ||
-        n_head / n_kv > 128)
-        return fail(nullptr, BK_ERR_INVALID, "bk_prefill_plan: bad argument");
-    *n_pieces = prefill_plan(n_sms, pos0, n_tokens, n_head, n_kv, capacity, pieces);
-    return BK_OK;
-}
-
 bk_status bk_kvq_lane_cells(int32_t bits, uint32_t *out) {
     if (!out || bits < 1 || bits > 4) return fail(nullptr, BK_ERR_INVALID, "bk_kvq_lane_cells: bits must be 1..4");
     float book[256];

@@ -352,7 +352,6 @@ bool prefill_mma_supported(const DecodeArgs &a);
 bk_status launch_prefill_mma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha);
 // The same on tcgen05 tensor cores with the accumulators in tensor memory (bk_prefill_umma.cu).
 bool prefill_umma_supported(const DecodeArgs &a);  // planar4 / planar3 / f16 caches
-int prefill_plan(int n_sms, int pos0, int n_tokens, int n_head, int n_kv, int capacity, int32_t *pieces);  // see bk_prefill_plan
 bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha);
 bk_status launch_lse_merge(bk_ctx *ctx, int n_parts, int n_rows, int hd, const float *parts, float *out);
 
@@ -370,3 +369,12 @@ bk_status launch_f32_to_half(bk_ctx *ctx, size_t n, const float *in, uint16_t *o
 bk_status launch_half_to_f32(bk_ctx *ctx, size_t n, const uint16_t *in, float *out);
 
 }  // namespace bk
+
+// ---- exported for the tests, no part of the interface: plans that are made on the host, to be checked without a GPU
+extern "C" {
+// How launch_prefill_umma spreads a block of n_tokens at position pos0 over n_sms processors.  A piece is four words: item = (blocks - 1 - block) *
+// n_kv + kv head, with blocks of 128 / (n_head / n_kv) tokens; first tile and end, in tiles of 32 rows; its place in the scratch, -1 for a whole
+// item.  Returns how many there are, in the order in which they are handed out; 0: every item whole, in the order of the items.  At most
+// `capacity` are written.
+BK_API int32_t bk_hook_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces);
+}

@@ -1100,18 +1100,6 @@ static void plan_pieces(int n_sms, int pos0, int n_tokens, int tq, int n_kv, Pie
     std::stable_sort(list.p + n_stretches, list.p + n, [&](const Piece &x, const Piece &y) { return length(x) > length(y); });
 }
 
-int prefill_plan(int n_sms, int pos0, int n_tokens, int n_head, int n_kv, int capacity, int32_t *pieces) {
-    PieceList list;
-    ItemParts parts;
-    plan_pieces(n_sms, pos0, n_tokens, kRows / (n_head / n_kv), n_kv, list, parts);
-    for (int i = 0; i < std::min(list.n, capacity); i++) {
-        const Piece &p = list.p[i];
-        const int32_t words[4] = {p.item, p.at, p.end, p.part};
-        std::copy(words, words + 4, pieces + 4 * i);
-    }
-    return list.n;
-}
-
 bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos0, int n_tokens, float alpha) {
     if (n_tokens <= 0) return BK_OK;
     const int n_rep = a.n_head / a.n_kv;
@@ -1149,3 +1137,15 @@ bk_status launch_prefill_umma(bk_ctx *ctx, const DecodeArgs &a, int seq, int pos
 }
 
 }  // namespace bk
+
+int32_t bk_hook_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces) {
+    bk::PieceList list;
+    bk::ItemParts parts;
+    bk::plan_pieces(n_sms, pos0, n_tokens, bk::kRows / (n_head / n_kv), n_kv, list, parts);
+    for (int i = 0; i < std::min(list.n, capacity); i++) {
+        const bk::Piece &p = list.p[i];
+        const int32_t words[4] = {p.item, p.at, p.end, p.part};
+        std::copy(words, words + 4, pieces + 4 * i);
+    }
+    return list.n;
+}
