@@ -71,6 +71,7 @@ constexpr size_t kPrefillRunFloats = 128 * 256;
 // place in the scratch, 128 query rows of (O, m, l).
 constexpr int kPrefillStretches = 160, kPrefillParts = 2 * kPrefillStretches, kPrefillPieces = 768;
 constexpr size_t kPrefillPartFloats = 128 * (256 + 2);
+constexpr int kGemmMaxSplit = 8;  // CTAs that share a tile of the PQ2_0 product, a cluster
 
 // What a kernel needs once per device (an attribute of it): `set_up` runs where it has not succeeded yet.  Racing first calls run it twice, and
 // devices beyond the table run it with every launch.
@@ -122,6 +123,7 @@ struct bk_ctx {
     size_t d_layer_floats = 0;
     float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention (the mma.sync form may grow it)
     size_t d_prefill_floats = 0;
+    int gemm_clusters[bk::kGemmMaxSplit + 1] = {};  // [0]: asked for; [n]: clusters of n CTAs of the PQ2_0 product that the device takes at once
     float *d_prefill_runs = nullptr;       // prefill attention: kPrefillRunFloats per SM, then an int per SM (taken or not)
     bk::HostPipe *pipe = nullptr;          // made by the first bulk host transfer
     uint8_t *d_pq2_x = nullptr;            // digits and block scales of x in the token-block PQ2_0 product (kPq2ScratchBytes)
@@ -377,4 +379,8 @@ extern "C" {
 // item.  Returns how many there are, in the order in which they are handed out; 0: every item whole, in the order of the items.  At most
 // `capacity` are written.
 BK_API int32_t bk_hook_prefill_plan(int32_t n_sms, int32_t pos0, int32_t n_tokens, int32_t n_head, int32_t n_kv, int32_t capacity, int32_t *pieces);
+// How launch_pq2_gemm tiles n_rows rows of n_blocks blocks: row tiles a CTA, token tiles in units of 16, CTAs that share a tile, tiles of the first
+// launch.  clusters[2..8]: how many clusters of that many CTAs are resident together, bk_hook_pq2_clusters() on the context's device.
+BK_API const int32_t *bk_hook_pq2_clusters(bk_ctx *ctx);
+BK_API int32_t bk_hook_pq2_plan(int32_t n_sms, const int32_t *clusters, int32_t n_rows, int32_t n_blocks, int32_t n_tok, int32_t *plan);
 }

@@ -58,7 +58,8 @@ constexpr uint32_t kGemmStageW = 2 * 2 * 128 * kGemmRowWords * 4;  // staged wei
 // Shared memory of the sums of the segments done, [row tile][token][row]; of a split tile every unit's, [unit of the CTA][token][row].
 __host__ __device__ constexpr uint32_t gemm_sum_bytes(int places, int n) { return (uint32_t)(places * n) * 512u; }
 // Pairs of units of a row of nb blocks, see the kernel.
-__host__ __device__ constexpr int gemm_pairs(int nb) { return (((nb + kGemmSegBlocks - 1) / kGemmSegBlocks + 1) / 2 + 1) / 2; }
+__host__ __device__ constexpr int gemm_halves(int nb) { return ((nb + kGemmSegBlocks - 1) / kGemmSegBlocks + 1) / 2; }
+__host__ __device__ constexpr int gemm_pairs(int nb) { return (gemm_halves(nb) + 1) / 2; }
 __host__ __device__ constexpr int gemm_places(int mt, int nb, int split) { return split > 1 ? 2 * ((gemm_pairs(nb) + split - 1) / split) : mt; }
 constexpr int kGemmFrac = 27;                     // X = round(x * 2^(kGemmFrac - e))
 // tensor-memory columns: per owner one or two pairs of sums (low | high, N columns each), then per owner two A stages (weights | times -64)
@@ -613,9 +614,17 @@ struct GemmPlan {
 // (row tile, block) takes what unpacking and draining issue, about 480 + 12 n clocks, or 700 + 11 n when two row tiles do not share a B block (L2).
 // Where two row tiles a CTA leave a last round nearly empty, its rows go out as tiles of half the size: q, k and v of 512 tokens are
 // 448 items for 148 SMs: 219 us in four rounds, 204 us as three rounds and one of half the length.
-static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n_tok) {
+static GemmPlan plan_gemm(int n_sms, const int *clusters, int n_seg, const int *n_rows, int nb, int n_tok) {
     GemmPlan plan;
     double best = 1e300;
+    const int n_pairs = gemm_pairs(nb), n_half = gemm_halves(nb);
+    int most[kGemmMaxSplit + 1] = {};  // segments of an owner of a cluster's busiest CTA: the pairs differ
+    for (int split = 2; split <= std::min(n_pairs, kGemmMaxSplit); split++)
+        for (int rank = 0; rank < split; rank++) {
+            int mine = 0;
+            for (int p = rank; p < n_pairs; p += split) mine += (p + 1) * n_half / n_pairs - p * n_half / n_pairs;
+            most[split] = std::max(most[split], mine);
+        }
     for (int nc = 1; nc <= 4; nc++) {
         const int n = 16 * nc;
         if (nc > 1 && n - 16 >= n_tok) break;
@@ -632,19 +641,46 @@ static GemmPlan plan_gemm(int n_sms, int n_seg, const int *n_rows, int nb, int n
         };
         for (int mt = 1; mt <= 2; mt++)
             if (gemm_stages(mt, n, nb) >= 2) take(mt, tiles[mt], rounds(tiles[mt]) * round[mt]);
-        // Where the tiles leave SMs without work, clusters of up to eight share a tile's pairs of units: the output projection of up to 64
-        // tokens is 40 tiles of three pairs, 27 us on
-        // 40 SMs and 16 us on 120 for 16 tokens, 32 and 25 for 64.  A cluster costs about 3000 clocks beside its steps.
-        const int n_pairs = gemm_pairs(nb), room = (int)std::min<int64_t>(std::min(n_pairs, 8), n_sms / std::max<int64_t>(1, tiles[1] * tok_tiles));
-        for (int split = 2; split <= room; split++) {
-            const int most = (n_pairs + split - 1) / split;  // pairs of the busiest CTA
-            if (gemm_stages(1, n, nb, split) >= 2) take(1, tiles[1], (700.0 + 11.0 * n) * nb * most / n_pairs + 9000.0, split);
-        }
+        // Where the tiles leave SMs without work, clusters of up to eight share a tile's pairs of units, as long as all of them fit on the device at
+        // once: the output projection of up to 64 tokens is 40 tiles of three pairs, 27 us on 40 SMs and 16 us on 120 for 16 tokens, 32 and 25 for
+        // 64.  A cluster lies within a group of SMs, so of 148 SMs 74 clusters of two find room, but 45 of three, 33, 26, 22, 15 and 15 of
+        // eight; one more is a second round: 24 tiles as 48 clusters of three 29 us, as 24 of wider tiles 18 (3072 rows, 32 tokens).  A cluster
+        // costs about 3000 clocks beside its steps, and the last places are dear (the CTAs of a cluster start together): 72 clusters of two 31.7
+        // us where 96 CTAs of their own take 29.7 (3072 rows, 100 tokens), 56 of them 27 against 29 (7168 rows, 40 tokens).
+        for (int split = 2; split <= std::min(n_pairs, kGemmMaxSplit); split++)
+            if (tiles[1] * tok_tiles <= clusters[split] && gemm_stages(1, n, nb, split) >= 2) {
+                const double last_places = std::max(0.0, (double)(tiles[1] * tok_tiles * split) / n_sms - 0.9);
+                take(1, tiles[1], (700.0 + 11.0 * n) * nb * most[split] / n_half + 9000.0 + 160000.0 * last_places, split);
+            }
         const int64_t whole = tiles[2] * tok_tiles / n_sms, main_tiles = whole * n_sms / tok_tiles;
         if (whole > 0 && main_tiles < tiles[2] && gemm_stages(2, n, nb) >= 2)
             take(2, main_tiles, (double)whole * round[2] + rounds(2 * (tiles[2] - main_tiles)) * round[1]);
     }
     return plan;
+}
+
+// How many clusters of 2, 3 .. kGemmMaxSplit CTAs the device takes at once (a CTA fills an SM); none where it does not say.
+static void pq2_gemm_clusters(int *clusters) {
+    const int smem = 227 * 1024;
+    std::fill(clusters, clusters + kGemmMaxSplit + 1, 0);
+    bool ok = cudaFuncSetAttribute(pq2_gemm_kernel<1, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+    for (int split = 2; ok && split <= kGemmMaxSplit; split++) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)split);
+        cfg.blockDim = dim3(kGemmThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)split;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        ok = cudaOccupancyMaxActiveClusters(&n, pq2_gemm_kernel<1, 1, true>, &cfg) == cudaSuccess;
+        clusters[split] = ok ? n : 0;
+    }
+    if (!ok) cudaGetLastError();
+    clusters[0] = 1;  // asked
 }
 
 // A token has 512 bytes of digits and a scale a block; a tile is filled up with up to 63 tokens of zeros.
@@ -674,7 +710,8 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
     if (used == 0) return BK_OK;
     const bk_status fit = pq2_rows_fit(ctx, ne0, n_tok);  // one limit for every number of tokens from two on
     if (fit != BK_OK) return fit;
-    const GemmPlan plan = plan_gemm(ctx->n_sms, used, rows_used, a.nb, n_tok);
+    if (!ctx->gemm_clusters[0]) pq2_gemm_clusters(ctx->gemm_clusters);
+    const GemmPlan plan = plan_gemm(ctx->n_sms, ctx->gemm_clusters, used, rows_used, a.nb, n_tok);
     const int n = 16 * plan.nc, tok_tiles = (n_tok + n - 1) / n;
     const size_t b_bytes = (size_t)n * 512, s_bytes = (size_t)a.nb * n * sizeof(float);
     // the digits, then one scale per block of every padded token
@@ -731,3 +768,14 @@ bk_status launch_pq2_gemm(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, co
 }
 
 }  // namespace bk
+
+const int32_t *bk_hook_pq2_clusters(bk_ctx *ctx) {
+    if (!ctx->gemm_clusters[0]) bk::pq2_gemm_clusters(ctx->gemm_clusters);
+    return ctx->gemm_clusters;
+}
+
+int32_t bk_hook_pq2_plan(int32_t n_sms, const int32_t *clusters, int32_t n_rows, int32_t n_blocks, int32_t n_tok, int32_t *plan) {
+    const bk::GemmPlan p = bk::plan_gemm(n_sms, clusters, 1, &n_rows, n_blocks, n_tok);
+    plan[0] = p.mt, plan[1] = p.nc, plan[2] = p.split, plan[3] = (int32_t)p.main_tiles;
+    return 4;
+}

@@ -320,8 +320,8 @@ def test_gpu_pq2_tiling_does_not_show(bk, gpu_ctx, nb):
 @pytest.mark.gpu
 @pytest.mark.parametrize("nb", [16, 17, 33, 36, 48, 49, 129])
 def test_gpu_pq2_clusters_on_a_tile_do_not_show(bk, gpu_ctx, nb):
-    """Few row tiles and few tokens: clusters of 2 to 8 share a tile's units (none with 16 blocks, which are one pair).  The same bits as among
-    so many tokens that nothing is shared, for tiles of 16 to 64 tokens and rows that do not fill their tile."""
+    """Few row tiles and few tokens: clusters share a tile's units (none with 16 blocks, which are one pair), up to eight CTAs of them with 129
+    blocks, which have nine pairs.  The same bits as among so many tokens that nothing is shared, with rows that do not fill their tile."""
     ne0, n_rows, n_all = nb * 128 - 40, 1000, 1024
     payload, _, _, x = synth(bk, nb, n_rows, ne0, n_all)
     t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
@@ -329,6 +329,59 @@ def test_gpu_pq2_clusters_on_a_tile_do_not_show(bk, gpu_ctx, nb):
     for n_tok in (5, 17, 33, 64):
         assert np.array_equal(t.matmul_n(x[:n_tok], n_tok), want[:n_tok]), n_tok
     assert np.array_equal(t.matmul_n(x[:9], 9, base_row=130, n_rows=150), want[:9, 130:280])
+    t.free()
+
+
+def pq2_plan(bk, n_sms, clusters, n_rows, nb, n_tok):
+    """(row tiles a CTA, token tile / 16, CTAs that share a tile, tiles of the first launch)"""
+    out = (ctypes.c_int32 * 4)()
+    bk._abi.load().bk_hook_pq2_plan(n_sms, (ctypes.c_int32 * 9)(*clusters), n_rows, nb, n_tok, out)
+    return tuple(out)
+
+
+def test_pq2_plan_keeps_to_the_clusters_that_fit(bk):
+    """A launch never has more clusters than the device takes at once, a tile's CTAs all have work, and the device decides: with room for none,
+    none are made.  The counts are a B200's, then fewer."""
+    b200 = [0, 0, 74, 45, 33, 26, 22, 15, 15]
+    assert pq2_plan(bk, 148, b200, 5120, 48, 16)[:3] == (1, 1, 3)
+    assert pq2_plan(bk, 148, b200, 3072, 40, 32)[:3] == (1, 2, 3)  # (48 clusters of three for tiles of 16 tokens)
+    forms = set()
+    for clusters in (b200, [0, 0, 9, 6, 4, 3, 3, 2, 2], [0] * 9):
+        for n_rows in (1, 150, 640, 1000, 2304, 3072, 5120, 5760, 9472, 14336):
+            for nb in (1, 16, 17, 33, 40, 48, 49, 72, 88, 104, 113, 120, 128, 129, 140):
+                for n_tok in (5, 16, 17, 33, 48, 49, 64, 100, 130, 256, 512):
+                    mt, nc, split, _ = pq2_plan(bk, 148, clusters, n_rows, nb, n_tok)
+                    if split > 1:
+                        assert mt == 1 and -(-n_rows // 128) * -(-n_tok // (16 * nc)) <= clusters[split]
+                        assert split <= (-(-(-(-nb // 4)) // 2) + 1) // 2
+                        forms.add((nc, split))
+    assert {nc for nc, _ in forms} == {1, 2, 3, 4} and {split for _, split in forms} == set(range(2, 9))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,n_rows,forms", [
+    (48, 5120, {(1, 3), (2, 3), (3, 3), (4, 3)}),  # the output projection
+    (17, 1000, {(1, 2)}), (64, 5100, {(1, 2), (2, 2)}), (49, 1000, {(1, 4), (2, 4), (3, 4)}), (72, 1000, {(1, 5), (2, 5)}), (88, 1000, {(1, 6), (2, 6), (4, 6)}),
+    (104, 1000, {(1, 7), (2, 7), (3, 7), (4, 7)}), (120, 1000, {(1, 8), (2, 8), (3, 8)})])
+def test_gpu_pq2_every_form_of_clusters(bk, gpu_ctx, nb, n_rows, forms):
+    """Tiles of 16, 32, 48 and 64 tokens in clusters of 2 to 8: bit for bit a block of so many tokens that no tile is shared, and that within
+    the bound of the token-block test.  Which forms a B200 gets is part of the test."""
+    ne0, n_all, counts = nb * 128 - 40, 1024, (5, 17, 33, 48, 50, 64, 100, 130)
+    clusters = (ctypes.c_int32 * 9)()
+    fn = bk._abi.load().bk_hook_pq2_clusters
+    fn.restype = ctypes.POINTER(ctypes.c_int32)
+    clusters[:] = [0, 0, *fn(gpu_ctx.h)[2:9]]
+    plans = {n: pq2_plan(bk, 148, clusters, n_rows, nb, n) for n in (*counts, n_all)}
+    assert plans[n_all][2] == 1
+    if list(clusters) == [0, 0, 74, 45, 33, 26, 22, 15, 15]:  # (a device with other groups of SMs has other forms)
+        assert {p[1:3] for p in plans.values() if p[2] > 1} >= forms
+    payload, codes, scales, x = synth(bk, nb, n_rows, ne0, n_all)
+    t = bk.Pq2Tensor(gpu_ctx, payload, ne0)
+    want = t.matmul_n(x, n_all)
+    w, x64 = dense(codes[:200], scales[:200], ne0), x[:130].astype(np.float64)
+    assert np.max(np.abs(want[:130, :200] - x64 @ w.T) / (np.abs(x64) @ np.abs(w).T + 1e-30)) <= 2e-6  # as in the token-block test
+    for n_tok in counts:
+        assert np.array_equal(t.matmul_n(x[:n_tok], n_tok), want[:n_tok]), (n_tok, plans[n_tok])
     t.free()
 
 
