@@ -189,6 +189,47 @@ def test_prefill_plan_covers_every_tile_once(bk, n_head, n_kv):
                 assert np.array_equal(w[:, 3], w[0, 3] + np.arange(len(w))) and (w[0, 3] >= 0 or len(w) == 1)
 
 
+def test_prefill_plan_cuts_where_it_gains(bk):
+    """A plan of pieces, each handed to the processor that is free first at seven tiles a piece beside its own, ends before whole items would, within
+    a fifth and a piece's seven tiles of an even spread; and blocks that go out whole would not have gained more than the cutting costs."""
+    import heapq
+    lib = bk._abi.load()
+
+    def end(lengths, n_sms):
+        free = [0] * n_sms
+        for n in lengths:
+            heapq.heapreplace(free, free[0] + n + 7)
+        return max(free)
+
+    seen = {True: 0, False: 0}
+    for n_sms in (148, 132, 16):
+        for n_head, n_kv in ((24, 4), (48, 8), (8, 8), (6, 1)):
+            tq = 128 // (n_head // n_kv)
+            for pos0 in (0, 500, 1024, 4096, 30000):
+                for n_tok in (4, 50, 130, 300, 400, 512, 600, 777, 1000, 1500, 2500):
+                    blocks = -(-n_tok // tq)
+                    if blocks * n_kv > 608:
+                        continue
+                    words = np.zeros((768, 4), np.int32)
+                    n = lib.bk_hook_prefill_plan(n_sms, pos0, n_tok, n_head, n_kv, 768, C.c_void_p(words.ctypes.data))
+                    items = [-(-(pos0 + min((blocks - i // n_kv) * tq, n_tok)) // 32) for i in range(blocks * n_kv)]
+                    whole, even = end(items, n_sms), sum(t + 7 for t in items) / n_sms
+                    what = (n_sms, n_head, n_kv, pos0, n_tok)
+                    if n:
+                        cut = end((words[:n, 2] - words[:n, 1]).tolist(), n_sms)
+                        assert cut < whole, (what, cut, whole)
+                        spread = (sum(items) + 7 * n) / n_sms
+                        assert cut <= 1.2 * max(spread, 11) + 7, (what, cut, spread)
+                    else:
+                        assert whole <= 1.05 * max(1.25 * even + 7, 11) + 3 + 320 / 45, (what, whole, even)
+                    seen[n > 0] += 1
+    assert min(seen.values()) > 50
+    for shape in ((0, 400, 24, 4), (4096, 512, 24, 4), (30000, 4, 6, 1)):
+        assert lib.bk_hook_prefill_plan(148, *shape, 0, None) > 0
+    for shape in ((0, 4, 24, 4), (0, 1000, 24, 4), (0, 600, 48, 8), (0, 3400, 24, 4)):
+        assert lib.bk_hook_prefill_plan(148, *shape, 0, None) == 0
+
+
 def test_read_only_loads_are_of_constants():
     """A kernel that is launched under the end of another one (it has a griddepcontrol.wait) may use the read-only path, which takes it for granted
     that nobody writes the data while the kernel lives, only for tables and weights: its other inputs may still be on their way when it starts."""
