@@ -282,9 +282,11 @@ bk_status launch_append(bk_ctx *ctx, const AppendArgs &a) {
     const int threads = kThreads;
     const size_t n_vec = (size_t)a.n_tokens * 2 * a.n_kv;
     const bool planar = a.k_kind == ROW_PLANAR || a.v_kind == ROW_PLANAR;
-    // More than ten small CTAs per SM: go for throughput.  Append and decode, us a layer, 8 / 16 vectors a CTA: planar4, 512 tokens 14.6 / 16.5,
-    // 1184 tokens 17.7 / 19.1, 1500 tokens 20.1 / 20.4, 2048 tokens 22.6 / 21.0; K only, 1500 tokens 19.4 / 18.7.  (32 vectors: 18.9 at 512.)
-    const bool bulk = n_vec > (size_t)8 * 10 * ctx->n_sms;
+    // More small CTAs than this per SM: go for throughput.  Up to 4 bits eight, the places of small CTAs on an SM twice: us a layer, 8 / 16
+    // vectors a CTA, append alone, and with a decode: planar4, 1050 tokens 6.7 / 6.3, 15.8 / 17.2; 1200 tokens 8.5 / 6.6, 17.6 / 17.7; 1400 tokens
+    // 9.7 / 7.3, 18.9 / 18.2 (with 32 vectors 7.1 and 18.5, 8.4 and 20.8, 9.5 and 21.5); K only, 1050 tokens 7.3 / 6.9, 16.8 / 16.5; 1200
+    // tokens 8.7 / 7.2, 17.3 / 16.6.  Wider rows ten: planar8, 1200 tokens 17.8 / 17.4, 32.9 / 34.2; 1600 tokens (24.2, 42.8 with 16).
+    const bool bulk = n_vec > (size_t)8 * (a.bits >= 1 && a.bits <= 4 ? 8 : 10) * ctx->n_sms;
     const int vecs = bulk && planar ? 16 : 8;
     const size_t smem = (size_t)(vecs * kVecPad + 64 + (a.bits > 4 ? 256 + kHd : 0)) * sizeof(float);
     const int per_warp = vecs / kWarps;

@@ -171,8 +171,10 @@ def test_append_bytes_bit_exact(bk, gpu_ctx, oracle, tag, mode, bits, vq):
 def test_bulk_append_of_ragged_token_counts(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv):
     """Calls on both sides of the line between small and bulk calls; warps with one or two tokens of a head, warps without any, numbers of heads
     that are no power of two: rows bit-exact."""
+    import torch
     rng = np.random.default_rng(n_kv)
-    n0 = 8 * 10 * 148 // (2 * n_kv)  # ten small CTAs an SM
+    n_sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n0 = 8 * (8 if 1 <= bits <= 4 else 10) * n_sms // (2 * n_kv)  # small CTAs an SM
     for n in (n0 - 1, n0 + 1, n0 + 2):
         k, v = rng.standard_normal((2, n, n_kv, HD)).astype(np.float32)
         cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n, n_head=n_head, n_kv=n_kv)
