@@ -350,9 +350,6 @@ bk_status bk_ctx_create(int device, bk_ctx **out) {
     const size_t run_bytes = (size_t)ctx->n_sms * kPrefillRunFloats * sizeof(float);
     if ((e = cudaMalloc(&ctx->d_prefill_runs, run_bytes + ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc prefill sums");
     if ((e = cudaMemset((char *)ctx->d_prefill_runs + run_bytes, 0, ctx->n_sms * sizeof(int))) != cudaSuccess) return bail(e, "clear prefill sums");
-    const size_t prefill_floats = (size_t)2 * std::min(ctx->n_sms, kPrefillStretches) * kPrefillPartFloats;
-    if ((e = cudaMalloc((void **)&ctx->d_prefill, prefill_floats * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc prefill scratch");
-    ctx->d_prefill_floats = prefill_floats;
     {
         void *herr = nullptr, *derr = nullptr;
         if ((e = cudaHostAlloc(&herr, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) return bail(e, "cudaHostAlloc error word");
@@ -577,6 +574,18 @@ bk_status bk_cache_create(bk_ctx *ctx, const bk_cache_config *cfg, bk_cache **ou
             return st;
         }
         c->has_tmaps = true;
+        // the prefill's scratch (39 MB on 148 SMs) comes with the context's first cache that can use it, so that no call allocates
+        if (!ctx->d_prefill && ctx->prefill_umma && !ctx->force_generic && n_rep != 8) {
+            const size_t floats = (size_t)2 * std::min(ctx->n_sms, kPrefillStretches) * kPrefillPartFloats;
+            const cudaError_t e = cudaMalloc((void **)&ctx->d_prefill, floats * sizeof(float));
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                ctx->d_prefill = nullptr;
+                bk_cache_destroy(c);
+                return cuda_fail(ctx, e, "cudaMalloc prefill scratch");
+            }
+            ctx->d_prefill_floats = floats;
+        }
     }
     *out = c;
     return BK_OK;

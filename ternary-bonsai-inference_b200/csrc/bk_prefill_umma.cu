@@ -991,6 +991,7 @@ bk_status launch_umma_one(bk_ctx *ctx, const PrefillUArgs &pa, const PieceList &
     }
     if (!pa.d.h_tmap_k || !pa.d.h_tmap_v) return fail(ctx, BK_ERR_INVALID, "prefill: the cache has no tensor maps");
     const int n_items = pa.n_blocks * pa.d.n_kv;
+    if (list.n > n_items && !pa.scratch) return fail(ctx, BK_ERR_INVALID, "prefill: no scratch for pieces");  // (made with the cache)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(list.n ? list.n : n_items));
     cfg.blockDim = dim3(kUT);

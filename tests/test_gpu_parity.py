@@ -1583,6 +1583,34 @@ def test_prefill_of_an_infinite_row(bk, gpu_ctx, oracle, tag, mode, bits, vq):
     assert 40 < seen < 160  # (20 tokens, 12 heads, about half)
 
 
+def test_prefill_scratch_comes_with_the_first_cache_that_can_use_it(bk):
+    """39 MB (two places of 129 KiB a SM) that a context without such a cache does not hold; a second cache brings no more."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    scratch = 2 * min(sms, 160) * 128 * 258 * 4
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    warm = bk.Context(0)
+    before = free()
+    ctx = bk.Context(0)
+    alone = before - free()
+    caches = []
+    grown = []
+    for tag, n_head in (("planar8", 24), ("f16", 32), ("planar4", 24), ("f32", 24)):  # (32 heads on 4 are not taken)
+        at = free()
+        caches.append(bk.AttnCache(ctx, bk.parse_mode(tag), n_layers=1, n_ctx=64, n_head=n_head))
+        grown.append(at - free())
+    slack = 8 << 20  # (what the driver rounds up to)
+    assert max(grown[0], grown[1], grown[3]) < slack and scratch - slack < grown[2] < scratch + slack, (alone, grown)
+    for c in caches:
+        c.close()
+    ctx.close()
+    warm.close()
+
+
 def test_prefill_of_more_items_than_are_cut(bk, gpu_ctx, oracle):
     """A prompt block of so many items that they go out whole: 153 blocks of 21 tokens."""
     rng = np.random.default_rng(3)
