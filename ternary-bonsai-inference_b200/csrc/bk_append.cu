@@ -30,15 +30,7 @@ constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 
 // Two f32 products in one instruction, each rounded as __fmul_rn does.
-__device__ __forceinline__ float2 mul_pair(float x, float y, float a, float b) {
-    uint64_t p, q;
-    float2 r;
-    asm("mov.b64 %0, {%1, %2};\n" : "=l"(p) : "f"(x), "f"(y));
-    asm("mov.b64 %0, {%1, %2};\n" : "=l"(q) : "f"(a), "f"(b));
-    asm("mul.rn.f32x2 %0, %0, %1;\n" : "+l"(p) : "l"(q));
-    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(p));
-    return r;
-}
+__device__ __forceinline__ float2 mul_pair(float x, float y, float a, float b) { return unpack2(mul2(pack2(x, y), pack2(a, b))); }
 
 // Eight consecutive coordinates of a staged vector for every lane without bank conflicts: two 128-bit reads
 // in the staging layout (coordinates 4 l .. 4 l + 3 and 128 + 4 l .. + 3), then lanes 2m and 2m + 1 swap

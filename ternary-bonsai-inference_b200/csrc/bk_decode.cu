@@ -229,32 +229,6 @@ __global__ void __launch_bounds__(kThreads) decode_kernel(DecodeArgs a, DecodeMe
 // 185 instructions a row now (215 with rows loaded into registers); the f32 pipe is the busiest.
 constexpr int kGroup = 4;  // positions a warp works on at a time
 
-__device__ __forceinline__ uint64_t pack2(float x, float y) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t r) {
-    float2 a;
-    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a.x), "=f"(a.y) : "l"(r));
-    return a;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // More than twelve warps do not fit with q and the sums of six heads in registers (168 each); eight heads, or rows of f32, want 255.
 template <int VK, int NREP>
 constexpr int kPlanarWarps = (VK == ROW_PLANAR && NREP <= 6) ? 12 : 8;

@@ -153,31 +153,8 @@ __device__ __forceinline__ void unpack16(uint32_t w, uint32_t *one, uint32_t *wi
     }
 }
 
-// Two f32 operations in one instruction (the draining warps are bound by what they issue).
-struct F2 {
-    float x, y;
-};
-__device__ __forceinline__ uint64_t join2(F2 a) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a.x), "f"(a.y));
-    return r;
-}
-__device__ __forceinline__ F2 split2(uint64_t r) {
-    F2 a;
-    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a.x), "=f"(a.y) : "l"(r));
-    return a;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t int2_to_f2(uint32_t a, uint32_t b) { return join2(F2{__int2float_rn((int)a), __int2float_rn((int)b)}); }
+// (Two f32 operations in one instruction: the draining warps are bound by what they issue.)
+__device__ __forceinline__ uint64_t int2_to_f2(uint32_t a, uint32_t b) { return pack2(__int2float_rn((int)a), __int2float_rn((int)b)); }
 
 // MT row tiles per CTA, N = 16 NC tokens.  Sixteen warps in two halves of eight ("owners") work on alternate steps, each with
 // its own sums and operand stages, so that the round trips of a step (operand stores, the MMAs, reading the sums back) are under
@@ -453,9 +430,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
                         const int k = 4 * c4 + 2 * j;
-                        const uint64_t sum = fma2(int2_to_f2(hi[c & 1][k], hi[c & 1][k + 1]), join2(F2{16384.0f, 16384.0f}),
+                        const uint64_t sum = fma2(int2_to_f2(hi[c & 1][k], hi[c & 1][k + 1]), pack2(16384.0f, 16384.0f),
                                                   int2_to_f2(lo[c & 1][k], lo[c & 1][k + 1]));
-                        acc[4 * c + k / 2] = fma2(mul2(join2(F2{sc, sc}), xv[j]), sum, acc[4 * c + k / 2]);
+                        acc[4 * c + k / 2] = fma2(mul2(pack2(sc, sc), xv[j]), sum, acc[4 * c + k / 2]);
                     }
                 }
             }
@@ -469,7 +446,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
                 float *own = reinterpret_cast<float *>(sm + off_t) + (size_t)(unit * N + half * NH) * 128 + r;
 #pragma unroll
                 for (int j = 0; j < NH / 2; j++) {
-                    const F2 v = split2(acc[j]);
+                    const float2 v = unpack2(acc[j]);
                     own[2 * j * 128] = v.x, own[(2 * j + 1) * 128] = v.y;
                     acc[j] = 0;
                 }
@@ -479,10 +456,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) pq2_gemm_kernel(const GemmArg
                 ok = ok && wait(bar_turn + 8 * (1 - owner), (uint32_t)((unit - 1) >> 1) & 1u);
                 __syncwarp();
             }
-            F2 v[NH / 2];
+            float2 v[NH / 2];
 #pragma unroll
             for (int j = 0; j < NH / 2; j++) {
-                v[j] = split2(acc[j]);
+                v[j] = unpack2(acc[j]);
                 acc[j] = 0;
                 if (unit > 0) v[j].x += tot[2 * j * 128], v[j].y += tot[(2 * j + 1) * 128];
             }

@@ -178,7 +178,7 @@ struct ItemParts {  // of every item: its first place in the scratch (they lie s
 };
 static_assert((size_t)kRows * (kHd + 2) == kPrefillPartFloats, "scratch of a piece: [row][coordinate], then [row](m, l)");
 
-// Two f32 operations in one instruction (the softmax warps are bound by what they issue).
+// Two f32 operations in one instruction (the softmax warps are bound by what they issue); scores come and go as words.
 __device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(a), "r"(b));
@@ -186,22 +186,6 @@ __device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ uint32_t first(uint64_t x) { return (uint32_t)x; }
 __device__ __forceinline__ uint32_t second(uint64_t x) { return (uint32_t)(x >> 32); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
 struct PrefillUArgs {
     DecodeArgs d;
     int seq, pos0, n_tokens, tq, n_blocks;
@@ -704,11 +688,11 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
         // 4608 tokens 6.2 -> 6.7 ms (four layers), 777 tokens 287 -> 309 us.  The same by shorter chunks: 7.1 ms and 341 us.
         // The sums so far come in a block of 32 coordinates ahead of their use, the first before the run's last product is awaited (one block
         // after the other, each with its trip to L2, made 4 us of it).
-        auto collect_o = [&](bool first, auto &&run_done) -> bool {
+        auto collect_o = [&](bool first_run, auto &&run_done) -> bool {
             float4 old[2][8];
             auto fetch = [&](int b, float4 (&dst)[8]) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) dst[j] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
+                for (int j = 0; j < 8; j++) dst[j] = first_run ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(run_sums() + (8 * b + j) * kRows + my_q);
             };
             fetch(0, old[0]);
             if (!run_done()) return false;
