@@ -519,6 +519,29 @@ def test_generic_planar_decode_in_groups_of_four(bk, gpu_ctx, oracle, tag, bits,
     cache.close()
 
 
+@pytest.mark.parametrize("tag,bits,vq", [("planar8", 8, True), ("planar1", 1, True), ("planar5k", 5, False)])
+@pytest.mark.parametrize("copies", [1, 4])
+def test_generic_planar_decode_of_a_batch_in_chunks(bk, gpu_ctx, oracle, tag, bits, vq, copies):
+    """Sequences of one and of many chunks in one launch, few of them (one wave) and 24 (two CTAs' time an SM)."""
+    rng = np.random.default_rng(bits)
+    lens = [2500, 5, 1200, 700, 145, 64] * copies
+    k, v = rng.standard_normal((2, max(lens), NKV, HD)).astype(np.float32)
+    q = rng.standard_normal((len(lens), NH, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_seqs=len(lens), n_ctx=max(lens))
+    ref = oracle.cache(MODE_PLANAR, bits, vq)
+    for p in range(max(lens)):
+        ref.append(0, k[p], v[p], p)
+    for s, n in enumerate(lens):
+        cache.append(0, k[:n], v[:n], seq=s)
+    launches = gpu_ctx.launch_count
+    got = cache.attend(0, q, n_seqs=len(lens))
+    assert gpu_ctx.launch_count - launches == 1
+    cache.close()
+    for s, n in enumerate(lens):
+        want = ref.attend(0, q[s], n - 1, n, threads=8)
+        assert np.max(np.abs(got[s] - want)) <= 1e-5 * np.max(np.abs(want)), (s, n)  # (as in the test of groups of four)
+
+
 def test_generic_decode_keeps_infinities_where_they_are(bk, gpu_ctx, oracle):
     """K-only rows: an infinite V coordinate in the last row, of which copies stand in for the rows a group lacks."""
     rng = np.random.default_rng(5)
@@ -1369,8 +1392,8 @@ def prefill_both(bk, gpu_ctx, oracle, tag, mode, bits, vq, n0, n_tok, seed, n_he
                                               MODES[4], ("planar3k", MODE_PLANAR, 3, False)])
 @pytest.mark.parametrize("n0,n_tok", [(0, 45), (300, 50), (3000, 100), (37, 3), (0, 1)])
 def test_prefill_attention_equals_token_by_token(bk, gpu_ctx, oracle, tag, mode, bits, vq, n0, n_tok):
-    """planar4 / planar3 / f16 take the batched tensor-core kernel (from 4 tokens on), the other
-    modes the decode kernels with one entry per token; every token must meet the decode bar."""
+    """All but 1-bit and 5- to 8-bit caches take the batched tensor-core kernel (from 4 tokens on), the others
+    the decode kernels with one entry per token; every token must meet the decode bar."""
     got, want = prefill_both(bk, gpu_ctx, oracle, tag, mode, bits, vq, n0, n_tok, seed=n0 + n_tok + bits)
     for i in range(n_tok):
         assert_close(got[i], want[i], f"{tag} n0={n0} token {i}")
@@ -1380,8 +1403,8 @@ def test_prefill_attention_equals_token_by_token(bk, gpu_ctx, oracle, tag, mode,
 def test_prefill_mma_sync_variant_and_empty_chunks(bk, oracle, monkeypatch, tag, mode, bits, vq):
     """The batched kernel exists twice: on tcgen05 with tensor-memory accumulators (default) and
     on mma.sync (BONSAI_KV_PREFILL=mma, read when the context is created).  A 700-token prompt
-    from the empty cache gives two context chunks, of which the second is empty for the early
-    query blocks; both kernels must handle it."""
+    from the empty cache gives the mma.sync form two context chunks, of which the second is empty for
+    the early query blocks (the pieces of the tcgen05 form end where their item ends)."""
     for env in ("mma", None):
         if env:
             monkeypatch.setenv("BONSAI_KV_PREFILL", env)
@@ -1609,6 +1632,69 @@ def test_prefill_scratch_comes_with_the_first_cache_that_can_use_it(bk):
         c.close()
     ctx.close()
     warm.close()
+
+
+def prefill_plan(bk, pos0, n_tok, n_head, n_kv):
+    """Pieces of a prompt block on this device, 0 where its items stay whole."""
+    import torch
+    return bk._abi.load().bk_hook_prefill_plan(torch.cuda.get_device_properties(0).multi_processor_count, pos0, n_tok, n_head, n_kv, 0, None)
+
+
+@pytest.mark.parametrize("tag,mode,bits,vq", [MODES[0], MODES[3], ("planar2", MODE_PLANAR, 2, True), MODES[4], ("planar3k", MODE_PLANAR, 3, False)])
+@pytest.mark.parametrize("n_head,n_kv,n0,n_tok", [(6, 1, 9000, 5), (24, 4, 2000, 300), (24, 4, 0, 400), (4, 4, 1000, 130)])
+def test_prefill_in_pieces_of_other_modes(bk, gpu_ctx, oracle, tag, mode, bits, vq, n_head, n_kv, n0, n_tok):
+    """The same for rows that are looked up by permutes, K-only rows and f32: an item over all SMs, items in one and two pieces side by side."""
+    assert prefill_plan(bk, n0, n_tok, n_head, n_kv) > -(-n_tok // (128 * n_kv // n_head)) * n_kv
+    rng = np.random.default_rng(n0 + n_tok + bits)
+    n = n0 + n_tok
+    k, v = rng.standard_normal((2, n, n_kv, HD)).astype(np.float32)
+    q = rng.standard_normal((n_tok, n_head, HD)).astype(np.float32)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n, n_head=n_head, n_kv=n_kv)
+    cache.append(0, k, v)
+    ref = oracle.cache(mode, bits, vq, n_head=n_head, n_kv=n_kv)
+    for p in range(n):
+        ref.append(0, k[p], v[p], p)
+    got = cache.prefill_attend(0, q, n0)
+    cache.close()
+    for i in sorted({0, 1, min(20, n_tok - 1), min(21, n_tok - 1), n_tok // 2, n_tok - 2, n_tok - 1}):
+        assert_close(got[i], ref.attend(0, q[i], n0 + i, n0 + i + 1, threads=8), f"{tag} token {i}")
+
+
+@pytest.mark.parametrize("tag", ["planar4", "planar3", "planar2"])
+@pytest.mark.parametrize("n0,n_tok", [(0, 90), (700, 40)])
+def test_prefill_of_v_rows_of_any_norm(bk, gpu_ctx, tag, n0, n_tok):
+    """A norm is a factor beside a weight of up to 2^114: V rows of zeros, of 1e-12 and 1e12 and of 1e-18 before one of 1e12, next to ordinary
+    ones and alone at the start, in whole and in cut items.  Bound: the 2-norm of the other tests, and 1e-29 where a result is all but zero (norms are taken
+    as 1e-30 at least)."""
+    assert (prefill_plan(bk, n0, n_tok, NH, NKV) > 0) == (n0 > 0)
+    rng = np.random.default_rng(n0 + int(tag[6]))
+    n = n0 + n_tok
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    v[:n // 3, 0] = 0                                   # nothing but zeros, then ordinary rows
+    v[:, 1] *= np.float32(1e-12)
+    v[::3, 2] = 0
+    v[1::3, 2] *= np.float32(1e12)
+    v[:n // 2, 3] *= np.float32(1e-18)                   # (a row's norms may span 1e32: weights go to 2^114 in f32)
+    v[n // 2 + 5, 3] *= np.float32(1e12)
+    cache = bk.AttnCache(gpu_ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    cache.append(0, k, v)
+    got = cache.prefill_attend(0, q[n0:], n0).astype(np.float64)
+    d = cache.dump_kv(0)
+    cache.close()
+    pq = bk.PlanarQuant(HD, int(tag[6]), gpu_ctx)
+    ks, unit = (pq.dequantize(d[x].reshape(n * NKV, -1), nrm).reshape(n, NKV, HD).astype(np.float64)
+                for x, nrm in (("kq", d["kn"].ravel()), ("vq", np.ones(n * NKV, np.float32))))
+    vs = unit * d["vn"].reshape(n, NKV, 1).astype(np.float64)
+    bound = 2e-4 if tag == "planar3" else 1e-5  # (f16 centroids without remainders: the 8 of 3 bits to 1e-4, on K and on V)
+    qr = roped(bk, gpu_ctx, q)[n0:].astype(np.float64)
+    for h in range(NH):
+        s = qr[:, h] @ ks[:, h // 6].T / 16.0
+        s[np.arange(n)[None, :] > np.arange(n0, n)[:, None]] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = (w / w.sum(1, keepdims=True)) @ vs[:, h // 6]
+        err = np.linalg.norm(got[:, h] - want, axis=1)
+        assert np.all(err <= bound * np.linalg.norm(want, axis=1) + 1e-29), (h, (err / (np.linalg.norm(want, axis=1) + 1e-30)).max())
 
 
 def test_prefill_of_more_items_than_are_cut(bk, gpu_ctx, oracle):
