@@ -127,7 +127,7 @@ __device__ __forceinline__ void store_f16_row(const float *sx, int lane, uint8_t
 // smaller calls (latency: one vector per warp) and for f32 and f16 rows, which have no norm: many small CTAs load while others store.
 // Us a layer of back-to-back calls of 2048 / 4096 / 8192 tokens: planar4 12.6 / 20.4 / 33.9 with 32 vectors a CTA, the head worked out per
 // vector, products one at a time and five CTAs an SM, 10.3 / 17.8 / 32.2 without that and four CTAs, 9.9 / 16.8 / 29.6 with the rows staged by
-// cp.async instead of through registers, 11.0 / 17.2 / 31.0 with 16 vectors (six CTAs an SM spill); f32 10.3 / 17.7 / 29.7 in CTAs of 32
+// cp.async instead of through registers, 11.0 / 17.2 / 31.0 with 16 vectors (five CTAs an SM leave 48 registers, of which 4 bits spill 28 bytes and 5 to 7 bits 4 to 8; six were slower); f32 10.3 / 17.7 / 29.7 in CTAs of 32
 // vectors, 7.8 / 13.5 / 25.0 of 8, 7.4 / 12.1 / 21.9 by cp.async; f16 11.1 / 17.3 / 29.5, 7.9 / 14.1 / 25.9 and 7.4 / 11.8 / 21.6.
 // Sixteen vectors a CTA are taken for what follows an append, a decode of the same layer: both together 21.0 / 27.8 / 43.4 against 21.2 / 28.5 /
 // 45.5 with 32 (planar4), 20.9 / 29.5 / 47.2 against 20.3 / 30.4 / 50.7 (K only).

@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(kThreads) decode_kernel(DecodeArgs a, DecodeMe
 //     waited for (8 bit, 131000 rows: 182 to 235 us a layer).
 // Measured (24 q heads on 4, us a layer of a 16-layer step, append included, a row a step before / now): 8 bit, 40 rows 23 / 15, 100 rows 27 / 17, 1000 rows
 // 28 / 20, 9000 rows 90 / 32, 32768 rows 155 / 55, 131000 rows 370 / 145; 5 bit, 9000 rows 103 / 31; 8 bit K beside f32 V, 9000 rows 87 / 33.
-// 185 instructions a row now (215 with rows loaded into registers); the f32 pipe is the busiest.
+// 177 instructions a row now (215 with rows loaded into registers); the f32 pipe is the busiest.  With twelve warps (168 registers) 56 to 84 bytes
+// spill for four and six heads, none for one and two.
 constexpr int kGroup = 4;  // positions a warp works on at a time
 
 // More than twelve warps do not fit with q and the sums of six heads in registers (168 each); eight heads, or rows of f32, want 255.

@@ -341,7 +341,8 @@ bk_status pq2_rows_fit(bk_ctx *ctx, int ne0, int n_tok);
 bk_status launch_pq2_matvec(bk_ctx *ctx, int n_seg, const uint8_t *const *rows, const int *n_rows, float *const *y, int ne0,
                             const float *x, int n_tok);
 // The same for a block of up to pq2_gemm_tokens() tokens on the tensor cores (bk_pq2_gemm.cu).
-// From 5 tokens on (q + k + v and output rows of a layer: 4 tokens 45 us in pairs, 52 us here; 5 tokens 62 and 52);
+// From 5 tokens on (q + k + v and output rows of a layer: 2 tokens 20.9 us in pairs and 39.1 here, 3 tokens 37.4 and 39.1, 4
+// tokens 41.0 and 39.1, from where pairs take 10 us and more a token and this 0.1).
 // The scratch is made with the context, so that no call allocates or waits for the stream: 1024 tokens of up to 59 blocks a
 // pass, fewer of longer rows.
 constexpr int kPq2GemmTokens = 1024, kPq2GemmMin = 5;

@@ -24,9 +24,9 @@
 //     pair are what the operand stages leave, hence at most 64 tokens a tile.
 //   * The two digits that meet the same weights are one B operand of 2 N columns, into both sums of a pair at once: half as many
 //     products as one digit each, and up to 32 tokens each costs the same 32 clocks (512 tokens: 298 us a layer before, 281 so).
-// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 tokens 40 us, 16 tokens 42 (62 and
-// 176 as pairs of tokens; 4 tokens as pairs take 41, which is where the line lies), 64 tokens 61 (702), 128 tokens 93 (1410), 512
-// tokens 281 (5750).  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
+// Measured (q, k, v and output projection of a layer, 14336 x 5120 and 5120 x 6144): 5 tokens 39 us, 16 tokens 41 (62 and
+// 176 as pairs of tokens; 4 tokens 41.0 as pairs and 39.1 here, 3 tokens 37.4 and 39.1, so the line could lie at 4), 64 tokens 61 (702),
+// 128 tokens 93 (1410), 512 tokens 281 (5750).  The form before, x as two f16 parts scaled per token and truncated f32 block sums, took
 // 57, 86, 129, 287 and 574.  Error against float64, 2-norm: 7.4e-8 on normal data, 8.0e-8 with x20 outliers in x, 4.5e-8 without
 // a bias on products of one sign; 1.02e-7, 2.4e-7 and 5.0e-8 as pairs of tokens; 1.01e-7, 1.0e-7 and 6.5e-8 (bias -5e-8) in the
 // form before, which also lost blocks that lie 2^40 below the token's largest element.

@@ -4,8 +4,9 @@
 //
 // One CTA = 128 query rows (M = 128) of one kv head over a piece of the context they see, tile by tile of 32 positions.  What
 // bounds it: for 4-bit and f32 rows six 128 x 32 x 256 products per tile (hi.hi, hi.lo, lo.hi twice), 1800 clocks of the tensor cores as
-// issued; softmax warps and producers each take 2000 to 2600 of a tile's 2800 clocks, and shared memory is about as busy; so nothing may
-// wait for anything else.  Thirteen warps in three roles, coupled by mbarriers only:
+// issued, of a tile's 3260 clocks (f32 rows 4200, f16 and 3 bit 2650: from blocks of 512 tokens after 4096 and 16384 rows; 1.66 us at full clocks, long
+// loops run into the power limit).  The tensor pipe is active for 47 % of them, tensor memory 52, shared memory about half, 44 % of the issue slots are
+// taken: no unit is full, the roles wait for one another, so nothing may wait for anything else.  About 20 us of a launch lie beside the tiles.  Thirteen warps in three roles, coupled by mbarriers only:
 //   * warps 4-11 (producers) turn packed rows into f16 operand tiles (for 4 bit with the rounding remainders, for
 //     f32 rows hi + lo parts) in a ring of five slots, in the order of use: K0, K1, V0, K2, V1, ...  A thread's four
 //     16-byte pieces of a packed row go out in an order that depends on its lane, or the eight lanes of a row would meet on
@@ -22,7 +23,8 @@
 // Measured (4 layers, append included): a 4608-token planar4 prompt in blocks of 512 11.3 ms with one role after the other per tile, 5.95 with the
 // roles and (query block, kv head, chunk) items of one length each, 4.95 in pieces (plan_pieces), 4.70 with less around the tiles of a piece
 // (q's preparation 5.6 -> 3.3 us, the first tile and the epilogue 2 us each), 4.50 when a producer's first use of a row no longer stood
-// right behind its load, 4.46 with all of q_hi in tensor memory; a 777-token f32 prompt in one block 741, 320, 302, 288, 255 us.
+// right behind its load, 4.46 with all of q_hi in tensor memory, 4.2 with the append's small CTAs; a 777-token f32 prompt in one block 741, 320, 302, 288, 255
+// and 233 us.  (128 registers a thread: 8 to 16 bytes spill.)
 // Every mbarrier wait is bounded: one that runs out raises the context's error flag, the others of the CTA stop
 // waiting, and the kernel runs on to its end, where the tensor memory is always released.
 #include <cuda_fp16.h>
@@ -319,7 +321,7 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
     uint32_t pk[4], pv[4];  // packed K of one tile and packed V of the tile before, on their way
     float pn = 0.f;
     // f32 rows: a warp takes four rows of the tile, a lane 32 bytes of each, which become a 16-byte operand piece.  (Eight lanes a row with 128 bytes
-    // each, as for packed rows, made every load touch 32 lines: 4096 of a tile's 3970 clocks.)
+    // each, as for packed rows, made every load touch 32 lines: 4096 clocks a tile of the load path, as much as a tile takes now.)
     [[maybe_unused]] float4 fk[kF32 ? 8 : 1], fv[kVRows32 ? 8 : 1];
     auto fetch_f32 = [&](float4 *dst, const uint8_t *rows, int tile) {
 #pragma unroll
@@ -684,8 +686,8 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
         // size of what it holds, so its error grows with the tiles it collects.  Against float64, channels with x20 outliers: 777
         // tokens into an f32 cache 1.36e-6 of the result (1.69e-6 without runs, 1.49e-6 with runs of up to 20 tiles), 4608 in blocks
         // of 512 2.0e-6 (3.5e-6, 2.2e-6); V of one sign, 4608 tokens, 2.8e-6 (7.9e-6).  Without lo tiles a run may be longer: fewer
-        // products.  The sums stay in L2; a launch pays 5 us for the first and the last pass over them and 4 for each between: the
-        // 4608 tokens 6.2 -> 6.7 ms (four layers), 777 tokens 287 -> 309 us.  The same by shorter chunks: 7.1 ms and 341 us.
+        // products.  The sums stay in L2.  Without runs the 4608 planar4 tokens take 4.03 ms instead of 4.19 (four layers), f16 3.26 instead of
+        // 3.55, the 777 tokens 215 us instead of 233; shorter chunks cost 15 to 20 % for the same when they were tried.
         // The sums so far come in a block of 32 coordinates ahead of their use, the first before the run's last product is awaited (one block
         // after the other, each with its trip to L2, made 4 us of it).
         auto collect_o = [&](bool first_run, auto &&run_done) -> bool {
@@ -790,7 +792,8 @@ prefill_umma_kernel(const __grid_constant__ PrefillUArgs pa, const __grid_consta
                 ref = new_ref;
             }
             // weights p ||v||, two positions a column: for each K-step of 16 positions eight columns of hi parts and eight of lo parts.
-            // (p = 2^(s - ref) stays below 2^114: the norms are taken as 1e-30 at least.)
+            // (p = 2^(s - ref) stays below 2^114: the norms are taken as 1e-30 at least.  The sum of p falls by the ratio of the norms when a row outweighs
+            // those before it, so the norms that a query sees may span a factor of 1e32.)
             const ulonglong2 *vn2 = reinterpret_cast<const ulonglong2 *>(ss.vn[tile % kNormTiles]);
             uint64_t l2 = 0;
 #pragma unroll
@@ -1024,7 +1027,8 @@ bool prefill_umma_supported(const DecodeArgs &a) {
 // With more than kPrefillItems items (four and more an SM) whole ones, longest first, are spread evenly enough.
 constexpr int kPrefillItems = kPrefillPieces - kPrefillStretches;
 static void plan_pieces(int n_sms, int pos0, int n_tokens, int tq, int n_kv, PieceList &list, ItemParts &parts) {
-    constexpr int kFixed = 7, kMerge = 3, kLeast = 4;  // (a piece has kLeast tiles or the rest of its item)
+    // A piece has kLeast tiles or the rest of its item.  kFixed is less than the 12 tiles' time that a launch spends beside its tiles; 5 to 20 give the same times within 0.6 % (six modes, 76 shapes each).
+    constexpr int kFixed = 7, kMerge = 3, kLeast = 4;
     const int most = std::min(n_sms, kPrefillStretches), n_blocks = (n_tokens + tq - 1) / tq, n_items = n_blocks * n_kv;
     list.n = 0;
     if (n_items > kPrefillItems || (int64_t)pos0 + n_tokens > UINT16_MAX * kTK) return;
