@@ -1606,6 +1606,38 @@ def test_prefill_of_an_infinite_row(bk, gpu_ctx, oracle, tag, mode, bits, vq):
     assert 40 < seen < 160  # (20 tokens, 12 heads, about half)
 
 
+@pytest.mark.parametrize("tag,n", [("planar4", 400), ("f16", 400), ("planar4", 1000)])
+def test_first_prompt_of_a_context_can_be_captured(bk, tag, n):
+    """Append and attention of a context's first prompt block, cut or whole, go into a CUDA graph: no call allocates or waits for the stream."""
+    import torch
+    assert (prefill_plan(bk, 0, n, NH, NKV) > 0) == (n == 400)
+    rng = np.random.default_rng(n)
+    ctx = bk.Context(0)
+    cache = bk.AttnCache(ctx, bk.parse_mode(tag), n_layers=1, n_ctx=n)
+    k, v = synth_kv(rng, n)
+    q = rng.standard_normal((n, NH, HD)).astype(np.float32)
+    dq, dk, dv, do = (ctx.to_device(x) for x in (q, k, v, np.zeros_like(q)))
+    ctx.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    stream = torch.cuda.ExternalStream(ctx.lib.bk_ctx_stream(ctx.h))
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        cache.prefill_step_device(0, dq.ptr, dk.ptr, dv.ptr, do.ptr, 0, n)
+    got = []
+    for _ in range(2):
+        do.zero()
+        ctx.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        ctx.synchronize()
+        got.append(do.download(q.shape, np.float32))
+    del graph
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], cache.prefill_attend(0, q, 0)) and np.abs(got[0]).max() > 0
+    cache.close()
+    for b in (dq, dk, dv, do):
+        b.free()
+    ctx.close()
+
+
 def test_prefill_scratch_comes_with_the_first_cache_that_can_use_it(bk):
     """39 MB (two places of 129 KiB a SM) that a context without such a cache does not hold; a second cache brings no more."""
     import torch
