@@ -121,7 +121,7 @@ struct bk_ctx {
     size_t d_stage_bytes = 0;
     float *d_layer = nullptr;              // normed q and k rows of the layer step (generic decode path)
     size_t d_layer_floats = 0;
-    float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention (the mma.sync form may grow it)
+    float *d_prefill = nullptr;            // (O, m, l) triples of the prefill attention, made with the first cache that can use them (the mma.sync form grows its own)
     size_t d_prefill_floats = 0;
     int gemm_clusters[bk::kGemmMaxSplit + 1] = {};  // [0]: asked for; [n]: clusters of n CTAs of the PQ2_0 product that the device takes at once
     float *d_prefill_runs = nullptr;       // prefill attention: kPrefillRunFloats per SM, then an int per SM (taken or not)
